@@ -190,16 +190,23 @@ struct OchiDev {
   double c[8][2];
 };
 
-__device__ __forceinline__ double rsqrt_fp64(double x)
+__device__ __forceinline__ double rsqrtFrom(double x, double y)
 {
-  // 1/sqrt(x) by two Newton-Raphson steps from the FP32 hardware estimate (quadratic convergence:
-  // ~2^-22 -> 2^-44 -> below FP64 rounding): y <- y (3 - x y^2) / 2, then the same step in the
-  // residual form y + y (1 - x y^2) / 2 with the residual by FMA, which rounds faithfully
-  double y = double(rsqrtf(float(x)));
-  double const h = x * y;
-  y = y * fma(-0.5 * h, y, 1.5);
-  double const r = fma(-x * y, y, 1.0);
-  return fma(0.5 * y, r, y);
+  // 1/sqrt(x) from an estimate y of FP32 accuracy (relative error e/2, e = 1 - x y^2 about 2^-22) by the
+  // cubic step y + y e (1/2 + 3/8 e): the next term is (5/16) e^3, below 2^-66, so one step of five FP64
+  // operations does what two quadratic Newton steps (seven operations) do
+  double const e = fma(-x * y, y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+__device__ __forceinline__ double rsqrt_fp64(double x) { return rsqrtFrom(x, double(rsqrtf(float(x)))); }
+
+// 1/r12 from r12^2 >= 0, 0 for an exactly coincident pair: the estimate is cleared on the ALU (the high word of
+// a non-negative double is 0 only for 0 and for values below 2^-1042), which leaves the FP64 pipe alone
+__device__ __forceinline__ double invR12(double r2)
+{
+  float const y = __double2hiint(r2) == 0 ? 0.0f : rsqrtf(float(r2));
+  return rsqrtFrom(r2, double(y));
 }
 
 }  // namespace tcscf
