@@ -15,13 +15,14 @@
 namespace tcscf {
 namespace {
 
-constexpr int BK = 32;    // r2 points per block step
-constexpr int BN = 128;   // columns per block
-constexpr int NT = 256;
+constexpr int BK = 32;        // r2 points per stage
+constexpr int kMaxCol = 128;  // columns per block at most
+constexpr int NT = 256;       // threads of the reductions
 
 struct KArgs {
   int64_t n1, n2, r2PerSplit;
-  int R, ncol, ldpsi, ldv, ldt, component, same;
+  int R, ncol, colsPerBlock, ldpsi, ldv, ldt, component, same;
+  int vec16;              // V rows may be copied in 16-byte chunks
   const double * p1;
   const double * p2;
   const double * psi1;
@@ -72,8 +73,8 @@ __device__ __forceinline__ double r12Kernel(KArgs const & a, double x1, double y
 {
   double const dx = x1 - x2, dy = y1 - y2, dz = z1 - z2;
   double const rr = fma(dx, dx, fma(dy, dy, dz * dz));
+  if constexpr (KIND == 0) return invR12(rr);
   if (rr == 0.0) return 0.0;
-  if (KIND == 0) return rsqrt_fp64(rr);
   if (KIND == 1) {
     double ax, ay, az, bx, by, bz;
     ochiGrad(a.u, x1, y1, z1, x2, y2, z2, a.same, ax, ay, az);
@@ -85,76 +86,93 @@ __device__ __forceinline__ double r12Kernel(KArgs const & a, double x1, double y
   return a.component == 0 ? gx : (a.component == 1 ? gy : gz);
 }
 
-__device__ __forceinline__ void cpAsync8(double * dst, const double * src, bool valid)
+// copies `bytes` (0, 8 or WIDTH) of a WIDTH-byte chunk and zero-fills the rest
+template <int WIDTH>
+__device__ __forceinline__ void cpAsync(double * dst, const double * src, int bytes)
 {
   unsigned const d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-  int const n = valid ? 8 : 0;   // src-size 0 zero-fills the destination
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(n) : "memory");
+  if constexpr (WIDTH == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void cpAsyncCommit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cpAsyncWait1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
 
-// Block: BMT = 16 RPT r1 rows x BN columns, 256 threads.  r2 streamed in BK blocks through a
-// two-stage cp.async pipeline (coordinates, Coulomb source, psi2 and V of block i+1 load while block i
-// computes).  Phase B: each thread generates VPT kernel values g(r1,r2) (and rho) of one row;
-// phase C: register-tiled FP64 GEMM, each thread RPT rows x BN/16 columns, columns interleaved in
-// pairs so that a half-warp reads 16 consecutive 16-byte chunks (conflict-free).  RPT = 8 (an 8 x 8
-// register tile: 16 shared-memory doubles per 64 FMAs) keeps the FP64 pipe ahead of shared-memory
-// bandwidth where RPT = 4 (12 per 32) does not; it holds one block per SM.
-template <int KIND, int BN, int RPT>
-__global__ void __launch_bounds__(NT, RPT == 8 ? 1 : 2) kContractFp64(KArgs a)
+// D += A B on the FP64 tensor cores: A[r][k] at lane 4 r + k, B[k][n] at lane 4 n + k, D[r][2 q + e] at
+// lane 4 r + q (element e)
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b)
 {
-  constexpr int CPT = BN / 16;            // columns per thread
-  constexpr int BMT = 16 * RPT;           // r1 rows per block
-  // the 128 x 128 tile's GEMM on the FP64 tensor cores (mma.m8n8k4): its operands come from registers,
-  // so shared memory stops limiting the FP64 rate as it does the 8 x 8 register tile on the CUDA cores
-  constexpr bool kDmma = BN == 128;
-  // row strides of the X and V tiles: the DMMA fragments read 4 rows (k) x 8 consecutive doubles per
-  // warp, which a stride of 8 (mod 16) doubles spreads over all 32 banks (two wavefronts, the minimum)
-  constexpr int XLD = kDmma ? BMT + 8 : BMT;
-  constexpr int VLD = kDmma ? BN + 8 : BN;
-  constexpr int VPT = BMT * BK / NT;      // phase-B values per thread
-  constexpr int TPR = BK / VPT;           // phase-B threads per row
-  extern __shared__ __align__(16) double sm[];
-  int const R = a.R;
-  double * sP1 = sm;                              // [R][BMT]
-  double * sC1 = sP1 + R * BMT;                   // [3][BMT]
-  double * sX = sC1 + 3 * BMT;                    // [BK][XLD]
-  double * stage0 = sX + BK * XLD;                // per stage: sV [BK][VLD], sC2 [4][BK], sP2 [R][BK]
-  int const stageSize = BK * VLD + 4 * BK + R * BK;
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(d[0]), "+d"(d[1]) : "d"(a), "d"(b));
+}
 
-  int const tid = threadIdx.x;
+// row stride (doubles) of a shared-memory operand with `n4` columns (a multiple of 4) whose fragments read 4
+// consecutive doubles of 8 rows: 4 or 12 mod 16 spreads a half-warp over all 16 bank pairs
+__host__ __device__ constexpr int fragStride(int n4) { return n4 % 8 == 4 ? n4 : n4 + 4; }
+// row stride of the V tile (2 mod 8: the 16-byte fragment loads below read rows 2 k + e)
+__host__ __device__ constexpr int vStride(int nt) { return 8 * nt + 2; }
+__host__ __device__ constexpr int contractWarps(int rt) { return rt == 1 ? 8 : 4; }
+
+// T += (g .* rho) V for 8 RT rows per warp and 8 NTL columns, everything between the shared-memory
+// operands and T in registers: per 8 r2 points a warp forms rho for its rows with FP64 MMAs (psi1 psi2^T),
+// whose D fragment gives each lane its row's values at points 2 q and 2 q + 1 (q = lane % 4); the lane
+// multiplies them by g of the same two pairs, and the products are the A fragments of the two MMA k-steps
+// that follow (step e takes the points 2 q + e, so V is read at rows 2 q + e).  X never passes through
+// shared memory and no barrier separates the generation of g from the GEMM: the warps of an SM
+// drift apart and one's FP64 chains fill the other's waits.  Columns are interleaved in pairs (n and
+// n + 1 of two tiles), so one 16-byte load serves two MMAs.  Blocks are 4 warps (8 where RT = 1), r2 in
+// stages of BK points through a two-stage cp.async pipeline.  Bound by the FP64 pipe, which the MMAs share
+// with g: against a kernel that passed X through
+// shared memory between two barriers, 59,000 points x 40 columns (rank 5, symmetric) 21.1 -> 9.95 ms and
+// 81,200 points x 120 columns (rank 18, symmetric) 58.6 -> 39.6 ms (0.70 of the FP64 matmul rate).
+template <int KIND, int NTL, int RT>
+__global__ void __launch_bounds__(32 * contractWarps(RT), RT == 1 ? 1 : (RT * NTL <= 20 ? 3 : 2)) kContractFp64(KArgs a)
+{
+  constexpr int kThreads = 32 * contractWarps(RT);
+  constexpr int BMT = 8 * RT * contractWarps(RT);   // r1 rows per block
+  constexpr int VLD = vStride(NTL);
+  extern __shared__ __align__(16) double sm[];
+  int const R = a.R, R4 = (R + 3) / 4 * 4, pld = fragStride(R4);
+  double * sP1 = sm;                                     // [BMT][pld]
+  double * stage0 = sP1 + (R ? BMT * pld : 0);           // per stage: sV [BK][VLD], sC2 [4][BK], sP2 [BK][pld]
+  int const stageSize = BK * VLD + 4 * BK + (R ? BK * pld : 0);
+
+  int const tid = threadIdx.x, lane = tid & 31, fr = lane >> 2, fq = lane & 3;
   int64_t const r1base = int64_t(blockIdx.x) * BMT;
-  int const cg = blockIdx.z;
+  int const col0 = blockIdx.z * a.colsPerBlock, ncol = min(a.ncol, col0 + a.colsPerBlock);
   // a symmetric contraction takes the r2 points from this block's own rows on (its own BMT x BMT
   // square at half weight in T); the Coulomb sums over the points before them come from kCoulombLowerFp64
   int64_t const r2split = int64_t(blockIdx.y) * a.r2PerSplit;
   int64_t const r2begin = a.sym ? max(r2split, r1base) : r2split;
   int64_t const r2end = min(a.n2, r2split + a.r2PerSplit);
-  int64_t const r2half = a.sym ? r1base + BMT : 0;   // r2 below this (and >= r2begin) at half weight
-  bool const doCoul = a.coul != nullptr && cg == 0;
+  int64_t const r2half = a.sym ? r1base + BMT : 0;   // r2 below this (and >= r2begin) at half weight: whole stages, both multiples of BK
+  bool const doCoul = a.coul != nullptr && blockIdx.z == 0;
 
   auto issue = [&](int64_t k0, int st) {
     double * sV = stage0 + st * stageSize;
     double * sC2 = sV + BK * VLD;
     double * sP2 = sC2 + 4 * BK;
     int const kn = int(min(int64_t(BK), r2end - k0));
-    for (int idx = tid; idx < BK * BN; idx += NT) {
-      int const k = idx / BN, c = idx % BN;
-      int const col = cg * BN + c;
-      bool const ok = k < kn && col < a.ncol;
-      cpAsync8(&sV[k * VLD + c], ok ? &a.V[(k0 + k) * a.ldv + col] : a.V, ok);
+    if (a.vec16) {
+      for (int idx = tid; idx < BK * NTL * 4; idx += kThreads) {
+        int const k = idx / (NTL * 4), c = 2 * (idx % (NTL * 4)), left = k < kn ? ncol - col0 - c : 0;
+        cpAsync<16>(&sV[k * VLD + c], left > 0 ? &a.V[(k0 + k) * a.ldv + col0 + c] : a.V, left > 1 ? 16 : (left > 0 ? 8 : 0));
+      }
+    } else {
+      for (int idx = tid; idx < BK * NTL * 8; idx += kThreads) {
+        int const k = idx / (NTL * 8), c = idx % (NTL * 8);
+        bool const ok = k < kn && col0 + c < ncol;
+        cpAsync<8>(&sV[k * VLD + c], ok ? &a.V[(k0 + k) * a.ldv + col0 + c] : a.V, ok ? 8 : 0);
+      }
     }
-    for (int idx = tid; idx < R * BK; idx += NT) {
-      int const k = idx / R, b = idx % R;
-      bool const ok = k < kn;
-      cpAsync8(&sP2[b * BK + k], ok ? &a.psi2[(k0 + k) * a.ldpsi + b] : a.psi2, ok);
+    for (int idx = tid; idx < R4 * BK; idx += kThreads) {
+      int const k = idx / R4, b = idx % R4;
+      bool const ok = k < kn && b < R;
+      cpAsync<8>(&sP2[k * pld + b], ok ? &a.psi2[(k0 + k) * a.ldpsi + b] : a.psi2, ok ? 8 : 0);
     }
-    if (tid < 4 * BK) {
-      int const d = tid / BK, k = tid % BK;
+    for (int idx = tid; idx < 4 * BK; idx += kThreads) {
+      int const d = idx / BK, k = idx % BK;
       bool const ok = k < kn && (d < 3 || doCoul);
       const double * src = d < 3 ? &a.p2[d * a.n2 + k0 + k] : (doCoul ? &a.coul[k0 + k] : a.p2);
-      cpAsync8(&sC2[d * BK + k], ok ? src : a.p2, ok);
+      cpAsync<8>(&sC2[d * BK + k], ok ? src : a.p2, ok ? 8 : 0);
     }
   };
 
@@ -162,28 +180,27 @@ __global__ void __launch_bounds__(NT, RPT == 8 ? 1 : 2) kContractFp64(KArgs a)
   if (nsteps > 0) issue(r2begin, 0);
   cpAsyncCommit();
 
-  for (int idx = tid; idx < R * BMT; idx += NT) {
-    int const r = idx / R, b = idx % R;
+  for (int idx = tid; idx < R4 * BMT; idx += kThreads) {
+    int const r = idx / R4, b = idx % R4;
     int64_t const g = r1base + r;
-    sP1[b * BMT + r] = g < a.n1 ? a.psi1[g * a.ldpsi + b] : 0.0;
+    sP1[r * pld + b] = b < R && g < a.n1 ? a.psi1[g * a.ldpsi + b] : 0.0;
   }
-  for (int idx = tid; idx < 3 * BMT; idx += NT) {
-    int const d = idx / BMT, r = idx % BMT;
-    int64_t const g = r1base + r;
-    sC1[idx] = g < a.n1 ? a.p1[d * a.n1 + g] : 1.0e6;
+  int const wrow = (tid >> 5) * 8 * RT + fr;   // this lane's row of the block in row tile 0
+  double x1[RT], y1[RT], z1[RT], vh[RT];
+#pragma unroll
+  for (int i = 0; i < RT; ++i) {
+    int64_t const g = r1base + wrow + 8 * i;
+    bool const ok = g < a.n1;
+    x1[i] = ok ? a.p1[g] : 1.0e6;
+    y1[i] = ok ? a.p1[a.n1 + g] : 1.0e6;
+    z1[i] = ok ? a.p1[2 * a.n1 + g] : 1.0e6;
+    vh[i] = 0.0;
   }
-  __syncthreads();
-
-  int const rB = tid / TPR;             // phase-B row
-  int const cB = (tid % TPR) * VPT;     // phase-B first column
-  double const x1 = sC1[rB], y1 = sC1[BMT + rB], z1 = sC1[2 * BMT + rB];
-  int const tr = tid >> 4, tc = tid & 15;
-  double acc[RPT][CPT];
+  double acc[RT][NTL][2];
 #pragma unroll
-  for (int i = 0; i < RPT; ++i)
+  for (int i = 0; i < RT; ++i)
 #pragma unroll
-    for (int j = 0; j < CPT; ++j) acc[i][j] = 0.0;
-  double vh = 0.0;
+    for (int j = 0; j < NTL; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 
   for (int64_t step = 0; step < nsteps; ++step) {
     int64_t const k0 = r2begin + step * BK;
@@ -197,106 +214,78 @@ __global__ void __launch_bounds__(NT, RPT == 8 ? 1 : 2) kContractFp64(KArgs a)
     double const * sC2 = sV + BK * VLD;
     double const * sP2 = sC2 + 4 * BK;
     int const kn = int(min(int64_t(BK), r2end - k0));
-    double rho[VPT];
+    bool const half = k0 < r2half;
+#pragma unroll 1
+    for (int p0 = 0; p0 < BK; p0 += 8) {
+      double x[RT][2];
 #pragma unroll
-    for (int j = 0; j < VPT; ++j) rho[j] = R > 0 ? 0.0 : 1.0;
-    for (int b = 0; b < R; ++b) {
-      // one psi1 value against VPT psi2 values
-      double const p = sP1[b * BMT + rB];
+      for (int i = 0; i < RT; ++i) x[i][0] = x[i][1] = R > 0 ? 0.0 : 1.0;
+      for (int b = fq; b < R4; b += 4) {
+        double const q = sP2[(p0 + fr) * pld + b];
 #pragma unroll
-      for (int j = 0; j < VPT; j += 2) {
-        double2 const q = *reinterpret_cast<double2 const *>(&sP2[b * BK + cB + j]);
-        rho[j] = fma(p, q.x, rho[j]);
-        rho[j + 1] = fma(p, q.y, rho[j + 1]);
+        for (int i = 0; i < RT; ++i) dmma(x[i], sP1[(wrow + 8 * i) * pld + b], q);
       }
-    }
+      int const c = p0 + 2 * fq;
+      double2 const px = *reinterpret_cast<double2 const *>(&sC2[c]);
+      double2 const py = *reinterpret_cast<double2 const *>(&sC2[BK + c]);
+      double2 const pz = *reinterpret_cast<double2 const *>(&sC2[2 * BK + c]);
+      double2 const pc = *reinterpret_cast<double2 const *>(&sC2[3 * BK + c]);
 #pragma unroll
-    for (int j = 0; j < VPT; ++j) {
-      int const c = cB + j;
-      double g = r12Kernel<KIND>(a, x1, y1, z1, sC2[c], sC2[BK + c], sC2[2 * BK + c]);
-      g = c < kn ? g : 0.0;
-      vh = fma(g, sC2[3 * BK + c], vh);
-      sX[c * XLD + rB] = (k0 + c < r2half ? 0.5 * g : g) * rho[j];
-    }
-    __syncthreads();
-    if constexpr (kDmma) {
-      // FP64 tensor cores: warp w owns rows BMT/2 (w & 1) .. + BMT/2 and columns 32 (w >> 1) .. + 32 of
-      // the block as RPT x 4 tiles of 8 x 8; mma.m8n8k4 fragments: A[r][k] at lane 4 r + k, B[k][n] at
-      // lane 4 n + k, C[r][2 q + e] at lane 4 r + q (element e)
-      int const lane = tid & 31, wr = ((tid >> 5) & 1) * (BMT / 2), wc = (tid >> 6) * 32;
-      int const fr = lane >> 2, fk = lane & 3;
-#pragma unroll 2
-      for (int k = 0; k < BK; k += 4) {
-        double av[RPT], bv[4];
-#pragma unroll
-        for (int i = 0; i < RPT; ++i) av[i] = sX[(k + fk) * XLD + wr + 8 * i + fr];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) bv[j] = sV[(k + fk) * VLD + wc + 8 * j + fr];
-#pragma unroll
-        for (int i = 0; i < RPT; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                         : "+d"(acc[i][2 * j]), "+d"(acc[i][2 * j + 1])
-                         : "d"(av[i]), "d"(bv[j]));
-      }
-      continue;
-    }
-#pragma unroll 4
-    for (int k = 0; k < BK; ++k) {
-      double av[RPT];
-#pragma unroll
-      for (int q = 0; q < RPT / 2; ++q) {
-        double2 const aa = *reinterpret_cast<double2 const *>(&sX[k * XLD + tr * RPT + 2 * q]);
-        av[2 * q] = aa.x;
-        av[2 * q + 1] = aa.y;
-      }
-      double bv[CPT];
-#pragma unroll
-      for (int q = 0; q < CPT / 2; ++q) {
-        double2 const bb = *reinterpret_cast<double2 const *>(&sV[k * VLD + 32 * q + 2 * tc]);
-        bv[2 * q] = bb.x;
-        bv[2 * q + 1] = bb.y;
+      for (int i = 0; i < RT; ++i) {
+        double g0 = r12Kernel<KIND>(a, x1[i], y1[i], z1[i], px.x, py.x, pz.x);
+        double g1 = r12Kernel<KIND>(a, x1[i], y1[i], z1[i], px.y, py.y, pz.y);
+        g0 = c < kn ? g0 : 0.0;
+        g1 = c + 1 < kn ? g1 : 0.0;
+        vh[i] = fma(g0, pc.x, fma(g1, pc.y, vh[i]));
+        if (half) { g0 *= 0.5; g1 *= 0.5; }
+        x[i][0] *= g0;
+        x[i][1] *= g1;
       }
 #pragma unroll
-      for (int i = 0; i < RPT; ++i)
+      for (int e = 0; e < 2; ++e) {
+        double const * v = sV + (c + e) * VLD;   // row 2 q + e: the k index of this lane's B fragments
 #pragma unroll
-        for (int j = 0; j < CPT; ++j) acc[i][j] = fma(av[i], bv[j], acc[i][j]);
+        for (int j = 0; j + 1 < NTL; j += 2) {
+          double2 const b = *reinterpret_cast<double2 const *>(&v[8 * j + 2 * fr]);
+#pragma unroll
+          for (int i = 0; i < RT; ++i) {
+            dmma(acc[i][j], x[i][e], b.x);
+            dmma(acc[i][j + 1], x[i][e], b.y);
+          }
+        }
+        if constexpr (NTL % 2) {
+          double const b = v[8 * (NTL - 1) + fr];
+#pragma unroll
+          for (int i = 0; i < RT; ++i) dmma(acc[i][NTL - 1], x[i][e], b);
+        }
+      }
     }
   }
 
   double * T = a.T + blockIdx.y * a.tStrideSplit;
-  if constexpr (kDmma) {
-    int const lane = tid & 31, wr = ((tid >> 5) & 1) * (BMT / 2), wc = (tid >> 6) * 32;
 #pragma unroll
-    for (int i = 0; i < RPT; ++i) {
-      int64_t const g = r1base + wr + 8 * i + (lane >> 2);
-      if (g >= a.n1) continue;
+  for (int i = 0; i < RT; ++i) {
+    int64_t const g = r1base + wrow + 8 * i;
+    if (g >= a.n1) continue;
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < NTL; ++j)
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          int const col = cg * BN + wc + 8 * j + 2 * (lane & 3) + e;
-          if (col < a.ncol) T[g * a.ldt + col] = acc[i][2 * j + e];
-        }
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < RPT; ++i) {
-      int64_t const g = r1base + tr * RPT + i;
-      if (g >= a.n1) continue;
-#pragma unroll
-      for (int j = 0; j < CPT; ++j) {
-        int const col = cg * BN + 32 * (j / 2) + 2 * tc + (j & 1);
-        if (col < a.ncol) T[g * a.ldt + col] = acc[i][j];
+      for (int e = 0; e < 2; ++e) {
+        // D column n = 2 q + e of tile j is column 8 (j - j % 2) + 2 n + j % 2 of the block (the last tile of an odd count: 8 j + n)
+        int const n = 2 * fq + e;
+        int const col = col0 + (NTL % 2 && j == NTL - 1 ? 8 * j + n : 8 * (j & ~1) + 2 * n + (j & 1));
+        if (col < ncol) T[g * a.ldt + col] = acc[i][j][e];
       }
-    }
   }
   if (doCoul) {
 #pragma unroll
-    for (int o = 1; o < TPR; o <<= 1) vh += __shfl_xor_sync(0xffffffffu, vh, o);
-    int64_t const g = r1base + rB;
-    if ((tid % TPR) == 0 && g < a.n1) a.VH[blockIdx.y * a.vhStrideSplit + g] = vh;
+    for (int i = 0; i < RT; ++i) {
+      double v = vh[i];
+      v += __shfl_xor_sync(0xffffffffu, v, 1);
+      v += __shfl_xor_sync(0xffffffffu, v, 2);
+      int64_t const g = r1base + wrow + 8 * i;
+      if (fq == 0 && g < a.n1) a.VH[blockIdx.y * a.vhStrideSplit + g] = v;
+    }
   }
 }
 
@@ -504,33 +493,67 @@ __global__ void __launch_bounds__(NT) kReduceComplex(int64_t n1, int nb, const d
   }
 }
 
-template <int KIND, int BNV, int RPT>
+template <int KIND, int NTL, int RT>
 int launchOne(tcscf_ctx * ctx, KArgs const & a, dim3 grid, size_t smem)
 {
-  TCSCF_CUDA(ctx, cudaFuncSetAttribute(kContractFp64<KIND, BNV, RPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-  TCSCF_CUDA(ctx, cudaFuncSetAttribute(kContractFp64<KIND, BNV, RPT>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-  kContractFp64<KIND, BNV, RPT><<<grid, NT, smem, ctx->stream>>>(a);
+  TCSCF_CUDA(ctx, cudaFuncSetAttribute(kContractFp64<KIND, NTL, RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  TCSCF_CUDA(ctx, cudaFuncSetAttribute(kContractFp64<KIND, NTL, RT>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+  kContractFp64<KIND, NTL, RT><<<grid, 32 * contractWarps(RT), smem, ctx->stream>>>(a);
   TCSCF_LAUNCH(ctx);
   return TCSCF_OK;
 }
 
+// the 8-column tiles of a block (contractTiles' result) and its row tiles per warp, as template parameters
 template <int KIND>
-int launchKind(tcscf_ctx * ctx, int bn, int rpt, KArgs const & a, dim3 grid, size_t smem)
+int launchKind(tcscf_ctx * ctx, int nt, int rt, KArgs const & a, dim3 grid, size_t smem)
 {
-  if (bn == 32) return launchOne<KIND, 32, 4>(ctx, a, grid, smem);
-  if (bn == 64) return launchOne<KIND, 64, 4>(ctx, a, grid, smem);
-  if constexpr (KIND == 0)
-    if (rpt == 8) return launchOne<KIND, 128, 8>(ctx, a, grid, smem);
-  return launchOne<KIND, 128, 4>(ctx, a, grid, smem);
+  if constexpr (KIND == 0) {
+    if (rt == 1) {
+      if (nt == 4) return launchOne<0, 4, 1>(ctx, a, grid, smem);
+      if (nt == 8) return launchOne<0, 8, 1>(ctx, a, grid, smem);
+      return launchOne<0, 16, 1>(ctx, a, grid, smem);
+    }
+    switch (nt) {
+      case 1: return launchOne<0, 1, 4>(ctx, a, grid, smem);
+      case 2: return launchOne<0, 2, 4>(ctx, a, grid, smem);
+      case 3: return launchOne<0, 3, 4>(ctx, a, grid, smem);
+      case 4: return launchOne<0, 4, 4>(ctx, a, grid, smem);
+      case 5: return launchOne<0, 5, 4>(ctx, a, grid, smem);
+      case 6: return launchOne<0, 6, 4>(ctx, a, grid, smem);
+      case 7: return launchOne<0, 7, 4>(ctx, a, grid, smem);
+      case 8: return launchOne<0, 8, 4>(ctx, a, grid, smem);
+      case 10: return launchOne<0, 10, 2>(ctx, a, grid, smem);
+      case 12: return launchOne<0, 12, 2>(ctx, a, grid, smem);
+      case 13: return launchOne<0, 13, 2>(ctx, a, grid, smem);
+      case 14: return launchOne<0, 14, 2>(ctx, a, grid, smem);
+      case 15: return launchOne<0, 15, 2>(ctx, a, grid, smem);
+      default: return launchOne<0, 16, 2>(ctx, a, grid, smem);
+    }
+  } else {
+    switch (nt) {
+      case 4: return launchOne<KIND, 4, 2>(ctx, a, grid, smem);
+      case 8: return launchOne<KIND, 8, 2>(ctx, a, grid, smem);
+      case 12: return launchOne<KIND, 12, 2>(ctx, a, grid, smem);
+      case 13: return launchOne<KIND, 13, 2>(ctx, a, grid, smem);
+      case 14: return launchOne<KIND, 14, 2>(ctx, a, grid, smem);
+      case 15: return launchOne<KIND, 15, 2>(ctx, a, grid, smem);
+      default: return launchOne<KIND, 16, 2>(ctx, a, grid, smem);
+    }
+  }
 }
 
-int launchContract(tcscf_ctx * ctx, int kind, int bn, int rpt, KArgs const & a, unsigned tiles, unsigned nsplit, size_t smem)
+// the smallest instantiated tile count that holds nt tiles
+int contractTiles(int kind, int rt, int nt)
 {
-  unsigned const cgroups = a.ncol <= 128 ? 1u : unsigned((a.ncol + BN - 1) / BN);
-  dim3 const grid{tiles, nsplit, cgroups};
-  if (kind == 0) return launchKind<0>(ctx, bn, rpt, a, grid, smem);
-  if (kind == 1) return launchKind<1>(ctx, bn, rpt, a, grid, smem);
-  return launchKind<2>(ctx, bn, rpt, a, grid, smem);
+  static int const direct[] = {1, 2, 3, 4, 5, 6, 7, 8, 10, 12, 13, 14, 15, 16}, wideRank[] = {4, 8, 16}, tc[] = {4, 8, 12, 13, 14, 15, 16};
+  auto pick = [&](auto const & v) { for (int t : v) if (t >= nt) return t; return 16; };
+  return kind != 0 ? pick(tc) : (rt == 1 ? pick(wideRank) : pick(direct));
+}
+
+size_t contractSmem(int nt, int rt, int R)
+{
+  int const bm = 8 * rt * contractWarps(rt), p = R > 0 ? fragStride((R + 3) / 4 * 4) : 0;
+  return sizeof(double) * (size_t(bm) * p + 2 * (size_t(BK) * vStride(nt) + 4 * BK + size_t(BK) * p));
 }
 
 }  // namespace
@@ -539,23 +562,29 @@ int contractFp64(tcscf_ctx * ctx, Contraction const & c)
 {
   TCSCF_CHECK(ctx, c.R >= 0 && c.R <= 128, TCSCF_ERR_UNSUPPORTED, "contraction rank must be <= 128");
   TCSCF_CHECK(ctx, c.ncol > 0 && c.n1 > 0 && c.n2 > 0, TCSCF_ERR_INVALID_ARGUMENT, "empty contraction");
-  int const bn = c.ncol <= 32 ? 32 : (c.ncol <= 64 ? 64 : 128);
   int const kind = c.kernel == TCSCF_K_INV_R12 ? 0 : (c.kernel <= TCSCF_K_TC_SCALAR_OPPO ? 1 : 2);
-  // 8 x 8 register tiles (128 r1 rows per block) for 1/r12 where the 128-column tile and the rank
-  // leave the shared memory room (R <= 64), else 4 x 8 (64 rows).  The transcorrelated kernels spend
-  // more of each block generating g, which the one block per SM of the 8 x 8 tile cannot hide: at Be-TC
-  // (24 STO, 65,536 x 65,536 points) their precompute took 4.37 s with 8 x 8 and 2.68 s with 4 x 8.
-  int const rpt = bn == 128 && c.R <= 64 && kind == 0 ? 8 : 4;
-  int const bm = 16 * rpt;
+  TCSCF_CHECK(ctx, kind == 0 || c.R == 0, TCSCF_ERR_UNSUPPORTED, "internal: the transcorrelated kernels come in the precompute form");
+  // columns in equal groups of at most 128 (g is generated once per group)
+  int const cgroups = (c.ncol + kMaxCol - 1) / kMaxCol;
+  int const colsPerBlock = ((c.ncol + cgroups - 1) / cgroups + 7) / 8 * 8;
+  // row tiles per warp: the accumulators (4 RT NT registers a thread) fit with RT = 4 up to 64 columns and RT = 2
+  // above; the transcorrelated kernels take RT = 2 (their g needs the registers); ranks whose factor rows
+  // would leave room for one block of 4 warps per SM take 8 warps of one row tile
+  int rt = kind == 0 && colsPerBlock <= 64 ? 4 : 2;
+  if (kind == 0 && contractSmem(contractTiles(kind, rt, colsPerBlock / 8), rt, c.R) > 112 * 1024) rt = 1;
+  int const nt = contractTiles(kind, rt, colsPerBlock / 8);
+  int const bm = 8 * rt * contractWarps(rt);
   int64_t const tiles = (c.n1 + bm - 1) / bm;
-  int const cgroups = c.ncol <= 128 ? 1 : (c.ncol + BN - 1) / BN;
   int dev = 0;
   cudaGetDevice(&dev);
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // split r2 so that small r1 sets still fill the machine (partials are summed deterministically)
-  int64_t const want = int64_t(sms) * (rpt == 8 ? 2 : 4);
+  // split r2 so that there are several waves of blocks (2 to 3 per SM; a symmetric contraction's first
+  // tiles take the whole range and its last ones almost nothing): partials are summed deterministically, and
+  // kept below 512 MiB
+  int64_t const want = int64_t(sms) * (c.sym ? 24 : 12);
   int64_t nsplit = (want + tiles * cgroups - 1) / (tiles * cgroups);
+  nsplit = std::min<int64_t>(nsplit, (int64_t(512) << 20) / (c.n1 * c.ldt * int64_t(sizeof(double))));
   nsplit = std::max<int64_t>(1, std::min<int64_t>(nsplit, (c.n2 + 4 * BK - 1) / (4 * BK)));
   nsplit = std::min<int64_t>(nsplit, 65535);
   int64_t perSplit = (c.n2 + nsplit - 1) / nsplit;
@@ -564,7 +593,7 @@ int contractFp64(tcscf_ctx * ctx, Contraction const & c)
 
   KArgs a{};
   a.n1 = c.n1; a.n2 = c.n2; a.r2PerSplit = perSplit;
-  a.R = c.R; a.ncol = c.ncol; a.ldpsi = c.ldpsi; a.ldv = c.ldv; a.ldt = c.ldt;
+  a.R = c.R; a.ncol = c.ncol; a.colsPerBlock = colsPerBlock; a.ldpsi = c.ldpsi; a.ldv = c.ldv; a.ldt = c.ldt;
   a.component = c.component; a.same = (c.kernel == TCSCF_K_TC_SCALAR_SAME || c.kernel == TCSCF_K_GRAD_U_SAME) ? 1 : 0;
   a.p1 = c.p1; a.p2 = c.p2; a.psi1 = c.psi1; a.psi2 = c.psi2; a.coul = c.coul; a.V = c.V;
   if (c.jastrow) {
@@ -591,11 +620,15 @@ int contractFp64(tcscf_ctx * ctx, Contraction const & c)
   TCSCF_CHECK(ctx, !c.sym || (c.p1 == c.p2 && c.n1 == c.n2 && c.psi1 == c.psi2 && c.R > 0 && (c.VH != nullptr) == (c.coul != nullptr)),
               TCSCF_ERR_INVALID_ARGUMENT, "internal: a symmetric contraction needs r1 = r2 and psi1 = psi2");
   a.sym = c.sym ? 1 : 0;
-  int const pad = bn == 128 ? 8 : 0;   // the DMMA tiles' padded X and V row strides
-  size_t const smem = sizeof(double) * (size_t(c.R) * bm + 3 * bm + BK * (bm + pad) + 2 * (size_t(BK) * (bn + pad) + 4 * BK + size_t(c.R) * BK));
+  // 16-byte copies of V: every chunk starts at an even column of a 16-byte aligned row
+  a.vec16 = c.ldv % 2 == 0 && reinterpret_cast<uintptr_t>(c.V) % 16 == 0;
+  size_t const smem = contractSmem(nt, rt, c.R);
+  TCSCF_CHECK(ctx, smem <= 227 * 1024, TCSCF_ERR_UNSUPPORTED, "internal: contraction tile beyond the shared memory");
   // the contraction kernel alone is bracketed by the context's timing events (tcscf_last_timing)
   if (!ctx->capturing) cudaEventRecord(ctx->ev[2], ctx->stream);
-  TCSCF_TRY(launchContract(ctx, kind, bn, rpt, a, unsigned(tiles), unsigned(nsplit), smem));
+  dim3 const grid{unsigned(tiles), unsigned(nsplit), unsigned(cgroups)};
+  TCSCF_TRY(kind == 0 ? launchKind<0>(ctx, nt, rt, a, grid, smem) : (kind == 1 ? launchKind<1>(ctx, nt, rt, a, grid, smem)
+                                                                                  : launchKind<2>(ctx, nt, rt, a, grid, smem)));
   if (!ctx->capturing) cudaEventRecord(ctx->ev[3], ctx->stream);
   if (nsplit > 1) {
     int64_t const n = c.n1 * c.ncol;
