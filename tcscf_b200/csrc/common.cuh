@@ -190,23 +190,19 @@ struct OchiDev {
   double c[8][2];
 };
 
-__device__ __forceinline__ double rsqrtFrom(double x, double y)
-{
-  // 1/sqrt(x) from an estimate y of FP32 accuracy (relative error e/2, e = 1 - x y^2 about 2^-22) by the
-  // cubic step y + y e (1/2 + 3/8 e): the next term is (5/16) e^3, below 2^-66, so one step of five FP64
-  // operations does what two quadratic Newton steps (seven operations) do
-  double const e = fma(-x * y, y, 1.0);
-  return fma(y * e, fma(0.375, e, 0.5), y);
-}
-
-__device__ __forceinline__ double rsqrt_fp64(double x) { return rsqrtFrom(x, double(rsqrtf(float(x)))); }
-
-// 1/r12 from r12^2 >= 0, 0 for an exactly coincident pair: the estimate is cleared on the ALU (the high word of
-// a non-negative double is 0 only for 0 and for values below 2^-1042), which leaves the FP64 pipe alone
+// 1/r12 from r12^2 >= 0, 0 for an exactly coincident pair.  The hardware estimate y (rsqrt.approx.ftz.f64 works
+// on the high word: no conversions, about 20 bits) is refined by the binomial series of (1 - e)^(-1/2) to
+// second order, y + y e (1/2 + 3/8 e) with e = 1 - x y^2 (Householder's third-order step): the next
+// term, (5/16) e^3, is below 2^-58, so one step of five FP64 operations does what two quadratic Newton
+// steps (seven) do.  The estimate of a zero is cleared on the ALU (the high word of a non-negative double is
+// 0 only for 0 and for values below 2^-1042), which leaves the FP64 pipe alone.
 __device__ __forceinline__ double invR12(double r2)
 {
-  float const y = __double2hiint(r2) == 0 ? 0.0f : rsqrtf(float(r2));
-  return rsqrtFrom(r2, double(y));
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2));
+  y = __hiloint2double(__double2hiint(r2) == 0 ? 0 : __double2hiint(y), 0);
+  double const e = fma(-r2 * y, y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
 }  // namespace tcscf

@@ -103,6 +103,17 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b)
 {
   asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(d[0]), "+d"(d[1]) : "d"(a), "d"(b));
 }
+// two row tiles (d0 and d1, rows 8 apart) in one instruction, k = 4 and k = 8 (the second half at a2, a3 and b1)
+__device__ __forceinline__ void dmma16(double (&d0)[2], double (&d1)[2], double a0, double a1, double b)
+{
+  asm("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};"
+      : "+d"(d0[0]), "+d"(d0[1]), "+d"(d1[0]), "+d"(d1[1]) : "d"(a0), "d"(a1), "d"(b));
+}
+__device__ __forceinline__ void dmma16k8(double (&d0)[2], double (&d1)[2], double a0, double a1, double a2, double a3, double b0, double b1)
+{
+  asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+d"(d0[0]), "+d"(d0[1]), "+d"(d1[0]), "+d"(d1[1]) : "d"(a0), "d"(a1), "d"(a2), "d"(a3), "d"(b0), "d"(b1));
+}
 
 // row stride (doubles) of a shared-memory operand with `n4` columns (a multiple of 4) whose fragments read 4
 // consecutive doubles of 8 rows: 4 or 12 mod 16 spreads a half-warp over all 16 bank pairs
@@ -111,31 +122,42 @@ __host__ __device__ constexpr int fragStride(int n4) { return n4 % 8 == 4 ? n4 :
 __host__ __device__ constexpr int vStride(int nt) { return 8 * nt + 2; }
 __host__ __device__ constexpr int contractWarps(int rt) { return rt == 1 ? 8 : 4; }
 
+// blocks per SM the register budget is cut for (65,536 / (threads x blocks) a thread); one more block each
+// below 8 tiles spilled and ran 1 to 20 % slower
+__host__ __device__ constexpr int contractBlocks(int nt, int rt)
+{
+  return rt == 1 ? 1 : (nt <= 3 ? 4 : (nt <= 6 ? 3 : 2));
+}
+
 // T += (g .* rho) V for 8 RT rows per warp and 8 NTL columns, everything between the shared-memory
 // operands and T in registers: per 8 r2 points a warp forms rho for its rows with FP64 MMAs (psi1 psi2^T),
 // whose D fragment gives each lane its row's values at points 2 q and 2 q + 1 (q = lane % 4); the lane
 // multiplies them by g of the same two pairs, and the products are the A fragments of the two MMA k-steps
 // that follow (step e takes the points 2 q + e, so V is read at rows 2 q + e).  X never passes through
 // shared memory and no barrier separates the generation of g from the GEMM: the warps of an SM
-// drift apart and one's FP64 chains fill the other's waits.  Columns are interleaved in pairs (n and
-// n + 1 of two tiles), so one 16-byte load serves two MMAs.  Blocks are 4 warps (8 where RT = 1), r2 in
-// stages of BK points through a two-stage cp.async pipeline.  Bound by the FP64 pipe, which the MMAs share
-// with g: against a kernel that passed X through
-// shared memory between two barriers, 59,000 points x 40 columns (rank 5, symmetric) 21.1 -> 9.95 ms and
-// 81,200 points x 120 columns (rank 18, symmetric) 58.6 -> 39.6 ms (0.70 of the FP64 matmul rate).
-template <int KIND, int NTL, int RT>
-__global__ void __launch_bounds__(32 * contractWarps(RT), RT == 1 ? 1 : (RT * NTL <= 20 ? 3 : 2)) kContractFp64(KArgs a)
+// drift apart.  Columns are interleaved in pairs (n and n + 1 of two tiles), so one 16-byte load serves two
+// MMAs.  Blocks are 4 warps (8 where RT = 1), r2 in stages of BK points through a two-stage cp.async
+// pipeline.  Bound by the FP64 pipe and the instruction issue together: an m8n8k4 MMA takes 16 issue cycles of its
+// scheduler and nothing overlaps it, so the time is 16 x MMAs plus the other instructions; they are kept
+// few (copies without index arithmetic, the rank a template parameter, no masks in full stages, the
+// half weight applied once).  Forming the next group's X beside the GEMM, MMAs of m8n8k4 or m16n8k8 and
+// volatile ordering all measured the same.  Against a kernel that passed X through shared memory between
+// two barriers: 59,000 points x 40 columns (rank 5, symmetric) 21.1 -> 7.2 ms; 81,200 points x 120
+// columns (rank 18, symmetric) 58.6 -> 32.1 ms, 0.81 of the FP64 matmul rate counting the padded MMAs.
+template <int KIND, int NTL, int RT, int KR>
+__global__ void __launch_bounds__(32 * contractWarps(RT), contractBlocks(NTL, RT)) kContractFp64(KArgs a)
 {
-  constexpr int kThreads = 32 * contractWarps(RT);
+  constexpr int kWarps = contractWarps(RT), kThreads = 32 * kWarps;
+  static_assert(BK == 32, "a warp copies one coordinate row of a stage");
   constexpr int BMT = 8 * RT * contractWarps(RT);   // r1 rows per block
   constexpr int VLD = vStride(NTL);
   extern __shared__ __align__(16) double sm[];
-  int const R = a.R, R4 = (R + 3) / 4 * 4, pld = fragStride(R4);
+  int const R = KR == 0 ? 0 : a.R, R4 = KR >= 0 ? 4 * KR : (R + 3) / 4 * 4, pld = fragStride(R4);
   double * sP1 = sm;                                     // [BMT][pld]
   double * stage0 = sP1 + (R ? BMT * pld : 0);           // per stage: sV [BK][VLD], sC2 [4][BK], sP2 [BK][pld]
   int const stageSize = BK * VLD + 4 * BK + (R ? BK * pld : 0);
 
-  int const tid = threadIdx.x, lane = tid & 31, fr = lane >> 2, fq = lane & 3;
+  int const tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, fr = lane >> 2, fq = lane & 3;
   int64_t const r1base = int64_t(blockIdx.x) * BMT;
   int const col0 = blockIdx.z * a.colsPerBlock, ncol = min(a.ncol, col0 + a.colsPerBlock);
   // a symmetric contraction takes the r2 points from this block's own rows on (its own BMT x BMT
@@ -146,33 +168,53 @@ __global__ void __launch_bounds__(32 * contractWarps(RT), RT == 1 ? 1 : (RT * NT
   int64_t const r2half = a.sym ? r1base + BMT : 0;   // r2 below this (and >= r2begin) at half weight: whole stages, both multiples of BK
   bool const doCoul = a.coul != nullptr && blockIdx.z == 0;
 
+  // The copies of a stage: warp w takes V and psi2 rows w, w + warps, ... (psi2: several rows at once where
+  // they are short) and coordinate row w, the lanes a row's chunks; a full stage's copies differ only by
+  // one pointer step from row to row, so a lane's pointers and byte counts are formed once.
+  constexpr int W = 8 * NTL;
+  int const cols = ncol - col0;
+  int const psiLanes = R4 <= 4 ? 4 : (R4 <= 8 ? 8 : (R4 <= 16 ? 16 : 32)), psiRows = 32 / psiLanes;
+  int const pk = warp * psiRows + lane / psiLanes, pb = lane % psiLanes;
+  int const vb0 = min(16, max(0, 8 * (cols - 2 * lane))), vb1 = min(16, max(0, 8 * (cols - 64 - 2 * lane)));
+  const double * const vsrc = a.V + int64_t(warp) * a.ldv + col0 + (vb0 ? 2 * lane : 0);
+  const double * const psrc = R ? a.psi2 + int64_t(pk) * a.ldpsi + (pb < R ? pb : 0) : nullptr;
+  const double * const csrc = warp < 3 ? a.p2 + int64_t(warp) * a.n2 + lane : (doCoul ? a.coul + lane : a.p2 + lane);
+  int64_t const vstep = int64_t(kWarps) * a.ldv, pstep = int64_t(kWarps) * psiRows * a.ldpsi;
   auto issue = [&](int64_t k0, int st) {
     double * sV = stage0 + st * stageSize;
     double * sC2 = sV + BK * VLD;
     double * sP2 = sC2 + 4 * BK;
-    int const kn = int(min(int64_t(BK), r2end - k0));
-    if (a.vec16) {
-      for (int idx = tid; idx < BK * NTL * 4; idx += kThreads) {
-        int const k = idx / (NTL * 4), c = 2 * (idx % (NTL * 4)), left = k < kn ? ncol - col0 - c : 0;
-        cpAsync<16>(&sV[k * VLD + c], left > 0 ? &a.V[(k0 + k) * a.ldv + col0 + c] : a.V, left > 1 ? 16 : (left > 0 ? 8 : 0));
+    if (a.vec16 && R4 <= 32 && r2end - k0 >= BK) {
+      const double * src = vsrc + k0 * a.ldv;
+      double * dst = sV + warp * VLD + 2 * lane;
+#pragma unroll
+      for (int k = 0; k < BK; k += kWarps, src += vstep) {
+        if (W >= 64 || 2 * lane < W) cpAsync<16>(dst + k * VLD, src, vb0);
+        if (W > 64 && 64 + 2 * lane < W) cpAsync<16>(dst + k * VLD + 64, vb1 ? src + 64 : src, vb1);
       }
-    } else {
-      for (int idx = tid; idx < BK * NTL * 8; idx += kThreads) {
-        int const k = idx / (NTL * 8), c = idx % (NTL * 8);
-        bool const ok = k < kn && col0 + c < ncol;
+      if (R4 > 0 && pb < R4) {
+        src = psrc + k0 * a.ldpsi;
+#pragma unroll
+        for (int k = 0; k < BK; k += kWarps * psiRows, src += pstep) cpAsync<8>(&sP2[(pk + k) * pld + pb], src, pb < R ? 8 : 0);
+      }
+      if (warp < 4) cpAsync<8>(&sC2[warp * BK + lane], csrc + k0, warp < 3 || doCoul ? 8 : 0);
+      return;
+    }
+    int const kn = int(min(int64_t(BK), r2end - k0));
+    for (int k = warp; k < BK; k += kWarps)
+#pragma unroll
+      for (int c = lane; c < W; c += 32) {
+        bool const ok = k < kn && c < cols;
         cpAsync<8>(&sV[k * VLD + c], ok ? &a.V[(k0 + k) * a.ldv + col0 + c] : a.V, ok ? 8 : 0);
       }
-    }
-    for (int idx = tid; idx < R4 * BK; idx += kThreads) {
-      int const k = idx / R4, b = idx % R4;
-      bool const ok = k < kn && b < R;
-      cpAsync<8>(&sP2[k * pld + b], ok ? &a.psi2[(k0 + k) * a.ldpsi + b] : a.psi2, ok ? 8 : 0);
-    }
-    for (int idx = tid; idx < 4 * BK; idx += kThreads) {
-      int const d = idx / BK, k = idx % BK;
-      bool const ok = k < kn && (d < 3 || doCoul);
-      const double * src = d < 3 ? &a.p2[d * a.n2 + k0 + k] : (doCoul ? &a.coul[k0 + k] : a.p2);
-      cpAsync<8>(&sC2[d * BK + k], ok ? src : a.p2, ok ? 8 : 0);
+    for (int k = pk; k < BK; k += kWarps * psiRows)
+      for (int b = pb; b < R4; b += psiLanes) {
+        bool const ok = k < kn && b < R;
+        cpAsync<8>(&sP2[k * pld + b], ok ? &a.psi2[(k0 + k) * a.ldpsi + b] : a.psi2, ok ? 8 : 0);
+      }
+    if (warp < 4) {
+      bool const ok = lane < kn && (warp < 3 || doCoul);
+      cpAsync<8>(&sC2[warp * BK + lane], ok ? csrc + k0 : a.p2, ok ? 8 : 0);
     }
   };
 
@@ -214,16 +256,26 @@ __global__ void __launch_bounds__(32 * contractWarps(RT), RT == 1 ? 1 : (RT * NT
     double const * sC2 = sV + BK * VLD;
     double const * sP2 = sC2 + 4 * BK;
     int const kn = int(min(int64_t(BK), r2end - k0));
-    bool const half = k0 < r2half;
-#pragma unroll 1
-    for (int p0 = 0; p0 < BK; p0 += 8) {
-      double x[RT][2];
+    // the own square's stages come first: once they are in, T holds them at half weight
+    if (step > 0 && k0 >= r2half && k0 - BK < r2half) {
+#pragma unroll
+      for (int i = 0; i < RT; ++i)
+#pragma unroll
+        for (int j = 0; j < NTL; ++j) { acc[i][j][0] *= 0.5; acc[i][j][1] *= 0.5; }
+    }
+    // X of the 8 points from p0: x[i][e] = g rho at row tile i, point 2 q + e.  Points past kn are zeros in
+    // V, psi2 and coul; 1/r12 is finite there, the transcorrelated kernels are masked
+    auto generate = [&](int p0, double (&x)[RT][2]) {
 #pragma unroll
       for (int i = 0; i < RT; ++i) x[i][0] = x[i][1] = R > 0 ? 0.0 : 1.0;
-      for (int b = fq; b < R4; b += 4) {
-        double const q = sP2[(p0 + fr) * pld + b];
 #pragma unroll
-        for (int i = 0; i < RT; ++i) dmma(x[i], sP1[(wrow + 8 * i) * pld + b], q);
+      for (int b = fq; b < R4 + fq; b += 4) {
+        double const q = sP2[(p0 + fr) * pld + b];
+        if constexpr (RT == 1) dmma(x[0], sP1[wrow * pld + b], q);
+        else {
+#pragma unroll
+          for (int i = 0; i < RT; i += 2) dmma16(x[i], x[i + 1], sP1[(wrow + 8 * i) * pld + b], sP1[(wrow + 8 * i + 8) * pld + b], q);
+        }
       }
       int const c = p0 + 2 * fq;
       double2 const px = *reinterpret_cast<double2 const *>(&sC2[c]);
@@ -234,33 +286,42 @@ __global__ void __launch_bounds__(32 * contractWarps(RT), RT == 1 ? 1 : (RT * NT
       for (int i = 0; i < RT; ++i) {
         double g0 = r12Kernel<KIND>(a, x1[i], y1[i], z1[i], px.x, py.x, pz.x);
         double g1 = r12Kernel<KIND>(a, x1[i], y1[i], z1[i], px.y, py.y, pz.y);
-        g0 = c < kn ? g0 : 0.0;
-        g1 = c + 1 < kn ? g1 : 0.0;
+        if constexpr (KIND != 0) {
+          g0 = c < kn ? g0 : 0.0;
+          g1 = c + 1 < kn ? g1 : 0.0;
+        }
         vh[i] = fma(g0, pc.x, fma(g1, pc.y, vh[i]));
-        if (half) { g0 *= 0.5; g1 *= 0.5; }
         x[i][0] *= g0;
         x[i][1] *= g1;
       }
+    };
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        double const * v = sV + (c + e) * VLD;   // row 2 q + e: the k index of this lane's B fragments
+    for (int p0 = 0; p0 < BK; p0 += 8) {
+      int const c = p0 + 2 * fq;
+      double x[RT][2];
+      generate(p0, x);
+      // B fragments: rows 2 q (step 0) and 2 q + 1 (step 1) of this 8-point group
+      double const * v = sV + c * VLD;
+      auto gemm = [&](int j, double b0, double b1) {
+        if constexpr (RT == 1) {
+          dmma(acc[0][j], x[0][0], b0);
+          dmma(acc[0][j], x[0][1], b1);
+        } else {
 #pragma unroll
-        for (int j = 0; j + 1 < NTL; j += 2) {
-          double2 const b = *reinterpret_cast<double2 const *>(&v[8 * j + 2 * fr]);
-#pragma unroll
-          for (int i = 0; i < RT; ++i) {
-            dmma(acc[i][j], x[i][e], b.x);
-            dmma(acc[i][j + 1], x[i][e], b.y);
-          }
+          for (int i = 0; i < RT; i += 2) dmma16k8(acc[i][j], acc[i + 1][j], x[i][0], x[i + 1][0], x[i][1], x[i + 1][1], b0, b1);
         }
-        if constexpr (NTL % 2) {
-          double const b = v[8 * (NTL - 1) + fr];
+      };
 #pragma unroll
-          for (int i = 0; i < RT; ++i) dmma(acc[i][NTL - 1], x[i][e], b);
-        }
+      for (int j = 0; j + 1 < NTL; j += 2) {
+        double2 const b0 = *reinterpret_cast<double2 const *>(&v[8 * j + 2 * fr]);
+        double2 const b1 = *reinterpret_cast<double2 const *>(&v[VLD + 8 * j + 2 * fr]);
+        gemm(j, b0.x, b1.x);
+        gemm(j + 1, b0.y, b1.y);
       }
+      if constexpr (NTL % 2) gemm(NTL - 1, v[8 * (NTL - 1) + fr], v[VLD + 8 * (NTL - 1) + fr]);
     }
   }
+  double const last = nsteps > 0 && r2begin + (nsteps - 1) * BK < r2half ? 0.5 : 1.0;   // only stages of the own square
 
   double * T = a.T + blockIdx.y * a.tStrideSplit;
 #pragma unroll
@@ -274,7 +335,7 @@ __global__ void __launch_bounds__(32 * contractWarps(RT), RT == 1 ? 1 : (RT * NT
         // D column n = 2 q + e of tile j is column 8 (j - j % 2) + 2 n + j % 2 of the block (the last tile of an odd count: 8 j + n)
         int const n = 2 * fq + e;
         int const col = col0 + (NTL % 2 && j == NTL - 1 ? 8 * j + n : 8 * (j & ~1) + 2 * n + (j & 1));
-        if (col < ncol) T[g * a.ldt + col] = acc[i][j][e];
+        if (col < ncol) T[g * a.ldt + col] = last * acc[i][j][e];
       }
   }
   if (doCoul) {
@@ -493,51 +554,70 @@ __global__ void __launch_bounds__(NT) kReduceComplex(int64_t n1, int nb, const d
   }
 }
 
-template <int KIND, int NTL, int RT>
+template <int KIND, int NTL, int RT, int KR>
 int launchOne(tcscf_ctx * ctx, KArgs const & a, dim3 grid, size_t smem)
 {
-  TCSCF_CUDA(ctx, cudaFuncSetAttribute(kContractFp64<KIND, NTL, RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-  TCSCF_CUDA(ctx, cudaFuncSetAttribute(kContractFp64<KIND, NTL, RT>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-  kContractFp64<KIND, NTL, RT><<<grid, 32 * contractWarps(RT), smem, ctx->stream>>>(a);
+  TCSCF_CUDA(ctx, cudaFuncSetAttribute(kContractFp64<KIND, NTL, RT, KR>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  TCSCF_CUDA(ctx, cudaFuncSetAttribute(kContractFp64<KIND, NTL, RT, KR>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+  kContractFp64<KIND, NTL, RT, KR><<<grid, 32 * contractWarps(RT), smem, ctx->stream>>>(a);
   TCSCF_LAUNCH(ctx);
   return TCSCF_OK;
 }
 
+// the rank in steps of 4 as a template parameter where small (its loops and strides are then constants): 0 (the
+// precompute form), 1, 2, 3, 5, or -1 for any other; contractSteps rounds 4 up to 5
+constexpr int kAnySteps = -1;
+int contractSteps(int rt, int R)
+{
+  int const k = (R + 3) / 4;
+  return rt == 1 || k > 5 ? kAnySteps : (k == 4 ? 5 : k);
+}
+
+template <int NTL>
+int launchDirect(tcscf_ctx * ctx, int kr, KArgs const & a, dim3 grid, size_t smem)
+{
+  switch (kr) {
+    case 0: return launchOne<0, NTL, 2, 0>(ctx, a, grid, smem);
+    case 1: return launchOne<0, NTL, 2, 1>(ctx, a, grid, smem);
+    case 2: return launchOne<0, NTL, 2, 2>(ctx, a, grid, smem);
+    case 3: return launchOne<0, NTL, 2, 3>(ctx, a, grid, smem);
+    case 5: return launchOne<0, NTL, 2, 5>(ctx, a, grid, smem);
+    default: return launchOne<0, NTL, 2, kAnySteps>(ctx, a, grid, smem);
+  }
+}
+
 // the 8-column tiles of a block (contractTiles' result) and its row tiles per warp, as template parameters
 template <int KIND>
-int launchKind(tcscf_ctx * ctx, int nt, int rt, KArgs const & a, dim3 grid, size_t smem)
+int launchKind(tcscf_ctx * ctx, int nt, int rt, int kr, KArgs const & a, dim3 grid, size_t smem)
 {
   if constexpr (KIND == 0) {
     if (rt == 1) {
-      if (nt == 4) return launchOne<0, 4, 1>(ctx, a, grid, smem);
-      if (nt == 8) return launchOne<0, 8, 1>(ctx, a, grid, smem);
-      return launchOne<0, 16, 1>(ctx, a, grid, smem);
+      if (nt == 4) return launchOne<0, 4, 1, kAnySteps>(ctx, a, grid, smem);
+      if (nt == 8) return launchOne<0, 8, 1, kAnySteps>(ctx, a, grid, smem);
+      return launchOne<0, 16, 1, kAnySteps>(ctx, a, grid, smem);
     }
     switch (nt) {
-      case 1: return launchOne<0, 1, 4>(ctx, a, grid, smem);
-      case 2: return launchOne<0, 2, 4>(ctx, a, grid, smem);
-      case 3: return launchOne<0, 3, 4>(ctx, a, grid, smem);
-      case 4: return launchOne<0, 4, 4>(ctx, a, grid, smem);
-      case 5: return launchOne<0, 5, 4>(ctx, a, grid, smem);
-      case 6: return launchOne<0, 6, 4>(ctx, a, grid, smem);
-      case 7: return launchOne<0, 7, 4>(ctx, a, grid, smem);
-      case 8: return launchOne<0, 8, 4>(ctx, a, grid, smem);
-      case 10: return launchOne<0, 10, 2>(ctx, a, grid, smem);
-      case 12: return launchOne<0, 12, 2>(ctx, a, grid, smem);
-      case 13: return launchOne<0, 13, 2>(ctx, a, grid, smem);
-      case 14: return launchOne<0, 14, 2>(ctx, a, grid, smem);
-      case 15: return launchOne<0, 15, 2>(ctx, a, grid, smem);
-      default: return launchOne<0, 16, 2>(ctx, a, grid, smem);
+      case 1: return launchDirect<1>(ctx, kr, a, grid, smem);
+      case 2: return launchDirect<2>(ctx, kr, a, grid, smem);
+      case 3: return launchDirect<3>(ctx, kr, a, grid, smem);
+      case 4: return launchDirect<4>(ctx, kr, a, grid, smem);
+      case 5: return launchDirect<5>(ctx, kr, a, grid, smem);
+      case 6: return launchDirect<6>(ctx, kr, a, grid, smem);
+      case 8: return launchDirect<8>(ctx, kr, a, grid, smem);
+      case 10: return launchDirect<10>(ctx, kr, a, grid, smem);
+      case 12: return launchDirect<12>(ctx, kr, a, grid, smem);
+      case 13: return launchDirect<13>(ctx, kr, a, grid, smem);
+      case 15: return launchDirect<15>(ctx, kr, a, grid, smem);
+      default: return launchDirect<16>(ctx, kr, a, grid, smem);
     }
   } else {
     switch (nt) {
-      case 4: return launchOne<KIND, 4, 2>(ctx, a, grid, smem);
-      case 8: return launchOne<KIND, 8, 2>(ctx, a, grid, smem);
-      case 12: return launchOne<KIND, 12, 2>(ctx, a, grid, smem);
-      case 13: return launchOne<KIND, 13, 2>(ctx, a, grid, smem);
-      case 14: return launchOne<KIND, 14, 2>(ctx, a, grid, smem);
-      case 15: return launchOne<KIND, 15, 2>(ctx, a, grid, smem);
-      default: return launchOne<KIND, 16, 2>(ctx, a, grid, smem);
+      case 4: return launchOne<KIND, 4, 2, 0>(ctx, a, grid, smem);
+      case 8: return launchOne<KIND, 8, 2, 0>(ctx, a, grid, smem);
+      case 12: return launchOne<KIND, 12, 2, 0>(ctx, a, grid, smem);
+      case 13: return launchOne<KIND, 13, 2, 0>(ctx, a, grid, smem);
+      case 15: return launchOne<KIND, 15, 2, 0>(ctx, a, grid, smem);
+      default: return launchOne<KIND, 16, 2, 0>(ctx, a, grid, smem);
     }
   }
 }
@@ -545,14 +625,14 @@ int launchKind(tcscf_ctx * ctx, int nt, int rt, KArgs const & a, dim3 grid, size
 // the smallest instantiated tile count that holds nt tiles
 int contractTiles(int kind, int rt, int nt)
 {
-  static int const direct[] = {1, 2, 3, 4, 5, 6, 7, 8, 10, 12, 13, 14, 15, 16}, wideRank[] = {4, 8, 16}, tc[] = {4, 8, 12, 13, 14, 15, 16};
+  static int const direct[] = {1, 2, 3, 4, 5, 6, 8, 10, 12, 13, 15, 16}, wideRank[] = {4, 8, 16}, tc[] = {4, 8, 12, 13, 15, 16};
   auto pick = [&](auto const & v) { for (int t : v) if (t >= nt) return t; return 16; };
   return kind != 0 ? pick(tc) : (rt == 1 ? pick(wideRank) : pick(direct));
 }
 
 size_t contractSmem(int nt, int rt, int R)
 {
-  int const bm = 8 * rt * contractWarps(rt), p = R > 0 ? fragStride((R + 3) / 4 * 4) : 0;
+  int const kr = contractSteps(rt, R), bm = 8 * rt * contractWarps(rt), p = R > 0 ? fragStride(kr > 0 ? 4 * kr : (R + 3) / 4 * 4) : 0;
   return sizeof(double) * (size_t(bm) * p + 2 * (size_t(BK) * vStride(nt) + 4 * BK + size_t(BK) * p));
 }
 
@@ -567,10 +647,10 @@ int contractFp64(tcscf_ctx * ctx, Contraction const & c)
   // columns in equal groups of at most 128 (g is generated once per group)
   int const cgroups = (c.ncol + kMaxCol - 1) / kMaxCol;
   int const colsPerBlock = ((c.ncol + cgroups - 1) / cgroups + 7) / 8 * 8;
-  // row tiles per warp: the accumulators (4 RT NT registers a thread) fit with RT = 4 up to 64 columns and RT = 2
-  // above; the transcorrelated kernels take RT = 2 (their g needs the registers); ranks whose factor rows
-  // would leave room for one block of 4 warps per SM take 8 warps of one row tile
-  int rt = kind == 0 && colsPerBlock <= 64 ? 4 : 2;
+  // two row tiles per warp (with four, 59,000 points x 40 columns took 9.8 ms against 8.5: half the warps, and
+  // the accumulators spilled); ranks whose factor rows would leave room for one block of 4 warps per
+  // SM take 8 warps of one row tile
+  int rt = 2;
   if (kind == 0 && contractSmem(contractTiles(kind, rt, colsPerBlock / 8), rt, c.R) > 112 * 1024) rt = 1;
   int const nt = contractTiles(kind, rt, colsPerBlock / 8);
   int const bm = 8 * rt * contractWarps(rt);
@@ -627,8 +707,8 @@ int contractFp64(tcscf_ctx * ctx, Contraction const & c)
   // the contraction kernel alone is bracketed by the context's timing events (tcscf_last_timing)
   if (!ctx->capturing) cudaEventRecord(ctx->ev[2], ctx->stream);
   dim3 const grid{unsigned(tiles), unsigned(nsplit), unsigned(cgroups)};
-  TCSCF_TRY(kind == 0 ? launchKind<0>(ctx, nt, rt, a, grid, smem) : (kind == 1 ? launchKind<1>(ctx, nt, rt, a, grid, smem)
-                                                                                  : launchKind<2>(ctx, nt, rt, a, grid, smem)));
+  TCSCF_TRY(kind == 0 ? launchKind<0>(ctx, nt, rt, contractSteps(rt, c.R), a, grid, smem) : (kind == 1 ? launchKind<1>(ctx, nt, rt, 0, a, grid, smem)
+              : launchKind<2>(ctx, nt, rt, 0, a, grid, smem)));
   if (!ctx->capturing) cudaEventRecord(ctx->ev[3], ctx->stream);
   if (nsplit > 1) {
     int64_t const n = c.n1 * c.ncol;
