@@ -81,7 +81,12 @@ struct tcscf_ctx {
   std::map<int, tcscf::Grid> grids;
   std::map<int, tcscf::Tensor> tensors;
   int nextId = 1;
-  cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
+  // ev[0] / ev[1] bracket a whole call; ev[2 + 2 k] / ev[3 + 2 k] the k-th contraction of a Fock build (up to two
+  // spins, real and imaginary parts), read after the call's last synchronisation
+  cudaEvent_t ev[10] = {};
+  int evPart = 0;
+  cudaEvent_t evStart() const { return ev[2 + 2 * evPart]; }
+  cudaEvent_t evStop() const { return ev[3 + 2 * evPart]; }
   double lastContractionMs = 0, lastTotalMs = 0;
   int lastLaunches = 0;
   int launchCount = 0;
@@ -204,5 +209,39 @@ __device__ __forceinline__ double invR12(double r2)
   double const e = fma(-r2 * y, y, 1.0);
   return fma(y * e, fma(0.375, e, 0.5), y);
 }
+
+// D += A B on the FP64 tensor cores: A[r][k] at lane 4 r + k, B[k][n] at lane 4 n + k, D[r][2 q + e] at
+// lane 4 r + q (element e)
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b)
+{
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(d[0]), "+d"(d[1]) : "d"(a), "d"(b));
+}
+// two row tiles (d0 and d1, rows 8 apart) in one instruction, k = 4 and k = 8 (the second half at a2, a3 and b1)
+__device__ __forceinline__ void dmma16(double (&d0)[2], double (&d1)[2], double a0, double a1, double b)
+{
+  asm("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};"
+      : "+d"(d0[0]), "+d"(d0[1]), "+d"(d1[0]), "+d"(d1[1]) : "d"(a0), "d"(a1), "d"(b));
+}
+__device__ __forceinline__ void dmma16k8(double (&d0)[2], double (&d1)[2], double a0, double a1, double a2, double a3, double b0, double b1)
+{
+  asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+d"(d0[0]), "+d"(d0[1]), "+d"(d1[0]), "+d"(d1[1]) : "d"(a0), "d"(a1), "d"(a2), "d"(a3), "d"(b0), "d"(b1));
+}
+
+// row stride (doubles) of a shared-memory operand with `n4` columns (a multiple of 4) whose fragments read 4
+// consecutive doubles of 8 rows: 4 or 12 mod 16 spreads a half-warp over all 16 bank pairs
+__host__ __device__ constexpr int fragStride(int n4) { return n4 % 8 == 4 ? n4 : n4 + 4; }
+
+// copies `bytes` (0, 8 or WIDTH) of a WIDTH-byte chunk and zero-fills the rest
+template <int WIDTH>
+__device__ __forceinline__ void cpAsync(double * dst, const double * src, int bytes)
+{
+  unsigned const d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+  if constexpr (WIDTH == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cpAsyncCommit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cpAsyncWait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 }  // namespace tcscf

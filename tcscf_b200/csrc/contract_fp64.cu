@@ -17,7 +17,7 @@ namespace {
 
 constexpr int BK = 32;        // r2 points per stage
 constexpr int kMaxCol = 128;  // columns per block at most
-constexpr int NT = 256;       // threads of the reductions
+constexpr int NT = 256;       // threads of the complex reduction
 
 struct KArgs {
   int64_t n1, n2, r2PerSplit;
@@ -86,38 +86,6 @@ __device__ __forceinline__ double r12Kernel(KArgs const & a, double x1, double y
   return a.component == 0 ? gx : (a.component == 1 ? gy : gz);
 }
 
-// copies `bytes` (0, 8 or WIDTH) of a WIDTH-byte chunk and zero-fills the rest
-template <int WIDTH>
-__device__ __forceinline__ void cpAsync(double * dst, const double * src, int bytes)
-{
-  unsigned const d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-  if constexpr (WIDTH == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(bytes) : "memory");
-  else asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void cpAsyncCommit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cpAsyncWait1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
-
-// D += A B on the FP64 tensor cores: A[r][k] at lane 4 r + k, B[k][n] at lane 4 n + k, D[r][2 q + e] at
-// lane 4 r + q (element e)
-__device__ __forceinline__ void dmma(double (&d)[2], double a, double b)
-{
-  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(d[0]), "+d"(d[1]) : "d"(a), "d"(b));
-}
-// two row tiles (d0 and d1, rows 8 apart) in one instruction, k = 4 and k = 8 (the second half at a2, a3 and b1)
-__device__ __forceinline__ void dmma16(double (&d0)[2], double (&d1)[2], double a0, double a1, double b)
-{
-  asm("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};"
-      : "+d"(d0[0]), "+d"(d0[1]), "+d"(d1[0]), "+d"(d1[1]) : "d"(a0), "d"(a1), "d"(b));
-}
-__device__ __forceinline__ void dmma16k8(double (&d0)[2], double (&d1)[2], double a0, double a1, double a2, double a3, double b0, double b1)
-{
-  asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-      : "+d"(d0[0]), "+d"(d0[1]), "+d"(d1[0]), "+d"(d1[1]) : "d"(a0), "d"(a1), "d"(a2), "d"(a3), "d"(b0), "d"(b1));
-}
-
-// row stride (doubles) of a shared-memory operand with `n4` columns (a multiple of 4) whose fragments read 4
-// consecutive doubles of 8 rows: 4 or 12 mod 16 spreads a half-warp over all 16 bank pairs
-__host__ __device__ constexpr int fragStride(int n4) { return n4 % 8 == 4 ? n4 : n4 + 4; }
 // row stride of the V tile (2 mod 8: the 16-byte fragment loads below read rows 2 k + e)
 __host__ __device__ constexpr int vStride(int nt) { return 8 * nt + 2; }
 __host__ __device__ constexpr int contractWarps(int rt) { return rt == 1 ? 8 : 4; }
@@ -250,7 +218,7 @@ __global__ void __launch_bounds__(32 * contractWarps(RT), contractBlocks(NTL, RT
     __syncthreads();   // every thread is done with the stage the next issue overwrites
     if (step + 1 < nsteps) issue(k0 + BK, st ^ 1);
     cpAsyncCommit();
-    cpAsyncWait1();
+    cpAsyncWait<1>();
     __syncthreads();
     double const * sV = stage0 + st * stageSize;
     double const * sC2 = sV + BK * VLD;
@@ -426,73 +394,120 @@ __global__ void kSumSplits(int64_t n, int nsplit, int64_t stride, const double *
   (void)rows;
 }
 
-// ---- real Fock reduction:  out[k][l] = sum_r w[r] phi[r][k] (cJ phi[r][l] VH[r] - sgnT T[r][l]) ----
+// ---- real Fock reduction:  out[k][l] = sum_r w[r] phi[r][k] (cJ phi[r][l] VH[r] - T[r][l]) ----
 constexpr int RB = 16;      // rows per step
 constexpr int RCH = 1024;   // rows per block (complex reduction; the real one sizes its row chunks per call)
 
-// one block: `rch` rows (a multiple of RB) into a W x W tile of out (W = 64 or 128; 16 x 16 threads, TT x TT each)
-template <int W>
-__global__ void __launch_bounds__(NT) kReduceReal(int64_t n1, int nb, int rch, const double * phi, const double * w, const double * VH,
-                                                  double cJ, const double * T, int ldt, double sgnT, double * part)
+struct ReduceArgs {
+  int64_t n1, tStride;        // rows; elements between the spins' T
+  int nb, ldt, rch;
+  const double * phi;
+  const double * w;
+  const double * VH;          // null: no Coulomb term
+  const double * T;
+  double cJ[2];               // per spin
+};
+
+// One block: `rch` rows (a multiple of RB) into a W x W tile of one spin's sum, W = 8 WT Q: Q x Q warps of (8 WT)^2 on
+// the FP64 tensor cores, whose fragments are 8 consecutive doubles of 4 rows (stride 4 mod 16:
+// conflict-free).  Rows pass through two shared-memory stages of RB, the next stage's values loaded into registers
+// while the current one is multiplied.  Q = 4 up to 128 columns reads phi and T once (Q = 2 would, above
+// 64 columns, read them once per 64-wide tile).  Bound by the FP64 MMAs.  The CUDA-core form (8 x 8 outputs a
+// thread, no prefetch) took, per call, 1.38 -> 1.09 ms for Kr (406,000
+// points, 120 columns) and 61 -> 36 us for Ne (59,000, 40), and symmetric builds called it twice.
+template <int WT, int Q>
+__global__ void __launch_bounds__(32 * Q * Q) kReduceReal(ReduceArgs a, double * part)
 {
-  constexpr int TT = W / 16;
-  __shared__ __align__(16) double sA[RB][W];
-  __shared__ __align__(16) double sY[RB][W];
-  int const tid = threadIdx.x;
-  int const kg = blockIdx.y * W, lg = blockIdx.z * W;
-  int64_t const rbeg = int64_t(blockIdx.x) * rch, rend = min(n1, rbeg + rch);
-  int const tk = tid >> 4, tl = tid & 15;
-  double acc[TT][TT];
+  constexpr int NTH = 32 * Q * Q, W = 8 * WT * Q, LD = W % 16 == 8 ? W + 12 : W + 4, VPT = RB * W / NTH;
+  static_assert(LD % 16 == 4 && RB * W % NTH == 0, "fragment stride; values per thread");
+  extern __shared__ __align__(16) double sm[];
+  auto sA = reinterpret_cast<double(*)[RB][LD]>(sm);   // [2][RB][LD]
+  auto sY = sA + 2;
+  int const tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, fr = lane >> 2, fq = lane & 3;
+  int const tilesW = (a.nb + W - 1) / W, spin = blockIdx.z;
+  int const kg = blockIdx.y / tilesW * W, lg = blockIdx.y % tilesW * W;
+  int const wk = warp / Q * 8 * WT, wl = warp % Q * 8 * WT;
+  double const * T = a.T + spin * a.tStride;
+  double const cJ = a.cJ[spin];
+  int64_t const rbeg = int64_t(blockIdx.x) * a.rch, rend = min(a.n1, rbeg + a.rch);
+  double acc[WT][WT][2];
 #pragma unroll
-  for (int i = 0; i < TT; ++i)
+  for (int i = 0; i < WT; ++i)
 #pragma unroll
-    for (int j = 0; j < TT; ++j) acc[i][j] = 0.0;
-  for (int64_t r0 = rbeg; r0 < rend; r0 += RB) {
-    __syncthreads();
-    for (int idx = tid; idx < RB * W; idx += NT) {
-      int const rr = idx / W, c = idx % W;
-      int64_t const r = r0 + rr;
-      double av = 0.0, yv = 0.0;
-      if (r < rend) {
-        int const k = kg + c, l = lg + c;
-        if (k < nb) av = w[r] * phi[r * nb + k];
-        if (l < nb) {
-          double y = 0.0;
-          if (VH) y = cJ * phi[r * nb + l] * VH[r];
-          if (T) y -= sgnT * T[r * ldt + l];
-          yv = y;
-        }
-      }
-      sA[rr][c] = av;
-      sY[rr][c] = yv;
+    for (int j = 0; j < WT; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  double av[VPT], yv[VPT];
+  auto load = [&](int64_t r0) {
+#pragma unroll
+    for (int q = 0; q < VPT; ++q) {
+      int const idx = tid + q * NTH, c = idx % W, k = kg + c, l = lg + c;
+      int64_t const r = r0 + idx / W;
+      bool const in = r < rend;
+      double const pk = in && k < a.nb ? a.phi[r * a.nb + k] : 0.0;
+      double const pl = kg == lg ? pk : (in && l < a.nb ? a.phi[r * a.nb + l] : 0.0);
+      double const t = in && l < a.nb ? T[r * a.ldt + l] : 0.0;
+      av[q] = in ? a.w[r] * pk : 0.0;
+      yv[q] = (in && a.VH ? cJ * pl * a.VH[r] : 0.0) - t;
     }
-    __syncthreads();
-#pragma unroll 2
-    for (int rr = 0; rr < RB; ++rr) {
-      double av[TT], bv[TT];
+  };
+  auto store = [&](int st) {
 #pragma unroll
-      for (int q = 0; q < TT / 2; ++q) {
-        double2 const x = *reinterpret_cast<double2 const *>(&sA[rr][tk * TT + 2 * q]);
-        double2 const y = *reinterpret_cast<double2 const *>(&sY[rr][tl * TT + 2 * q]);
-        av[2 * q] = x.x; av[2 * q + 1] = x.y;
-        bv[2 * q] = y.x; bv[2 * q + 1] = y.y;
-      }
-#pragma unroll
-      for (int i = 0; i < TT; ++i)
-#pragma unroll
-        for (int j = 0; j < TT; ++j) acc[i][j] = fma(av[i], bv[j], acc[i][j]);
+    for (int q = 0; q < VPT; ++q) {
+      int const idx = tid + q * NTH;
+      sA[st][idx / W][idx % W] = av[q];
+      sY[st][idx / W][idx % W] = yv[q];
     }
+  };
+  if (rbeg < rend) {
+    load(rbeg);
+    store(0);
   }
-  double * out = part + int64_t(blockIdx.x) * nb * nb;
+  __syncthreads();
+  int st = 0;
+  for (int64_t r0 = rbeg; r0 < rend; r0 += RB, st ^= 1) {
+    bool const more = r0 + RB < rend;
+    if (more) load(r0 + RB);
 #pragma unroll
-  for (int i = 0; i < TT; ++i) {
-    int const k = kg + tk * TT + i;
-    if (k >= nb) continue;
+    for (int rr = 0; rr < RB; rr += 4) {
+      double af[WT], bf[WT];
 #pragma unroll
-    for (int j = 0; j < TT; ++j) {
-      int const l = lg + tl * TT + j;
-      if (l < nb) out[k * nb + l] = acc[i][j];
+      for (int i = 0; i < WT; ++i) { af[i] = sA[st][rr + fq][wk + 8 * i + fr]; bf[i] = sY[st][rr + fq][wl + 8 * i + fr]; }
+#pragma unroll
+      for (int i = 0; i < WT; ++i)
+#pragma unroll
+        for (int j = 0; j < WT; ++j) dmma(acc[i][j], af[i], bf[j]);
     }
+    if (more) store(st ^ 1);   // the stage before's buffer: every warp finished it before the last barrier
+    __syncthreads();
+  }
+  double * out = part + (int64_t(spin) * gridDim.x + blockIdx.x) * a.nb * a.nb;
+#pragma unroll
+  for (int i = 0; i < WT; ++i)
+#pragma unroll
+    for (int j = 0; j < WT; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        int const k = kg + wk + 8 * i + fr, l = lg + wl + 8 * j + 2 * fq + e;
+        if (k < a.nb && l < a.nb) out[k * a.nb + l] = acc[i][j][e];
+      }
+}
+
+// out[s][e] = the sum over the chunks k of part[s][k][e], e < n: 32 elements per block, 8 warps taking every eighth chunk each
+// (their sums added in warp order), so that a few hundred chunks of a small matrix are not one thread's chain
+__global__ void __launch_bounds__(256) kReduceSum(int n, int nchunk, const double * part, double * out)
+{
+  __shared__ double red[8][32];
+  int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5, e = blockIdx.x * 32 + lane;
+  part += int64_t(blockIdx.y) * nchunk * n;
+  double s = 0.0;
+  if (e < n)
+#pragma unroll 4
+    for (int k = warp; k < nchunk; k += 8) s += part[int64_t(k) * n + e];
+  red[warp][lane] = s;
+  __syncthreads();
+  if (warp == 0 && e < n) {
+#pragma unroll
+    for (int k = 1; k < 8; ++k) s += red[k][lane];
+    out[int64_t(blockIdx.y) * n + e] = s;
   }
 }
 
@@ -705,11 +720,11 @@ int contractFp64(tcscf_ctx * ctx, Contraction const & c)
   size_t const smem = contractSmem(nt, rt, c.R);
   TCSCF_CHECK(ctx, smem <= 227 * 1024, TCSCF_ERR_UNSUPPORTED, "internal: contraction tile beyond the shared memory");
   // the contraction kernel alone is bracketed by the context's timing events (tcscf_last_timing)
-  if (!ctx->capturing) cudaEventRecord(ctx->ev[2], ctx->stream);
+  if (!ctx->capturing) cudaEventRecord(ctx->evStart(), ctx->stream);
   dim3 const grid{unsigned(tiles), unsigned(nsplit), unsigned(cgroups)};
   TCSCF_TRY(kind == 0 ? launchKind<0>(ctx, nt, rt, contractSteps(rt, c.R), a, grid, smem) : (kind == 1 ? launchKind<1>(ctx, nt, rt, 0, a, grid, smem)
               : launchKind<2>(ctx, nt, rt, 0, a, grid, smem)));
-  if (!ctx->capturing) cudaEventRecord(ctx->ev[3], ctx->stream);
+  if (!ctx->capturing) cudaEventRecord(ctx->evStop(), ctx->stream);
   if (nsplit > 1) {
     int64_t const n = c.n1 * c.ncol;
     kSumSplits<<<gridBlocks(n, 256), 256, 0, ctx->stream>>>(n, int(nsplit), c.n1 * c.ldt, Tpart, c.T, c.n1, c.ncol, c.ldt, c.ldt);
@@ -745,28 +760,40 @@ int sumSplitsLaunch(tcscf_ctx * ctx, int64_t n, int nsplit, int64_t stride, cons
   return TCSCF_OK;
 }
 
-int reduceFockReal(tcscf_ctx * ctx, int64_t n1, int nb, const double * phi, const double * w1, const double * VH, double cJ,
-                   const double * T, int ldt, double sgnT, double * out)
+int reduceFockReal(tcscf_ctx * ctx, int64_t n1, int nb, int nspin, const double * phi, const double * w1, const double * VH,
+                   const double * cJ, const double * T, int64_t tStride, int ldt, double * out)
 {
-  // output tiles 64 wide (70 registers a thread: three blocks per SM, where the 128-wide tile's 168
-  // allowed one, whose global-to-shared staging then stalled its FP64 FMAs); row chunks sized for about
-  // two blocks per SM per output tile (16 to 1024 rows)
-  int const W = 64;
-  int const g = (nb + W - 1) / W;
+  // tiles 16, 32, 48 or 64 wide with 4 warps up to 64 columns, 96 or 128 wide with 16 warps above: the least padding
+  int const Q = nb <= 64 ? 2 : 4;
+  int const wt = Q == 2 ? (nb + 15) / 16 : (nb <= 96 ? 3 : 4);
+  int const W = 8 * wt * Q, g = (nb + W - 1) / W;
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-  int64_t const want = (n1 + 2 * sms * g * g - 1) / (2 * sms * g * g);
-  int const rch = int(std::min<int64_t>(1024, std::max<int64_t>(RB, (want + RB - 1) / RB * RB)));
+  // row chunks for four small or two large blocks per SM (16 to 1024 rows a chunk)
+  int64_t const blocks = std::max<int64_t>(1, (Q == 2 ? 4 : 2) * int64_t(sms) / (int64_t(g) * g * nspin));
+  int64_t const rows = (n1 + blocks - 1) / blocks;
+  int const rch = int(std::min<int64_t>(1024, std::max<int64_t>(RB, (rows + RB - 1) / RB * RB)));
   int64_t const chunks = (n1 + rch - 1) / rch;
   void * p = nullptr;
-  TCSCF_TRY(scratch(ctx, "reduce_real", size_t(chunks) * nb * nb * sizeof(double), &p));
+  TCSCF_TRY(scratch(ctx, "reduce_real", size_t(nspin) * chunks * nb * nb * sizeof(double), &p));
   double * part = static_cast<double *>(p);
-  dim3 grid{unsigned(chunks), unsigned(g), unsigned(g)};
-  if (W == 64) kReduceReal<64><<<grid, NT, 0, ctx->stream>>>(n1, nb, rch, phi, w1, VH, cJ, T, ldt, sgnT, part);
-  else kReduceReal<128><<<grid, NT, 0, ctx->stream>>>(n1, nb, rch, phi, w1, VH, cJ, T, ldt, sgnT, part);
+  ReduceArgs a{n1, tStride, nb, ldt, rch, phi, w1, VH, T, {cJ[0], nspin > 1 ? cJ[1] : 0.0}};
+  dim3 const grid{unsigned(chunks), unsigned(g * g), unsigned(nspin)};
+  auto launch = [&](auto kernel) {
+    size_t const smem = sizeof(double) * 4 * RB * (W % 16 == 8 ? W + 12 : W + 4);
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    kernel<<<grid, 32 * Q * Q, smem, ctx->stream>>>(a, part);
+  };
+  if (Q == 2) {
+    if (wt == 1) launch(kReduceReal<1, 2>);
+    else if (wt == 2) launch(kReduceReal<2, 2>);
+    else if (wt == 3) launch(kReduceReal<3, 2>);
+    else launch(kReduceReal<4, 2>);
+  } else if (wt == 3) launch(kReduceReal<3, 4>);
+  else launch(kReduceReal<4, 4>);
   TCSCF_LAUNCH(ctx);
   int const n = nb * nb;
-  kSumChunks<<<(n + 255) / 256, 256, 0, ctx->stream>>>(n, int(chunks), part, out);
+  kReduceSum<<<dim3(unsigned((n + 31) / 32), unsigned(nspin)), 256, 0, ctx->stream>>>(n, int(chunks), part, out);
   TCSCF_LAUNCH(ctx);
   return TCSCF_OK;
 }

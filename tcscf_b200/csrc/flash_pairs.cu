@@ -552,7 +552,7 @@ int contractPairsTensor(tcscf_ctx * ctx, Contraction const & c, int precision)
   P.tStride = int64_t(c.n1) * c.ldt;
   P.status = dStatus;
   int const grid = int(std::min<int64_t>(items * nSplit, sms));
-  cudaEventRecord(ctx->ev[2], ctx->stream);
+  cudaEventRecord(ctx->evStart(), ctx->stream);
   int st = TCSCF_OK;
   if (NB == 64) {
     st = P.kind == 0 ? tc::launchPairs<64, 0>(ctx, P, maps, grid)
@@ -561,7 +561,7 @@ int contractPairsTensor(tcscf_ctx * ctx, Contraction const & c, int precision)
     st = P.kind == 0 ? tc::launchPairs<128, 0>(ctx, P, maps, grid)
                      : (P.kind == 1 ? tc::launchPairs<128, 1>(ctx, P, maps, grid) : tc::launchPairs<128, 2>(ctx, P, maps, grid));
   }
-  cudaEventRecord(ctx->ev[3], ctx->stream);
+  cudaEventRecord(ctx->evStop(), ctx->stream);
   TCSCF_TRY(st);
   int hs = 0;
   TCSCF_CUDA(ctx, cudaMemcpyAsync(&hs, dStatus, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));

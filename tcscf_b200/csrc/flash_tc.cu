@@ -1218,7 +1218,7 @@ int tensorRun(tcscf_ctx * ctx, TensorPrep * const * preps, int count, bool recor
   };
   std::vector<Launch> launches;
   size_t offset = 0;
-  if (recordStart) cudaEventRecord(ctx->ev[2], ctx->stream);
+  if (recordStart) cudaEventRecord(ctx->evStart(), ctx->stream);
   for (auto const & cl : kClasses) {
     int const NB = cl[0], RP = cl[1], XS = cl[2], NS = cl[3];
     std::vector<int4> items;
@@ -1274,7 +1274,7 @@ int tensorRun(tcscf_ctx * ctx, TensorPrep * const * preps, int count, bool recor
     }
     TCSCF_CUDA(ctx, cudaGraphLaunch(ctx->tensorGraph, ctx->stream));
   }
-  cudaEventRecord(ctx->ev[3], ctx->stream);
+  cudaEventRecord(ctx->evStop(), ctx->stream);
   int st = 0;
   TCSCF_CUDA(ctx, cudaMemcpyAsync(&st, dStatus, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   TCSCF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -1504,7 +1504,7 @@ int contractTensor(tcscf_ctx * ctx, Contraction const & c, int precision)
   }
   // rho is linear in the density factor: a rank beyond what one launch's psi tiles hold (32 for TF32
   // or with nb > 64, 64 otherwise) is contracted in column chunks whose T add up (the Coulomb potential,
-  // which does not depend on the factor, with the first); ev[2] / ev[3] span all chunks
+  // which does not depend on the factor, with the first); evStart() / evStop() span all chunks
   double * tmp = nullptr;
   TCSCF_TRY(scratch(ctx, "flash_tc_rank_chunk", sizeof(double) * size_t(c.n1) * c.ldt, reinterpret_cast<void **>(&tmp)));
   for (int r0 = 0; r0 < c.R; r0 += lim) {
@@ -1520,7 +1520,7 @@ int contractTensor(tcscf_ctx * ctx, Contraction const & c, int precision)
       TCSCF_LAUNCH(ctx);
     }
   }
-  cudaEventRecord(ctx->ev[3], ctx->stream);
+  cudaEventRecord(ctx->evStop(), ctx->stream);
   return nearCorrect(ctx, c);
 }
 

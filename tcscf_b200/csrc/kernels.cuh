@@ -147,9 +147,10 @@ int tensorPlanLaunch(tcscf_ctx * ctx, TensorPlan const & plan);
 int sumSplitsLaunch(tcscf_ctx * ctx, int64_t n, int nsplit, int64_t stride, const double * part, double * out, int64_t rows, int cols,
                     int ldOut, int ldPart);
 
-// G_s[k][l] (+)= sum_r1 w1 phi[r1][k] * (cJ * phi[r1][l] * VH[r1] - sgnT * T[r1][l]); real, out [nb][nb]
-int reduceFockReal(tcscf_ctx * ctx, int64_t n1, int nb, const double * phi, const double * w1, const double * VH, double cJ,
-                   const double * T, int ldt, double sgnT, double * out);
+// out_s[k][l] = sum_r1 w1 phi[r1][k] (cJ[s] phi[r1][l] VH[r1] - T_s[r1][l]) for s < nspin (T_s at T + s tStride); real, out [nspin][nb][nb].
+// A symmetric contraction's T' gives M with G = M + M^T when cJ is halved (the Coulomb part is symmetric)
+int reduceFockReal(tcscf_ctx * ctx, int64_t n1, int nb, int nspin, const double * phi, const double * w1, const double * VH,
+                   const double * cJ, const double * T, int64_t tStride, int ldt, double * out);
 
 // complex reduction G(j,i) = sum_r w[r] conj(A[r][j]) Y[r][i] with Y = cJ * A[r][i] * Faa[r] - Fai[r][i]
 int reduceFockComplex(tcscf_ctx * ctx, int64_t n1, int nb, const double * A, const double * w, const double * Faa, double cJ,

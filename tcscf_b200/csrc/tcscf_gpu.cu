@@ -256,31 +256,6 @@ __device__ __forceinline__ double2 urow(const DevSto * s, int k, int i)
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) { return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
 __device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -a.y); }
 
-// DR = conj(U) D U^T for each spin; D complex [nspin][nb][nb] (reference basis)
-__global__ void kDensityToReal(int nspin, int nb, const DevSto * s, const double2 * D, double2 * DR)
-{
-  int const total = nspin * nb * nb;
-  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
-    int const sp = idx / (nb * nb), k = (idx / nb) % nb, l = idx % nb;
-    int const ik[2] = {k, s[k].partner};
-    int const jl[2] = {l, s[l].partner};
-    double2 acc = make_double2(0, 0);
-    for (int a = 0; a < 2; ++a) {
-      int const i = ik[a];
-      if (i < 0) continue;
-      double2 const u1 = cconj(urow(s, k, i));
-      for (int b = 0; b < 2; ++b) {
-        int const j = jl[b];
-        if (j < 0) continue;
-        double2 const t = cmul(cmul(u1, D[sp * nb * nb + i * nb + j]), urow(s, l, j));
-        acc.x += t.x;
-        acc.y += t.y;
-      }
-    }
-    DR[idx] = acc;
-  }
-}
-
 // symmetric real part (column-major == row-major) and the imaginary magnitude, per spin
 __global__ void kSplitDensity(int nb, const double2 * DR, double * A, double * maxAbs)
 {
@@ -313,41 +288,118 @@ __global__ void kHermitianCopy(int nb, const double2 * DR, double2 * Z)
   }
 }
 
-// factor matrices X1, X2 [nb][ldx] from the kept eigenpairs (real case): X2 = v sqrt|l|, X1 = sign(l) X2
 constexpr int kCholeskyMaxNb = 128;
 
-// Pivoted (diagonal-pivoting) Cholesky factorisation of the real symmetric density A [nb][nb]:
-// A = L L^T with the R columns of L written to X1 and X2 ([nb][ldx], both L).  Stops when the largest
-// remaining diagonal is <= 1e-12 of the largest initial diagonal; info = {R, 0}, or {R, 1} when the
-// remainder is not negligible (largest |entry| above 1e-10 of the largest initial diagonal: the
-// density is not positive semi-definite and the caller factors it by eigen-decomposition).  One
-// block of 256 threads; shared memory nb * nb doubles (nb <= 128).
-__global__ void __launch_bounds__(256) kPivotedCholesky(int nb, const double * A, int ldx, double * X1, double * X2, int * info)
+// One density factorisation (FactorBufs below): D complex [nb][nb] in the reference basis, DR its real-harmonic form,
+// A the symmetrised real part, X1 and X2 the factors [nb][ldx], status {max |Re DR|, max |Im DR|, rank, indefinite}
+struct FactorStatus {
+  double maxAbs[2];
+  int rank, indefinite;
+};
+struct FactorJob {
+  int nb, ldx;
+  const DevSto * sto;
+  const double2 * D;
+  double2 * DR;
+  double * A, * X1, * X2;
+  FactorStatus * status;
+};
+
+// element (k, l) of conj(U) D U^T
+__device__ __forceinline__ double2 densityToReal(int nb, const DevSto * s, const double2 * D, int k, int l)
+{
+  int const ik[2] = {k, s[k].partner};
+  int const jl[2] = {l, s[l].partner};
+  double2 acc = make_double2(0, 0);
+  for (int a = 0; a < 2; ++a) {
+    int const i = ik[a];
+    if (i < 0) continue;
+    double2 const u1 = cconj(urow(s, k, i));
+    for (int b = 0; b < 2; ++b) {
+      int const j = jl[b];
+      if (j < 0) continue;
+      double2 const t = cmul(cmul(u1, D[i * nb + j]), urow(s, l, j));
+      acc.x += t.x;
+      acc.y += t.y;
+    }
+  }
+  return acc;
+}
+
+// DR = conj(U) D U^T; D complex [nb][nb] (reference basis)
+__global__ void kDensityToReal(int nb, const DevSto * s, const double2 * D, double2 * DR)
+{
+  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < nb * nb; idx += gridDim.x * blockDim.x) DR[idx] = densityToReal(nb, s, D, idx / nb, idx % nb);
+}
+
+// The whole factorisation of a density in one block of 256 threads (one block per job: a batch's densities in one
+// launch), so that a single build pays one launch for what four kernels did and a batch does not run one block
+// at a time.  (1) DR, A and the magnitudes.  (2) Pivoted (diagonal-pivoting) Cholesky factorisation of A:
+// A = L L^T with the R columns of L written to X1 and X2; stops when the largest remaining diagonal is <=
+// 1e-12 of the largest initial one; indefinite = 1 when the remainder is not negligible (largest |entry|
+// above 1e-10 of the largest initial diagonal: the caller factors the density by eigen-decomposition).
+// (3) One-sided Jacobi (Hestenes) orthogonalisation of L's columns (skipped when indefinite): L <- L W
+// with W orthogonal; X X^T = L L^T is unchanged and X's columns become the density's eigenvectors
+// scaled by the square roots of its eigenvalues (the factor the fixed-point and TF32 contractions are
+// accurate with: no cancellation between columns).  Column pairs in round-robin order, one pair per warp
+// at a time; at most 30 sweeps, ending when every pair is orthogonal to 1e-15 of its norms.  Bound by the
+// latency of its chain of barriers (a few per pivot and Jacobi step); shared memory nb * nb doubles;
+// bases above kCholeskyMaxNb take step (1) only and are marked indefinite.
+__global__ void __launch_bounds__(256) kFactorDensity(FactorJob one, const FactorJob * jobs)
 {
   extern __shared__ double S[];
   __shared__ double lcol[kCholeskyMaxNb];
   __shared__ int done[kCholeskyMaxNb];
-  __shared__ double rv[256];
-  __shared__ int ri[256];
-  int const t = threadIdx.x;
-  for (int i = t; i < nb * nb; i += 256) S[i] = A[i];
+  __shared__ double rv[8], rw[8];
+  __shared__ int ri[8];
+  __shared__ int rotated;
+  FactorJob const f = jobs ? jobs[blockIdx.x] : one;
+  int const nb = f.nb, ldx = f.ldx, t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  double mr = 0, mi = 0;
+  for (int idx = t; idx < nb * nb; idx += 256) {
+    double2 const d = densityToReal(nb, f.sto, f.D, idx / nb, idx % nb);
+    f.DR[idx] = d;
+    mr = fmax(mr, fabs(d.x));
+    mi = fmax(mi, fabs(d.y));
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    mr = fmax(mr, __shfl_xor_sync(0xffffffffu, mr, o));
+    mi = fmax(mi, __shfl_xor_sync(0xffffffffu, mi, o));
+  }
+  if (lane == 0) { rv[warp] = mr; rw[warp] = mi; }
+  __syncthreads();   // and DR is visible to the block
+  if (t == 0) {
+    for (int k = 1; k < 8; ++k) { mr = fmax(mr, rv[k]); mi = fmax(mi, rw[k]); }
+    f.status->maxAbs[0] = mr;
+    f.status->maxAbs[1] = mi;
+  }
+  bool const small = nb <= kCholeskyMaxNb;
+  for (int idx = t; idx < nb * nb; idx += 256) {
+    int const k = idx / nb, l = idx % nb;
+    double const v = 0.5 * (f.DR[idx].x + f.DR[l * nb + k].x);
+    f.A[idx] = v;
+    if (small) S[idx] = v;
+  }
+  if (!small) {
+    if (t == 0) { f.status->rank = 0; f.status->indefinite = 1; }
+    return;
+  }
   for (int i = t; i < nb; i += 256) done[i] = 0;
   __syncthreads();
   // block reduction of (value, index): largest value, smallest index among equals
+  auto better = [](double w, int wi, double v, int i) { return w > v || (w == v && wi >= 0 && (i < 0 || wi < i)); };
   auto argmax = [&](double v, int idx, double & bv, int & bi) {
-    rv[t] = v;
-    ri[t] = idx;
-    __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-      if (t < o) {
-        double const w = rv[t + o];
-        int const wi = ri[t + o];
-        if (w > rv[t] || (w == rv[t] && wi >= 0 && (ri[t] < 0 || wi < ri[t]))) { rv[t] = w; ri[t] = wi; }
-      }
-      __syncthreads();
+    for (int o = 16; o > 0; o >>= 1) {
+      double const w = __shfl_xor_sync(0xffffffffu, v, o);
+      int const wi = __shfl_xor_sync(0xffffffffu, idx, o);
+      if (better(w, wi, v, idx)) { v = w; idx = wi; }
     }
+    if (lane == 0) { rv[warp] = v; ri[warp] = idx; }
+    __syncthreads();
     bv = rv[0];
     bi = ri[0];
+    for (int k = 1; k < 8; ++k)
+      if (better(rv[k], ri[k], bv, bi)) { bv = rv[k]; bi = ri[k]; }
     __syncthreads();
   };
   double d0 = 0;
@@ -372,8 +424,7 @@ __global__ void __launch_bounds__(256) kPivotedCholesky(int nb, const double * A
     for (int i = t; i < nb; i += 256) {
       double const l = done[i] ? 0.0 : (i == p ? sq : S[i * nb + p] * inv);
       lcol[i] = l;
-      X1[int64_t(i) * ldx + R] = l;
-      X2[int64_t(i) * ldx + R] = l;
+      f.X1[int64_t(i) * ldx + R] = l;
     }
     __syncthreads();
     for (int idx = t; idx < nb * nb; idx += 256) S[idx] -= lcol[idx / nb] * lcol[idx % nb];
@@ -385,30 +436,17 @@ __global__ void __launch_bounds__(256) kPivotedCholesky(int nb, const double * A
     if (!done[idx / nb] && !done[idx % nb]) r = fmax(r, fabs(S[idx]));
   double rmax;
   argmax(r, -1, rmax, unused);
+  bool const indefinite = rmax > 1e-10 * d0 || !(rmax == rmax);
   if (t == 0) {
-    info[0] = R;
-    info[1] = (rmax > 1e-10 * d0 || !(rmax == rmax)) ? 1 : 0;
+    f.status->rank = R;
+    f.status->indefinite = indefinite ? 1 : 0;
   }
-}
-
-// One-sided Jacobi (Hestenes) orthogonalisation of the R = info[0] factor columns L [nb][ldx] of X1
-// (skipped when info[1] flags an indefinite density): L <- L W with W orthogonal, chosen so that the
-// columns of L W are mutually orthogonal; X X^T = L L^T is unchanged and X's columns become the
-// density's eigenvectors scaled by the square roots of its eigenvalues (the factor the fixed-point
-// and TF32 contractions are accurate with: no cancellation between columns).  The result goes to
-// X1 and X2.  One block of 256 threads: column pairs in round-robin order, one pair per warp at a
-// time; at most 30 sweeps, ending when every pair is orthogonal to 1e-15 of its norms.
-__global__ void __launch_bounds__(256) kOrthogonalizeFactor(int nb, int ldx, double * X1, double * X2, const int * info)
-{
-  extern __shared__ double Lc[];   // [R][nb]: column a at Lc + a * nb
-  __shared__ int rotated;
-  int const R = info[0];
-  if (info[1] || R < 2) return;
-  int const t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  for (int idx = t; idx < R * nb; idx += 256) Lc[idx] = X1[int64_t(idx % nb) * ldx + idx / nb];
+  if (indefinite) return;
+  double * Lc = S;   // [R][nb]: column a at Lc + a * nb (argmax ended with a barrier)
+  for (int idx = t; idx < R * nb; idx += 256) Lc[idx] = f.X1[int64_t(idx % nb) * ldx + idx / nb];
   __syncthreads();
   int const Rp = R + (R & 1);   // an even number of slots (the last one idle when R is odd)
-  for (int sweep = 0; sweep < 30; ++sweep) {
+  for (int sweep = 0; sweep < 30 && R > 1; ++sweep) {
     if (t == 0) rotated = 0;
     __syncthreads();
     for (int step = 0; step < Rp - 1; ++step) {
@@ -447,17 +485,12 @@ __global__ void __launch_bounds__(256) kOrthogonalizeFactor(int nb, int ldx, dou
   }
   for (int idx = t; idx < R * nb; idx += 256) {
     int64_t const o = int64_t(idx % nb) * ldx + idx / nb;
-    X1[o] = Lc[idx];
-    X2[o] = Lc[idx];
+    f.X1[o] = Lc[idx];
+    f.X2[o] = Lc[idx];
   }
 }
 
-// status of a density the pivoted Cholesky does not take (nb > 128): factor by eigen-decomposition
-__global__ void kMarkIndefinite(int * info)
-{
-  if (threadIdx.x == 0) { info[0] = 0; info[1] = 1; }
-}
-
+// factor matrices X1, X2 [nb][ldx] from the kept eigenpairs (real case): X2 = v sqrt|l|, X1 = sign(l) X2
 __global__ void kRealFactors(int nb, int nkeep, const int * keep, const double * W, const double * V, int ldx, double * X1, double * X2)
 {
   for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < nb * nkeep; idx += gridDim.x * blockDim.x) {
@@ -489,35 +522,104 @@ __global__ void kComplexFactors(int nb, int nkeep, const int * keep, const doubl
   }
 }
 
-// psi[r][b] = sum_k phi[r][k] X[k][b]  (FP64), b < R, row stride ld
-__global__ void kOrbitals(int64_t n, int nb, int R, const double * __restrict__ phi, const double * __restrict__ X, int ldx,
-                          double * __restrict__ psi, int ld)
+// One side of a contraction from one read of the basis values phi [n][nb]: psi[r][b] = sum_k phi[r][k] X[k][b] for
+// b < R (row stride ld); with coul, coul[r] = scale w[r] sum_b psi'[r][b] psi[r][b], psi' from the factor Xc (null: psi
+// itself); with V, V[r][l] = scale w[r] phi[r][l].  A block takes `rows` points (8 per warp): phi rows and the factors in
+// shared memory (rows 4 mod 16 doubles apart: conflict-free fragments), the products on the FP64 tensor
+// cores, four column tiles at a time.  Bound by HBM.  As three kernels, each reading its operands again (one
+// thread per (r, b), the phi row from global memory): Kr (406,000 points, 120 columns, rank 18) 984 -> 375 us.
+struct OrbitalArgs {
+  int64_t n;
+  int nb, R, ldx, ld, rows;
+  double scale;
+  const double * phi;
+  const double * w;
+  const double * X;
+  const double * Xc;
+  double * psi;
+  double * coul;
+  double * V;
+};
+__global__ void __launch_bounds__(256) kOrbitals(OrbitalArgs a)
 {
-  extern __shared__ double sXo[];
-  for (int i = threadIdx.x; i < nb * R; i += blockDim.x) sXo[i] = X[(i / R) * ldx + (i % R)];
+  extern __shared__ double sm[];
+  int const nb = a.nb, nb4 = (nb + 3) / 4 * 4, R8 = (a.R + 7) / 8 * 8, lp = fragStride(nb4), lx = fragStride(R8);
+  int const t = threadIdx.x, warp = t >> 5, lane = t & 31, fr = lane >> 2, fq = lane & 3;
+  double * sX = sm;                                // [nb4][lx], then the same of Xc
+  double * sXc = sX + nb4 * lx;
+  double * sPhi = sXc + (a.Xc ? nb4 * lx : 0);     // [rows][lp]
+  int64_t const r0 = int64_t(blockIdx.x) * a.rows;
+  int const nr = int(min(int64_t(a.rows), a.n - r0));
+  for (int k = warp; k < nb4; k += 8)
+    for (int b = lane; b < R8; b += 32) {
+      bool const in = k < nb && b < a.R;
+      sX[k * lx + b] = in ? a.X[int64_t(k) * a.ldx + b] : 0.0;
+      if (a.Xc) sXc[k * lx + b] = in ? a.Xc[int64_t(k) * a.ldx + b] : 0.0;
+    }
+  // the block's phi rows are one contiguous range: every load in flight at once
+  for (int r = warp; r < a.rows; r += 8)
+#pragma unroll 4
+    for (int c = lane; c < nb4; c += 32) {
+      bool const in = r < nr && c < nb;
+      cpAsync<8>(&sPhi[r * lp + c], in ? a.phi + (r0 + r) * nb + c : a.phi, in ? 8 : 0);
+    }
+  cpAsyncCommit();
+  cpAsyncWait<0>();
   __syncthreads();
-  int64_t const total = n * R;
-  for (int64_t idx = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; idx < total; idx += int64_t(gridDim.x) * blockDim.x) {
-    int64_t const r = idx / R;
-    int const b = int(idx % R);
-    double s = 0;
-    const double * pr = phi + r * nb;
-    for (int k = 0; k < nb; ++k) s = fma(pr[k], sXo[k * R + b], s);
-    psi[r * ld + b] = s;
+  if (a.V)
+    for (int r = warp; r < nr; r += 8) {
+      double const f = a.scale * a.w[r0 + r];
+#pragma unroll 4
+      for (int c = lane; c < nb; c += 32) a.V[(r0 + r) * nb + c] = f * sPhi[r * lp + c];
+    }
+  if (8 * warp >= a.rows) return;
+  int const row = 8 * warp + fr;
+  double s = 0;
+  for (int b0 = 0; b0 < R8; b0 += 32) {
+    double q[4][2], qc[4][2];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) q[j][0] = q[j][1] = qc[j][0] = qc[j][1] = 0.0;
+    for (int k = fq; k < nb4; k += 4) {
+      double const p = sPhi[row * lp + k];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (b0 + 8 * j < R8) dmma(q[j], p, sX[k * lx + b0 + 8 * j + fr]);
+      if (a.Xc) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (b0 + 8 * j < R8) dmma(qc[j], p, sXc[k * lx + b0 + 8 * j + fr]);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        int const b = b0 + 8 * j + 2 * fq + e;
+        if (row < nr && b < a.R) a.psi[(r0 + row) * a.ld + b] = q[j][e];
+        s = fma(a.Xc ? qc[j][e] : q[j][e], q[j][e], s);   // columns past R are zero
+      }
   }
+  if (!a.coul) return;
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  if (fq == 0 && row < nr) a.coul[r0 + row] = a.scale * a.w[r0 + row] * s;
 }
 
-// coul[r] = scale w[r] sum_b psiA[r][b] psiB[r][b]
-__global__ void kCoulombSource(int64_t n, int R, const double * psiA, const double * psiB, int ld, const double * w, double scale, double * coul)
+int orbitals(tcscf_ctx * ctx, OrbitalArgs a)
 {
-  for (int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; r < n; r += int64_t(gridDim.x) * blockDim.x) {
-    double s = 0;
-    for (int b = 0; b < R; ++b) s = fma(psiA[r * ld + b], psiB[r * ld + b], s);
-    coul[r] = scale * w[r] * s;
-  }
+  TCSCF_CHECK(ctx, size_t(a.nb) * a.R * sizeof(double) <= 48 * 1024, TCSCF_ERR_CUDA, "orbital factor (basis size x density rank) above 6144 elements");
+  int const nb4 = (a.nb + 3) / 4 * 4, R8 = (a.R + 7) / 8 * 8;
+  auto bytes = [&](int rows) { return sizeof(double) * (size_t(nb4) * fragStride(R8) * (a.Xc ? 2 : 1) + size_t(rows) * fragStride(nb4)); };
+  a.rows = 64;
+  while (a.rows > 8 && bytes(a.rows) > 200 * 1024) a.rows /= 2;
+  TCSCF_CHECK(ctx, bytes(a.rows) <= 227 * 1024, TCSCF_ERR_UNSUPPORTED, "basis too large for the orbital kernel");
+  TCSCF_CUDA(ctx, cudaFuncSetAttribute(kOrbitals, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes(a.rows))));
+  kOrbitals<<<unsigned((a.n + a.rows - 1) / a.rows), 256, bytes(a.rows), ctx->stream>>>(a);
+  TCSCF_LAUNCH(ctx);
+  return TCSCF_OK;
 }
 
-// V[r][l] = scale w[r] phi[r][l]
+// V[r][l] = scale w[r] phi[r][l] (kOrbitals writes it beside a factor's orbitals)
 __global__ void kWeightedBasis(int64_t n, int nb, const double * phi, const double * w, double scale, double * V)
 {
   for (int64_t idx = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; idx < n * nb; idx += int64_t(gridDim.x) * blockDim.x)
@@ -577,44 +679,69 @@ __global__ void kPairsToReference(int64_t n1, int nb, const DevSto * s, const do
   }
 }
 
-// G(j,i) = sum_{k,l} U[k][j] GR(k,l) conj(U[l][i]); GR complex [nspin][nb][nb] given as re/im planes
+// element (j, i) of U^T GR conj(U) for one spin's GR (re / im planes, im may be null), GR + tr^T in its place where tr is given
+__device__ __forceinline__ double2 realToReference(int nb, const DevSto * s, const double * re, const double * im, const double * tr, int j, int i)
+{
+  int const kj[2] = {j, s[j].partner};
+  int const li[2] = {i, s[i].partner};
+  double2 acc = make_double2(0, 0);
+  for (int a = 0; a < 2; ++a) {
+    int const k = kj[a];
+    if (k < 0) continue;
+    double2 const uk = urow(s, k, j);
+    for (int b = 0; b < 2; ++b) {
+      int const l = li[b];
+      if (l < 0) continue;
+      double2 g = make_double2(re[k * nb + l], im ? im[k * nb + l] : 0.0);
+      if (tr) g.x += tr[l * nb + k];
+      double2 const t = cmul(cmul(uk, g), cconj(urow(s, l, i)));
+      acc.x += t.x;
+      acc.y += t.y;
+    }
+  }
+  return acc;
+}
+// G(j,i) = sum_{k,l} U[k][j] GR(k,l) conj(U[l][i]); GR [nspin][nb][nb] given as re/im planes
 __global__ void kRealToReference(int nspin, int nb, const DevSto * s, const double * GRre, const double * GRim, double2 * G)
 {
-  int const total = nspin * nb * nb;
-  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
-    int const sp = idx / (nb * nb), j = (idx / nb) % nb, i = idx % nb;
-    int const kj[2] = {j, s[j].partner};
-    int const li[2] = {i, s[i].partner};
-    double2 acc = make_double2(0, 0);
-    for (int a = 0; a < 2; ++a) {
-      int const k = kj[a];
-      if (k < 0) continue;
-      double2 const uk = urow(s, k, j);
-      for (int b = 0; b < 2; ++b) {
-        int const l = li[b];
-        if (l < 0) continue;
-        int64_t const o = int64_t(sp) * nb * nb + k * nb + l;
-        double2 const g = make_double2(GRre[o], GRim ? GRim[o] : 0.0);
-        double2 const t = cmul(cmul(uk, g), cconj(urow(s, l, i)));
-        acc.x += t.x;
-        acc.y += t.y;
-      }
-    }
-    G[idx] = acc;
+  int const nn = nb * nb;
+  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < nspin * nn; idx += gridDim.x * blockDim.x) {
+    int const sp = idx / nn, ji = idx % nn;
+    G[idx] = realToReference(nb, s, GRre + sp * nn, GRim ? GRim + sp * nn : nullptr, nullptr, ji / nb, ji % nb);
   }
 }
 
-// enforceOneElectronSymmetry (HartreeFock.cpp:758-780) and constructSCFOperator (:48-98) with a
-// compensated FP64 energy sum.  One block.  energy = factor * Re sum D(i,j) (h(j,i) + G(j,i)/2 - G3(j,i)/3)
-__global__ void kFinalize(int nspin, int nb, const double * h, double2 * G, const double2 * G3, const double2 * D, int respectSym,
-                          double factor, double2 * fock, double * energy)
+// The end of a Fock build: G from the real-harmonic sums (gr.re; symSpin bit s: G = M + M^T there, or M + tr^T) or as given (gr.re null),
+// enforceOneElectronSymmetry (HartreeFock.cpp:758-780), constructSCFOperator (:48-98) and the
+// compensated FP64 energy, factor * Re sum D(i,j) (h(j,i) + G(j,i)/2 - G3(j,i)/3): every thread sums its terms with
+// TwoSum, warps and blocks are combined in a fixed order.  parts[block] = {sum, compensation}; one block
+// alone writes the energy, several leave it to kEnergySum
+struct RealSums {
+  const double * re;
+  const double * im;
+  const DevSto * sto;
+  int symSpin;
+  const double * tr = nullptr;
+};
+__device__ __forceinline__ void addPair(double & s, double & c, double s2, double c2)
 {
-  __shared__ double ss[512], se[512];
+  double t, err;
+  twoSum(s, s2, t, err);
+  s = t;
+  c += err + c2;
+}
+constexpr int kFinishThreads = 256;
+__global__ void __launch_bounds__(kFinishThreads) kFockFinish(int nspin, int nb, RealSums gr, const double * h, double2 * G, const double2 * G3,
+                                                            const double2 * D, int respectSym, double factor, double2 * fock, double2 * parts,
+                                                            double * energy)
+{
+  __shared__ double2 red[kFinishThreads / 32];
   double s = 0, c = 0;
   int const nn = nb * nb;
-  for (int idx = threadIdx.x; idx < nspin * nn; idx += blockDim.x) {
+  for (int idx = blockIdx.x * kFinishThreads + threadIdx.x; idx < nspin * nn; idx += gridDim.x * kFinishThreads) {
     int const sp = idx / nn, ji = idx % nn, j = ji / nb, i = ji % nb;
-    double2 g = G[idx];
+    double2 g = gr.re ? realToReference(nb, gr.sto, gr.re + sp * nn, gr.im ? gr.im + sp * nn : nullptr,
+                                             (gr.symSpin >> sp) & 1 ? (gr.tr ? gr.tr : gr.re) + sp * nn : nullptr, j, i) : G[idx];
     double2 g3 = G3 ? G3[idx] : make_double2(0, 0);
     if (respectSym && !(fabs(h[ji]) > 0)) { g = make_double2(0, 0); g3 = make_double2(0, 0); }
     G[idx] = g;
@@ -622,25 +749,39 @@ __global__ void kFinalize(int nspin, int nb, const double * h, double2 * G, cons
     if (fock) fock[idx] = f;
     double2 const e = make_double2(h[ji] + g.x / 2 - g3.x / 3, g.y / 2 - g3.y / 3);
     double2 const d = D[int64_t(sp) * nn + i * nb + j];
-    double const term = d.x * e.x - d.y * e.y;
-    double t, err;
-    twoSum(s, term, t, err);
-    s = t;
-    c += err;
+    addPair(s, c, d.x * e.x - d.y * e.y, 0.0);
   }
-  ss[threadIdx.x] = s;
-  se[threadIdx.x] = c;
+  for (int o = 16; o > 0; o >>= 1) addPair(s, c, __shfl_down_sync(0xffffffffu, s, o), __shfl_down_sync(0xffffffffu, c, o));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = make_double2(s, c);
   __syncthreads();
   if (threadIdx.x == 0) {
-    double tot = 0, comp = 0;
-    for (int k = 0; k < int(blockDim.x); ++k) {
-      double t, err;
-      twoSum(tot, ss[k], t, err);
-      tot = t;
-      comp += err + se[k];
-    }
-    energy[0] = factor * (tot + comp);
+    for (int k = 1; k < kFinishThreads / 32; ++k) addPair(s, c, red[k].x, red[k].y);
+    if (gridDim.x == 1) energy[0] = factor * (s + c);
+    else parts[blockIdx.x] = make_double2(s, c);
   }
+}
+__global__ void kEnergySum(int n, const double2 * parts, double factor, double * energy)
+{
+  double s = 0, c = 0;
+  for (int k = threadIdx.x; k < n; k += 32) addPair(s, c, parts[k].x, parts[k].y);
+  for (int o = 16; o > 0; o >>= 1) addPair(s, c, __shfl_down_sync(0xffffffffu, s, o), __shfl_down_sync(0xffffffffu, c, o));
+  if (threadIdx.x == 0) energy[0] = factor * (s + c);
+}
+int fockFinish(tcscf_ctx * ctx, int nspin, int nb, RealSums const & gr, const double * h, double2 * G, const double2 * G3, const double2 * D,
+               int respectSym, double factor, double2 * fock, double * energy)
+{
+  // one block up to four elements a thread (a second launch costs more than they do), else up to 64
+  int const n = nspin * nb * nb, blocks = n <= 4 * kFinishThreads ? 1 : std::min(64, (n + kFinishThreads - 1) / kFinishThreads);
+  void * p = nullptr;
+  TCSCF_TRY(scratch(ctx, "fock_finish", sizeof(double2) * 64, &p));
+  double2 * parts = static_cast<double2 *>(p);
+  kFockFinish<<<blocks, kFinishThreads, 0, ctx->stream>>>(nspin, nb, gr, h, G, G3, D, respectSym, factor, fock, parts, energy);
+  TCSCF_LAUNCH(ctx);
+  if (blocks > 1) {
+    kEnergySum<<<1, 32, 0, ctx->stream>>>(blocks, parts, factor, energy);
+    TCSCF_LAUNCH(ctx);
+  }
+  return TCSCF_OK;
 }
 
 // Faa(r) (+)= sum_ji F(r,j,i) D(i,j) ; Fai(r,i) (+)= sum_j (sum_k D(k,j) vals(r,k)) F(r,j,i)
@@ -692,15 +833,15 @@ __global__ void kFaaFai(int64_t n1, int nb, const double * F, const double2 * va
   }
 }
 
+// the Coulomb potential of both spins
+__global__ void kAddSpins(int64_t n, const double * a, const double * b, double * out)
+{
+  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) out[i] = a[i] + b[i];
+}
+
 __global__ void kAddInto(int64_t n, const double * a, double * out)
 {
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) out[i] += a[i];
-}
-
-// out[i][j] += a[j][i] (nb x nb, row-major)
-__global__ void kAddTransposed(int nb, const double * a, double * out)
-{
-  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < nb * nb; idx += gridDim.x * blockDim.x) out[idx] += a[(idx % nb) * nb + idx / nb];
 }
 
 // column-major complex copy of the row-major (j,i) Fock matrix, and of a real row-major S
@@ -840,9 +981,7 @@ bool solveDiis(int m, std::vector<double> const & B, int ld, std::vector<double>
 int finalizeLaunch(tcscf_ctx * ctx, int nspin, int nb, const double * h, double2 * G, const double2 * G3, const double2 * D, int respectSym,
                    double factor, double2 * fock, double * energy)
 {
-  kFinalize<<<1, 512, 0, ctx->stream>>>(nspin, nb, h, G, G3, D, respectSym, factor, fock, energy);
-  TCSCF_LAUNCH(ctx);
-  return TCSCF_OK;
+  return fockFinish(ctx, nspin, nb, RealSums{}, h, G, G3, D, respectSym, factor, fock, energy);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -863,10 +1002,6 @@ struct Factor {
 // Device buffers of one density factorisation: the real-harmonic density DR, its symmetrised real
 // part A, the factors X1 (X1im) and X2 [nb][ldx], and the status {max |Re DR|, max |Im DR|} with the
 // pivoted-Cholesky rank and flag behind it (FactorStatus).
-struct FactorStatus {
-  double maxAbs[2];
-  int rank, indefinite;
-};
 struct FactorBufs {
   double2 * DR = nullptr;
   double * A = nullptr;
@@ -892,27 +1027,17 @@ FactorBufs carveFactorBufs(void * p, int nb)
   return b;
 }
 
-// Launches (no host synchronisation) the real-harmonic transform of the spin density, its split
-// into real and imaginary magnitudes, and the pivoted Cholesky factorisation of its real part.
-int factorLaunch(tcscf_ctx * ctx, Grid & g, const double2 * dD, FactorBufs const & b)
+FactorJob factorJob(Grid const & g, const double2 * dD, FactorBufs const & b)
 {
-  int const nb = g.nb;
-  size_t const nn = size_t(nb) * nb;
-  kDensityToReal<<<gridBlocks(nn, 256), 256, 0, ctx->stream>>>(1, nb, g.dsto, dD, b.DR);
+  return {g.nb, 2 * g.nb, g.dsto, dD, b.DR, b.A, b.X1, b.X2, b.status};
+}
+// Launches (no host synchronisation) the factorisations: `one`, or the `count` jobs of a device array; maxNb: their largest basis
+int factorLaunch(tcscf_ctx * ctx, FactorJob const & one, const FactorJob * jobs, int count, int maxNb)
+{
+  TCSCF_CUDA(ctx, cudaFuncSetAttribute(kFactorDensity, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(double) * kCholeskyMaxNb * kCholeskyMaxNb)));
+  int const nb = std::min(maxNb, kCholeskyMaxNb);
+  kFactorDensity<<<count, 256, sizeof(double) * nb * nb, ctx->stream>>>(one, jobs);
   TCSCF_LAUNCH(ctx);
-  kSplitDensity<<<1, 256, 0, ctx->stream>>>(nb, b.DR, b.A, b.status->maxAbs);
-  TCSCF_LAUNCH(ctx);
-  if (nb <= kCholeskyMaxNb) {
-    TCSCF_CUDA(ctx, cudaFuncSetAttribute(kPivotedCholesky, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(double) * kCholeskyMaxNb * kCholeskyMaxNb)));
-    kPivotedCholesky<<<1, 256, sizeof(double) * nn, ctx->stream>>>(nb, b.A, 2 * nb, b.X1, b.X2, &b.status->rank);
-    TCSCF_LAUNCH(ctx);
-    TCSCF_CUDA(ctx, cudaFuncSetAttribute(kOrthogonalizeFactor, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(double) * kCholeskyMaxNb * kCholeskyMaxNb)));
-    kOrthogonalizeFactor<<<1, 256, sizeof(double) * nn, ctx->stream>>>(nb, 2 * nb, b.X1, b.X2, &b.status->rank);
-    TCSCF_LAUNCH(ctx);
-  } else {
-    kMarkIndefinite<<<1, 32, 0, ctx->stream>>>(&b.status->rank);
-    TCSCF_LAUNCH(ctx);
-  }
   return TCSCF_OK;
 }
 
@@ -997,7 +1122,7 @@ int factorDensity(tcscf_ctx * ctx, Grid & g, const double2 * dD, int spin, Facto
   void * p = nullptr;
   TCSCF_TRY(scratch(ctx, spin ? "fac1" : "fac0", factorBufBytes(g.nb), &p));
   FactorBufs const b = carveFactorBufs(p, g.nb);
-  TCSCF_TRY(factorLaunch(ctx, g, dD, b));
+  TCSCF_TRY(factorLaunch(ctx, factorJob(g, dD, b), nullptr, 1, g.nb));
   FactorStatus st;
   TCSCF_CUDA(ctx, cudaMemcpyAsync(&st, b.status, sizeof(FactorStatus), cudaMemcpyDeviceToHost, ctx->stream));
   TCSCF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -1030,7 +1155,7 @@ int fockBuildDevice(tcscf_ctx * ctx, Grid & g1, Grid & g2, int nspin, const doub
   int const ldt = nb;
   int const ldpsi = 2 * nb;
   size_t const bytes = sizeof(double) * (size_t(n2) * nb                 // V
-                                         + size_t(n1) * ldpsi + 2 * size_t(n2) * ldpsi  // psi1, psi2, psi1 on r2
+                                         + size_t(n1) * ldpsi + size_t(n2) * ldpsi  // psi1, psi2
                                          + size_t(n2)                              // coul
                                          + size_t(nspin) * n1 * ldt                // T re
                                          + size_t(nspin) * n1 * ldt                // T im
@@ -1041,8 +1166,7 @@ int fockBuildDevice(tcscf_ctx * ctx, Grid & g1, Grid & g2, int nspin, const doub
   double * V = static_cast<double *>(p);
   double * psi1 = V + size_t(n2) * nb;
   double * psi2 = psi1 + size_t(n1) * ldpsi;
-  double * psi1at2 = psi2 + size_t(n2) * ldpsi;
-  double * coul = psi1at2 + size_t(n2) * ldpsi;
+  double * coul = psi2 + size_t(n2) * ldpsi;
   double * Tre = coul + n2;
   double * Tim = Tre + size_t(nspin) * n1 * ldt;
   double * VH = Tim + size_t(nspin) * n1 * ldt;
@@ -1052,15 +1176,9 @@ int fockBuildDevice(tcscf_ctx * ctx, Grid & g1, Grid & g2, int nspin, const doub
 
   cudaEventRecord(ctx->ev[0], ctx->stream);
   int const launch0 = ctx->launchCount;
-  kWeightedBasis<<<gridBlocks(n2 * nb, 256), 256, 0, ctx->stream>>>(n2, nb, g2.phiR, g2.w, scale, V);
-  TCSCF_LAUNCH(ctx);
-  TCSCF_CUDA(ctx, cudaMemsetAsync(VH, 0, sizeof(double) * (size_t(nspin) * n1 + n1), ctx->stream));
-  TCSCF_CUDA(ctx, cudaMemsetAsync(GRre, 0, sizeof(double) * size_t(nspin) * nb * nb * 2, ctx->stream));
-  bool anyComplex = false;
-  bool symSpin[2] = {false, false};
-  double contractionMs = 0;
+  int nparts = 0, symSpin = 0, complexSpin = 0;
+  double const * Vdone = nullptr;   // V once a spin has formed it
   const void * vtPacked = nullptr;
-  if (precision == TCSCF_PREC_BF16X3) TCSCF_TRY(tensorPackedV(ctx, g2, V, scale, &vtPacked));
   for (int s = 0; s < nspin; ++s) {
     Factor f;
     if (given && given[s].X1) f = given[s];   // the caller's factor of this spin's density (its occupied orbitals)
@@ -1069,6 +1187,7 @@ int fockBuildDevice(tcscf_ctx * ctx, Grid & g1, Grid & g2, int nspin, const doub
     double * Ti = Tim + size_t(s) * n1 * ldt;
     if (f.R == 0) {
       TCSCF_CUDA(ctx, cudaMemsetAsync(Ts, 0, sizeof(double) * n1 * ldt, ctx->stream));
+      TCSCF_CUDA(ctx, cudaMemsetAsync(VH + size_t(s) * n1, 0, sizeof(double) * n1, ctx->stream));
       continue;
     }
     int const R = f.R;
@@ -1076,19 +1195,24 @@ int fockBuildDevice(tcscf_ctx * ctx, Grid & g1, Grid & g2, int nspin, const doub
     // FP64 contractions compute only the pairs on and above each r1 tile's diagonal (T'), and the
     // exchange matrix is sum W T' plus its transpose (TF32 keeps the full form: tensorPrepare)
     bool const sym = precision != TCSCF_PREC_TF32 && &g1 == &g2 && f.same;
-    symSpin[s] = sym;
+    if (sym) symSpin |= 1 << s;
+    if (f.complex) complexSpin |= 1 << s;
     for (int part = 0; part < (f.complex ? 2 : 1); ++part) {
       double const * X1 = part == 0 ? f.X1 : f.X1im;
-      size_t const sm = sizeof(double) * size_t(nb) * R;
-      kOrbitals<<<gridBlocks(n1 * R, 256), 256, sm, ctx->stream>>>(n1, nb, R, g1.phiR, X1, f.ldx, psi1, ldpsi);
-      TCSCF_LAUNCH(ctx);
-      if (part == 0 && !sym) {
-        kOrbitals<<<gridBlocks(n2 * R, 256), 256, sm, ctx->stream>>>(n2, nb, R, g2.phiR, f.X2, f.ldx, psi2, ldpsi);
-        TCSCF_LAUNCH(ctx);
-        // rho(r2, r2) needs the r1-side factor evaluated on the r2 points
-        kOrbitals<<<gridBlocks(n2 * R, 256), 256, sm, ctx->stream>>>(n2, nb, R, g2.phiR, f.X1, f.ldx, psi1at2, ldpsi);
-        TCSCF_LAUNCH(ctx);
+      OrbitalArgs o1{n1, nb, R, f.ldx, ldpsi, 0, scale, g1.phiR, g1.w, X1, nullptr, psi1, nullptr, nullptr};
+      // the r2 side (the r1 side where the two are one): psi2, the Coulomb source with the r1-side factor on
+      // the r2 points (rho(r2, r2)), and V for the first spin
+      OrbitalArgs o2 = o1;
+      o2.n = n2; o2.phi = g2.phiR; o2.w = g2.w; o2.coul = coul;
+      o2.V = Vdone ? nullptr : V;
+      if (sym) TCSCF_TRY(orbitals(ctx, o2));
+      else {
+        TCSCF_TRY(orbitals(ctx, o1));
+        o2.X = f.X2; o2.Xc = f.same ? nullptr : f.X1; o2.psi = psi2;
+        if (part == 0) TCSCF_TRY(orbitals(ctx, o2));
       }
+      Vdone = V;
+      if (precision == TCSCF_PREC_BF16X3 && !vtPacked) TCSCF_TRY(tensorPackedV(ctx, g2, V, scale, &vtPacked));
       double const * p2side = sym ? psi1 : psi2;
       Contraction c;
       c.n1 = n1; c.n2 = n2; c.R = R; c.ncol = nb;
@@ -1098,54 +1222,46 @@ int fockBuildDevice(tcscf_ctx * ctx, Grid & g1, Grid & g2, int nspin, const doub
       c.sym = sym ? 1 : 0;
       if (precision != TCSCF_PREC_FP64) TCSCF_TRY(nearPairsFor(ctx, g1, g2, &c.near));
       if (part == 0) {
-        kCoulombSource<<<gridBlocks(n2, 256), 256, 0, ctx->stream>>>(n2, R, sym ? psi1 : psi1at2, p2side, ldpsi, g2.w, scale, coul);
-        TCSCF_LAUNCH(ctx);
         c.coul = coul;
         c.VH = VH + size_t(s) * n1;
       }
-      // the contraction routines bracket their main kernel with ev[2] / ev[3]
-      if (precision == TCSCF_PREC_FP64) TCSCF_TRY(contractFp64(ctx, c));
-      else TCSCF_TRY(contractTensor(ctx, c, precision));
-      TCSCF_CUDA(ctx, cudaEventSynchronize(ctx->ev[3]));
-      float ms = 0;
-      cudaEventElapsedTime(&ms, ctx->ev[2], ctx->ev[3]);
-      contractionMs += ms;
+      // the contraction routines bracket their main kernel with evStart() / evStop()
+      ctx->evPart = nparts++;
+      int const st = precision == TCSCF_PREC_FP64 ? contractFp64(ctx, c) : contractTensor(ctx, c, precision);
+      ctx->evPart = 0;
+      TCSCF_TRY(st);
     }
-    if (f.complex) anyComplex = true;
-    else TCSCF_CUDA(ctx, cudaMemsetAsync(Ti, 0, sizeof(double) * n1 * ldt, ctx->stream));
   }
-  for (int s = 0; s < nspin; ++s) {
-    kAddInto<<<gridBlocks(n1, 256), 256, 0, ctx->stream>>>(n1, VH + size_t(s) * n1, VHtot);
+  if (nspin == 2) {
+    kAddSpins<<<gridBlocks(n1, 256), 256, 0, ctx->stream>>>(n1, VH, VH + n1, VHtot);
     TCSCF_LAUNCH(ctx);
   }
-  double const cJ = nspin == 1 ? 2.0 : 1.0;
-  double * GRhalf = nullptr;
-  if (symSpin[0] || symSpin[1]) TCSCF_TRY(scratch(ctx, "fock_sym_half", sizeof(double) * size_t(nb) * nb, reinterpret_cast<void **>(&GRhalf)));
-  for (int s = 0; s < nspin; ++s) {
-    TCSCF_TRY(reduceFockReal(ctx, n1, nb, g1.phiR, g1.w, VHtot, cJ, Tre + size_t(s) * n1 * ldt, ldt, 1.0, GRre + size_t(s) * nb * nb));
-    if (symSpin[s]) {
-      // the exchange of the pairs below the diagonal tiles: the transpose of T's own contribution
-      // (reduceFockReal adds into its output)
-      TCSCF_CUDA(ctx, cudaMemsetAsync(GRhalf, 0, sizeof(double) * size_t(nb) * nb, ctx->stream));
-      TCSCF_TRY(reduceFockReal(ctx, n1, nb, g1.phiR, g1.w, nullptr, 0.0, Tre + size_t(s) * n1 * ldt, ldt, 1.0, GRhalf));
-      kAddTransposed<<<gridBlocks(int64_t(nb) * nb, 256), 256, 0, ctx->stream>>>(nb, GRhalf, GRre + size_t(s) * nb * nb);
-      TCSCF_LAUNCH(ctx);
-    }
-    if (anyComplex)
-      TCSCF_TRY(reduceFockReal(ctx, n1, nb, g1.phiR, g1.w, nullptr, 0.0, Tim + size_t(s) * n1 * ldt, ldt, 1.0, GRim + size_t(s) * nb * nb));
+  double const * potential = nspin == 2 ? VHtot : VH;
+  // a symmetric spin's G is M + M^T of the sums over T', with the (symmetric) Coulomb part at half weight in M
+  double const cJ0 = nspin == 1 ? 2.0 : 1.0;
+  double const cJ[2] = {symSpin & 1 ? 0.5 * cJ0 : cJ0, symSpin & 2 ? 0.5 * cJ0 : cJ0};
+  TCSCF_TRY(reduceFockReal(ctx, n1, nb, nspin, g1.phiR, g1.w, potential, cJ, Tre, int64_t(n1) * ldt, ldt, GRre));
+  if (complexSpin) {
+    double const none[2] = {0.0, 0.0};
+    for (int s = 0; s < nspin; ++s)
+      if (!((complexSpin >> s) & 1)) TCSCF_CUDA(ctx, cudaMemsetAsync(Tim + size_t(s) * n1 * ldt, 0, sizeof(double) * n1 * ldt, ctx->stream));
+    TCSCF_TRY(reduceFockReal(ctx, n1, nb, nspin, g1.phiR, g1.w, nullptr, none, Tim, int64_t(n1) * ldt, ldt, GRim));
   }
-  ctx->lastVH = VHtot;
+  ctx->lastVH = potential;
   ctx->lastT = Tre;
   ctx->lastN1 = n1;
   ctx->lastNb = nb;
-  kRealToReference<<<gridBlocks(int64_t(nspin) * nb * nb, 256), 256, 0, ctx->stream>>>(nspin, nb, g1.dsto, GRre, anyComplex ? GRim : nullptr, dG);
-  TCSCF_LAUNCH(ctx);
-  kFinalize<<<1, 512, 0, ctx->stream>>>(nspin, nb, dH, dG, nullptr, dD, respectSym, nspin == 1 ? 2.0 : 1.0, dFock, dE);
-  TCSCF_LAUNCH(ctx);
+  TCSCF_TRY(fockFinish(ctx, nspin, nb, {GRre, complexSpin ? GRim : nullptr, g1.dsto, symSpin}, dH, dG, nullptr, dD, respectSym, cJ0, dFock, dE));
   cudaEventRecord(ctx->ev[1], ctx->stream);
   TCSCF_CUDA(ctx, cudaEventSynchronize(ctx->ev[1]));
   float tot = 0;
   cudaEventElapsedTime(&tot, ctx->ev[0], ctx->ev[1]);
+  double contractionMs = 0;
+  for (int k = 0; k < nparts; ++k) {
+    float ms = 0;
+    cudaEventElapsedTime(&ms, ctx->ev[2 + 2 * k], ctx->ev[3 + 2 * k]);
+    contractionMs += ms;
+  }
   ctx->lastTotalMs = tot;
   ctx->lastContractionMs = contractionMs;
   ctx->lastLaunches = ctx->launchCount - launch0;
@@ -1170,14 +1286,13 @@ int fockBuildBatch(tcscf_ctx * ctx, int count, Grid * const * g1s, Grid * const 
     maxN2 = std::max(maxN2, g2s[k]->n);
     maxNb = std::max(maxNb, g1s[k]->nb);
   }
-  size_t const tmpBytes = sizeof(double) * (size_t(maxN2) * maxNb + size_t(maxN1) * maxNb + 2 * size_t(maxN2) * maxNb + size_t(maxN2));
+  size_t const tmpBytes = sizeof(double) * (2 * size_t(maxN2) * maxNb + size_t(maxN1) * maxNb + size_t(maxN2));
   void * tp = nullptr;
   TCSCF_TRY(scratch(ctx, "batch_tmp", tmpBytes, &tp));
   double * V = static_cast<double *>(tp);
   double * psi1 = V + size_t(maxN2) * maxNb;
   double * psi2 = psi1 + size_t(maxN1) * maxNb;
-  double * psi1at2 = psi2 + size_t(maxN2) * maxNb;
-  double * coul = psi1at2 + size_t(maxN2) * maxNb;
+  double * coul = psi2 + size_t(maxN2) * maxNb;
 
   // per-instance persistent buffers: T, VH, GR and the tensor arena
   std::vector<Contraction> cs(count);
@@ -1198,20 +1313,25 @@ int fockBuildBatch(tcscf_ctx * ctx, int count, Grid * const * g1s, Grid * const 
   }
   void * bp = nullptr;
   TCSCF_TRY(scratch(ctx, "batch_arena", offs[count] + 256, &bp));
-  // every instance's density factorisation is launched first, with one host synchronisation for all
+  // every instance's density is factored in one launch (a block each), with one host synchronisation for all
   std::vector<size_t> fOffs(count + 1, 0);
   for (int k = 0; k < count; ++k) fOffs[k + 1] = fOffs[k] + ((factorBufBytes(g1s[k]->nb) + 255) & ~size_t(255));
   void * fp = nullptr;
   TCSCF_TRY(scratch(ctx, "batch_factors", fOffs[count] + 256, &fp));
+  size_t const jobBytes = (sizeof(FactorJob) * count + 255) & ~size_t(255);
   void * sp = nullptr;
-  TCSCF_TRY(scratch(ctx, "batch_factor_status", sizeof(FactorStatus) * count + 256, &sp));
-  auto * dStatus = static_cast<FactorStatus *>(sp);
+  TCSCF_TRY(scratch(ctx, "batch_factor_status", jobBytes + sizeof(FactorStatus) * count + 256, &sp));
+  auto * dJobs = static_cast<FactorJob *>(sp);
+  auto * dStatus = reinterpret_cast<FactorStatus *>(static_cast<char *>(sp) + jobBytes);
   std::vector<FactorBufs> fbufs(count);
+  std::vector<FactorJob> jobs(count);
   for (int k = 0; k < count; ++k) {
     fbufs[k] = carveFactorBufs(static_cast<char *>(fp) + fOffs[k], g1s[k]->nb);
-    TCSCF_TRY(factorLaunch(ctx, *g1s[k], dDs[k], fbufs[k]));
-    TCSCF_CUDA(ctx, cudaMemcpyAsync(dStatus + k, fbufs[k].status, sizeof(FactorStatus), cudaMemcpyDeviceToDevice, ctx->stream));
+    fbufs[k].status = dStatus + k;
+    jobs[k] = factorJob(*g1s[k], dDs[k], fbufs[k]);
   }
+  TCSCF_CUDA(ctx, cudaMemcpyAsync(dJobs, jobs.data(), sizeof(FactorJob) * count, cudaMemcpyHostToDevice, ctx->stream));
+  TCSCF_TRY(factorLaunch(ctx, FactorJob{}, dJobs, count, maxNb));
   std::vector<FactorStatus> hStatus(count);
   TCSCF_CUDA(ctx, cudaMemcpyAsync(hStatus.data(), dStatus, sizeof(FactorStatus) * count, cudaMemcpyDeviceToHost, ctx->stream));
   TCSCF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -1246,22 +1366,17 @@ int fockBuildBatch(tcscf_ctx * ctx, int count, Grid * const * g1s, Grid * const 
       eligible = nl->count == 0;
     }
     if (!eligible) continue;
-    kWeightedBasis<<<gridBlocks(n2 * nb, 256), 256, 0, ctx->stream>>>(n2, nb, g2.phiR, g2.w, scale, V);
-    TCSCF_LAUNCH(ctx);
+    OrbitalArgs o1{n1, nb, f.R, f.ldx, nb, 0, scale, g1.phiR, g1.w, f.X1, nullptr, psi1, nullptr, nullptr};
+    OrbitalArgs o2 = o1;
+    o2.n = n2; o2.phi = g2.phiR; o2.w = g2.w; o2.coul = coul; o2.V = V;
+    if (!sym) {
+      TCSCF_TRY(orbitals(ctx, o1));
+      o2.X = f.X2; o2.Xc = f.same ? nullptr : f.X1; o2.psi = psi2;
+    }
+    TCSCF_TRY(orbitals(ctx, o2));
     const void * vtPacked = nullptr;
     if (precision == TCSCF_PREC_BF16X3) TCSCF_TRY(tensorPackedV(ctx, g2, V, scale, &vtPacked));
     c.vtPacked = vtPacked;
-    size_t const sm = sizeof(double) * size_t(nb) * f.R;
-    kOrbitals<<<gridBlocks(n1 * f.R, 256), 256, sm, ctx->stream>>>(n1, nb, f.R, g1.phiR, f.X1, f.ldx, psi1, nb);
-    TCSCF_LAUNCH(ctx);
-    if (!sym) {
-      kOrbitals<<<gridBlocks(n2 * f.R, 256), 256, sm, ctx->stream>>>(n2, nb, f.R, g2.phiR, f.X2, f.ldx, psi2, nb);
-      TCSCF_LAUNCH(ctx);
-      kOrbitals<<<gridBlocks(n2 * f.R, 256), 256, sm, ctx->stream>>>(n2, nb, f.R, g2.phiR, f.X1, f.ldx, psi1at2, nb);
-      TCSCF_LAUNCH(ctx);
-    }
-    kCoulombSource<<<gridBlocks(n2, 256), 256, 0, ctx->stream>>>(n2, f.R, sym ? psi1 : psi1at2, c.psi2, nb, g2.w, scale, coul);
-    TCSCF_LAUNCH(ctx);
     TCSCF_TRY(tensorPrepare(ctx, c, precision, arena, arenaBytes[k], preps[k]));
     tensorOk[k] = 1;
     ready.push_back(&preps[k]);
@@ -1269,11 +1384,9 @@ int fockBuildBatch(tcscf_ctx * ctx, int count, Grid * const * g1s, Grid * const 
   if (!ready.empty()) TCSCF_TRY(tensorRun(ctx, ready.data(), int(ready.size())));
   float contractionMs = 0;
   if (!ready.empty()) {
-    TCSCF_CUDA(ctx, cudaEventSynchronize(ctx->ev[3]));
-    cudaEventElapsedTime(&contractionMs, ctx->ev[2], ctx->ev[3]);
+    TCSCF_CUDA(ctx, cudaEventSynchronize(ctx->evStop()));
+    cudaEventElapsedTime(&contractionMs, ctx->evStart(), ctx->evStop());
   }
-  double * GRhalf = nullptr;
-  TCSCF_TRY(scratch(ctx, "batch_sym_half", sizeof(double) * size_t(maxNb) * maxNb, reinterpret_cast<void **>(&GRhalf)));
   for (int k = 0; k < count; ++k) {
     Grid & g1 = *g1s[k];
     int const nb = g1.nb;
@@ -1283,18 +1396,9 @@ int fockBuildBatch(tcscf_ctx * ctx, int count, Grid * const * g1s, Grid * const 
     }
     Contraction const & c = cs[k];
     double * GR = c.VH + g1.n;
-    TCSCF_CUDA(ctx, cudaMemsetAsync(GR, 0, sizeof(double) * nb * nb, ctx->stream));
-    TCSCF_TRY(reduceFockReal(ctx, g1.n, nb, g1.phiR, g1.w, c.VH, 2.0, c.T, nb, 1.0, GR));
-    if (c.sym) {
-      TCSCF_CUDA(ctx, cudaMemsetAsync(GRhalf, 0, sizeof(double) * nb * nb, ctx->stream));
-      TCSCF_TRY(reduceFockReal(ctx, g1.n, nb, g1.phiR, g1.w, nullptr, 0.0, c.T, nb, 1.0, GRhalf));
-      kAddTransposed<<<gridBlocks(int64_t(nb) * nb, 256), 256, 0, ctx->stream>>>(nb, GRhalf, GR);
-      TCSCF_LAUNCH(ctx);
-    }
-    kRealToReference<<<gridBlocks(int64_t(nb) * nb, 256), 256, 0, ctx->stream>>>(1, nb, g1.dsto, GR, nullptr, dGs[k]);
-    TCSCF_LAUNCH(ctx);
-    kFinalize<<<1, 512, 0, ctx->stream>>>(1, nb, dHs[k], dGs[k], nullptr, dDs[k], respectSym, 2.0, dFs[k], dEs[k]);
-    TCSCF_LAUNCH(ctx);
+    double const cJ[2] = {c.sym ? 1.0 : 2.0, 0.0};
+    TCSCF_TRY(reduceFockReal(ctx, g1.n, nb, 1, g1.phiR, g1.w, c.VH, cJ, c.T, 0, nb, GR));
+    TCSCF_TRY(fockFinish(ctx, 1, nb, {GR, nullptr, g1.dsto, c.sym}, dHs[k], dGs[k], nullptr, dDs[k], respectSym, 2.0, dFs[k], dEs[k]));
   }
   cudaEventRecord(ctx->ev[1], ctx->stream);
   TCSCF_CUDA(ctx, cudaEventSynchronize(ctx->ev[1]));
@@ -1591,7 +1695,7 @@ __global__ void kScfCheck(ScfGraphState * st, const double * E, const int * tsta
 // One RCS SCF on the device (tcscf_scf_graph).  Every iteration is the same launch sequence on fixed
 // buffers: orbitals of the current occupied coefficients C on both grids, the Coulomb source, the r12
 // contraction (FP64 or tensor cores) from those factors (D = C C^T, rank nocc), the real Fock
-// reduction, the reference-basis G, F and energy (kFinalize), the convergence test, then the new C from
+// reduction, the reference-basis G, F and energy (kFockFinish), the convergence test, then the new C from
 // the Fock matrix: real-harmonic F, Xc^T F Xc with the canonical orthogonaliser Xc of S, Jacobi, the
 // nocc lowest eigenvectors.  The first two iterations run directly (the zero-density one, F = h, with
 // no contraction; the second allocates every buffer); with capture the rest run as one graph launch
@@ -1652,7 +1756,7 @@ int scfGraph(tcscf_ctx * ctx, Grid & g1, Grid & g2, int nocc, const double * S, 
   TCSCF_CUDA(ctx, cudaMemcpyAsync(dH, h, sizeof(double) * nn, cudaMemcpyHostToDevice, ctx->stream));
   kRealToComplex<<<gridBlocks(int64_t(nn), 256), 256, 0, ctx->stream>>>(int64_t(nn), SR, Sc);
   TCSCF_LAUNCH(ctx);
-  kDensityToReal<<<gridBlocks(nn, 256), 256, 0, ctx->stream>>>(1, nb, g1.dsto, Sc, SRc);
+  kDensityToReal<<<gridBlocks(nn, 256), 256, 0, ctx->stream>>>(nb, g1.dsto, Sc, SRc);
   TCSCF_LAUNCH(ctx);
   kSplitDensity<<<1, 256, 0, ctx->stream>>>(nb, SRc, SR, fmaxv);
   TCSCF_LAUNCH(ctx);
@@ -1725,19 +1829,16 @@ int scfGraph(tcscf_ctx * ctx, Grid & g1, Grid & g2, int nocc, const double * S, 
   // zeroDensity: the first iteration's density is zero, so its exchange and Coulomb potentials are
   // zero without a contraction (as tcscf_scf skips a rank-0 factor)
   auto body = [&](cudaGraphConditionalHandle handle, int useHandle, bool zeroDensity) -> int {
-    size_t const sm = sizeof(double) * size_t(nb) * nocc;
     if (zeroDensity) {
       TCSCF_CUDA(ctx, cudaMemsetAsync(Tb, 0, sizeof(double) * size_t(n1) * nb, ctx->stream));
       TCSCF_CUDA(ctx, cudaMemsetAsync(VH, 0, sizeof(double) * size_t(n1), ctx->stream));
     } else {
-    kOrbitals<<<gridBlocks(n1 * nocc, 256), 256, sm, ctx->stream>>>(n1, nb, nocc, g1.phiR, C, nocc, psi1, ldpsi);
-    TCSCF_LAUNCH(ctx);
+    OrbitalArgs o{n2, nb, nocc, nocc, ldpsi, 0, scale, g2.phiR, g2.w, C, nullptr, sym ? psi1 : psi2, coul, nullptr};
+    TCSCF_TRY(orbitals(ctx, o));
     if (!sym) {
-      kOrbitals<<<gridBlocks(n2 * nocc, 256), 256, sm, ctx->stream>>>(n2, nb, nocc, g2.phiR, C, nocc, psi2, ldpsi);
-      TCSCF_LAUNCH(ctx);
+      o.n = n1; o.phi = g1.phiR; o.w = g1.w; o.psi = psi1; o.coul = nullptr;
+      TCSCF_TRY(orbitals(ctx, o));
     }
-    kCoulombSource<<<gridBlocks(n2, 256), 256, 0, ctx->stream>>>(n2, nocc, c.psi2, c.psi2, ldpsi, g2.w, scale, coul);
-    TCSCF_LAUNCH(ctx);
     if (tensor) {
       TCSCF_TRY(tensorPrepare(ctx, c, precision, arena, arenaBytes, tp));
       TCSCF_TRY(tensorPlanLaunch(ctx, plan));
@@ -1746,23 +1847,19 @@ int scfGraph(tcscf_ctx * ctx, Grid & g1, Grid & g2, int nocc, const double * S, 
       TCSCF_TRY(contractFp64(ctx, c));
     }
     }
-    TCSCF_CUDA(ctx, cudaMemsetAsync(FR, 0, sizeof(double) * nn, ctx->stream));
-    TCSCF_TRY(reduceFockReal(ctx, n1, nb, g1.phiR, g1.w, VH, 2.0, Tb, nb, 1.0, FR));
-    if (sym && !zeroDensity) {
-      TCSCF_CUDA(ctx, cudaMemsetAsync(FRhalf, 0, sizeof(double) * nn, ctx->stream));
-      TCSCF_TRY(reduceFockReal(ctx, n1, nb, g1.phiR, g1.w, nullptr, 0.0, Tb, nb, 1.0, FRhalf));
-      kAddTransposed<<<gridBlocks(int64_t(nn), 256), 256, 0, ctx->stream>>>(nb, FRhalf, FR);
-      TCSCF_LAUNCH(ctx);
-    }
-    kRealToReference<<<gridBlocks(int64_t(nn), 256), 256, 0, ctx->stream>>>(1, nb, g1.dsto, FR, nullptr, dG);
-    TCSCF_LAUNCH(ctx);
-    kFinalize<<<1, 512, 0, ctx->stream>>>(1, nb, dH, dG, nullptr, dD, respectSym, 2.0, dF, dE);
-    TCSCF_LAUNCH(ctx);
+    // the exchange of T' and of the skipped pairs in sums of their own, not M + M^T as the single builds: that G is
+    // symmetric to the last bit, so the Jacobi solver never turns a degenerate shell, and split-BF16 loops (whose
+    // energies carry a few 1e-8 Eh of rounding per build) can sit in a cycle (Ne, 40 x 110 points: no two
+    // energies within 1e-9 in 60 iterations, against 13 to 16)
+    double const cJ[2] = {2.0, 0.0}, none[2] = {0.0, 0.0};
+    TCSCF_TRY(reduceFockReal(ctx, n1, nb, 1, g1.phiR, g1.w, VH, cJ, Tb, 0, nb, FR));
+    if (sym) TCSCF_TRY(reduceFockReal(ctx, n1, nb, 1, g1.phiR, g1.w, nullptr, none, Tb, 0, nb, FRhalf));
+    TCSCF_TRY(fockFinish(ctx, 1, nb, {FR, nullptr, g1.dsto, sym ? 1 : 0, FRhalf}, dH, dG, nullptr, dD, respectSym, 2.0, dF, dE));
     kScfCheck<<<1, 256, 0, ctx->stream>>>(st, dE, tensor ? plan.status : nullptr, maxIter, tol, int(nn), dD, Dres, nb, Ws, Wres, handle,
                                           useHandle);
     TCSCF_LAUNCH(ctx);
     // the next density from this Fock matrix (real in the real-harmonic basis)
-    kDensityToReal<<<gridBlocks(nn, 256), 256, 0, ctx->stream>>>(1, nb, g1.dsto, dF, FRc);
+    kDensityToReal<<<gridBlocks(nn, 256), 256, 0, ctx->stream>>>(nb, g1.dsto, dF, FRc);
     TCSCF_LAUNCH(ctx);
     kSplitDensity<<<1, 256, 0, ctx->stream>>>(nb, FRc, FR, fmaxv);
     TCSCF_LAUNCH(ctx);
@@ -2385,8 +2482,7 @@ int tcscf_fock_build_precomputed(tcscf_ctx * ctx, int r1, int fji, int nspin, co
   for (int s = 0; s < nspin; ++s)
     TCSCF_TRY(reduceFockComplex(ctx, n1, nb, g1->vals, g1->w, reinterpret_cast<double *>(FaaTot), cJ,
                                 reinterpret_cast<double *>(Fai + s * n1 * nb), reinterpret_cast<double *>(dG + s * nn)));
-  kFinalize<<<1, 512, 0, ctx->stream>>>(nspin, nb, dH, dG, nullptr, dD, respect_symmetry, nspin == 1 ? 2.0 : 1.0, dF, dE);
-  TCSCF_LAUNCH(ctx);
+  TCSCF_TRY(fockFinish(ctx, nspin, nb, RealSums{}, dH, dG, nullptr, dD, respect_symmetry, nspin == 1 ? 2.0 : 1.0, dF, dE));
   cudaEventRecord(ctx->ev[1], ctx->stream);
   if (G) TCSCF_CUDA(ctx, cudaMemcpyAsync(G, dG, sizeof(double2) * nn * nspin, cudaMemcpyDeviceToHost, ctx->stream));
   if (fock) TCSCF_CUDA(ctx, cudaMemcpyAsync(fock, dF, sizeof(double2) * nn * nspin, cudaMemcpyDeviceToHost, ctx->stream));
@@ -2493,7 +2589,7 @@ int tcscf_scf(tcscf_ctx * ctx, int r1, int r2, int nspin, int n_up, int n_down, 
   int lworkR = 0;
   void * wkR = nullptr;
   {
-    kDensityToReal<<<gridBlocks(nn, 256), 256, 0, ctx->stream>>>(1, nb, g1->dsto, Sc, SRc);
+    kDensityToReal<<<gridBlocks(nn, 256), 256, 0, ctx->stream>>>(nb, g1->dsto, Sc, SRc);
     TCSCF_LAUNCH(ctx);
     kSplitDensity<<<1, 256, 0, ctx->stream>>>(nb, SRc, SRre, fmax);
     TCSCF_LAUNCH(ctx);
@@ -2568,7 +2664,7 @@ int tcscf_scf(tcscf_ctx * ctx, int r1, int r2, int nspin, int n_up, int n_down, 
     given[0] = given[1] = Factor{};
     for (int s = 0; s < nspin; ++s) {
       if (realPath) {
-        kDensityToReal<<<gridBlocks(nn, 256), 256, 0, ctx->stream>>>(1, nb, g1->dsto, Fuse + s * nn, FR);
+        kDensityToReal<<<gridBlocks(nn, 256), 256, 0, ctx->stream>>>(nb, g1->dsto, Fuse + s * nn, FR);
         TCSCF_LAUNCH(ctx);
         kSplitDensity<<<1, 256, 0, ctx->stream>>>(nb, FR, Ar, fmax);
         TCSCF_LAUNCH(ctx);
