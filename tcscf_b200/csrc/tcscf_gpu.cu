@@ -180,49 +180,164 @@ __device__ __forceinline__ void twoSum(double a, double b, double & s, double & 
   e = (a - (s - bb)) + (b - bb);
 }
 
-// S_ij / H_ij quadrature, one block per (i, j); complex reference-basis values and gradients.
-__global__ void kQuadOverlapCore(int64_t n, int nb, int Z, const double * pts, const double * w, const double2 * vals,
-                                 const double2 * grads, double2 * S, double2 * H)
+// S_ij = sum_p w conj(v_i) v_j and, with gradients, H_ij = sum_p w (conj(g_i) . g_j / 2 - Z conj(v_i) v_j / r) over complex
+// reference-basis values and gradients: a complex A^H B with two rows (S), or five (S; three gradient
+// components and the value of H), per point, on the FP64 tensor cores.  A k step of 4 holds two complex
+// rows, re and im apart: A is read as stored, the B fragments of the real and the imaginary result are
+// (b.re, b.im) and (b.im, -b.re).  One block: a 32 x 32 tile (i tile <= j tile: S and H are Hermitian, the rest
+// is mirrored) over a chunk of points, 4 warps of 8 x 32; the points' values pass through shared memory 8 at
+// a time, the next ones loaded into registers meanwhile.  chunks == 1 writes S and H, else the partials
+// [chunk][S, H][nb][nb] for kQuadSum.  Bound by the FP64 MMAs.  One block per element, reading two columns with
+// a stride of nb: QUAD_FIGURES
+constexpr int kQuadPts = 8;
+struct QuadArgs {
+  int64_t n, chunk;
+  int nb, Z;
+  const double * pts;
+  const double * w;
+  const double2 * vals;
+  const double2 * grads;   // null: S only
+  double2 * S;             // [nb][nb], or the partials of chunk 0 (chunk c at S + c stride)
+  double2 * H;
+  int64_t stride;
+};
+template <bool GRAD>
+__global__ void __launch_bounds__(128, 3) kQuadOverlapCore(QuadArgs a)
 {
-  int const i = blockIdx.x / nb, j = blockIdx.x % nb;
-  double sRe = 0, sIm = 0, hRe = 0, hIm = 0;
-  for (int64_t p = threadIdx.x; p < n; p += blockDim.x) {
-    double2 const a = vals[p * nb + i], b = vals[p * nb + j];
-    double const ovRe = a.x * b.x + a.y * b.y, ovIm = a.x * b.y - a.y * b.x;  // conj(a) b
-    sRe += w[p] * ovRe;
-    sIm += w[p] * ovIm;
-    if (grads) {
-      double const r = norm3d(pts[p], pts[n + p], pts[2 * n + p]);
-      double kRe = 0, kIm = 0;
-      for (int d = 0; d < 3; ++d) {
-        double2 const ga = grads[(p * nb + i) * 3 + d], gb = grads[(p * nb + j) * 3 + d];
-        kRe += ga.x * gb.x + ga.y * gb.y;
-        kIm += ga.x * gb.y - ga.y * gb.x;
+  constexpr int ROW = GRAD ? 128 : 32;   // a point's 32 values, then its 32 x 3 gradient components as stored
+  constexpr int LD = ROW + 1, VPT = kQuadPts * ROW / 128;
+  __shared__ double2 sA[kQuadPts][LD], sB[kQuadPts][LD];
+  __shared__ double sw[kQuadPts], sz[kQuadPts];
+  int const nb = a.nb, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, fr = lane >> 2, fq = lane & 3;
+  int ti = 0, tj = blockIdx.y;         // tile pair of the upper triangle, row by row
+  for (int left = (nb + 31) / 32; tj >= left; --left, ++ti) tj -= left;
+  tj += ti;
+  int const i0 = ti * 32, j0 = tj * 32;
+  int64_t const pbeg = int64_t(blockIdx.x) * a.chunk, pend = min(a.n, pbeg + a.chunk);
+  double acc[GRAD ? 2 : 1][4][2][2];   // S / H, column tile, re / im, fragment element
+#pragma unroll
+  for (int m = 0; m < (GRAD ? 2 : 1); ++m)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[m][j][0][0] = acc[m][j][0][1] = acc[m][j][1][0] = acc[m][j][1][1] = 0.0;
+  double2 av[VPT], bv[VPT];
+  double wv = 0, zv = 0;
+  // element e of a point's row for the tile from column c0: contiguous over the lanes in both arrays
+  auto value = [&](int64_t p, int e, int c0) {
+    if (e < 32) return p < pend && c0 + e < nb ? a.vals[p * nb + c0 + e] : make_double2(0, 0);
+    return p < pend && 3 * c0 + e - 32 < 3 * nb ? a.grads[(p * nb + c0) * 3 + e - 32] : make_double2(0, 0);
+  };
+  auto load = [&](int64_t p0) {
+#pragma unroll
+    for (int q = 0; q < VPT; ++q) {
+      int const idx = tid + 128 * q;
+      av[q] = value(p0 + idx / ROW, idx % ROW, i0);
+      if (i0 != j0) bv[q] = value(p0 + idx / ROW, idx % ROW, j0);
+    }
+    if (tid < kQuadPts) {
+      int64_t const p = p0 + tid;
+      bool const in = p < pend;
+      wv = in ? a.w[p] : 0.0;
+      zv = in && GRAD ? -a.Z * wv / norm3d(a.pts[p], a.pts[a.n + p], a.pts[2 * a.n + p]) : 0.0;
+    }
+  };
+  load(pbeg);
+  int const part = fq & 1, half = fq >> 1;   // k = 4 rows: complex row 2 s + half, re (0) or im (1)
+  double2(*const sJ)[LD] = i0 != j0 ? sB : sA;
+  for (int64_t p0 = pbeg; p0 < pend; p0 += kQuadPts) {
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < VPT; ++q) {
+      int const idx = tid + 128 * q;
+      sA[idx / ROW][idx % ROW] = av[q];
+      if (i0 != j0) sB[idx / ROW][idx % ROW] = bv[q];
+    }
+    if (tid < kQuadPts) { sw[tid] = wv; sz[tid] = zv; }
+    __syncthreads();
+    if (p0 + kQuadPts < pend) load(p0 + kQuadPts);
+    // one k step: of point p the complex row whose column c is element e0 + es c, weight f
+    auto step = [&](int m, int p, int e0, int es, double f) {
+      double2 const x = sA[p][e0 + es * (8 * warp + fr)];
+      double const af = f * (part ? x.y : x.x);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        double2 const y = sJ[p][e0 + es * (8 * j + fr)];
+        dmma(acc[m][j][0], af, part ? y.y : y.x);
+        dmma(acc[m][j][1], af, part ? -y.x : y.y);
       }
-      hRe += w[p] * (0.5 * kRe - Z * ovRe / r);
-      hIm += w[p] * (0.5 * kIm - Z * ovIm / r);
+    };
+#pragma unroll 2
+    for (int p = 0; p < kQuadPts; p += 2) step(0, p + half, 0, 1, sw[p + half]);   // S: the values of two points
+    if constexpr (GRAD) {
+#pragma unroll 2
+      for (int p = 0; p < kQuadPts; ++p) {
+        step(1, p, half ? 33 : 0, half ? 3 : 1, half ? 0.5 * sw[p] : sz[p]);   // H: value and second component,
+        step(1, p, half ? 34 : 32, 3, 0.5 * sw[p]);                            // first and third
+      }
     }
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    sRe += __shfl_xor_sync(0xffffffffu, sRe, o);
-    sIm += __shfl_xor_sync(0xffffffffu, sIm, o);
-    hRe += __shfl_xor_sync(0xffffffffu, hRe, o);
-    hIm += __shfl_xor_sync(0xffffffffu, hIm, o);
-  }
-  __shared__ double red[4][32];
-  int const wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0) { red[0][wid] = sRe; red[1][wid] = sIm; red[2][wid] = hRe; red[3][wid] = hIm; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double a[4] = {0, 0, 0, 0};
-    for (int k = 0; k < int(blockDim.x >> 5); ++k)
-      for (int q = 0; q < 4; ++q) a[q] += red[q][k];
-    S[blockIdx.x] = make_double2(a[0], a[1]);
-    if (H) H[blockIdx.x] = make_double2(a[2], a[3]);
+#pragma unroll
+  for (int m = 0; m < (GRAD ? 2 : 1); ++m) {
+    double2 * out = (m ? a.H : a.S) + blockIdx.x * a.stride;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        int const i = i0 + 8 * warp + fr, c = j0 + 8 * j + 2 * fq + e;
+        if (i >= nb || c >= nb) continue;
+        double2 const v = make_double2(acc[m][j][0][e], acc[m][j][1][e]);
+        out[i * nb + c] = v;
+        if (ti != tj) out[c * nb + i] = make_double2(v.x, -v.y);
+      }
   }
 }
 
-// Fixed scratch of tcscf_overlap_core_quadrature_static: S block results, then H (2 MiB).
+// out[e] = sum over the chunks c of part[c n + e], in chunk order
+__global__ void kQuadSum(int n, int chunks, const double2 * part, double2 * out)
+{
+  int const e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= n) return;
+  double2 s = make_double2(0, 0);
+#pragma unroll 4
+  for (int c = 0; c < chunks; ++c) {
+    double2 const v = part[int64_t(c) * n + e];
+    s.x += v.x;
+    s.y += v.y;
+  }
+  out[e] = s;
+}
+
+// S and (withH) H of a grid into out[0 .. nb^2) and out[nb^2 .. 2 nb^2); the partial sums of up to maxChunks point chunks
+// go behind them (maxChunks 1: none).  Two blocks per SM where the chunks allow
+constexpr int kQuadMaxChunks = 256;
+int quadChunks(tcscf_ctx * ctx, Grid const & g)
+{
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+  int const t = (g.nb + 31) / 32, pairs = t * (t + 1) / 2;
+  int64_t const want = (2 * int64_t(sms) + pairs - 1) / pairs;
+  return int(std::max<int64_t>(1, std::min<int64_t>({want, kQuadMaxChunks, (g.n + 4 * kQuadPts - 1) / (4 * kQuadPts)})));
+}
+int quadLaunch(tcscf_ctx * ctx, Grid const & g, int Z, bool withH, double2 * out, int maxChunks)
+{
+  int const nb = g.nb, nn = nb * nb, t = (nb + 31) / 32;
+  int const want = std::min(maxChunks, quadChunks(ctx, g));
+  int64_t const chunk = ((g.n + want - 1) / want + kQuadPts - 1) / kQuadPts * kQuadPts;
+  int const chunks = int((g.n + chunk - 1) / chunk);
+  double2 * part = chunks == 1 ? out : out + 2 * nn;
+  QuadArgs a{g.n, chunk, nb, Z, g.pts, g.w, reinterpret_cast<const double2 *>(g.vals), withH ? reinterpret_cast<const double2 *>(g.grads) : nullptr,
+             part, part + nn, 2 * int64_t(nn)};
+  dim3 const grid{unsigned(chunks), unsigned(t * (t + 1) / 2)};
+  if (withH) kQuadOverlapCore<true><<<grid, 128, 0, ctx->stream>>>(a);
+  else kQuadOverlapCore<false><<<grid, 128, 0, ctx->stream>>>(a);
+  TCSCF_LAUNCH(ctx);
+  if (chunks > 1) {
+    kQuadSum<<<gridBlocks(2 * nn, 128), 128, 0, ctx->stream>>>(2 * nn, chunks, part, out);
+    TCSCF_LAUNCH(ctx);
+  }
+  return TCSCF_OK;
+}
+
+// Fixed scratch of tcscf_overlap_core_quadrature_static: S, H and the chunk partials that fit behind them (2 MiB).
 constexpr int kQuadStaticMaxNb = 256;
 static __device__ __align__(256) double2 gQuadStaticScratch[2 * kQuadStaticMaxNb * kQuadStaticMaxNb];
 
@@ -2218,19 +2333,18 @@ int tcscf_overlap_core_quadrature(tcscf_ctx * ctx, int grid, int Z, double * S, 
   TCSCF_CHECK(ctx, !H || g->grads, TCSCF_ERR_INVALID_ARGUMENT, "H needs stored gradients");
   int const nb = g->nb;
   void * p = nullptr;
-  TCSCF_TRY(scratch(ctx, "quad_sh", sizeof(double2) * nb * nb * 2, &p));
+  int const chunks = quadChunks(ctx, *g);
+  TCSCF_TRY(scratch(ctx, "quad_sh", sizeof(double2) * nb * nb * 2 * (size_t(chunks) + 1), &p));
   double2 * dS = static_cast<double2 *>(p);
   double2 * dH = dS + nb * nb;
-  kQuadOverlapCore<<<nb * nb, 256, 0, ctx->stream>>>(g->n, nb, Z, g->pts, g->w, reinterpret_cast<double2 *>(g->vals),
-                                                      H ? reinterpret_cast<double2 *>(g->grads) : nullptr, dS, H ? dH : nullptr);
-  TCSCF_LAUNCH(ctx);
+  TCSCF_TRY(quadLaunch(ctx, *g, Z, H != nullptr, dS, chunks));
   TCSCF_CUDA(ctx, cudaMemcpyAsync(S, dS, sizeof(double2) * nb * nb, cudaMemcpyDeviceToHost, ctx->stream));
   if (H) TCSCF_CUDA(ctx, cudaMemcpyAsync(H, dH, sizeof(double2) * nb * nb, cudaMemcpyDeviceToHost, ctx->stream));
   TCSCF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return TCSCF_OK;
 }
 
-// Fixed-scratch form of the S/H quadrature: the block results go to a file-scope device array
+// Fixed-scratch form of the S/H quadrature: results and partial sums go to a file-scope device array
 // instead of context scratch, so this entry point allocates nothing.  It serves callers that cannot
 // allocate device memory at this point: a host whose device memory is already handed out to its own
 // pool (grids and tensors sized to fill HBM), and a host that cannot accept the device-wide
@@ -2241,7 +2355,7 @@ int tcscf_overlap_core_quadrature(tcscf_ctx * ctx, int grid, int Z, double * S, 
 //     context's device current), so a call of this entry point does no set-up of its own.
 //   * Sharing: every call on a device uses the same array, so overlapping calls on one device (other
 //     streams or other contexts) race; callers serialise them.  Nothing in the array needs to start
-//     at zero: kQuadOverlapCore writes every element it returns (one block per (i, j)).
+//     at zero: every element is written before it is read.
 int tcscf_overlap_core_quadrature_static(tcscf_ctx * ctx, int grid, int Z, double * S, double * H)
 {
   if (!ctx) return TCSCF_ERR_INVALID_ARGUMENT;
@@ -2256,10 +2370,10 @@ int tcscf_overlap_core_quadrature_static(tcscf_ctx * ctx, int grid, int Z, doubl
   TCSCF_CUDA(ctx, cudaSetDevice(ctx->device));
   double2 * dS = nullptr;
   TCSCF_TRY(quadStaticScratch(ctx, &dS));
-  double2 * dH = dS + kQuadStaticMaxNb * kQuadStaticMaxNb;
-  kQuadOverlapCore<<<nb * nb, 256, 0, ctx->stream>>>(g->n, nb, Z, g->pts, g->w, reinterpret_cast<double2 *>(g->vals),
-                                                      H ? reinterpret_cast<double2 *>(g->grads) : nullptr, dS, H ? dH : nullptr);
-  TCSCF_LAUNCH(ctx);
+  double2 * dH = dS + nb * nb;
+  // as many chunks of partial sums as the array holds behind S and H (none at nb = 256)
+  int const room = (kQuadStaticMaxNb * kQuadStaticMaxNb) / (nb * nb) - 1;
+  TCSCF_TRY(quadLaunch(ctx, *g, Z, H != nullptr, dS, std::max(1, room)));
   TCSCF_CUDA(ctx, cudaMemcpyAsync(S, dS, sizeof(double2) * nb * nb, cudaMemcpyDeviceToHost, ctx->stream));
   if (H) TCSCF_CUDA(ctx, cudaMemcpyAsync(H, dH, sizeof(double2) * nb * nb, cudaMemcpyDeviceToHost, ctx->stream));
   TCSCF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
