@@ -100,29 +100,73 @@ __device__ double sphLegendre(int l, int m, double x, double s)
 
 // QMCGrid::setBasisFunctions (integrateAll.hpp:88-137) with SlaterTypeOrbital::operator() and
 // ::gradient (SlaterTypeOrbital.hpp:51-106), or the Ochi / hydrogen-like radial parts (basisRadial;
-// OchiBasisFunction::gradient, OchiBasis.hpp:58-107, shares the angular terms of the STO gradient).  One thread per (point, function), function index
-// fastest, so every store is coalesced.  Also writes the real-harmonic values phiR used by the
-// contraction kernels: cos-type sqrt2 R P cos(|m| phi) for m > 0, sin-type sqrt2 R P sin(|m| phi)
-// for m < 0, R P for m == 0.
-__global__ void kBasis(int64_t n, int nb, int ndim, const double * __restrict__ pts, const DevSto * __restrict__ sto,
-                       double * __restrict__ phiR, double * __restrict__ vals, double * __restrict__ grads)
+// OchiBasisFunction::gradient, OchiBasis.hpp:58-107, shares the angular terms of the STO gradient).  Also writes
+// the real-harmonic values phiR used by the contraction kernels: cos-type sqrt2 R P cos(|m| phi) for m > 0,
+// sin-type sqrt2 R P sin(|m| phi) for m < 0, R P for m == 0.
+// A block takes `npts` points.  What depends on the point alone (angles, unit vectors, cos / sin of m phi, the associated
+// Legendre functions of every l <= lmax) is formed once in shared memory; then one thread per (point,
+// function), function index fastest so that every store is coalesced, has the radial part and products left.
+// Bound by its stores and the FP64 exponentials.  With every thread forming the angles for itself: 59,000
+// points x 40 functions with gradients 224 -> 57 us.
+constexpr int kBasisHead = 12;   // doubles per point before the tables
+__host__ __device__ inline int basisPointDoubles(int lmax) { return kBasisHead + 2 * (lmax + 2) + (lmax + 1) * (lmax + 2) / 2; }
+__global__ void __launch_bounds__(256) kBasis(int64_t n, int nb, int ndim, int lmax, int npts, const double * __restrict__ pts,
+                                            const DevSto * __restrict__ sto, double * __restrict__ phiR, double * __restrict__ vals,
+                                            double * __restrict__ grads)
 {
-  int64_t const total = n * nb;
-  for (int64_t idx = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; idx < total; idx += int64_t(gridDim.x) * blockDim.x) {
-    int64_t const i = idx / nb;
-    int const b = int(idx % nb);
-    double const x = pts[i], y = pts[n + i], z = pts[2 * n + i];
+  extern __shared__ double sm[];
+  int const per = basisPointDoubles(lmax), nm = lmax + 2, nlm = (lmax + 1) * (lmax + 2) / 2, tid = threadIdx.x;
+  int64_t const i0 = int64_t(blockIdx.x) * npts;
+  int const np = int(min(int64_t(npts), n - i0));
+  // per point: r, cos and sin theta of the Legendre functions, phi (replaced below), then for the gradients 1/r, cot theta,
+  // 1/(r sin theta) and the unit vectors' sines and cosines; cos, sin (m phi); P(l, m)
+  for (int t = tid; t < np; t += 256) {
+    double * q = sm + t * per;
+    double const x = pts[i0 + t], y = pts[n + i0 + t], z = pts[2 * n + i0 + t];
     double const r = norm3d(x, y, z);
-    double const ct = z / r;
-    double const st = sqrt(x * x + y * y) / r;
-    double const ph = atan2(y, x);
+    q[0] = r;
+    q[1] = z / r;
+    q[2] = sqrt(x * x + y * y) / r;
+    q[3] = atan2(y, x);
+    if (grads) {
+      double const th = acos(q[1]);
+      double sth, cth;
+      sincos(th, &sth, &cth);
+      q[4] = 1.0 / r;
+      q[5] = 1.0 / tan(th);
+      q[6] = 1.0 / (r * sth);
+      q[7] = sth;
+      q[8] = cth;
+    }
+  }
+  __syncthreads();
+  for (int t = tid; t < np * (nm + nlm); t += 256) {
+    int const k = t / np;
+    double * q = sm + (t % np) * per;
+    if (k < nm) {
+      double sn, cs;
+      sincos(double(k) * q[3], &sn, &cs);
+      q[kBasisHead + 2 * k] = cs;
+      q[kBasisHead + 2 * k + 1] = sn;
+    } else {
+      int l = 0, m = k - nm;
+      while (m > l) { m -= l + 1; ++l; }
+      q[kBasisHead + 2 * nm + k - nm] = sphLegendre(l, m, q[1], q[2]);
+    }
+  }
+  __syncthreads();
+  for (int t = tid; t < np * nb; t += 256) {
+    int const b = t % nb;
+    double const * q = sm + (t / nb) * per;
+    double const * ang = q + kBasisHead;
+    double const * leg = ang + 2 * nm;
+    int64_t const idx = i0 * nb + t;
     DevSto const s = sto[b];
     double R, dR;
-    basisRadial(s, r, R, dR);
+    basisRadial(s, q[0], R, dR);
     int const am = s.m < 0 ? -s.m : s.m;
-    double const P = sphLegendre(s.l, am, ct, st);
-    double sn, cs;
-    sincos(double(s.m) * ph, &sn, &cs);
+    double const P = leg[s.l * (s.l + 1) / 2 + am];
+    double const cs = ang[2 * am], sn = s.m < 0 ? -ang[2 * am + 1] : ang[2 * am + 1];   // of m phi
     double const rp = R * P;
     double pr;
     if (s.rtype == 0) pr = rp;
@@ -130,44 +174,34 @@ __global__ void kBasis(int64_t n, int nb, int ndim, const double * __restrict__ 
     else pr = -1.4142135623730950488 * rp * sn;
     phiR[idx] = pr;
     if (vals) {
-      if (ndim == 3) { vals[2 * idx] = rp * cs; vals[2 * idx + 1] = rp * sn; }
+      if (ndim == 3) reinterpret_cast<double2 *>(vals)[idx] = make_double2(rp * cs, rp * sn);
       else vals[idx] = rp * cs;
     }
     if (grads) {
-      // SlaterTypeOrbital.hpp:63-106, arithmetic kept (including its m < 0 and pole behaviour)
-      double const th = acos(ct);
+      // SlaterTypeOrbital.hpp:63-106 (including its m < 0 and pole behaviour), its quotients by the point's reciprocals
       double const l = s.l, m = s.m;
-      double const dRadialPart = dR;
       double const ylmRe = P * cs, ylmIm = P * sn;
       double const c1 = (s.l != s.m) ? sqrt((l - m) * (l + m + 1)) : 0.0;
-      int const m1 = s.m + 1;
-      double const P1 = sphLegendre(s.l, m1 < 0 ? -m1 : m1, ct, st);
-      double sn1, cs1, snm, csm;
-      sincos(double(m1) * ph, &sn1, &cs1);
-      sincos(-ph, &snm, &csm);
+      int const m1 = s.m + 1, am1 = m1 < 0 ? -m1 : m1;
+      double const P1 = am1 > s.l ? 0.0 : leg[s.l * (s.l + 1) / 2 + am1];
+      double const cs1 = ang[2 * am1], sn1 = m1 < 0 ? -ang[2 * am1 + 1] : ang[2 * am1 + 1];
+      double const cp = ang[2], sp = ang[3];   // of phi
       // cExp(-phi) * Y_l^{m+1}
       double const y1Re = P1 * cs1, y1Im = P1 * sn1;
-      double const ylmp1Re = c1 * (csm * y1Re - snm * y1Im);
-      double const ylmp1Im = c1 * (csm * y1Im + snm * y1Re);
-      double const rHatRe = dRadialPart * ylmRe, rHatIm = dRadialPart * ylmIm;
-      double const tnt = tan(th), sth = sin(th), cth = cos(th);
-      double const thRe = (m * ylmRe / tnt + ylmp1Re) * R / r;
-      double const thIm = (m * ylmIm / tnt + ylmp1Im) * R / r;
+      double const ylmp1Re = c1 * (cp * y1Re + sp * y1Im);
+      double const ylmp1Im = c1 * (cp * y1Im - sp * y1Re);
+      double const rHatRe = dR * ylmRe, rHatIm = dR * ylmIm;
+      double const Rr = R * q[4], sth = q[7], cth = q[8];
+      double const thRe = (m * ylmRe * q[5] + ylmp1Re) * Rr;
+      double const thIm = (m * ylmIm * q[5] + ylmp1Im) * Rr;
       // i m Ylm R / (r sin t)
-      double const phRe = -m * ylmIm * R / (r * sth);
-      double const phIm = m * ylmRe * R / (r * sth);
-      double sp, cp;
-      sincos(ph, &sp, &cp);
-      double const rx = cp * sth, ry = sp * sth, rz = cth;
-      double const tx = cp * cth, ty = sp * cth, tz = -sth;
-      double const px = -sp, py = cp;
-      double * g = grads + 6 * idx;
-      g[0] = rHatRe * rx + thRe * tx + phRe * px;
-      g[1] = rHatIm * rx + thIm * tx + phIm * px;
-      g[2] = rHatRe * ry + thRe * ty + phRe * py;
-      g[3] = rHatIm * ry + thIm * ty + phIm * py;
-      g[4] = rHatRe * rz + thRe * tz;
-      g[5] = rHatIm * rz + thIm * tz;
+      double const phRe = -m * ylmIm * R * q[6];
+      double const phIm = m * ylmRe * R * q[6];
+      double const rx = cp * sth, ry = sp * sth, tx = cp * cth, ty = sp * cth;
+      double2 * g = reinterpret_cast<double2 *>(grads) + 3 * idx;
+      g[0] = make_double2(rHatRe * rx + thRe * tx - phRe * sp, rHatIm * rx + thIm * tx - phIm * sp);
+      g[1] = make_double2(rHatRe * ry + thRe * ty + phRe * cp, rHatIm * ry + thIm * ty + phIm * cp);
+      g[2] = make_double2(rHatRe * cth - thRe * sth, rHatIm * cth - thIm * sth);
     }
   }
 }
@@ -183,12 +217,12 @@ __device__ __forceinline__ void twoSum(double a, double b, double & s, double & 
 // S_ij = sum_p w conj(v_i) v_j and, with gradients, H_ij = sum_p w (conj(g_i) . g_j / 2 - Z conj(v_i) v_j / r) over complex
 // reference-basis values and gradients: a complex A^H B with two rows (S), or five (S; three gradient
 // components and the value of H), per point, on the FP64 tensor cores.  A k step of 4 holds two complex
-// rows, re and im apart: A is read as stored, the B fragments of the real and the imaginary result are
-// (b.re, b.im) and (b.im, -b.re).  One block: a 32 x 32 tile (i tile <= j tile: S and H are Hermitian, the rest
+// rows, re and im apart: the real result multiplies (a.re, a.im) by (b.re, b.im), the imaginary one (a.re, -a.im) by
+// (b.im, b.re), so fragments are plain 8-byte loads and the sign goes with the weight of A.  One block: a 32 x 32 tile (i tile <= j tile: S and H are Hermitian, the rest
 // is mirrored) over a chunk of points, 4 warps of 8 x 32; the points' values pass through shared memory 8 at
 // a time, the next ones loaded into registers meanwhile.  chunks == 1 writes S and H, else the partials
 // [chunk][S, H][nb][nb] for kQuadSum.  Bound by the FP64 MMAs.  One block per element, reading two columns with
-// a stride of nb: QUAD_FIGURES
+// a stride of nb: 59,000 points x 40 functions 2,995 -> 334 us.
 constexpr int kQuadPts = 8;
 struct QuadArgs {
   int64_t n, chunk;
@@ -256,13 +290,13 @@ __global__ void __launch_bounds__(128, 3) kQuadOverlapCore(QuadArgs a)
     if (p0 + kQuadPts < pend) load(p0 + kQuadPts);
     // one k step: of point p the complex row whose column c is element e0 + es c, weight f
     auto step = [&](int m, int p, int e0, int es, double f) {
-      double2 const x = sA[p][e0 + es * (8 * warp + fr)];
-      double const af = f * (part ? x.y : x.x);
+      const double * x = reinterpret_cast<const double *>(&sA[p][e0 + es * (8 * warp + fr)]);
+      const double * y = reinterpret_cast<const double *>(&sJ[p][e0 + es * fr]);
+      double const af = f * x[part], ai = part ? -af : af;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        double2 const y = sJ[p][e0 + es * (8 * j + fr)];
-        dmma(acc[m][j][0], af, part ? y.y : y.x);
-        dmma(acc[m][j][1], af, part ? -y.x : y.y);
+        dmma(acc[m][j][0], af, y[16 * es * j + part]);
+        dmma(acc[m][j][1], ai, y[16 * es * j + 1 - part]);
       }
     };
 #pragma unroll 2
@@ -291,30 +325,35 @@ __global__ void __launch_bounds__(128, 3) kQuadOverlapCore(QuadArgs a)
   }
 }
 
-// out[e] = sum over the chunks c of part[c n + e], in chunk order
-__global__ void kQuadSum(int n, int chunks, const double2 * part, double2 * out)
+// out[e] = sum over the chunks c of part[c n + e]: 32 elements per block, 8 warps taking every eighth chunk each, added in warp order
+__global__ void __launch_bounds__(256) kQuadSum(int n, int chunks, const double2 * part, double2 * out)
 {
-  int const e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n) return;
+  __shared__ double2 red[8][32];
+  int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5, e = blockIdx.x * 32 + lane;
   double2 s = make_double2(0, 0);
+  if (e < n)
 #pragma unroll 4
-  for (int c = 0; c < chunks; ++c) {
-    double2 const v = part[int64_t(c) * n + e];
-    s.x += v.x;
-    s.y += v.y;
-  }
+    for (int c = warp; c < chunks; c += 8) {
+      double2 const v = part[int64_t(c) * n + e];
+      s.x += v.x;
+      s.y += v.y;
+    }
+  red[warp][lane] = s;
+  __syncthreads();
+  if (warp != 0 || e >= n) return;
+  for (int k = 1; k < 8; ++k) { s.x += red[k][lane].x; s.y += red[k][lane].y; }
   out[e] = s;
 }
 
 // S and (withH) H of a grid into out[0 .. nb^2) and out[nb^2 .. 2 nb^2); the partial sums of up to maxChunks point chunks
-// go behind them (maxChunks 1: none).  Two blocks per SM where the chunks allow
+// go behind them (maxChunks 1: none).  Three blocks per SM (as many as are resident) where the chunks allow
 constexpr int kQuadMaxChunks = 256;
 int quadChunks(tcscf_ctx * ctx, Grid const & g)
 {
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
   int const t = (g.nb + 31) / 32, pairs = t * (t + 1) / 2;
-  int64_t const want = (2 * int64_t(sms) + pairs - 1) / pairs;
+  int64_t const want = 3 * int64_t(sms) / pairs;
   return int(std::max<int64_t>(1, std::min<int64_t>({want, kQuadMaxChunks, (g.n + 4 * kQuadPts - 1) / (4 * kQuadPts)})));
 }
 int quadLaunch(tcscf_ctx * ctx, Grid const & g, int Z, bool withH, double2 * out, int maxChunks)
@@ -331,7 +370,7 @@ int quadLaunch(tcscf_ctx * ctx, Grid const & g, int Z, bool withH, double2 * out
   else kQuadOverlapCore<false><<<grid, 128, 0, ctx->stream>>>(a);
   TCSCF_LAUNCH(ctx);
   if (chunks > 1) {
-    kQuadSum<<<gridBlocks(2 * nn, 128), 128, 0, ctx->stream>>>(2 * nn, chunks, part, out);
+    kQuadSum<<<unsigned((2 * nn + 31) / 32), 256, 0, ctx->stream>>>(2 * nn, chunks, part, out);
     TCSCF_LAUNCH(ctx);
   }
   return TCSCF_OK;
@@ -2299,7 +2338,12 @@ int tcscf_grid_set_basis(tcscf_ctx * ctx, int grid, const tcscf_sto * basis, int
   TCSCF_TRY(gridAlloc(ctx, &g->vals, sizeof(double) * g->n * nb * (g->ndim == 3 ? 2 : 1)));
   if (gradients) TCSCF_TRY(gridAlloc(ctx, &g->grads, sizeof(double) * g->n * nb * 6));
   TCSCF_CUDA(ctx, cudaMemcpyAsync(g->dsto, ds.data(), sizeof(DevSto) * nb, cudaMemcpyHostToDevice, ctx->stream));
-  kBasis<<<gridBlocks(g->n * nb, 256), 256, 0, ctx->stream>>>(g->n, nb, g->ndim, g->pts, g->dsto, g->phiR, g->vals, g->grads);
+  int lmax = 0;
+  for (DevSto const & d : ds) lmax = std::max(lmax, d.l);
+  // about four (point, function) pairs a thread, the tables within 48 KB (8 points of lmax = 12 take 8.4 KB)
+  int const npts = std::min(std::max(8, std::min(64, 1024 / nb)), int(48 * 1024 / (sizeof(double) * basisPointDoubles(lmax))));
+  kBasis<<<unsigned((g->n + npts - 1) / npts), 256, sizeof(double) * npts * basisPointDoubles(lmax), ctx->stream>>>(
+    g->n, nb, g->ndim, lmax, npts, g->pts, g->dsto, g->phiR, g->vals, g->grads);
   TCSCF_LAUNCH(ctx);
   TCSCF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   g->nb = nb;

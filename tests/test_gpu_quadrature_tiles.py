@@ -31,3 +31,20 @@ def test_overlap_core_tile_edges(ctx, n, counts):
     G.close()
     for a, r in ((S, Sr), (Ss, Sr), (S0, Sr), (H, Hr), (Hs, Hr)):
         assert np.abs(a - r).max() <= 1e-11 * np.abs(r).max()
+
+
+# per-point tables: one function of the highest l (the largest tables, the most points a block would take), one point
+# over a block's share, and many functions (fewest points a block)
+@pytest.mark.parametrize("n,basis", [(3, [(0.8, 13, 12, 0)]), (129, [(0.8, 13, 12, 0)]), (65, wl.expand(0, [0.7])), (33, wl.expand(12, [0.9, 1.4])),
+                                     (17, wl.expand(0, [0.5 * 1.02 ** k for k in range(150)]))])
+def test_basis_values_and_gradients_by_block(ctx, n, basis):
+    rng = np.random.default_rng(n)
+    g = grids.QuadratureGrid(rng.normal(size=(3, n)) * 1.5, np.ones(n))
+    v, gr = oracle.basis_values(g.points, basis, gradients=True)
+    G = api.QMCGrid(ctx, g)
+    G.setBasisFunctions(basis, storeGradients=True)
+    a, b = G.basisValues, G.basisGradients
+    G.close()
+    # sums of a few dozen products of functions good to a few eps; the l = 12 recurrence loses another digit
+    assert np.abs(a - v).max() <= 1e-12 * np.abs(v).max()
+    assert np.abs(b - gr).max() <= 1e-12 * np.abs(gr).max()
