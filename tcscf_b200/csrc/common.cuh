@@ -46,13 +46,21 @@ struct Grid {
   double vtScale = 0;
 };
 
+// A kept Fji / Vji tensor.  The r12 kernels are real and each element integrates a product of two basis functions, so in the
+// real-harmonic basis the tensor is real and symmetric: it is kept as planes [n1][1 or 3][plane] of nb rows
+// (tensorStride(nb) doubles apart, zeros behind and below), half the complex [nb][nb](3) layout of the reference basis, which
+// tensorToReference forms where a routine or the host wants it
 struct Tensor {
   double * d = nullptr;
   int64_t n1 = 0;
   int nb = 0;
-  int isComplex = 1;
-  int vec = 0;  // 3 components (Vji)
+  int isComplex = 1;   // of the reference layout (0: a 2-D r2 grid's real Fji)
+  int vec = 0;         // 3 components (Vji)
 };
+// row stride of a plane, and doubles per plane: 4 (mod 8), which puts the fragments of 8 planes on different shared-memory
+// banks and every plane on a 16-byte boundary
+__host__ __device__ constexpr int tensorStride(int nb) { return (nb + 3) / 4 * 4; }
+__host__ __device__ constexpr int tensorPlane(int nb) { return tensorStride(nb) * tensorStride(nb) + 4; }
 
 struct Scratch {
   void * p = nullptr;
@@ -184,6 +192,15 @@ inline unsigned gridBlocks(int64_t n, int threads)
 {
   int64_t b = (n + threads - 1) / threads;
   return unsigned(b < 1 ? 1 : (b > 1048576 ? 1048576 : b));
+}
+
+// U coefficient U[k][i] of the unitary complex -> real-harmonic map phiR_k = sum_i U[k][i] phi_i (i = k or its partner)
+__device__ __forceinline__ double2 uRow(const DevSto * s, int k, int i)
+{
+  double const h = 0.70710678118654752440;
+  int const t = s[k].rtype;
+  if (i == k) return t == 0 ? make_double2(1, 0) : (t == 1 ? make_double2(h, 0) : make_double2(0, h));
+  return t == 1 ? make_double2(h, 0) : make_double2(0, -h);
 }
 
 // ---- kernels shared between translation units -------------------------------------------------

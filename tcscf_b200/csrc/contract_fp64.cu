@@ -17,7 +17,6 @@ namespace {
 
 constexpr int BK = 32;        // r2 points per stage
 constexpr int kMaxCol = 128;  // columns per block at most
-constexpr int NT = 256;       // threads of the complex reduction
 
 struct KArgs {
   int64_t n1, n2, r2PerSplit;
@@ -190,10 +189,12 @@ __global__ void __launch_bounds__(32 * contractWarps(RT), contractBlocks(NTL, RT
   if (nsteps > 0) issue(r2begin, 0);
   cpAsyncCommit();
 
-  for (int idx = tid; idx < R4 * BMT; idx += kThreads) {
-    int const r = idx / R4, b = idx % R4;
-    int64_t const g = r1base + r;
-    sP1[r * pld + b] = b < R && g < a.n1 ? a.psi1[g * a.ldpsi + b] : 0.0;
+  if constexpr (KR != 0) {
+    for (int idx = tid; idx < R4 * BMT; idx += kThreads) {
+      int const r = idx / R4, b = idx % R4;
+      int64_t const g = r1base + r;
+      sP1[r * pld + b] = b < R && g < a.n1 ? a.psi1[g * a.ldpsi + b] : 0.0;
+    }
   }
   int const wrow = (tid >> 5) * 8 * RT + fr;   // this lane's row of the block in row tile 0
   double x1[RT], y1[RT], z1[RT], vh[RT];
@@ -396,7 +397,6 @@ __global__ void kSumSplits(int64_t n, int nsplit, int64_t stride, const double *
 
 // ---- real Fock reduction:  out[k][l] = sum_r w[r] phi[r][k] (cJ phi[r][l] VH[r] - T[r][l]) ----
 constexpr int RB = 16;      // rows per step
-constexpr int RCH = 1024;   // rows per block (complex reduction; the real one sizes its row chunks per call)
 
 struct ReduceArgs {
   int64_t n1, tStride;        // rows; elements between the spins' T
@@ -508,64 +508,6 @@ __global__ void __launch_bounds__(256) kReduceSum(int n, int nchunk, const doubl
 #pragma unroll
     for (int k = 1; k < 8; ++k) s += red[k][lane];
     out[int64_t(blockIdx.y) * n + e] = s;
-  }
-}
-
-__global__ void kSumChunks(int n, int nchunk, const double * part, double * out)
-{
-  int const i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double s = 0.0;
-  for (int k = 0; k < nchunk; ++k) s += part[int64_t(k) * n + i];
-  out[i] += s;
-}
-
-// ---- complex Fock reduction (precompute form): out(j,i) += sum_r w conj(A[r][j]) (cJ A[r][i] Faa[r] - Fai[r][i])
-constexpr int CRB = 16;
-__global__ void __launch_bounds__(NT) kReduceComplex(int64_t n1, int nb, const double2 * A, const double * w, const double2 * Faa,
-                                                     double cJ, const double2 * Fai, double2 * part)
-{
-  extern __shared__ double2 csm[];
-  double2 * sA = csm;              // [CRB][nb]
-  double2 * sY = csm + CRB * nb;   // [CRB][nb]
-  int const tid = threadIdx.x;
-  int64_t const rbeg = int64_t(blockIdx.x) * RCH, rend = min(n1, rbeg + RCH);
-  int const nn = nb * nb;
-  int const per = (nn + NT - 1) / NT;
-  double2 acc[16];
-  for (int q = 0; q < 16; ++q) acc[q] = make_double2(0, 0);
-  for (int64_t r0 = rbeg; r0 < rend; r0 += CRB) {
-    __syncthreads();
-    for (int idx = tid; idx < CRB * nb; idx += NT) {
-      int const rr = idx / nb, c = idx % nb;
-      int64_t const r = r0 + rr;
-      double2 av = make_double2(0, 0), yv = make_double2(0, 0);
-      if (r < rend) {
-        double2 const x = A[r * nb + c];
-        av = make_double2(w[r] * x.x, -w[r] * x.y);   // w conj(A)
-        double2 const f = Faa[r];
-        double2 const t = Fai[r * nb + c];
-        yv.x = cJ * (x.x * f.x - x.y * f.y) - t.x;
-        yv.y = cJ * (x.x * f.y + x.y * f.x) - t.y;
-      }
-      sA[idx] = av;
-      sY[idx] = yv;
-    }
-    __syncthreads();
-    for (int rr = 0; rr < CRB; ++rr)
-      for (int q = 0; q < per && q < 16; ++q) {
-        int const e = tid + q * NT;
-        if (e >= nn) break;
-        int const j = e / nb, i = e % nb;
-        double2 const x = sA[rr * nb + j], y = sY[rr * nb + i];
-        acc[q].x = fma(x.x, y.x, fma(-x.y, y.y, acc[q].x));
-        acc[q].y = fma(x.x, y.y, fma(x.y, y.x, acc[q].y));
-      }
-  }
-  double2 * out = part + int64_t(blockIdx.x) * nn;
-  for (int q = 0; q < per && q < 16; ++q) {
-    int const e = tid + q * NT;
-    if (e < nn) out[e] = acc[q];
   }
 }
 
@@ -794,24 +736,6 @@ int reduceFockReal(tcscf_ctx * ctx, int64_t n1, int nb, int nspin, const double 
   TCSCF_LAUNCH(ctx);
   int const n = nb * nb;
   kReduceSum<<<dim3(unsigned((n + 31) / 32), unsigned(nspin)), 256, 0, ctx->stream>>>(n, int(chunks), part, out);
-  TCSCF_LAUNCH(ctx);
-  return TCSCF_OK;
-}
-
-int reduceFockComplex(tcscf_ctx * ctx, int64_t n1, int nb, const double * A, const double * w, const double * Faa, double cJ,
-                      const double * Fai, double * out)
-{
-  TCSCF_CHECK(ctx, nb * nb <= 16 * NT, TCSCF_ERR_UNSUPPORTED, "precompute-form Fock reduction supports nb <= 64");
-  int64_t const chunks = (n1 + RCH - 1) / RCH;
-  void * p = nullptr;
-  TCSCF_TRY(scratch(ctx, "reduce_complex", size_t(chunks) * nb * nb * 2 * sizeof(double), &p));
-  size_t const smem = size_t(2) * CRB * nb * sizeof(double2);
-  kReduceComplex<<<unsigned(chunks), NT, smem, ctx->stream>>>(n1, nb, reinterpret_cast<const double2 *>(A), w,
-                                                              reinterpret_cast<const double2 *>(Faa), cJ,
-                                                              reinterpret_cast<const double2 *>(Fai), static_cast<double2 *>(p));
-  TCSCF_LAUNCH(ctx);
-  int const n = 2 * nb * nb;
-  kSumChunks<<<(n + 255) / 256, 256, 0, ctx->stream>>>(n, int(chunks), static_cast<double *>(p), out);
   TCSCF_LAUNCH(ctx);
   return TCSCF_OK;
 }

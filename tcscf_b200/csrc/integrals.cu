@@ -239,10 +239,9 @@ int tcscf_integrate_all_r1r2(tcscf_ctx * ctx, int r1, int r2, int use_gradient, 
   double * B = nullptr;
   if (!use_gradient) {
     TCSCF_TRY(tcscf_compute_F(ctx, r1, r2, kernel, jastrow, TCSCF_PREC_FP64, nullptr, 1, &fid));
-    B = ctx->tensors[fid].d;
   }
   size_t const bytesA = sizeof(double2) * size_t(n1) * nn;
-  size_t const bytesB = use_gradient ? sizeof(double2) * size_t(n1) * nn * 2 + sizeof(double2) * size_t(n2) * nn : 0;
+  size_t const bytesB = use_gradient ? sizeof(double2) * size_t(n1) * nn * 2 + sizeof(double2) * size_t(n2) * nn : sizeof(double) * size_t(n1) * nn;
   size_t const bytesC = sizeof(double2) * size_t(nn) * nn * 2;
   void * p = nullptr;
   int st = scratch(ctx, "integrate_all", bytesA + bytesB + bytesC, &p);
@@ -266,6 +265,10 @@ int tcscf_integrate_all_r1r2(tcscf_ctx * ctx, int r1, int r2, int use_gradient, 
       TCSCF_LAUNCH(ctx);
     }
     B = Bsum;
+  } else {
+    B = reinterpret_cast<double *>(out + size_t(nn) * nn);   // F [n1][nn] in the reference basis
+    int const est = tensorToReference(ctx, ctx->tensors[fid], g1->dsto, 0, n1, B);
+    if (est != TCSCF_OK) { tcscf_tensor_destroy(ctx, fid); return est; }
   }
   kR1Pairs<<<gridBlocks(n1 * nn, 256), 256, 0, ctx->stream>>>(0, n1, nb, reinterpret_cast<const double2 *>(g1->vals), g1->w, A);
   TCSCF_LAUNCH(ctx);
@@ -307,10 +310,9 @@ int tcscf_three_electron_integrals(tcscf_ctx * ctx, int r1, int r2, const tcscf_
   TCSCF_TRY(blasHandle(ctx, &h));
   int vid = 0;
   TCSCF_TRY(tcscf_compute_V(ctx, r1, r2, TCSCF_K_GRAD_U_SAME, jastrow, TCSCF_PREC_FP64, nullptr, 1, &vid));
-  const double2 * V = reinterpret_cast<const double2 *>(ctx->tensors[vid].d);
   // r1 chunk so that the (q,t,r,u) operand stays below ~1 GB
   int64_t const chunk = std::max<int64_t>(1, std::min<int64_t>(n1, (int64_t(1) << 26) / n4));
-  size_t const bytes = sizeof(double2) * (size_t(chunk) * nn + size_t(chunk) * n4 + 2 * size_t(n6));
+  size_t const bytes = sizeof(double2) * (size_t(chunk) * nn * 4 + size_t(chunk) * n4 + 2 * size_t(n6));
   void * p = nullptr;
   int st = scratch(ctx, "three_electron", bytes, &p);
   if (st != TCSCF_OK) { tcscf_tensor_destroy(ctx, vid); return st; }
@@ -318,12 +320,15 @@ int tcscf_three_electron_integrals(tcscf_ctx * ctx, int r1, int r2, const tcscf_
   double2 * Y = X + size_t(chunk) * nn;
   double2 * C = Y + size_t(chunk) * n4;
   double2 * out = C + size_t(n6);
+  double2 * V = out + size_t(n6);   // the chunk's Vji in the reference basis
   cuDoubleComplex const one = make_cuDoubleComplex(1, 0), zero = make_cuDoubleComplex(0, 0);
   for (int64_t a0 = 0; a0 < n1 && st == TCSCF_OK; a0 += chunk) {
     int64_t const rows = std::min(chunk, n1 - a0);
+    st = tensorToReference(ctx, ctx->tensors[vid], g1->dsto, a0, rows, reinterpret_cast<double *>(V));
+    if (st != TCSCF_OK) break;
     kR1Pairs<<<gridBlocks(rows * nn, 256), 256, 0, ctx->stream>>>(a0, rows, nb, reinterpret_cast<const double2 *>(g1->vals), g1->w, X);
     ctx->launchCount++;
-    kVDotV<<<gridBlocks(rows * n4, 256), 256, 0, ctx->stream>>>(a0, rows, nb, V, Y);
+    kVDotV<<<gridBlocks(rows * n4, 256), 256, 0, ctx->stream>>>(0, rows, nb, V, Y);
     ctx->launchCount++;
     // C [(p,s)][(q,t,r,u)] (column-major) += X^T Y over this chunk of r1
     cublasStatus_t const bs = cublasZgemm(h, CUBLAS_OP_N, CUBLAS_OP_T, int(nn), int(n4), int(rows), &one,
@@ -370,27 +375,29 @@ int tcscf_tc_compute_q(tcscf_ctx * ctx, int r1, int vsame, int voppo, double * Q
               TCSCF_ERR_INVALID_ARGUMENT, "computeQ: the tensors do not match the r1 grid");
   TCSCF_CHECK(ctx, nb <= 46, TCSCF_ERR_UNSUPPORTED, "computeQ: nb <= 46 (nb^4 stays an int GEMM dimension)");
   int64_t const nn = int64_t(nb) * nb, n4 = nn * nn, n6 = n4 * nn, n1 = g1->n;
-  const double2 * Vs = reinterpret_cast<const double2 *>(itS->second.d);
-  const double2 * Vo = reinterpret_cast<const double2 *>(itO->second.d);
   cublasHandle_t h = nullptr;
   TCSCF_TRY(blasHandle(ctx, &h));
   int64_t const chunk = std::max<int64_t>(1, std::min<int64_t>(n1, (int64_t(1) << 26) / n4));
-  size_t const bytes = sizeof(double2) * (size_t(chunk) * nn + size_t(chunk) * n4 + 4 * size_t(n6));
-  TCSCF_TRY(sixIndexFits(ctx, bytes, "computeQ"));
+  size_t const bytes = sizeof(double2) * (size_t(chunk) * nn * 7 + size_t(chunk) * n4 + 4 * size_t(n6));
+  TCSCF_TRY(sixIndexFits(ctx, sizeof(double2) * (size_t(chunk) * nn + size_t(chunk) * n4 + 4 * size_t(n6)), "computeQ"));
   void * p = nullptr;
   TCSCF_TRY(scratch(ctx, "compute_q", bytes, &p));
   double2 * X = static_cast<double2 *>(p);
   double2 * Y = X + size_t(chunk) * nn;
   double2 * C = Y + size_t(chunk) * n4;        // [3][n6]: same-same, same-opposite, opposite-opposite
   double2 * out = C + 3 * size_t(n6);
+  double2 * Vs = out + size_t(n6);             // the chunk's Vji in the reference basis
+  double2 * Vo = Vs + size_t(chunk) * nn * 3;
   const double2 * pairs[3][2] = {{Vs, Vs}, {Vs, Vo}, {Vo, Vo}};
   cuDoubleComplex const one = make_cuDoubleComplex(1, 0), zero = make_cuDoubleComplex(0, 0);
   for (int64_t a0 = 0; a0 < n1; a0 += chunk) {
     int64_t const rows = std::min(chunk, n1 - a0);
     kR1Pairs<<<gridBlocks(rows * nn, 256), 256, 0, ctx->stream>>>(a0, rows, nb, reinterpret_cast<const double2 *>(g1->vals), g1->w, X);
     TCSCF_LAUNCH(ctx);
+    TCSCF_TRY(tensorToReference(ctx, itS->second, g1->dsto, a0, rows, reinterpret_cast<double *>(Vs)));
+    TCSCF_TRY(tensorToReference(ctx, itO->second, g1->dsto, a0, rows, reinterpret_cast<double *>(Vo)));
     for (int t = 0; t < 3; ++t) {
-      kVDotV2<<<gridBlocks(rows * n4, 256), 256, 0, ctx->stream>>>(a0, rows, nb, pairs[t][0], pairs[t][1], Y);
+      kVDotV2<<<gridBlocks(rows * n4, 256), 256, 0, ctx->stream>>>(0, rows, nb, pairs[t][0], pairs[t][1], Y);
       TCSCF_LAUNCH(ctx);
       // C_t [(ji)][(pq,rs)] (column-major) += X^T Y over this chunk of r1
       cublasStatus_t const bs = cublasZgemm(h, CUBLAS_OP_N, CUBLAS_OP_T, int(nn), int(n4), int(rows), &one,

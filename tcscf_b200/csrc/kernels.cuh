@@ -86,6 +86,14 @@ int tensorPackedV(tcscf_ctx * ctx, Grid & g2, const double * V, double scale, co
 int finalizeLaunch(tcscf_ctx * ctx, int nspin, int nb, const double * h, double2 * G, const double2 * G3, const double2 * D, int respectSym,
                    double factor, double2 * fock, double * energy);
 
+// DR = conj(U) D U^T (complex [nb][nb], reference to real-harmonic basis)
+int densityToRealLaunch(tcscf_ctx * ctx, int nb, const DevSto * sto, const double2 * D, double2 * DR);
+
+// rows [r0, r0 + rows) of a kept tensor in the reference layout: complex [rows][nb][nb](3), or real [rows][nb][nb]
+int tensorToReference(tcscf_ctx * ctx, Tensor const & t, const DevSto * sto, int64_t r0, int64_t rows, double * out);
+int tensorAlloc(tcscf_ctx * ctx, Tensor & t, size_t bytes);
+void tensorRelease(tcscf_ctx * ctx, Tensor & t);
+
 // One contraction problem as the tensor kernel sees it (device pointers); a launch covers one or many
 // of them (batched builds), all with the same tile shapes NB, RP.
 struct TensorInstance {
@@ -151,9 +159,5 @@ int sumSplitsLaunch(tcscf_ctx * ctx, int64_t n, int nsplit, int64_t stride, cons
 // A symmetric contraction's T' gives M with G = M + M^T when cJ is halved (the Coulomb part is symmetric)
 int reduceFockReal(tcscf_ctx * ctx, int64_t n1, int nb, int nspin, const double * phi, const double * w1, const double * VH,
                    const double * cJ, const double * T, int64_t tStride, int ldt, double * out);
-
-// complex reduction G(j,i) = sum_r w[r] conj(A[r][j]) Y[r][i] with Y = cJ * A[r][i] * Faa[r] - Fai[r][i]
-int reduceFockComplex(tcscf_ctx * ctx, int64_t n1, int nb, const double * A, const double * w, const double * Faa, double cJ,
-                      const double * Fai, double * out);
 
 }  // namespace tcscf

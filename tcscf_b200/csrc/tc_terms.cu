@@ -330,25 +330,35 @@ __global__ void kRealToZ(int n, const double * in, double2 * out)
 }
 
 // ---- fused per-point build (nb <= kFusedMaxNb) -------------------------------------------------------
-// The kernels above keep every per-point intermediate in HBM and read the Fji / Vji tensors several
-// times over (once per intermediate, then again in the reduction, with each thread walking its own
-// point's rows).  kTcFused reads them once: one block of kFusedThreads per SM walks the r1 points
-// (p = block, block + grid, ...); a point's Vs, Vo ([nb][nb][3] complex), Fs, Fo ([nb][nb]) rows, basis
-// values and gradients arrive in shared memory by bulk copies (double-buffered when two points fit);
-// all intermediates of kTcPoint ... kTcSvd are formed there for both spins from that one copy, and
-// each thread adds the w-weighted scalar, vector and three-body terms of kTcReduce for its fixed
-// (spin, j, i) elements in registers.  The per-block sums go to part[block][3][2][nb][nb] and
-// kTcPartials adds them in block order (deterministic).  Same terms as kTcReduce, grouped per point:
-//   scalar  += conj(v_j) Pw(i)
-//   vector  += conj(v_j) Qw(i) + Vs(j,i).w SG_s + Vo(j,i).w SG_o - Vja_s(j).w g_i
-//   three   += conj(v_j) Rw(i) + Tw(j) v_i + 2w VTs(i).conj(VTs(j))
-//              - 2w occ_s sum_b Vjbs(j,b).conj(Vjbs(i,b)) - 2w occ_o sum_b Vjbo(j,b).conj(Vjbo(i,b))
-//              + Vs(j,i).w (2 occ_s VT_s - 2 SCV_s) + Vo(j,i).w (2 occ_o VT_o - 2 SCV_o)
-// with Pw = w (Faa v_i - Fai(i)), Qw = w (VT.g_i - Vai(i)), Rw = w ((|VT|^2 - sumNs_s - sumNo_o) v_i
-// + 2 (SVD(i) - VT.VTs(i))), Tw = 2w (conj(SVD(j)) - conj(VTs(j)).VT).
-constexpr int kFusedThreads = 512;
-constexpr int kFusedMaxNb = 32;   // 2 nb^2 elements over 512 threads: at most 4 register slots
+// The kernels above keep every per-point intermediate in HBM and read the tensors several times over.  kTcFused
+// reads them once, in the form they are kept in: real symmetric [nb][nb] planes in the real-harmonic
+// basis, where the basis values are real too and only densities, orbitals and gradients are complex
+// (every term pairs one conjugated and one plain index, so the sums transform back as one matrix each,
+// kSumsToReference).  A block walks the points p = block, block + grid, ...; one point's planes (Vs, Vo
+// components, Fs, Fo) arrive in shared memory by bulk copies while the block before them is still at its
+// outer products.  Everything that is a contraction runs on the FP64 tensor cores:
+//   (1) V(j,i) x_i for all vectors x at once (columns: sum_k D(k,i) v_k, sum_k D(i,k) v_k, sum_k D(k,i) g_k and the
+//       occupied orbitals of both spins), and Fs(j,i) x_i
+//   (2) the traces of the 8 planes with both densities: [8][nb^2] x [nb^2][4]
+//   (3) V(j,i) ell_i
+//   (4) the terms V(j,i) W linear in the planes, accumulated over the points: [nb (nb+1)/2][8] x [8][8]
+//   (5) the outer products of per-point vectors, accumulated over the points: per spin a [nb][K] x [K][nb] product
+//       for the scalar (K = 1 complex term), vector (4) and three-body sums (5 + 6 nel); k rows are re and im parts, the
+//       fragments of the real and the imaginary result plain 8-byte loads with the sign in A's weight.
+// The (spin, j tile) warps keep (5)'s accumulators, the others (4)'s, in registers over all points.  Terms, with
+// v, g the point's basis values and gradients, occ_s the occupied density:
+//   scalar  w v_j (Faa v_i - Fai_i)
+//   vector  w v_j (VT.g_i - Vai_i) - w Vja_j . g_i + w (Vs(j,i).SG_s + Vo(j,i).SG_o)
+//   three   w v_j ((|VT|^2 - sumN_s - sumN_o) v_i + 2 SVD_i - 2 VT.VTs_i) + 2w (conj(SVD_j) - conj(VTs_j).VT) v_i
+//           + 2w conj(VTs_j).VTs_i - 2w occ_s Vjbs_jb . conj(Vjbs_ib) - 2w occ_o Vjbo_jb . conj(Vjbo_ib)
+//           + w Vs(j,i).(2 occ_s VT_s - 2 SCV_s) + w Vo(j,i).(2 occ_o VT_o - 2 SCV_o)
+// The per-block sums go to part[block][3][2][nb][nb], added in block order.  Bound by the FP64 MMAs and the
+// barriers between the phases (two blocks per SM fill each other's): TCFUSED_FIGURES
+constexpr int kFusedMaxNb = 32;
 constexpr int kFusedWaitCode = 60;
+__host__ __device__ constexpr int fusedWarps(int ntb) { return ntb == 4 ? 16 : 8; }
+// column tiles (5) or row tiles (4) a warp accumulates
+__host__ __device__ constexpr int fusedElemTiles(int ntb) { return ntb == 1 ? 1 : (ntb == 2 ? 5 : (ntb == 3 ? 19 : 9)); }
 
 __device__ __forceinline__ double2 zfma(double2 a, double2 b, double2 c)   // a b + c
 {
@@ -358,452 +368,473 @@ __device__ __forceinline__ double2 zcfma(double2 a, double2 b, double2 c)  // co
 {
   return make_double2(fma(a.x, b.x, fma(a.y, b.y, c.x)), fma(a.x, b.y, fma(-a.y, b.x, c.y)));
 }
+__device__ __forceinline__ double2 zrfma(double a, double2 b, double2 c) { return make_double2(fma(a, b.x, c.x), fma(a, b.y, c.y)); }
 
-// shared-memory layout of kTcFused in double2 units (per-spin arrays are [2][...]); the same
-// arithmetic on the host sizes the launch
+// Shared-memory layout of kTcFused in doubles.  NB: the basis size rounded up to 4, the planes' row stride; every vector is
+// padded to it with zeros, so that the loops and offsets are constants.  What depends on the electron counts comes last
+template <int NB>
 struct FusedLayout {
-  int ldD, fU;
-  int D, C, kv, kc, kg, colF, colV, Fai, VTs, Vai, Vja, Vjb, nP, ell, sc, Pw, Qw, Rw, Tw, Xw, Jw, gw, ws;
-  int buf, bufStride, total;
-  __host__ __device__ FusedLayout(int nb, int nm, int fcx, int nbuf)
-  {
-    int const nn = nb * nb;
-    ldD = (nb & 1) ? nb : nb + 1;   // odd row stride: a warp walking a column of D hits distinct banks
-    fU = fcx ? nn : nn / 2;         // real Fji rows (nb even) take half the double2 slots
-    int o = 0;
-    D = o;    o += 2 * nb * ldD;     // D_s(i, j) at [s][i][j]
-    C = o;    o += 2 * nm * nb;      // C_s(i, b) at [s][b][i], zero for b >= nel[s]
-    kv = o;   o += 2 * nb;           // sum_k D(k, j) v_k
-    kc = o;   o += 2 * nb;           // sum_k D(j, k) conj(v_k)
-    kg = o;   o += 6 * nb;           // sum_k D(k, j) g_k
-    colF = o; o += 2 * nb;           // column i of the Faa trace
-    colV = o; o += 6 * nb;           // column i of the V-tilde trace
-    Fai = o;  o += 2 * nb;
-    VTs = o;  o += 6 * nb;
-    Vai = o;  o += 2 * nb;
-    Vja = o;  o += 6 * nb;
-    Vjb = o;  o += 12 * nb * nm;     // [s][tensor][j][b][3]
-    nP = o;   o += 4 * nm * nm;      // |sum_j conj(C(j,a)) Vjb(j,b)|^2 at [s][tensor][a][b] (.x)
-    ell = o;  o += 6 * nb;           // sum_l D(l, k) VTs(l)
-    sc = o;   o += 24;               // per spin: Faa, VT[3], SG[3], SCV[3], occ (.x), sumN (.x same, .y oppo)
-    Pw = o;   o += 2 * nb;
-    Qw = o;   o += 2 * nb;
-    Rw = o;   o += 2 * nb;
-    Tw = o;   o += 2 * nb;
-    Xw = o;   o += 6 * nb;
-    Jw = o;   o += 12 * nb * nm;
-    gw = o;   o += 3 * nb;
-    ws = o;   o += 24;               // per spin: w SG_s, w SG_o, w (2 occ_s VT_s - 2 SCV_s), w (2 occ_o VT_o - 2 SCV_o)
-    buf = o;
-    bufStride = 6 * nn + 2 * fU + 4 * nb;   // Vs, Vo, Fs, Fo, vals, grads
-    total = buf + nbuf * bufStride;
-  }
-  __host__ __device__ size_t bytes() const { return size_t(total) * sizeof(double2) + 32; }   // + 2 mbarriers, abort word
+  static constexpr int NTB = (NB + 7) / 8, NW = fusedWarps(NTB), PS = tensorPlane(NB), NS = 8 * NTB + 4;   // NS: complex per slot, two slots on different banks
+  static constexpr int planes = 0;                            // and zeros: fragments past a plane's last rows
+  static constexpr int D = planes + 8 * PS + 4 * 32 + 16;     // {D0, D1}(i, j) at 4 (i NB + j), zeros behind
+  static constexpr int X0 = D + 4 * (PS + 4);                 // {kv0, kv1, kc0, kc1} per row
+  static constexpr int KG = X0 + NB * 12 + 8;                 // {kg0, kg1} per component and row
+  static constexpr int EL = KG + 3 * (NB * 4 + 8);            // {ell0, ell1}
+  static constexpr int Pw = EL + 3 * (NB * 4 + 8);
+  static constexpr int Fai = Pw + 4 * NS;
+  static constexpr int vai = Fai + 4 * NB;                    // [spin][component][i]
+  static constexpr int SVD = vai + 12 * NB;
+  static constexpr int tp = SVD + 4 * NB;                     // trace partials [warp][plane][8]
+  static constexpr int tr = tp + NW * 64;                     // traces [plane][D0, D1]
+  static constexpr int sc = tr + 32;                          // per spin: SG[3], SCV[3], occ, sumN (same, opposite)
+  static constexpr int W = sc + 40;
+  static constexpr int g = W + 96;
+  static constexpr int v = g + 6 * NB;
+  static constexpr int slot = v + NB;
+  // per spin 16 + 6 max(nel) slots of NS complex: A 0..5, B 6..11, then the shared ones (VTs, Vjb, a zero); the occupied orbitals
+  // [NB][ldc], spin 0's columns then spin 1's, ldc = 4 mod 8
+  static int spinStride(int nel0, int nel1) { return 2 * NS * (16 + 6 * std::max(nel0, nel1)); }
+  static int ldc(int nel0, int nel1) { return (2 * (nel0 + nel1) + 7) / 8 * 8 + 4; }
+  static int total(int nel0, int nel1) { return slot + 2 * spinStride(nel0, nel1) + NB * ldc(nel0, nel1); }
+  static size_t bytes(int nel0, int nel1) { return size_t(total(nel0, nel1)) * sizeof(double) + 32; }   // + mbarrier, abort word
 };
 
 struct TcFusedArgs {
   int64_t n1;
-  int nb, nm, nbuf, fcx;
-  int nel[2];
-  const double * Fs;
+  int nb, nel[2];
+  int spinStride, ldc, CB, total;   // FusedLayout
+  const double * Fs;        // [n1][ps]
   const double * Fo;
-  const double2 * Vs;
-  const double2 * Vo;
-  const double2 * vals;
-  const double2 * grads;
+  const double * Vs;        // [n1][3][ps]
+  const double * Vo;
+  const double * phi;       // [n1][nb]
+  const double2 * grads;    // [n1][nb][3], reference basis
   const double * w;
-  const double2 * D;
-  const double2 * C0;
+  const DevSto * sto;
+  const double2 * D;        // [2][nb][nb], real-harmonic basis
+  const double2 * C0;       // occupied orbitals [nel][nb], reference basis
   const double2 * C1;
-  double2 * part;   // [gridDim.x][3][2][nb][nb]
+  double2 * part;           // [gridDim.x][3][2][nb][nb]
   int * status;
 };
 
-template <int SLOTS>
-__global__ void __launch_bounds__(kFusedThreads, 1) kTcFused(TcFusedArgs t)
+template <int NB>
+__global__ void __launch_bounds__(32 * FusedLayout<NB>::NW, FusedLayout<NB>::NTB == 4 ? 1 : 2) kTcFused(const __grid_constant__ TcFusedArgs t)
 {
-  extern __shared__ __align__(16) double2 sm[];
-  int const nb = t.nb, nn = nb * nb, nm = t.nm, tid = threadIdx.x;
-  FusedLayout const L(nb, nm, t.fcx, t.nbuf);
-  int const ld = L.ldD;
-  uint64_t * bars = reinterpret_cast<uint64_t *>(sm + L.total);
-  int * abortWord = reinterpret_cast<int *>(bars + 2);
+  using L = FusedLayout<NB>;
+  constexpr int NTB = L::NTB, NW = L::NW, PS = L::PS, NS = L::NS, NTH = 32 * NW, ET = fusedElemTiles(NTB), NACC = 6 * NTB > ET ? 6 * NTB : ET;
+  extern __shared__ __align__(16) double sm[];
+  int const nb = t.nb, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, fr = lane >> 2, fq = lane & 3;
+  uint64_t * bar = reinterpret_cast<uint64_t *>(sm + t.total);
+  int * abortWord = reinterpret_cast<int *>(bar + 1);
   double2 const zero = make_double2(0, 0);
+  auto z2 = [&](int o) -> double2 & { return *reinterpret_cast<double2 *>(sm + o); };
+  // complex entry i of a slot of spin s: A 0..5, B 6..11, shared 12.. (VTs 12 + c, Vjb 15 + (t nel + b) 3 + c)
+  auto slotAt = [&](int s, int k, int i) { return L::slot + s * t.spinStride + 2 * (k * NS + i); };
 
-  for (int e = tid; e < 2 * nn; e += kFusedThreads) {
-    int const s = e / nn, r = e - s * nn;
-    sm[L.D + (s * nb + r / nb) * ld + r % nb] = t.D[e];
+  for (int e = tid; e < t.total; e += NTH) sm[e] = 0.0;
+  __syncthreads();
+  for (int e = tid; e < 2 * nb * nb; e += NTH) {
+    int const s = e / (nb * nb), r = e - s * nb * nb;
+    z2(L::D + 4 * (r / nb * NB + r % nb) + 2 * s) = t.D[e];
   }
-  for (int e = tid; e < 2 * nm * nb; e += kFusedThreads) {
-    int const s = e / (nm * nb), b = (e / nb) % nm, i = e % nb;
-    sm[L.C + e] = b < t.nel[s] ? (s == 0 ? t.C0 : t.C1)[b * nb + i] : zero;
+  for (int e = tid; e < (t.nel[0] + t.nel[1]) * nb; e += NTH) {
+    // C_R(k, b) = sum_i conj(U[k][i]) C(i, b)
+    int const m = e / nb, k = e % nb;
+    const double2 * C = m < t.nel[0] ? t.C0 + m * nb : t.C1 + (m - t.nel[0]) * nb;
+    double2 c = zmul(zconj(uRow(t.sto, k, k)), C[k]);
+    if (t.sto[k].partner >= 0) c = zadd(c, zmul(zconj(uRow(t.sto, k, t.sto[k].partner)), C[t.sto[k].partner]));
+    z2(t.CB + k * t.ldc + 2 * m) = c;
   }
-  uint32_t const vBytes = uint32_t(nn) * 48u, fBytes = uint32_t(nn) * (t.fcx ? 16u : 8u);
-  uint32_t const txBytes = 2u * vBytes + 2u * fBytes + uint32_t(nb) * 64u;
-  auto issue = [&](int64_t p, int b) {
-    double2 * B = sm + L.buf + b * L.bufStride;
-    tc::mbarArriveTx(&bars[b], txBytes);
-    tc::bulkLoad(B, t.Vs + p * nn * 3, vBytes, &bars[b]);
-    tc::bulkLoad(B + 3 * nn, t.Vo + p * nn * 3, vBytes, &bars[b]);
-    tc::bulkLoad(B + 6 * nn, reinterpret_cast<const char *>(t.Fs) + p * fBytes, fBytes, &bars[b]);
-    tc::bulkLoad(B + 6 * nn + L.fU, reinterpret_cast<const char *>(t.Fo) + p * fBytes, fBytes, &bars[b]);
-    tc::bulkLoad(B + 6 * nn + 2 * L.fU, t.vals + p * nb, uint32_t(nb) * 16u, &bars[b]);
-    tc::bulkLoad(B + 6 * nn + 2 * L.fU + nb, t.grads + p * nb * 3, uint32_t(nb) * 48u, &bars[b]);
-  };
   if (tid == 0) {
-    tc::mbarInit(&bars[0], 1);
-    tc::mbarInit(&bars[1], 1);
+    tc::mbarInit(bar, 1);
     *abortWord = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  tc::fenceProxyAsync();   // the zeros above are written before the first copies land
   __syncthreads();
+  constexpr uint32_t pB = uint32_t(PS) * 8u;
+  auto issue = [&](int64_t p) {
+    tc::mbarArriveTx(bar, 8u * pB + uint32_t(nb) * 48u);
+    tc::bulkLoad(sm + L::planes, t.Vs + p * 3 * PS, 3 * pB, bar);
+    tc::bulkLoad(sm + L::planes + 3 * PS, t.Vo + p * 3 * PS, 3 * pB, bar);
+    tc::bulkLoad(sm + L::planes + 6 * PS, t.Fs + p * PS, pB, bar);
+    tc::bulkLoad(sm + L::planes + 7 * PS, t.Fo + p * PS, pB, bar);
+    tc::bulkLoad(sm + L::g, t.grads + p * nb * 3, uint32_t(nb) * 48u, bar);
+  };
   int const G = gridDim.x;
-  if (tid == 0) {
-    if (blockIdx.x < t.n1) issue(blockIdx.x, 0);
-    if (t.nbuf == 2 && blockIdx.x + G < t.n1) issue(blockIdx.x + G, 1);
-  }
+  if (tid == 0 && blockIdx.x < t.n1) issue(blockIdx.x);
 
-  double2 acc[SLOTS][3];
+  // roles of the accumulating phases: warps 0 .. 2 NTB - 1 hold (spin, j tile) outer products, the others row tiles of (4)
+  bool const outer = warp < 2 * NTB;
+  int const os = warp / NTB, oj = 8 * (warp % NTB) + fr;
+  constexpr int EW = NW - 2 * NTB;
+  int const np = nb * (nb + 1) / 2, ew = warp - 2 * NTB;
+  // offsets j NB + i of the upper-triangle elements this lane reads (row p of tile ew + q EW; rows past the last repeat it and
+  // are not written), two per register
+  uint32_t eoff[(ET + 1) / 2];
 #pragma unroll
-  for (int q = 0; q < SLOTS; ++q) acc[q][0] = acc[q][1] = acc[q][2] = zero;
+  for (int q = 0; q < ET; ++q) {
+    int p = min((ew + q * EW) * 8 + fr, np - 1), j = 0;
+    if (!outer)
+      while (p >= nb - j) { p -= nb - j; ++j; }
+    uint32_t const o = outer ? 0 : uint32_t(j * NB + j + p);
+    if (q & 1) eoff[q / 2] |= o << 16;
+    else eoff[q / 2] = o;
+  }
+  auto elem = [&](int q) { return int((eoff[q / 2] >> (q & 1 ? 16 : 0)) & 0xffffu); };
+  double acc[NACC][2];
+#pragma unroll
+  for (int q = 0; q < NACC; ++q) acc[q][0] = acc[q][1] = 0.0;
 
   int k = 0;
   for (int64_t p = blockIdx.x; p < t.n1; p += G, ++k) {
-    int const bi = k % t.nbuf;
-    bool const ok = tc::waitBar(&bars[bi], uint32_t(k / t.nbuf) & 1u, abortWord, t.status, kFusedWaitCode);
-    if (__syncthreads_or(!ok)) return;
-    const double2 * Vs = sm + L.buf + bi * L.bufStride;
-    const double2 * Vo = Vs + 3 * nn;
-    const double2 * F0 = Vo + 3 * nn;
-    const double2 * F1 = F0 + L.fU;
-    const double2 * vals = F1 + L.fU;
-    const double2 * grads = vals + nb;
-    auto F = [&](const double2 * base, int o) -> double2 {
-      return t.fcx ? base[o] : make_double2(reinterpret_cast<const double *>(base)[o], 0.0);
-    };
-
-    // phase 1: kv, kc, kg (per spin, j); the Faa and V-tilde traces by column; Vjb (per spin, tensor, b, j)
-    for (int it = tid; it < 8 * nb + 4 * nb * nm; it += kFusedThreads) {
-      int const grp = it / (2 * nb);
-      if (grp < 4) {
-        int const s = (it / nb) & 1, j = it % nb;
-        const double2 * Ds = sm + L.D + s * nb * ld;
-        const double2 * Do = sm + L.D + (1 - s) * nb * ld;
-        if (grp == 0) {
-          double2 kv = zero, kc = zero;
-          for (int kk = 0; kk < nb; ++kk) {
-            kv = zfma(Ds[kk * ld + j], vals[kk], kv);
-            kc = zfma(Ds[j * ld + kk], zconj(vals[kk]), kc);
-          }
-          sm[L.kv + s * nb + j] = kv;
-          sm[L.kc + s * nb + j] = kc;
-        } else if (grp == 1) {
-          double2 g0 = zero, g1 = zero, g2 = zero;
-          for (int kk = 0; kk < nb; ++kk) {
-            double2 const d = Ds[kk * ld + j];
-            g0 = zfma(d, grads[kk * 3], g0);
-            g1 = zfma(d, grads[kk * 3 + 1], g1);
-            g2 = zfma(d, grads[kk * 3 + 2], g2);
-          }
-          double2 * o = sm + L.kg + (s * nb + j) * 3;
-          o[0] = g0; o[1] = g1; o[2] = g2;
-        } else if (grp == 2) {
-          int const i = j;
-          double2 f = zero;
-          for (int jj = 0; jj < nb; ++jj) {
-            f = zfma(F(F0, jj * nb + i), Ds[i * ld + jj], f);
-            f = zfma(F(F1, jj * nb + i), Do[i * ld + jj], f);
-          }
-          sm[L.colF + s * nb + i] = f;
-        } else {
-          int const i = j;
-          double2 v0 = zero, v1 = zero, v2 = zero;
-          for (int jj = 0; jj < nb; ++jj) {
-            double2 const ds = Ds[i * ld + jj], dop = Do[i * ld + jj];
-            const double2 * a = Vs + (jj * nb + i) * 3;
-            const double2 * c = Vo + (jj * nb + i) * 3;
-            v0 = zfma(c[0], dop, zfma(a[0], ds, v0));
-            v1 = zfma(c[1], dop, zfma(a[1], ds, v1));
-            v2 = zfma(c[2], dop, zfma(a[2], ds, v2));
-          }
-          double2 * o = sm + L.colV + (s * nb + i) * 3;
-          o[0] = v0; o[1] = v1; o[2] = v2;
-        }
-      } else {
-        int const q = it - 8 * nb;
-        int const j = q % nb, b = (q / nb) % nm, st = q / (nb * nm), s = st >> 1, tt = st & 1;
-        double2 r0 = zero, r1 = zero, r2 = zero;
-        if (b < t.nel[s]) {
-          const double2 * V = tt ? Vo : Vs;
-          const double2 * Cb = sm + L.C + (s * nm + b) * nb;
-          for (int kk = 0; kk < nb; ++kk) {
-            int i = kk + j;   // each lane starts on its own column: rows j of a warp hit distinct banks
-            if (i >= nb) i -= nb;
-            double2 const c = Cb[i];
-            const double2 * v = V + (j * nb + i) * 3;
-            r0 = zfma(c, v[0], r0);
-            r1 = zfma(c, v[1], r1);
-            r2 = zfma(c, v[2], r2);
-          }
-        }
-        double2 * o = sm + L.Vjb + (((s * 2 + tt) * nb + j) * nm + b) * 3;
-        o[0] = r0; o[1] = r1; o[2] = r2;
-      }
-    }
-    __syncthreads();
-
-    // phase 2: Fai, VTs (per spin, i); Vai, Vja (per spin, i); occ, SG, Faa, VT (per spin); the |Vab|^2 terms
-    for (int it = tid; it < 4 * nb + 8 + 4 * nm * nm; it += kFusedThreads) {
-      if (it < 2 * nb) {
-        int const s = it / nb, i = it % nb;
-        double2 fa = zero, a0 = zero, a1 = zero, a2 = zero;
-        for (int j = 0; j < nb; ++j) {
-          double2 const kv = sm[L.kv + s * nb + j];
-          const double2 * v = Vs + (j * nb + i) * 3;
-          fa = zfma(kv, F(F0, j * nb + i), fa);
-          a0 = zfma(kv, v[0], a0);
-          a1 = zfma(kv, v[1], a1);
-          a2 = zfma(kv, v[2], a2);
-        }
-        sm[L.Fai + s * nb + i] = fa;
-        double2 * o = sm + L.VTs + (s * nb + i) * 3;
-        o[0] = a0; o[1] = a1; o[2] = a2;
-      } else if (it < 4 * nb) {
-        int const q = it - 2 * nb, s = q / nb, i = q % nb;
-        double2 c0 = zero, c1 = zero, c2 = zero, j0 = zero, j1 = zero, j2 = zero;
-        for (int jj = 0; jj < nb; ++jj) {
-          const double2 * kg = sm + L.kg + (s * nb + jj) * 3;
-          const double2 * v = Vs + (jj * nb + i) * 3;
-          c0 = zfma(v[0], kg[0], c0);
-          c1 = zfma(v[1], kg[1], c1);
-          c2 = zfma(v[2], kg[2], c2);
-          int j = jj + i;   // skewed walk along row i of Vs
-          if (j >= nb) j -= nb;
-          double2 const kc = sm[L.kc + s * nb + j];
-          const double2 * u = Vs + (i * nb + j) * 3;
-          j0 = zfma(kc, u[0], j0);
-          j1 = zfma(kc, u[1], j1);
-          j2 = zfma(kc, u[2], j2);
-        }
-        sm[L.Vai + s * nb + i] = zadd(zadd(c0, c1), c2);
-        double2 * o = sm + L.Vja + (s * nb + i) * 3;
-        o[0] = j0; o[1] = j1; o[2] = j2;
-      } else if (it < 4 * nb + 8) {
-        int const q = it - 4 * nb, s = q >> 2, which = q & 3;
-        double2 * S = sm + L.sc + s * 12;
-        if (which == 0) {
-          double2 oc = zero;
-          for (int kk = 0; kk < nb; ++kk) oc = zcfma(vals[kk], sm[L.kv + s * nb + kk], oc);
-          S[10] = make_double2(oc.x, 0.0);
-        } else if (which == 1) {
-          double2 g0 = zero, g1 = zero, g2 = zero;
-          for (int i = 0; i < nb; ++i) {
-            double2 const kc = sm[L.kc + s * nb + i];
-            g0 = zfma(kc, grads[i * 3], g0);
-            g1 = zfma(kc, grads[i * 3 + 1], g1);
-            g2 = zfma(kc, grads[i * 3 + 2], g2);
-          }
-          S[4] = g0; S[5] = g1; S[6] = g2;
-        } else if (which == 2) {
-          double2 f = zero;
-          for (int i = 0; i < nb; ++i) f = zadd(f, sm[L.colF + s * nb + i]);
-          S[0] = f;
-        } else {
-          double2 v0 = zero, v1 = zero, v2 = zero;
-          for (int i = 0; i < nb; ++i) {
-            const double2 * c = sm + L.colV + (s * nb + i) * 3;
-            v0 = zadd(v0, c[0]); v1 = zadd(v1, c[1]); v2 = zadd(v2, c[2]);
-          }
-          S[1] = v0; S[2] = v1; S[3] = v2;
-        }
-      } else {
-        int const q = it - 4 * nb - 8;
-        int const b = q % nm, a = (q / nm) % nm, st = q / (nm * nm), s = st >> 1, tt = st & 1;
-        double n = 0;
-        if (a < t.nel[s] && b < t.nel[s]) {
-          double2 r0 = zero, r1 = zero, r2 = zero;
-          for (int j = 0; j < nb; ++j) {
-            double2 const c = sm[L.C + (s * nm + a) * nb + j];
-            const double2 * v = sm + L.Vjb + (((s * 2 + tt) * nb + j) * nm + b) * 3;
-            r0 = zcfma(c, v[0], r0);
-            r1 = zcfma(c, v[1], r1);
-            r2 = zcfma(c, v[2], r2);
-          }
-          n = r0.x * r0.x + r0.y * r0.y + r1.x * r1.x + r1.y * r1.y + r2.x * r2.x + r2.y * r2.y;
-        }
-        sm[L.nP + q] = make_double2(n, 0.0);
-      }
-    }
-    __syncthreads();
-
-    // phase 3: ell (per spin, k), SCV (per spin), sum over a, b of the |Vab|^2 terms (per spin, tensor)
-    for (int it = tid; it < 2 * nb + 6; it += kFusedThreads) {
-      if (it < 2 * nb) {
-        int const s = it / nb, kk = it % nb;
-        const double2 * Ds = sm + L.D + s * nb * ld;
-        double2 e0 = zero, e1 = zero, e2 = zero;
-        for (int l = 0; l < nb; ++l) {
-          double2 const d = Ds[l * ld + kk];
-          const double2 * v = sm + L.VTs + (s * nb + l) * 3;
-          e0 = zfma(d, v[0], e0);
-          e1 = zfma(d, v[1], e1);
-          e2 = zfma(d, v[2], e2);
-        }
-        double2 * o = sm + L.ell + (s * nb + kk) * 3;
-        o[0] = e0; o[1] = e1; o[2] = e2;
-      } else if (it < 2 * nb + 2) {
-        int const s = it - 2 * nb;
-        double2 c0 = zero, c1 = zero, c2 = zero;
-        for (int kk = 0; kk < nb; ++kk) {
-          double2 const kv = sm[L.kv + s * nb + kk];
-          const double2 * v = sm + L.VTs + (s * nb + kk) * 3;
-          c0 = zcfma(v[0], kv, c0);
-          c1 = zcfma(v[1], kv, c1);
-          c2 = zcfma(v[2], kv, c2);
-        }
-        double2 * S = sm + L.sc + s * 12;
-        S[7] = c0; S[8] = c1; S[9] = c2;
-      } else {
-        int const q = it - 2 * nb - 2, s = q >> 1, tt = q & 1;
-        double n = 0;
-        for (int ab = 0; ab < nm * nm; ++ab) n += sm[L.nP + (s * 2 + tt) * nm * nm + ab].x;
-        double * S11 = reinterpret_cast<double *>(sm + L.sc + s * 12 + 11);
-        S11[tt] = n;
-      }
-    }
-    __syncthreads();
-
-    // phase 4: SVD and the w-scaled per-(spin, i) operands of the element sums; w g_i; the per-spin 3-vectors
+    double const vnew = tid < nb ? t.phi[p * nb + tid] : 0.0;
     double const w = t.w[p];
-    for (int it = tid; it < 3 * nb + 2; it += kFusedThreads) {
-      if (it < 2 * nb) {
-        int const s = it / nb, i = it % nb, o = 1 - s;
-        const double2 * S = sm + L.sc + s * 12;
-        const double2 * So = sm + L.sc + o * 12;
-        double2 s0 = zero, s1 = zero, s2 = zero;
-        for (int kk = 0; kk < nb; ++kk) {
-          const double2 * v = Vs + (kk * nb + i) * 3;
-          const double2 * e = sm + L.ell + (s * nb + kk) * 3;
-          s0 = zfma(v[0], e[0], s0);
-          s1 = zfma(v[1], e[1], s1);
-          s2 = zfma(v[2], e[2], s2);
+    bool const ok = tc::waitBar(bar, uint32_t(k) & 1u, abortWord, t.status, kFusedWaitCode);
+    if (tid < nb) {
+      // v; as a complex slot entry it is A 0 and 4 and B 5 of both spins
+      sm[L::v + tid] = vnew;
+      for (int s = 0; s < 2; ++s) sm[slotAt(s, 0, tid)] = sm[slotAt(s, 4, tid)] = sm[slotAt(s, 11, tid)] = vnew;
+    }
+    if (__syncthreads_or(!ok)) return;
+    const double2 * graw = reinterpret_cast<const double2 *>(sm + L::g);
+
+    // phase 0: kv, kc per spin; gradients in the real-harmonic basis (B 1..3).  A warp per vector, lane = i
+    for (int kind = warp; kind < 7; kind += NW) {
+      int const i = lane;
+      if (i >= nb) continue;
+      if (kind < 2) {
+        double2 a = zero;
+        const double * d = sm + L::D + 4 * i + 2 * kind;
+#pragma unroll
+        for (int kk = 0; kk < NB; ++kk) a = zrfma(sm[L::v + kk], *reinterpret_cast<const double2 *>(d + 4 * kk * NB), a);
+        z2(L::X0 + 12 * i + 2 * kind) = a;
+      } else if (kind < 4) {
+        double2 a = zero;
+        const double * d = sm + L::D + 4 * i * NB + 2 * (kind - 2);
+#pragma unroll 8
+        for (int kk = 0; kk < NB; ++kk) {
+          int l = kk + i;   // skewed: the lanes' rows of D fall on different banks
+          l = l >= NB ? l - NB : l;
+          a = zrfma(sm[L::v + l], *reinterpret_cast<const double2 *>(d + 4 * l), a);
         }
-        double2 const svd = zadd(zadd(s0, s1), s2);
-        double2 const vi = vals[i];
-        const double2 * g = grads + i * 3;
-        const double2 * vts = sm + L.VTs + (s * nb + i) * 3;
-        double2 vtg = zero, vtv = zero, cvv = zero;
+        z2(L::X0 + 12 * i + 4 + 2 * (kind - 2)) = a;
+      } else {
+        int const c = kind - 4, q = t.sto[i].partner;
+        double2 gr = zmul(uRow(t.sto, i, i), graw[3 * i + c]);
+        if (q >= 0) gr = zadd(gr, zmul(uRow(t.sto, i, q), graw[3 * q + c]));
+        z2(slotAt(0, 7 + c, i)) = gr;
+        z2(slotAt(1, 7 + c, i)) = gr;
+      }
+    }
+    __syncthreads();
+    // phase 1: kg per (spin, component), a warp each, lane = i
+    for (int it = warp; it < 6; it += NW) {
+      int const s = it / 3, c = it % 3;
+      if (lane >= nb) continue;
+      double2 a = zero;
+      const double * d = sm + L::D + 4 * lane + 2 * s;
+      const double * x = sm + slotAt(0, 7 + c, 0);
+#pragma unroll
+      for (int kk = 0; kk < NB; ++kk) a = zfma(*reinterpret_cast<const double2 *>(d + 4 * kk * NB), *reinterpret_cast<const double2 *>(x + 2 * kk), a);
+      z2(L::KG + c * (NB * 4 + 8) + 4 * lane + 2 * s) = a;
+    }
+    __syncthreads();
+    // phase 2: planes times vectors, one (plane, row tile) at a time, its fragments loaded once; then this warp's share of
+    // the traces
+    auto loadTile = [&](int plane, int jt, double (&A)[NB / 4]) {
+      const double * x = sm + L::planes + plane * PS + 8 * jt + fr + fq * NB;
+#pragma unroll
+      for (int u = 0; u < NB / 4; ++u) A[u] = x[4 * u * NB];
+    };
+    auto rowTile = [&](double const (&A)[NB / 4], int b, int ldb, double (&d)[2]) {
+      const double * x = sm + b + fq * ldb + fr;
+#pragma unroll
+      for (int u = 0; u < NB / 4; ++u) dmma(d, A[u], x[4 * u * ldb]);
+    };
+    for (int it = warp; it < 7 * NTB; it += NW) {
+      int const plane = it / NTB, jt = it % NTB, j = 8 * jt + fr;   // Vs 0..2, Vo 3..5, Fs 6: the costly ones first
+      bool const in = j < nb;
+      double A[NB / 4];
+      loadTile(plane, jt, A);
+      if (plane < 3) {
+        double d[2] = {0, 0}, e[2] = {0, 0};
+        rowTile(A, L::X0, 12, d);
+        rowTile(A, L::KG + plane * (NB * 4 + 8), 4, e);
+        if (in) {
+          // columns kv0, kv1: V-tilde_i of both spins; kc0, kc1: Vja
+          z2(fq < 2 ? slotAt(fq, 12 + plane, j) : slotAt(fq - 2, 1 + plane, j)) = make_double2(d[0], d[1]);
+          if (fq < 2) z2(L::vai + 2 * ((fq * 3 + plane) * NB + j)) = make_double2(e[0], e[1]);
+        }
+      } else if (plane == 6) {
+        double d[2] = {0, 0};
+        rowTile(A, L::X0, 12, d);
+        if (in && fq < 2) z2(L::Fai + 2 * (fq * NB + j)) = make_double2(d[0], d[1]);
+      }
+      if (plane < 6)
+        for (int n = 0; 8 * n + 4 < t.ldc; ++n) {
+          double d[2] = {0, 0};
+          rowTile(A, t.CB + 8 * n, t.ldc, d);
+          int const m = 4 * n + fq, s = m < t.nel[0] ? 0 : 1, b = s ? m - t.nel[0] : m;
+          if (in && m < t.nel[0] + t.nel[1]) z2(slotAt(s, 15 + (plane / 3 * t.nel[s] + b) * 3 + plane % 3, j)) = make_double2(d[0], d[1]);
+        }
+    }
+    {
+      double d[3][2] = {};
+      const double * A = sm + L::planes + fr * PS + fq + 4 * warp;
+      const double * B = sm + L::D + 4 * (fq + 4 * warp) + fr;
+      constexpr int KS = NB * NB / 4, EACH = (KS + NW - 1) / NW;
+#pragma unroll
+      for (int u = 0; u < EACH; ++u)
+        if ((u + 1) * NW <= KS || u * NW + warp < KS) dmma(d[u % 3], A[4 * NW * u], B[16 * NW * u]);
+      z2(L::tp + 64 * warp + 8 * fr + 2 * fq) = make_double2(d[0][0] + d[1][0] + d[2][0], d[0][1] + d[1][1] + d[2][1]);
+    }
+    __syncthreads();
+    // phase 3, a warp per item: ell per (spin, component), lane = k; sumN = sum_ab |sum_j conj(C(j,a)) Vjb(j,b)|^2 per (spin, tensor);
+    // SG and occ; SCV per spin; the traces
+    for (int it = warp; it < 14; it += NW) {
+      if (it < 6) {
+        int const s = it / 3, c = it % 3;
+        if (lane < nb) {
+          double2 a = zero;
+          const double * d = sm + L::D + 4 * lane + 2 * s;
+          const double * x = sm + slotAt(s, 12 + c, 0);
+#pragma unroll
+          for (int l = 0; l < NB; ++l) a = zfma(*reinterpret_cast<const double2 *>(d + 4 * l * NB), *reinterpret_cast<const double2 *>(x + 2 * l), a);
+          z2(L::EL + c * (NB * 4 + 8) + 4 * lane + 2 * s) = a;
+        }
+      } else if (it < 10) {
+        // rows: re and im of 4 orbitals a; columns: re and im of 4 of the 3 nel vectors Vjb(b, c)
+        int const s = (it - 6) >> 1, tt = (it - 6) & 1, ne = t.nel[s];
+        double sum = 0;
+        for (int a0 = 0; a0 < ne; a0 += 4)
+          for (int q0 = 0; q0 < 3 * ne; q0 += 4) {
+            double d[2] = {0, 0};
+            const double * A = sm + t.CB + 2 * ((s ? t.nel[0] : 0) + a0) + fr + fq * t.ldc;
+            const double * B = sm + slotAt(s, 15 + tt * 3 * ne + q0, 0) + (fr >> 1) * 2 * NS + (fr & 1) + 2 * fq;
+            bool const aIn = a0 + (fr >> 1) < ne, qIn = q0 + (fr >> 1) < 3 * ne;
+#pragma unroll
+            for (int u = 0; u < NB / 4; ++u) dmma(d, aIn ? A[4 * u * t.ldc] : 0.0, qIn ? B[8 * u] : 0.0);
+            // rows 2 a (C.re) and 2 a + 1 (C.im), this lane's column pair (V.re, V.im)
+            double const x = __shfl_down_sync(0xffffffffu, d[0], 4), y = __shfl_down_sync(0xffffffffu, d[1], 4);
+            double const re = d[0] + y, im = d[1] - x;
+            if (!(fr & 1)) sum += re * re + im * im;
+          }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (lane == 0) sm[L::sc + 20 * s + 14 + tt] = sum;
+      } else if (it < 13) {
+        // rows: kv0, kv1, kc0, kc1 (re, im); columns: the three components of g and v, or of VTs_s (re, im)
+        int const s = it - 11;   // -1: g
+        double d[2] = {0, 0};
+        const double * A = sm + L::X0 + 12 * fq + fr;
+        const double * B = fr < 6 ? sm + slotAt(s < 0 ? 0 : s, (s < 0 ? 7 : 12) + (fr >> 1), 0) + (fr & 1) + 2 * fq : sm + L::v + fq;
+        int const bs = fr < 6 ? 2 : 1;
+#pragma unroll
+        for (int u = 0; u < NB / 4; ++u) dmma(d, A[48 * u], fr == 7 ? 0.0 : B[4 * u * bs]);
+        double const x = __shfl_down_sync(0xffffffffu, d[0], 4), y = __shfl_down_sync(0xffffffffu, d[1], 4);
+        if (s < 0) {
+          if (fq < 3 && (fr == 4 || fr == 6)) z2(L::sc + 20 * ((fr - 4) >> 1) + 2 * fq) = make_double2(d[0] - y, d[1] + x);   // SG = kc g
+          if (fq == 3 && (fr == 0 || fr == 2)) sm[L::sc + 20 * (fr >> 1) + 12] = d[0];                                    // occ = Re kv v
+        } else if (fq < 3 && fr == 2 * s) z2(L::sc + 20 * s + 2 * (3 + fq)) = make_double2(d[0] + y, x - d[1]);              // SCV = conj(VTs) kv
+      } else {
+        double a = 0;
+        for (int u = 0; u < NW; ++u) a += sm[L::tp + 64 * u + 8 * (lane / 4) + lane % 4];
+        sm[L::tr + lane] = a;
+      }
+    }
+    __syncthreads();
+    // phase 4: V ell (the first warps); the weights of the terms linear in the planes (the last warp)
+    auto trace = [&](int plane, int s) { return z2(L::tr + 4 * plane + 2 * s); };
+    if (warp < NTB) {
+      double d[3][2] = {};
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        double A[NB / 4];
+        loadTile(c, warp, A);
+        rowTile(A, L::EL + c * (NB * 4 + 8), 4, d[c]);
+      }
+      int const j = 8 * warp + fr;
+      if (j < nb && fq < 2) z2(L::SVD + 2 * (fq * NB + j)) = make_double2(d[0][0] + d[1][0] + d[2][0], d[0][1] + d[1][1] + d[2][1]);
+    } else if (warp == NW - 1 && lane < 24) {
+      // W[plane][spin, vector / three, re / im] at 12 plane + 4 spin + 2 kind
+      int const plane = lane >> 2, s = (lane >> 1) & 1, kind = lane & 1, c = plane % 3, u = plane < 3 ? s : 1 - s;
+      double2 x = z2(L::sc + 20 * u + 2 * c);
+      if (kind) {
+        double2 const vt = zadd(trace(c, u), trace(3 + c, 1 - u)), scv = z2(L::sc + 20 * u + 2 * (3 + c));
+        double const oc = sm[L::sc + 20 * u + 12];
+        x = make_double2(2.0 * oc * vt.x - 2.0 * scv.x, 2.0 * oc * vt.y - 2.0 * scv.y);
+      }
+      z2(L::W + 12 * plane + 4 * s + 2 * kind) = zscale(w, x);
+    }
+    __syncthreads();
+    // phase 5: the vectors of the outer products (the outer-product warps); the terms linear in the planes (the others)
+    if (outer) {
+      for (int it = warp; it < 8; it += 2 * NTB) {
+        int const kind = it >> 1, s = it & 1, i = lane, u = 1 - s;
+        if (i >= nb) continue;
+        double const vi = sm[L::v + i];
+        double2 const svd = z2(L::SVD + 2 * (s * NB + i));
+        double2 x = zero;
+        if (kind == 0) {
+          double2 const faa = zadd(trace(6, s), trace(7, u));
+          x = zsub(zscale(vi, faa), z2(L::Fai + 2 * (s * NB + i)));
+          z2(L::Pw + 2 * (s * NS + i)) = x;
+          continue;
+        }
         double nvt = 0;
         for (int c = 0; c < 3; ++c) {
-          vtg = zfma(S[1 + c], g[c], vtg);
-          vtv = zfma(S[1 + c], vts[c], vtv);
-          cvv = zcfma(vts[c], S[1 + c], cvv);
-          nvt += S[1 + c].x * S[1 + c].x + S[1 + c].y * S[1 + c].y;
+          double2 const vt = zadd(trace(c, s), trace(3 + c, u)), vts = z2(slotAt(s, 12 + c, i));
+          if (kind == 1) x = zsub(zfma(vt, z2(slotAt(0, 7 + c, i)), x), z2(L::vai + 2 * ((s * 3 + c) * NB + i)));
+          else if (kind == 2) { x = zfma(vt, vts, x); nvt += vt.x * vt.x + vt.y * vt.y; }
+          else x = zcfma(vts, vt, x);
         }
-        double const coef = nvt - S[11].x - So[11].y;
-        sm[L.Pw + s * nb + i] = zscale(w, zsub(zmul(S[0], vi), sm[L.Fai + s * nb + i]));
-        sm[L.Qw + s * nb + i] = zscale(w, zsub(vtg, sm[L.Vai + s * nb + i]));
-        sm[L.Rw + s * nb + i] = zscale(w, zadd(zscale(coef, vi), zscale(2.0, zsub(svd, vtv))));
-        sm[L.Tw + s * nb + i] = zscale(2.0 * w, zsub(zconj(svd), cvv));
-        for (int c = 0; c < 3; ++c) sm[L.Xw + (s * nb + i) * 3 + c] = zscale(2.0 * w, vts[c]);
-        for (int tt = 0; tt < 2; ++tt) {
-          double const f = -2.0 * w * (tt ? So[10].x : S[10].x);
-          for (int b = 0; b < nm; ++b) {
-            int const o3 = (((s * 2 + tt) * nb + i) * nm + b) * 3;
-            for (int c = 0; c < 3; ++c) sm[L.Jw + o3 + c] = zscale(f, sm[L.Vjb + o3 + c]);
-          }
-        }
-      } else if (it < 3 * nb) {
-        int const i = it - 2 * nb;
-        for (int c = 0; c < 3; ++c) sm[L.gw + i * 3 + c] = zscale(-w, grads[i * 3 + c]);
-      } else {
-        int const s = it - 3 * nb, o = 1 - s;
-        const double2 * S = sm + L.sc + s * 12;
-        const double2 * So = sm + L.sc + o * 12;
-        double2 * W = sm + L.ws + s * 12;
-        for (int c = 0; c < 3; ++c) {
-          W[c] = zscale(w, S[4 + c]);
-          W[3 + c] = zscale(w, So[4 + c]);
-          W[6 + c] = zscale(w, zsub(zscale(2.0 * S[10].x, S[1 + c]), zscale(2.0, S[7 + c])));
-          W[9 + c] = zscale(w, zsub(zscale(2.0 * So[10].x, So[1 + c]), zscale(2.0, So[7 + c])));
-        }
+        if (kind == 1) z2(slotAt(s, 6, i)) = x;                                                  // B 0
+        else if (kind == 2) {
+          double const coef = nvt - sm[L::sc + 20 * s + 14] - sm[L::sc + 20 * u + 15];
+          z2(slotAt(s, 10, i)) = zadd(make_double2(coef * vi, 0.0), zscale(2.0, zsub(svd, x)));   // B 4
+        } else z2(slotAt(s, 5, i)) = zsub(zconj(svd), x);                                        // A 5
+      }
+    } else {
+      double const b0 = sm[L::W + 12 * fq + fr], b1 = sm[L::W + 12 * (4 + fq) + fr];
+      const double * A = sm + L::planes + fq * PS;
+#pragma unroll
+      for (int q = 0; q < ET; ++q) {
+        dmma(acc[q], A[elem(q)], b0);
+        dmma(acc[q], A[4 * PS + elem(q)], b1);
       }
     }
     __syncthreads();
-
-    // phase 5: this thread's (spin, j, i) elements
+    // the planes and raw gradients are free: the next point's copies run under the outer products
+    if (tid == 0 && p + G < t.n1) {
+      tc::fenceProxyAsync();
+      issue(p + G);
+    }
+    // phase 6: outer products.  k step u: terms 2 u + (fq >> 1), part fq & 1; offsets in doubles
+    if (outer) {
+      int const part = fq & 1, half = fq >> 1, ne = t.nel[os];
+      double const occS = sm[L::sc + 20 * os + 12], occO = sm[L::sc + 20 * (1 - os) + 12];
+      auto step = [&](int o, int a, int b, double fre, double fim) {
+        double const x = sm[a], xr = fre * x, xi = fim * x;
 #pragma unroll
-    for (int q = 0; q < SLOTS; ++q) {
-      int const e = tid + q * kFusedThreads;
-      if (e < 2 * nn) {
-        int const s = e / nn, r = e - s * nn, j = r / nb, i = r - j * nb;
-        const double2 * vs = Vs + r * 3;
-        const double2 * vo = Vo + r * 3;
-        const double2 * W = sm + L.ws + s * 12;
-        const double2 * vja = sm + L.Vja + (s * nb + j) * 3;
-        const double2 * gw = sm + L.gw + i * 3;
-        const double2 * xw = sm + L.Xw + (s * nb + i) * 3;
-        const double2 * vtj = sm + L.VTs + (s * nb + j) * 3;
-        double2 const vj = vals[j], vi = vals[i];
-        acc[q][0] = zcfma(vj, sm[L.Pw + s * nb + i], acc[q][0]);
-        double2 ve = zcfma(vj, sm[L.Qw + s * nb + i], acc[q][1]);
-        double2 s3 = zcfma(vj, sm[L.Rw + s * nb + i], acc[q][2]);
-        s3 = zfma(sm[L.Tw + s * nb + j], vi, s3);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          double2 const a = vs[c], b = vo[c];
-          ve = zfma(a, W[c], ve);
-          ve = zfma(b, W[3 + c], ve);
-          ve = zfma(vja[c], gw[c], ve);
-          s3 = zfma(a, W[6 + c], s3);
-          s3 = zfma(b, W[9 + c], s3);
-          s3 = zfma(xw[c], zconj(vtj[c]), s3);
+        for (int n = 0; n < NTB; ++n) {
+          dmma(acc[(2 * o) * NTB + n], xr, sm[b + 16 * n + part]);
+          dmma(acc[(2 * o + 1) * NTB + n], xi, sm[b + 16 * n + 1 - part]);
         }
-        for (int tt = 0; tt < 2; ++tt)
-          for (int b = 0; b < t.nel[s]; ++b) {
-            const double2 * jw = sm + L.Jw + (((s * 2 + tt) * nb + j) * nm + b) * 3;
-            const double2 * vb = sm + L.Vjb + (((s * 2 + tt) * nb + i) * nm + b) * 3;
-            s3 = zfma(jw[0], zconj(vb[0]), s3);
-            s3 = zfma(jw[1], zconj(vb[1]), s3);
-            s3 = zfma(jw[2], zconj(vb[2]), s3);
-          }
-        acc[q][1] = ve;
-        acc[q][2] = s3;
+      };
+      int const aj = slotAt(os, 0, oj) + part, bi = slotAt(os, 6, fr), term = 2 * NS;
+      double const sgn = part ? -1.0 : 1.0;   // of the real part of a plain product
+      step(0, aj, L::Pw + 2 * (os * NS + fr), half ? 0.0 : sgn * w, half ? 0.0 : w);            // scalar: v Pw
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {                                                             // vector: v Qw, -Vja g
+        double const f = u == 0 && half == 0 ? w : -w;
+        step(1, aj + (2 * u + half) * term, bi + (2 * u + half) * term, sgn * f, f);
+      }
+      {                                                                                          // three: v Rw, 2 Tw v
+        double const f = half ? 2.0 * w : w;
+        step(2, aj + (4 + half) * term, bi + (4 + half) * term, sgn * f, f);
+      }
+      int const sj = slotAt(os, 12, oj) + part, si = slotAt(os, 12, fr), last = 3 + 6 * ne;
+      for (int u = 0; u < last; u += 2) {
+        // conj(VTs_j) VTs_i (a conjugated), Vjb_j conj(Vjb_i) (b conjugated), then the zero slot
+        int const q = u + half;
+        double const f = q < 3 ? 2.0 * w : (q < last ? -2.0 * w * (q < 3 + 3 * ne ? occS : occO) : 0.0);
+        step(2, sj + q * term, si + q * term, f, (q < 3) == (part == 1) ? -f : f);
       }
     }
-    __syncthreads();   // the buffer and the intermediates are free again
-    int64_t const next = p + int64_t(t.nbuf) * G;
-    if (tid == 0 && next < t.n1) issue(next, bi);
+    // the next point's first writes (v in A 0, A 4, B 5) must not overtake phase 6
+    __syncthreads();
   }
-  double2 * out = t.part + int64_t(blockIdx.x) * 6 * nn;
+
+  // the sums linear in the planes to shared memory (both triangles), added by the warps that hold the outer products
+  double * E = sm + L::planes;   // [8][PS], every copy has landed and been consumed
+  if (!outer) {
 #pragma unroll
-  for (int q = 0; q < SLOTS; ++q) {
-    int const e = tid + q * kFusedThreads;
-    if (e < 2 * nn) {
-      out[e] = acc[q][0];
-      out[2 * nn + e] = acc[q][1];
-      out[4 * nn + e] = acc[q][2];
+    for (int q = 0; q < ET; ++q) {
+      int const r = (ew + q * EW) * 8 + fr;
+      if (r >= np) continue;
+      int const j = elem(q) / NB, i = elem(q) % NB;
+      for (int e = 0; e < 2; ++e) E[(2 * fq + e) * PS + j * NB + i] = E[(2 * fq + e) * PS + i * NB + j] = acc[q][e];
     }
   }
+  __syncthreads();
+  if (!outer || oj >= nb) return;
+  int const nn = nb * nb;
+  double2 * out = t.part + int64_t(blockIdx.x) * 6 * nn + os * nn + oj * nb;
+#pragma unroll
+  for (int n = 0; n < NTB; ++n)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      int const i = 8 * n + 2 * fq + e;
+      if (i >= nb) continue;
+      const double * x = E + 4 * os * PS + oj * NB + i;
+      out[i] = make_double2(acc[n][e], acc[NTB + n][e]);
+      out[2 * nn + i] = make_double2(acc[2 * NTB + n][e] + x[0], acc[3 * NTB + n][e] + x[PS]);
+      out[4 * nn + i] = make_double2(acc[4 * NTB + n][e] + x[2 * PS], acc[5 * NTB + n][e] + x[3 * PS]);
+    }
 }
 
-// out[e] = sum over blocks of part[block][e], e < n, in block order
-__global__ void kTcPartials(int nparts, int n, const double2 * part, double2 * out)
+// out[e] = sum over blocks of part[block][e], e < n: 32 elements per block, 8 warps taking every eighth part each, added in warp order
+__global__ void __launch_bounds__(256) kTcPartials(int nparts, int n, const double2 * part, double2 * out)
 {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-    double2 a = make_double2(0, 0);
-    for (int b = 0; b < nparts; ++b) a = zadd(a, part[int64_t(b) * n + e]);
-    out[e] = a;
+  __shared__ double2 red[8][32];
+  int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5, e = blockIdx.x * 32 + lane;
+  double2 a = make_double2(0, 0);
+  if (e < n)
+#pragma unroll 4
+    for (int b = warp; b < nparts; b += 8) a = zadd(a, part[int64_t(b) * n + e]);
+  red[warp][lane] = a;
+  __syncthreads();
+  if (warp != 0 || e >= n) return;
+  for (int k = 1; k < 8; ++k) a = zadd(a, red[k][lane]);
+  out[e] = a;
+}
+
+// X(j,i) = sum_{k,l} U[k][j] XR(k,l) conj(U[l][i]) of `count` complex matrices
+__global__ void kSumsToReference(int count, int nb, const DevSto * s, const double2 * XR, double2 * X)
+{
+  int const nn = nb * nb;
+  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < count * nn; idx += gridDim.x * blockDim.x) {
+    int const m = idx / nn, j = idx % nn / nb, i = idx % nb;
+    int const kj[2] = {j, s[j].partner}, li[2] = {i, s[i].partner};
+    double2 acc = make_double2(0, 0);
+    for (int a = 0; a < 2; ++a)
+      for (int b = 0; b < 2; ++b)
+        if (kj[a] >= 0 && li[b] >= 0)
+          acc = zadd(acc, zmul(zmul(uRow(s, kj[a], j), XR[m * nn + kj[a] * nb + li[b]]), zconj(uRow(s, li[b], i))));
+    X[idx] = acc;
   }
 }
 
-template <int SLOTS>
-int launchFused(tcscf_ctx * ctx, TcFusedArgs const & a, int grid, size_t smem)
+// bytes of shared memory, or the launch, of kTcFused for this basis size
+template <int NB>
+int launchFused(tcscf_ctx * ctx, TcFusedArgs a, int grid)
 {
-  TCSCF_CUDA(ctx, cudaFuncSetAttribute(kTcFused<SLOTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-  kTcFused<SLOTS><<<grid, kFusedThreads, smem, ctx->stream>>>(a);
+  using L = FusedLayout<NB>;
+  a.spinStride = L::spinStride(a.nel[0], a.nel[1]);
+  a.ldc = L::ldc(a.nel[0], a.nel[1]);
+  a.CB = L::slot + 2 * a.spinStride;
+  a.total = L::total(a.nel[0], a.nel[1]);
+  size_t const smem = L::bytes(a.nel[0], a.nel[1]);
+  TCSCF_CUDA(ctx, cudaFuncSetAttribute(kTcFused<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  kTcFused<NB><<<grid, 32 * L::NW, smem, ctx->stream>>>(a);
   TCSCF_LAUNCH(ctx);
   return TCSCF_OK;
+}
+template <class F>
+auto fusedDispatch(int nb, F && f)
+{
+  switch ((nb + 3) / 4) {
+    case 1: return f(std::integral_constant<int, 4>{});
+    case 2: return f(std::integral_constant<int, 8>{});
+    case 3: return f(std::integral_constant<int, 12>{});
+    case 4: return f(std::integral_constant<int, 16>{});
+    case 5: return f(std::integral_constant<int, 20>{});
+    case 6: return f(std::integral_constant<int, 24>{});
+    case 7: return f(std::integral_constant<int, 28>{});
+    default: return f(std::integral_constant<int, 32>{});
+  }
 }
 
 Tensor const * findTensor(tcscf_ctx * ctx, int id)
@@ -847,40 +878,40 @@ int tcFockBuildDevice(tcscf_ctx * ctx, TcInputs const & in, int nup, int ndown, 
   int const nb = g.nb, nm = std::max(1, std::max(nup, ndown));
   int64_t const n1 = g.n;
   *hostStatus = 0;
-  int const fcx = in.F[0]->isComplex;
-  int nbuf = 0;
-  if (nb <= kFusedMaxNb && (fcx || nb % 2 == 0)) {
-    int optin = 0;
+  int const ntb = (nb + 7) / 8;
+  size_t smem = 0;
+  int optin = 0;
+  if (nb <= kFusedMaxNb) {
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
-    for (int q = 2; q >= 1 && !nbuf; --q)
-      if (FusedLayout(nb, nm, fcx, q).bytes() <= size_t(optin)) nbuf = q;
+    smem = fusedDispatch(nb, [&](auto n) { return FusedLayout<decltype(n)::value>::bytes(nup, ndown); });
   }
-  if (nbuf) {
+  if (smem > 0 && smem <= size_t(optin)) {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-    int const grid = int(std::max<int64_t>(1, std::min<int64_t>(sms, n1)));
-    size_t const nn6 = 6 * size_t(nb) * nb;
+    // two blocks per SM where shared memory allows (1 KB of each block's share is the system's)
+    int const perSm = ntb < 4 && 2 * (smem + 1024) <= 228 * 1024 ? 2 : 1;
+    int const grid = int(std::max<int64_t>(1, std::min<int64_t>(int64_t(sms) * perSm, n1)));
+    size_t const nn = size_t(nb) * nb, nn6 = 6 * nn;
     void * p = nullptr;
-    TCSCF_TRY(scratch(ctx, "tc_fused", sizeof(double2) * nn6 * (size_t(grid) + 1) + 256, &p));
+    TCSCF_TRY(scratch(ctx, "tc_fused", sizeof(double2) * (nn6 * (size_t(grid) + 2) + 2 * nn) + 256, &p));
     double2 * part = static_cast<double2 *>(p);
-    double2 * sums = part + nn6 * grid;
-    int * dStatus = reinterpret_cast<int *>(sums + nn6);
+    double2 * sumsR = part + nn6 * grid;
+    double2 * sums = sumsR + nn6;
+    double2 * DR = sums + nn6;
+    int * dStatus = reinterpret_cast<int *>(DR + 2 * nn);
     TCSCF_CUDA(ctx, cudaMemsetAsync(dStatus, 0, sizeof(int), ctx->stream));
+    for (int s = 0; s < 2; ++s) TCSCF_TRY(densityToRealLaunch(ctx, nb, g.dsto, dD + s * nn, DR + s * nn));
     TcFusedArgs a{};
-    a.n1 = n1; a.nb = nb; a.nm = nm; a.nbuf = nbuf; a.fcx = fcx;
+    a.n1 = n1; a.nb = nb;
     a.nel[0] = nup; a.nel[1] = ndown;
-    a.Fs = in.F[0]->d; a.Fo = in.F[1]->d;
-    a.Vs = reinterpret_cast<const double2 *>(in.V[0]->d); a.Vo = reinterpret_cast<const double2 *>(in.V[1]->d);
-    a.vals = reinterpret_cast<const double2 *>(g.vals); a.grads = reinterpret_cast<const double2 *>(g.grads); a.w = g.w;
-    a.D = dD; a.C0 = dC0; a.C1 = dC1;
+    a.Fs = in.F[0]->d; a.Fo = in.F[1]->d; a.Vs = in.V[0]->d; a.Vo = in.V[1]->d;
+    a.phi = g.phiR; a.grads = reinterpret_cast<const double2 *>(g.grads); a.w = g.w; a.sto = g.dsto;
+    a.D = DR; a.C0 = dC0; a.C1 = dC1;
     a.part = part; a.status = dStatus;
-    size_t const smem = FusedLayout(nb, nm, fcx, nbuf).bytes();
-    int const slots = (2 * nb * nb + kFusedThreads - 1) / kFusedThreads;
-    if (slots <= 1) TCSCF_TRY(launchFused<1>(ctx, a, grid, smem));
-    else if (slots == 2) TCSCF_TRY(launchFused<2>(ctx, a, grid, smem));
-    else if (slots == 3) TCSCF_TRY(launchFused<3>(ctx, a, grid, smem));
-    else TCSCF_TRY(launchFused<4>(ctx, a, grid, smem));
-    kTcPartials<<<gridBlocks(int64_t(nn6), 256), 256, 0, ctx->stream>>>(grid, int(nn6), part, sums);
+    TCSCF_TRY(fusedDispatch(nb, [&](auto n) { return launchFused<decltype(n)::value>(ctx, a, grid); }));
+    kTcPartials<<<unsigned((nn6 + 31) / 32), 256, 0, ctx->stream>>>(grid, int(nn6), part, sumsR);
+    TCSCF_LAUNCH(ctx);
+    kSumsToReference<<<gridBlocks(int64_t(nn6), 256), 256, 0, ctx->stream>>>(6, nb, g.dsto, sumsR, sums);
     TCSCF_LAUNCH(ctx);
     kTcAssemble<<<gridBlocks(2 * nb * nb, 256), 256, 0, ctx->stream>>>(nb, sums, dH, respectSym, dG2, dG3);
     TCSCF_LAUNCH(ctx);
@@ -888,39 +919,60 @@ int tcFockBuildDevice(tcscf_ctx * ctx, TcInputs const & in, int nup, int ndown, 
     TCSCF_CUDA(ctx, cudaMemcpyAsync(hostStatus, dStatus, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     return TCSCF_OK;
   }
+  // larger bases: the tensors in the reference's layout, a chunk of points (at most 1 GiB of them) at a time
+  size_t const nn = size_t(nb) * nb, fElem = in.F[0]->isComplex ? 2 : 1;
+  size_t const perRow = sizeof(double) * nn * (2 * fElem + 12);
+  int64_t const chunk = std::max<int64_t>(1, std::min<int64_t>(n1, int64_t((size_t(1) << 30) / perRow)));
+  int const chunks = int((n1 + chunk - 1) / chunk);
   size_t const perPoint = 1 + nb + 3 + 3 + nb + 3 * nb + 3 * nb + 2 * 3 * size_t(nb) * nm + nb + 3;   // double2 units
-  size_t const bytes = sizeof(double2) * (2 * size_t(n1) * perPoint + 6 * size_t(nb) * nb) + sizeof(double) * 2 * 3 * size_t(n1) + 1024;
+  size_t const bytes = sizeof(double2) * (2 * size_t(chunk) * perPoint + 6 * nn * (size_t(chunks) + 1)) + sizeof(double) * 2 * 3 * size_t(chunk) +
+                       perRow * chunk + 1024;
   void * p = nullptr;
   TCSCF_TRY(scratch(ctx, "tc_terms", bytes, &p));
   double2 * z = static_cast<double2 *>(p);
   auto take = [&](size_t n) { double2 * r = z; z += n; return r; };
+  size_t const n2 = 2 * size_t(chunk);
   TcView t{};
-  t.n1 = n1; t.nb = nb; t.nelMax = nm; t.nel[0] = nup; t.nel[1] = ndown;
+  t.nb = nb; t.nelMax = nm; t.nel[0] = nup; t.nel[1] = ndown;
   t.fcx = in.F[0]->isComplex;
-  t.Fs = in.F[0]->d; t.Fo = in.F[1]->d;
-  t.Vs = reinterpret_cast<const double2 *>(in.V[0]->d); t.Vo = reinterpret_cast<const double2 *>(in.V[1]->d);
-  t.vals = reinterpret_cast<const double2 *>(g.vals); t.grads = reinterpret_cast<const double2 *>(g.grads); t.w = g.w;
   t.D = dD; t.C0 = dC0; t.C1 = dC1;
-  size_t const n2 = 2 * size_t(n1);
+  double2 * V[2] = {take(size_t(chunk) * nn * 3), take(size_t(chunk) * nn * 3)};
+  t.Vs = V[0]; t.Vo = V[1];
   t.Faa = take(n2); t.Fai = take(n2 * nb); t.VT = take(n2 * 3); t.SG = take(n2 * 3);
   t.Vai = take(n2 * nb); t.Vja = take(n2 * nb * 3); t.VTs = take(n2 * nb * 3);
   t.Vjbs = take(n2 * nb * nm * 3); t.Vjbo = take(n2 * nb * nm * 3); t.SVD = take(n2 * nb); t.SCV = take(n2 * 3);
-  double2 * sums = take(6 * size_t(nb) * nb);
+  double2 * part = take(6 * nn * chunks);
+  double2 * sums = take(6 * nn);
   double * dr = reinterpret_cast<double *>(z);
   t.occD = dr; t.sumNs = dr + n2; t.sumNo = dr + 2 * n2;
-  TCSCF_CHECK(ctx, reinterpret_cast<char *>(dr + 3 * n2) <= static_cast<char *>(p) + bytes, TCSCF_ERR_INVALID_ARGUMENT, "internal: tc scratch");
-
-  kTcPoint<<<gridBlocks(2 * n1, 128), 128, 0, ctx->stream>>>(t);
-  TCSCF_LAUNCH(ctx);
-  kTcPointI<<<gridBlocks(2 * n1 * nb, 128), 128, 0, ctx->stream>>>(t);
-  TCSCF_LAUNCH(ctx);
-  kTcVjb<<<gridBlocks(2 * n1 * nb * nm, 128), 128, 0, ctx->stream>>>(t);
-  TCSCF_LAUNCH(ctx);
-  kTcVab<<<gridBlocks(2 * n1, 128), 128, 0, ctx->stream>>>(t);
-  TCSCF_LAUNCH(ctx);
-  kTcSvd<<<gridBlocks(2 * n1 * nb, 128), 128, 0, ctx->stream>>>(t);
-  TCSCF_LAUNCH(ctx);
-  kTcReduce<<<unsigned(2 * nb * nb), 256, 0, ctx->stream>>>(t, sums);
+  double * F[2] = {dr + 3 * n2, dr + 3 * n2 + size_t(chunk) * nn * fElem};
+  t.Fs = F[0]; t.Fo = F[1];
+  TCSCF_CHECK(ctx, reinterpret_cast<char *>(F[1] + size_t(chunk) * nn * fElem) <= static_cast<char *>(p) + bytes, TCSCF_ERR_INVALID_ARGUMENT,
+              "internal: tc scratch");
+  for (int c = 0; c < chunks; ++c) {
+    int64_t const r0 = c * chunk, rows = std::min(chunk, n1 - r0);
+    for (int k = 0; k < 2; ++k) {
+      TCSCF_TRY(tensorToReference(ctx, *in.F[k], g.dsto, r0, rows, F[k]));
+      TCSCF_TRY(tensorToReference(ctx, *in.V[k], g.dsto, r0, rows, reinterpret_cast<double *>(V[k])));
+    }
+    t.n1 = rows;
+    t.vals = reinterpret_cast<const double2 *>(g.vals) + r0 * nb;
+    t.grads = reinterpret_cast<const double2 *>(g.grads) + r0 * nb * 3;
+    t.w = g.w + r0;
+    kTcPoint<<<gridBlocks(2 * rows, 128), 128, 0, ctx->stream>>>(t);
+    TCSCF_LAUNCH(ctx);
+    kTcPointI<<<gridBlocks(2 * rows * nb, 128), 128, 0, ctx->stream>>>(t);
+    TCSCF_LAUNCH(ctx);
+    kTcVjb<<<gridBlocks(2 * rows * nb * nm, 128), 128, 0, ctx->stream>>>(t);
+    TCSCF_LAUNCH(ctx);
+    kTcVab<<<gridBlocks(2 * rows, 128), 128, 0, ctx->stream>>>(t);
+    TCSCF_LAUNCH(ctx);
+    kTcSvd<<<gridBlocks(2 * rows * nb, 128), 128, 0, ctx->stream>>>(t);
+    TCSCF_LAUNCH(ctx);
+    kTcReduce<<<unsigned(2 * nb * nb), 256, 0, ctx->stream>>>(t, part + 6 * nn * c);
+    TCSCF_LAUNCH(ctx);
+  }
+  kTcPartials<<<unsigned((6 * nn + 31) / 32), 256, 0, ctx->stream>>>(chunks, int(6 * nn), part, sums);
   TCSCF_LAUNCH(ctx);
   kTcAssemble<<<gridBlocks(2 * nb * nb, 256), 256, 0, ctx->stream>>>(nb, sums, dH, respectSym, dG2, dG3);
   TCSCF_LAUNCH(ctx);

@@ -399,14 +399,6 @@ int quadStaticScratch(tcscf_ctx * ctx, double2 ** out)
   return TCSCF_OK;
 }
 
-// U coefficient U[k][i] of the unitary complex -> real-harmonic map phiR_k = sum_i U[k][i] phi_i
-__device__ __forceinline__ double2 urow(const DevSto * s, int k, int i)
-{
-  double const h = 0.70710678118654752440;
-  int const t = s[k].rtype;
-  if (i == k) return t == 0 ? make_double2(1, 0) : (t == 1 ? make_double2(h, 0) : make_double2(0, h));
-  return t == 1 ? make_double2(h, 0) : make_double2(0, -h);
-}
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) { return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
 __device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -a.y); }
 
@@ -468,11 +460,11 @@ __device__ __forceinline__ double2 densityToReal(int nb, const DevSto * s, const
   for (int a = 0; a < 2; ++a) {
     int const i = ik[a];
     if (i < 0) continue;
-    double2 const u1 = cconj(urow(s, k, i));
+    double2 const u1 = cconj(uRow(s, k, i));
     for (int b = 0; b < 2; ++b) {
       int const j = jl[b];
       if (j < 0) continue;
-      double2 const t = cmul(cmul(u1, D[i * nb + j]), urow(s, l, j));
+      double2 const t = cmul(cmul(u1, D[i * nb + j]), uRow(s, l, j));
       acc.x += t.x;
       acc.y += t.y;
     }
@@ -800,36 +792,48 @@ __device__ __forceinline__ int pairIndex(int nb, int k, int l)
   return k * nb - k * (k - 1) / 2 + (l - k);
 }
 
-// F(j,i) = sum_{k,l} U[k][j] FR(k,l) conj(U[l][i]) per r1 row; FR packed symmetric [n1][np] (component c of ncomp)
-// out complex [n1][nb][nb](*ncomp) or real (x 1) when realOut
-__global__ void kPairsToReference(int64_t n1, int nb, const DevSto * s, const double * FR, int ncomp, int comp, int realOut, double * out)
+// plane `comp` of a kept tensor (Tensor): the symmetric nb x nb matrices of the packed pair sums FR [n1][np]
+__global__ void kPairsToPlanes(int64_t n1, int nb, const double * FR, int ncomp, int comp, double * out)
 {
-  int const np = nb * (nb + 1) / 2;
-  int64_t const total = n1 * nb * nb;
+  int const np = nb * (nb + 1) / 2, ps = tensorPlane(nb), ld = tensorStride(nb);
+  int64_t const total = n1 * ps;
   for (int64_t idx = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; idx < total; idx += int64_t(gridDim.x) * blockDim.x) {
-    int64_t const r = idx / (nb * nb);
-    int const j = int((idx / nb) % nb), i = int(idx % nb);
+    int64_t const r = idx / ps;
+    int const e = int(idx % ps);
+    int const k = e / ld, l = e % ld;
+    out[(r * ncomp + comp) * ps + e] = k < nb && l < nb ? FR[r * np + pairIndex(nb, k, l)] : 0.0;
+  }
+}
+
+// F(j,i) = sum_{k,l} U[k][j] FR(k,l) conj(U[l][i]) for `rows` points of a kept tensor's planes: out complex [rows][nb][nb][ncomp],
+// or real [rows][nb][nb] when realOut
+__global__ void kPlanesToReference(int64_t rows, int nb, const DevSto * s, const double * FR, int ncomp, int realOut, double * out)
+{
+  int const ps = tensorPlane(nb), ld = tensorStride(nb);
+  int64_t const total = rows * nb * nb * ncomp;
+  for (int64_t idx = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; idx < total; idx += int64_t(gridDim.x) * blockDim.x) {
+    int const comp = int(idx % ncomp);
+    int64_t const e = idx / ncomp, r = e / (nb * nb);
+    int const j = int((e / nb) % nb), i = int(e % nb);
+    double const * F = FR + (r * ncomp + comp) * ps;
     int const kj[2] = {j, s[j].partner};
     int const li[2] = {i, s[i].partner};
     double2 acc = make_double2(0, 0);
     for (int a = 0; a < 2; ++a) {
       int const k = kj[a];
       if (k < 0) continue;
-      double2 const uk = urow(s, k, j);
+      double2 const uk = uRow(s, k, j);
       for (int b = 0; b < 2; ++b) {
         int const l = li[b];
         if (l < 0) continue;
-        double const f = FR[r * np + pairIndex(nb, k, l)];
-        double2 const t = cmul(uk, cconj(urow(s, l, i)));
+        double const f = F[k * ld + l];
+        double2 const t = cmul(uk, cconj(uRow(s, l, i)));
         acc.x += f * t.x;
         acc.y += f * t.y;
       }
     }
     if (realOut) out[idx] = acc.x;
-    else {
-      out[2 * (idx * ncomp + comp)] = acc.x;
-      out[2 * (idx * ncomp + comp) + 1] = acc.y;
-    }
+    else reinterpret_cast<double2 *>(out)[idx] = acc;
   }
 }
 
@@ -842,13 +846,13 @@ __device__ __forceinline__ double2 realToReference(int nb, const DevSto * s, con
   for (int a = 0; a < 2; ++a) {
     int const k = kj[a];
     if (k < 0) continue;
-    double2 const uk = urow(s, k, j);
+    double2 const uk = uRow(s, k, j);
     for (int b = 0; b < 2; ++b) {
       int const l = li[b];
       if (l < 0) continue;
       double2 g = make_double2(re[k * nb + l], im ? im[k * nb + l] : 0.0);
       if (tr) g.x += tr[l * nb + k];
-      double2 const t = cmul(cmul(uk, g), cconj(urow(s, l, i)));
+      double2 const t = cmul(cmul(uk, g), cconj(uRow(s, l, i)));
       acc.x += t.x;
       acc.y += t.y;
     }
@@ -938,52 +942,82 @@ int fockFinish(tcscf_ctx * ctx, int nspin, int nb, RealSums const & gr, const do
   return TCSCF_OK;
 }
 
-// Faa(r) (+)= sum_ji F(r,j,i) D(i,j) ; Fai(r,i) (+)= sum_j (sum_k D(k,j) vals(r,k)) F(r,j,i)
-// (calculateIaa / calculateFai, HartreeFock.cpp:144-213) for one spin density; one block per row.
-template <bool CX>
-__global__ void kFaaFai(int64_t n1, int nb, const double * F, const double2 * vals, const double2 * D, double2 * Faa, double2 * Fai)
+// Faa(r) = sum_ji F(r,j,i) D(i,j) (summed over the spins) and Fai_s(r,i) = sum_j (sum_k D_s(k,j) phi(r,k)) F(r,j,i)
+// (calculateIaa / calculateFai, HartreeFock.cpp:144-213) in the real-harmonic basis, from a kept tensor's real
+// planes, for complex D = DR [nspin][nb][nb]; re and im parts apart.  One block of 8 warps per point at a time: warp w
+// takes plane rows k = w, w + 8, ... with the lanes over the columns; from the row of D^T it forms q_k = sum_m
+// D(m,k) phi_m (lanes, then shuffles), the row's share of Faa, and adds q_k F(k, .) to the lanes' columns of Fai; the warps'
+// sums meet in shared memory.  Every plane is read once for both spins.  Bound by HBM and the shuffles; the
+// complex layout, read once per spin and sum: FAI_FIGURES
+constexpr int kFaiMaxNb = 64;
+template <int NSPIN>
+__global__ void __launch_bounds__(256) kFaaFai(int64_t n1, int nb, const double * __restrict__ F, const double * __restrict__ phi, const double2 * DR,
+                                              double * FaaRe, double * FaaIm, double * FaiRe, double * FaiIm)
 {
-  extern __shared__ double2 sk[];
-  int64_t const r = blockIdx.x;
-  int const tid = threadIdx.x;
-  for (int j = tid; j < nb; j += blockDim.x) {
-    double2 a = make_double2(0, 0);
-    for (int k = 0; k < nb; ++k) {
-      double2 const t = cmul(D[k * nb + j], vals[r * nb + k]);
-      a.x += t.x; a.y += t.y;
-    }
-    sk[j] = a;
+  extern __shared__ double2 sDT[];   // [NSPIN][nb][nb]: D_s(m, k) at [s][k][m]
+  __shared__ double2 sFai[8][NSPIN][kFaiMaxNb];
+  __shared__ double2 sFaa[8];
+  int const nn = nb * nb, ps = tensorPlane(nb), ld = tensorStride(nb), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  for (int e = tid; e < NSPIN * nn; e += 256) {
+    int const s = e / nn, k = e % nn / nb, m = e % nb;
+    sDT[e] = DR[s * nn + m * nb + k];
   }
   __syncthreads();
-  int64_t const base = r * nb * nb;
-  auto fval = [&](int j, int i) -> double2 {
-    if (CX) return reinterpret_cast<const double2 *>(F)[base + j * nb + i];
-    return make_double2(F[base + j * nb + i], 0.0);
-  };
-  for (int i = tid; i < nb; i += blockDim.x) {
-    double2 a = make_double2(0, 0);
-    for (int j = 0; j < nb; ++j) {
-      double2 const t = cmul(sk[j], fval(j, i));
-      a.x += t.x; a.y += t.y;
+  bool const in0 = lane < nb, in1 = lane + 32 < nb;
+  for (int64_t r = blockIdx.x; r < n1; r += gridDim.x) {
+    double const p0 = in0 ? phi[r * nb + lane] : 0.0, p1 = in1 ? phi[r * nb + lane + 32] : 0.0;
+    const double * Fr = F + r * ps;
+    double2 fai[NSPIN][2], faa = make_double2(0, 0);
+#pragma unroll
+    for (int s = 0; s < NSPIN; ++s) fai[s][0] = fai[s][1] = make_double2(0, 0);
+#pragma unroll 4
+    for (int k = warp; k < nb; k += 8) {
+      double const f0 = in0 ? Fr[k * ld + lane] : 0.0, f1 = in1 ? Fr[k * ld + lane + 32] : 0.0;
+#pragma unroll
+      for (int s = 0; s < NSPIN; ++s) {
+        double2 const d0 = in0 ? sDT[s * nn + k * nb + lane] : make_double2(0, 0), d1 = in1 ? sDT[s * nn + k * nb + lane + 32] : make_double2(0, 0);
+        faa.x = fma(f0, d0.x, fma(f1, d1.x, faa.x));
+        faa.y = fma(f0, d0.y, fma(f1, d1.y, faa.y));
+        double2 q = make_double2(fma(p0, d0.x, p1 * d1.x), fma(p0, d0.y, p1 * d1.y));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          q.x += __shfl_xor_sync(0xffffffffu, q.x, o);
+          q.y += __shfl_xor_sync(0xffffffffu, q.y, o);
+        }
+        fai[s][0].x = fma(q.x, f0, fai[s][0].x);
+        fai[s][0].y = fma(q.y, f0, fai[s][0].y);
+        fai[s][1].x = fma(q.x, f1, fai[s][1].x);
+        fai[s][1].y = fma(q.y, f1, fai[s][1].y);
+      }
     }
-    Fai[r * nb + i].x += a.x;
-    Fai[r * nb + i].y += a.y;
-  }
-  double sr = 0, si = 0;
-  for (int e = tid; e < nb * nb; e += blockDim.x) {
-    int const j = e / nb, i = e % nb;
-    double2 const t = cmul(fval(j, i), D[i * nb + j]);
-    sr += t.x; si += t.y;
-  }
-  for (int o = 16; o > 0; o >>= 1) { sr += __shfl_xor_sync(0xffffffffu, sr, o); si += __shfl_xor_sync(0xffffffffu, si, o); }
-  __shared__ double red[2][32];
-  if ((tid & 31) == 0) { red[0][tid >> 5] = sr; red[1][tid >> 5] = si; }
-  __syncthreads();
-  if (tid == 0) {
-    double a = 0, b = 0;
-    for (int k = 0; k < int(blockDim.x >> 5); ++k) { a += red[0][k]; b += red[1][k]; }
-    Faa[r].x += a;
-    Faa[r].y += b;
+#pragma unroll
+    for (int s = 0; s < NSPIN; ++s) {
+      if (in0) sFai[warp][s][lane] = fai[s][0];
+      if (in1) sFai[warp][s][lane + 32] = fai[s][1];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      faa.x += __shfl_xor_sync(0xffffffffu, faa.x, o);
+      faa.y += __shfl_xor_sync(0xffffffffu, faa.y, o);
+    }
+    if (lane == 0) sFaa[warp] = faa;
+    __syncthreads();
+    for (int e = tid; e < NSPIN * nb; e += 256) {
+      int const s = e / nb, i = e % nb;
+      double2 a = make_double2(0, 0);
+#pragma unroll
+      for (int w = 0; w < 8; ++w) { a.x += sFai[w][s][i].x; a.y += sFai[w][s][i].y; }
+      int64_t const o = (s * n1 + r) * nb + i;
+      FaiRe[o] = a.x;
+      FaiIm[o] = a.y;
+    }
+    if (tid == 255) {
+      double2 a = make_double2(0, 0);
+      for (int w = 0; w < 8; ++w) { a.x += sFaa[w].x; a.y += sFaa[w].y; }
+      FaaRe[r] = a.x;
+      FaaIm[r] = a.y;
+    }
+    __syncthreads();
   }
 }
 
@@ -991,11 +1025,6 @@ __global__ void kFaaFai(int64_t n1, int nb, const double * F, const double2 * va
 __global__ void kAddSpins(int64_t n, const double * a, const double * b, double * out)
 {
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) out[i] = a[i] + b[i];
-}
-
-__global__ void kAddInto(int64_t n, const double * a, double * out)
-{
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) out[i] += a[i];
 }
 
 // column-major complex copy of the row-major (j,i) Fock matrix, and of a real row-major S
@@ -1136,6 +1165,43 @@ int finalizeLaunch(tcscf_ctx * ctx, int nspin, int nb, const double * h, double2
                    double factor, double2 * fock, double * energy)
 {
   return fockFinish(ctx, nspin, nb, RealSums{}, h, G, G3, D, respectSym, factor, fock, energy);
+}
+
+int densityToRealLaunch(tcscf_ctx * ctx, int nb, const DevSto * sto, const double2 * D, double2 * DR)
+{
+  kDensityToReal<<<gridBlocks(int64_t(nb) * nb, 256), 256, 0, ctx->stream>>>(nb, sto, D, DR);
+  TCSCF_LAUNCH(ctx);
+  return TCSCF_OK;
+}
+
+int tensorToReference(tcscf_ctx * ctx, Tensor const & t, const DevSto * sto, int64_t r0, int64_t rows, double * out)
+{
+  int const ncomp = t.vec ? 3 : 1;
+  kPlanesToReference<<<gridBlocks(rows * t.nb * t.nb * ncomp, 256), 256, 0, ctx->stream>>>(rows, t.nb, sto, t.d + r0 * ncomp * tensorPlane(t.nb), ncomp,
+                                                                                           t.isComplex ? 0 : 1, out);
+  TCSCF_LAUNCH(ctx);
+  return TCSCF_OK;
+}
+
+// Tensor memory comes from the context's pool: a precompute per geometry or per Jastrow trial frees and takes the same sizes
+// again, which cudaMalloc and cudaFree of gigabytes made cost milliseconds to hundreds of milliseconds a call.
+// A request that the pool cannot grow to is tried once more with the pool's cached memory given back
+int tensorAlloc(tcscf_ctx * ctx, Tensor & t, size_t bytes)
+{
+  void * p = nullptr;
+  if (gridAllocBytes(ctx, &p, bytes) != TCSCF_OK) {
+    cudaGetLastError();
+    cudaStreamSynchronize(ctx->stream);
+    cudaMemPoolTrimTo(ctx->gridPool, 0);
+    TCSCF_TRY(gridAllocBytes(ctx, &p, bytes));
+  }
+  t.d = static_cast<double *>(p);
+  return TCSCF_OK;
+}
+void tensorRelease(tcscf_ctx * ctx, Tensor & t)
+{
+  gridRelease(ctx, t.d);
+  t.d = nullptr;
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1639,50 +1705,60 @@ int precomputeTensor(tcscf_ctx * ctx, int r1, int r2, int kernel, const tcscf_oc
   TCSCF_TRY(scratch(ctx, "computeF", sizeof(double) * (size_t(n2) * np + size_t(n1) * np), &p));
   double * pairs = static_cast<double *>(p);
   double * FR = pairs + size_t(n2) * np;
-  size_t const outElems = size_t(n1) * nb * nb * (realOut ? 1 : 2) * ncomp;
-  double * dOut = nullptr;
-  TCSCF_CUDA(ctx, cudaMalloc(&dOut, sizeof(double) * outElems));
+  Tensor t;
+  t.n1 = n1; t.nb = nb; t.isComplex = realOut ? 0 : 1; t.vec = ncomp == 3 ? 1 : 0;
+  TCSCF_TRY(tensorAlloc(ctx, t, sizeof(double) * size_t(n1) * ncomp * tensorPlane(nb)));
   cudaEventRecord(ctx->ev[0], ctx->stream);
   int const launch0 = ctx->launchCount;
   kPairProducts<<<gridBlocks(n2 * np, 256), 256, 0, ctx->stream>>>(n2, nb, g2->phiR, g2->w, scale, pairs);
   ctx->launchCount++;
   int st = TCSCF_OK;
-  if (cudaError_t const e = cudaGetLastError(); e != cudaSuccess)   // dOut is released below
+  if (cudaError_t const e = cudaGetLastError(); e != cudaSuccess)   // the tensor is released below
     st = fail(ctx, TCSCF_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
   c.V = pairs;
   c.T = FR;
-  float contraction = 0;
   for (int comp = 0; comp < ncomp && st == TCSCF_OK; ++comp) {
     c.component = comp;
-    // the contraction alone is bracketed by ev[2] / ev[3]; tcscf_last_timing reports the components' sum
-    cudaEventRecord(ctx->ev[2], ctx->stream);
+    // the contractions alone are bracketed by evStart() / evStop(); tcscf_last_timing reports the components' sum
+    ctx->evPart = comp;
+    cudaEventRecord(ctx->evStart(), ctx->stream);
     st = precision == TCSCF_PREC_FP64 ? contractFp64(ctx, c) : contractPairsTensor(ctx, c, precision);
-    cudaEventRecord(ctx->ev[3], ctx->stream);
+    cudaEventRecord(ctx->evStop(), ctx->stream);
     if (st == TCSCF_OK) {
-      kPairsToReference<<<gridBlocks(n1 * nb * nb, 256), 256, 0, ctx->stream>>>(n1, nb, g1->dsto, FR, ncomp, comp, realOut ? 1 : 0, dOut);
+      kPairsToPlanes<<<gridBlocks(n1 * tensorPlane(nb), 256), 256, 0, ctx->stream>>>(n1, nb, FR, ncomp, comp, t.d);
       ctx->launchCount++;
       cudaError_t const e = cudaGetLastError();
       if (e != cudaSuccess) st = fail(ctx, TCSCF_ERR_CUDA, cudaGetErrorString(e));
     }
-    cudaStreamSynchronize(ctx->stream);
-    float a = 0;
-    cudaEventElapsedTime(&a, ctx->ev[2], ctx->ev[3]);
-    contraction += a;
   }
+  ctx->evPart = 0;
   if (st == TCSCF_OK && out) {
-    cudaError_t const e = cudaMemcpyAsync(out, dOut, sizeof(double) * outElems, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e != cudaSuccess) st = fail(ctx, TCSCF_ERR_CUDA, cudaGetErrorString(e));
+    // the reference layout for the host, in pieces of at most 1 GiB
+    size_t const row = sizeof(double) * size_t(nb) * nb * ncomp * (realOut ? 1 : 2);
+    int64_t const chunk = std::max<int64_t>(1, std::min<int64_t>(n1, int64_t((size_t(1) << 30) / row)));
+    void * q = nullptr;
+    st = scratch(ctx, "tensor_out", row * chunk, &q);
+    for (int64_t r0 = 0; r0 < n1 && st == TCSCF_OK; r0 += chunk) {
+      int64_t const rows = std::min(chunk, n1 - r0);
+      st = tensorToReference(ctx, t, g1->dsto, r0, rows, static_cast<double *>(q));
+      cudaError_t const e = st == TCSCF_OK ? cudaMemcpyAsync(reinterpret_cast<char *>(out) + row * r0, q, row * rows, cudaMemcpyDeviceToHost, ctx->stream)
+                                           : cudaSuccess;
+      if (e != cudaSuccess) st = fail(ctx, TCSCF_ERR_CUDA, cudaGetErrorString(e));
+    }
   }
   cudaEventRecord(ctx->ev[1], ctx->stream);
   cudaStreamSynchronize(ctx->stream);
-  float b = 0;
+  float contraction = 0, b = 0;
+  for (int comp = 0; comp < ncomp; ++comp) {
+    float a = 0;
+    if (st == TCSCF_OK) cudaEventElapsedTime(&a, ctx->ev[2 + 2 * comp], ctx->ev[3 + 2 * comp]);
+    contraction += a;
+  }
   cudaEventElapsedTime(&b, ctx->ev[0], ctx->ev[1]);
   ctx->lastContractionMs = contraction;
   ctx->lastTotalMs = b;
   ctx->lastLaunches = ctx->launchCount - launch0;
-  if (st != TCSCF_OK || !keep) { cudaFree(dOut); return st; }
-  Tensor t;
-  t.d = dOut; t.n1 = n1; t.nb = nb; t.isComplex = realOut ? 0 : 1; t.vec = ncomp == 3 ? 1 : 0;
+  if (st != TCSCF_OK || !keep) { tensorRelease(ctx, t); return st; }
   int const id = ctx->nextId++;
   ctx->tensors[id] = t;
   if (handle) *handle = id;
@@ -2171,9 +2247,9 @@ int tcscf_ctx_destroy(tcscf_ctx * ctx)
   cudaSetDevice(ctx->device);
   cudaStreamSynchronize(ctx->stream);
   for (auto & kv : ctx->grids) gridReleaseAll(ctx, kv.second);
+  for (auto & kv : ctx->tensors) tensorRelease(ctx, kv.second);
   cudaStreamSynchronize(ctx->stream);
   if (ctx->gridPool) cudaMemPoolDestroy(ctx->gridPool);
-  for (auto & kv : ctx->tensors) cudaFree(kv.second.d);
   for (auto & kv : ctx->scratch) cudaFree(kv.second.p);
   for (auto & kv : ctx->nearPairs)
     if (kv.second.d) cudaFree(kv.second.d);
@@ -2508,8 +2584,7 @@ int tcscf_tensor_destroy(tcscf_ctx * ctx, int handle)
   if (!ctx) return TCSCF_ERR_INVALID_ARGUMENT;
   auto it = ctx->tensors.find(handle);
   TCSCF_CHECK(ctx, it != ctx->tensors.end(), TCSCF_ERR_INVALID_ARGUMENT, "unknown tensor handle");
-  cudaStreamSynchronize(ctx->stream);
-  cudaFree(it->second.d);
+  tensorRelease(ctx, it->second);
   ctx->tensors.erase(it);
   return TCSCF_OK;
 }
@@ -2611,36 +2686,43 @@ int tcscf_fock_build_precomputed(tcscf_ctx * ctx, int r1, int fji, int nspin, co
   int64_t const n1 = g1->n;
   size_t const nn = size_t(nb) * nb;
   void * p = nullptr;
-  TCSCF_TRY(scratch(ctx, "fock_pre", sizeof(double2) * (nn * nspin * 3 + size_t(nspin) * n1 * (nb + 1) + n1) + sizeof(double) * (nn + 8), &p));
+  TCSCF_CHECK(ctx, nb <= kFaiMaxNb, TCSCF_ERR_UNSUPPORTED, "precompute-form Fock reduction supports nb <= 64");
+  size_t const fai = size_t(nspin) * n1 * nb;
+  TCSCF_TRY(scratch(ctx, "fock_pre", sizeof(double2) * nn * nspin * 4 + sizeof(double) * (2 * fai + 2 * n1 + 2 * nn * nspin + nn + 8), &p));
   double2 * dD = static_cast<double2 *>(p);
   double2 * dG = dD + nn * nspin;
   double2 * dF = dG + nn * nspin;
-  double2 * Faa = dF + nn * nspin;
-  double2 * FaaTot = Faa + size_t(nspin) * n1;
-  double2 * Fai = FaaTot + n1;
-  double * dH = reinterpret_cast<double *>(Fai + size_t(nspin) * n1 * nb);
+  double2 * DR = dF + nn * nspin;
+  double * FaiRe = reinterpret_cast<double *>(DR + nn * nspin);
+  double * FaiIm = FaiRe + fai;
+  double * FaaRe = FaiIm + fai;
+  double * FaaIm = FaaRe + n1;
+  double * GRre = FaaIm + n1;
+  double * GRim = GRre + nn * nspin;
+  double * dH = GRim + nn * nspin;
   double * dE = dH + nn;
   TCSCF_CUDA(ctx, cudaMemcpyAsync(dD, density, sizeof(double2) * nn * nspin, cudaMemcpyHostToDevice, ctx->stream));
   TCSCF_CUDA(ctx, cudaMemcpyAsync(dH, h, sizeof(double) * nn, cudaMemcpyHostToDevice, ctx->stream));
-  TCSCF_CUDA(ctx, cudaMemsetAsync(Faa, 0, sizeof(double2) * (size_t(nspin) * n1 * (nb + 1) + n1), ctx->stream));
-  TCSCF_CUDA(ctx, cudaMemsetAsync(dG, 0, sizeof(double2) * nn * nspin, ctx->stream));
   cudaEventRecord(ctx->ev[0], ctx->stream);
   int const launch0 = ctx->launchCount;
-  for (int s = 0; s < nspin; ++s) {
-    size_t const sm = sizeof(double2) * nb;
-    if (t.isComplex)
-      kFaaFai<true><<<unsigned(n1), 128, sm, ctx->stream>>>(n1, nb, t.d, reinterpret_cast<double2 *>(g1->vals), dD + s * nn, Faa + s * n1, Fai + s * n1 * nb);
-    else
-      kFaaFai<false><<<unsigned(n1), 128, sm, ctx->stream>>>(n1, nb, t.d, reinterpret_cast<double2 *>(g1->vals), dD + s * nn, Faa + s * n1, Fai + s * n1 * nb);
-    TCSCF_LAUNCH(ctx);
-    kAddInto<<<gridBlocks(2 * n1, 256), 256, 0, ctx->stream>>>(2 * n1, reinterpret_cast<double *>(Faa + s * n1), reinterpret_cast<double *>(FaaTot));
-    TCSCF_LAUNCH(ctx);
-  }
-  double const cJ = nspin == 1 ? 2.0 : 1.0;
-  for (int s = 0; s < nspin; ++s)
-    TCSCF_TRY(reduceFockComplex(ctx, n1, nb, g1->vals, g1->w, reinterpret_cast<double *>(FaaTot), cJ,
-                                reinterpret_cast<double *>(Fai + s * n1 * nb), reinterpret_cast<double *>(dG + s * nn)));
-  TCSCF_TRY(fockFinish(ctx, nspin, nb, RealSums{}, dH, dG, nullptr, dD, respect_symmetry, nspin == 1 ? 2.0 : 1.0, dF, dE));
+  for (int s = 0; s < nspin; ++s) TCSCF_TRY(densityToRealLaunch(ctx, nb, g1->dsto, dD + s * nn, DR + s * nn));
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+  size_t const sm = sizeof(double2) * nn * nspin;
+  auto launch = [&](auto kernel) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm));
+    int per = 1;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, 256, sm);
+    kernel<<<unsigned(std::min<int64_t>(n1, int64_t(sms) * std::max(per, 1))), 256, sm, ctx->stream>>>(n1, nb, t.d, g1->phiR, DR, FaaRe, FaaIm, FaiRe, FaiIm);
+  };
+  if (nspin == 1) launch(kFaaFai<1>);
+  else launch(kFaaFai<2>);
+  TCSCF_LAUNCH(ctx);
+  // G = sum_r w phi (cJ phi Faa - Fai), real and imaginary parts apart
+  double const cJ0 = nspin == 1 ? 2.0 : 1.0, cJ[2] = {cJ0, cJ0};
+  TCSCF_TRY(reduceFockReal(ctx, n1, nb, nspin, g1->phiR, g1->w, FaaRe, cJ, FaiRe, int64_t(n1) * nb, nb, GRre));
+  TCSCF_TRY(reduceFockReal(ctx, n1, nb, nspin, g1->phiR, g1->w, FaaIm, cJ, FaiIm, int64_t(n1) * nb, nb, GRim));
+  TCSCF_TRY(fockFinish(ctx, nspin, nb, {GRre, GRim, g1->dsto, 0}, dH, dG, nullptr, dD, respect_symmetry, cJ0, dF, dE));
   cudaEventRecord(ctx->ev[1], ctx->stream);
   if (G) TCSCF_CUDA(ctx, cudaMemcpyAsync(G, dG, sizeof(double2) * nn * nspin, cudaMemcpyDeviceToHost, ctx->stream));
   if (fock) TCSCF_CUDA(ctx, cudaMemcpyAsync(fock, dF, sizeof(double2) * nn * nspin, cudaMemcpyDeviceToHost, ctx->stream));
