@@ -66,13 +66,29 @@ __device__ __forceinline__ void ochiGrad(OchiDev const & u, double px, double py
   gz = r12L * dz + r1L * pz;
 }
 
-// g(r1, r2): KIND 0 = 1/r12, 1 = TC scalar, 2 = one component of grad_1 u.  0 for r1 == r2.
+// (1/r12) du/dr12 of a Jastrow factor of r12 alone (every S[k] = (i, 0, 0)) from r12^2 and y = 1/r12:
+// a12 t y^2 sum_k i_k c_k (r12 t)^i_k with t = 1 / (r12 + a12); grad_1 u is this times r1 - r2
+__device__ __forceinline__ double ochiR12(OchiDev const & u, double rr, double y, int same)
+{
+  double const r = rr * y, t = 1.0 / (r + u.a12), z = r * t;
+  double s = 0;
+  for (int k = 0; k < u.nterms; ++k) s = fma(u.c[k][same] * u.S[k][0], ipow(z, u.S[k][0]), s);
+  return u.a12 * t * y * y * s;
+}
+
+// g(r1, r2), 0 for r1 == r2.  KIND 0 = 1/r12, 1 = TC scalar, 2 = one component of grad_1 u; 3, 4 = 1, 2 for a Jastrow factor of
+// r12 alone, where grad_2 u = -grad_1 u and no other distance enters (a fifth of the FP64 operations)
 template <int KIND>
 __device__ __forceinline__ double r12Kernel(KArgs const & a, double x1, double y1, double z1, double x2, double y2, double z2)
 {
   double const dx = x1 - x2, dy = y1 - y2, dz = z1 - z2;
   double const rr = fma(dx, dx, fma(dy, dy, dz * dz));
   if constexpr (KIND == 0) return invR12(rr);
+  if constexpr (KIND == 3 || KIND == 4) {
+    double const y = invR12(rr), q = y == 0.0 ? 0.0 : ochiR12(a.u, rr, y, a.same);
+    if constexpr (KIND == 3) return 2.0 * (y - q * q * rr);
+    return q * (a.component == 0 ? dx : (a.component == 1 ? dy : dz));
+  }
   if (rr == 0.0) return 0.0;
   if (KIND == 1) {
     double ax, ay, az, bx, by, bz;
@@ -91,9 +107,9 @@ __host__ __device__ constexpr int contractWarps(int rt) { return rt == 1 ? 8 : 4
 
 // blocks per SM the register budget is cut for (65,536 / (threads x blocks) a thread); one more block each
 // below 8 tiles spilled and ran 1 to 20 % slower
-__host__ __device__ constexpr int contractBlocks(int nt, int rt)
+__host__ __device__ constexpr int contractBlocks(int nt, int rt, int kind)
 {
-  return rt == 1 ? 1 : (nt <= 3 ? 4 : (nt <= 6 ? 3 : 2));
+  return rt == 1 ? (kind == 0 ? 1 : 2) : (nt <= 3 ? 4 : (nt <= 6 ? 3 : 2));
 }
 
 // T += (g .* rho) V for 8 RT rows per warp and 8 NTL columns, everything between the shared-memory
@@ -112,7 +128,7 @@ __host__ __device__ constexpr int contractBlocks(int nt, int rt)
 // two barriers: 59,000 points x 40 columns (rank 5, symmetric) 21.1 -> 7.2 ms; 81,200 points x 120
 // columns (rank 18, symmetric) 58.6 -> 32.1 ms, 0.81 of the FP64 matmul rate counting the padded MMAs.
 template <int KIND, int NTL, int RT, int KR>
-__global__ void __launch_bounds__(32 * contractWarps(RT), contractBlocks(NTL, RT)) kContractFp64(KArgs a)
+__global__ void __launch_bounds__(32 * contractWarps(RT), contractBlocks(NTL, RT, KIND)) kContractFp64(KArgs a)
 {
   constexpr int kWarps = contractWarps(RT), kThreads = 32 * kWarps;
   static_assert(BK == 32, "a warp copies one coordinate row of a stage");
@@ -568,13 +584,12 @@ int launchKind(tcscf_ctx * ctx, int nt, int rt, int kr, KArgs const & a, dim3 gr
       default: return launchDirect<16>(ctx, kr, a, grid, smem);
     }
   } else {
+    constexpr int RT = KIND >= 3 ? 2 : 1;
     switch (nt) {
-      case 4: return launchOne<KIND, 4, 2, 0>(ctx, a, grid, smem);
-      case 8: return launchOne<KIND, 8, 2, 0>(ctx, a, grid, smem);
-      case 12: return launchOne<KIND, 12, 2, 0>(ctx, a, grid, smem);
-      case 13: return launchOne<KIND, 13, 2, 0>(ctx, a, grid, smem);
-      case 15: return launchOne<KIND, 15, 2, 0>(ctx, a, grid, smem);
-      default: return launchOne<KIND, 16, 2, 0>(ctx, a, grid, smem);
+      case 4: return launchOne<KIND, 4, RT, 0>(ctx, a, grid, smem);
+      case 8: return launchOne<KIND, 8, RT, 0>(ctx, a, grid, smem);
+      case 13: return launchOne<KIND, 13, RT, 0>(ctx, a, grid, smem);
+      default: return launchOne<KIND, 16, RT, 0>(ctx, a, grid, smem);
     }
   }
 }
@@ -582,7 +597,7 @@ int launchKind(tcscf_ctx * ctx, int nt, int rt, int kr, KArgs const & a, dim3 gr
 // the smallest instantiated tile count that holds nt tiles
 int contractTiles(int kind, int rt, int nt)
 {
-  static int const direct[] = {1, 2, 3, 4, 5, 6, 8, 10, 12, 13, 15, 16}, wideRank[] = {4, 8, 16}, tc[] = {4, 8, 12, 13, 15, 16};
+  static int const direct[] = {1, 2, 3, 4, 5, 6, 8, 10, 12, 13, 15, 16}, wideRank[] = {4, 8, 16}, tc[] = {4, 8, 13, 16};
   auto pick = [&](auto const & v) { for (int t : v) if (t >= nt) return t; return 16; };
   return kind != 0 ? pick(tc) : (rt == 1 ? pick(wideRank) : pick(direct));
 }
@@ -599,15 +614,18 @@ int contractFp64(tcscf_ctx * ctx, Contraction const & c)
 {
   TCSCF_CHECK(ctx, c.R >= 0 && c.R <= 128, TCSCF_ERR_UNSUPPORTED, "contraction rank must be <= 128");
   TCSCF_CHECK(ctx, c.ncol > 0 && c.n1 > 0 && c.n2 > 0, TCSCF_ERR_INVALID_ARGUMENT, "empty contraction");
-  int const kind = c.kernel == TCSCF_K_INV_R12 ? 0 : (c.kernel <= TCSCF_K_TC_SCALAR_OPPO ? 1 : 2);
+  bool r12Only = c.jastrow != nullptr;
+  for (int k = 0; r12Only && k < c.jastrow->nterms; ++k) r12Only = c.jastrow->S[k][1] == 0 && c.jastrow->S[k][2] == 0 && c.jastrow->S[k][0] >= 0;
+  int const kind = c.kernel == TCSCF_K_INV_R12 ? 0 : (c.kernel <= TCSCF_K_TC_SCALAR_OPPO ? 1 : 2) + (r12Only ? 2 : 0);
   TCSCF_CHECK(ctx, kind == 0 || c.R == 0, TCSCF_ERR_UNSUPPORTED, "internal: the transcorrelated kernels come in the precompute form");
   // columns in equal groups of at most 128 (g is generated once per group)
   int const cgroups = (c.ncol + kMaxCol - 1) / kMaxCol;
   int const colsPerBlock = ((c.ncol + cgroups - 1) / cgroups + 7) / 8 * 8;
   // two row tiles per warp (with four, 59,000 points x 40 columns took 9.8 ms against 8.5: half the warps, and
   // the accumulators spilled); ranks whose factor rows would leave room for one block of 4 warps per
-  // SM take 8 warps of one row tile
-  int rt = 2;
+  // SM take 8 warps of one row tile, and so do the general transcorrelated kernels, whose long chains of roots and
+  // quotients want 16 warps per SM
+  int rt = kind == 1 || kind == 2 ? 1 : 2;
   if (kind == 0 && contractSmem(contractTiles(kind, rt, colsPerBlock / 8), rt, c.R) > 112 * 1024) rt = 1;
   int const nt = contractTiles(kind, rt, colsPerBlock / 8);
   int const bm = 8 * rt * contractWarps(rt);
@@ -664,8 +682,13 @@ int contractFp64(tcscf_ctx * ctx, Contraction const & c)
   // the contraction kernel alone is bracketed by the context's timing events (tcscf_last_timing)
   if (!ctx->capturing) cudaEventRecord(ctx->evStart(), ctx->stream);
   dim3 const grid{unsigned(tiles), unsigned(nsplit), unsigned(cgroups)};
-  TCSCF_TRY(kind == 0 ? launchKind<0>(ctx, nt, rt, contractSteps(rt, c.R), a, grid, smem) : (kind == 1 ? launchKind<1>(ctx, nt, rt, 0, a, grid, smem)
-              : launchKind<2>(ctx, nt, rt, 0, a, grid, smem)));
+  switch (kind) {
+    case 0: TCSCF_TRY(launchKind<0>(ctx, nt, rt, contractSteps(rt, c.R), a, grid, smem)); break;
+    case 1: TCSCF_TRY(launchKind<1>(ctx, nt, rt, 0, a, grid, smem)); break;
+    case 2: TCSCF_TRY(launchKind<2>(ctx, nt, rt, 0, a, grid, smem)); break;
+    case 3: TCSCF_TRY(launchKind<3>(ctx, nt, rt, 0, a, grid, smem)); break;
+    default: TCSCF_TRY(launchKind<4>(ctx, nt, rt, 0, a, grid, smem)); break;
+  }
   if (!ctx->capturing) cudaEventRecord(ctx->evStop(), ctx->stream);
   if (nsplit > 1) {
     int64_t const n = c.n1 * c.ncol;
