@@ -26,9 +26,9 @@
 // work items are (r1 tile of 128, column chunk, r2 split); the T accumulators are double-buffered in
 // TMEM so the MMAs of block g overlap the flush of block g - 1.
 //
-// Warp roles (384 threads, one persistent CTA per SM): warp 0 TMA producer (Vp slices by TMA, r2
+// Warp roles (640 threads, one persistent CTA per SM): warp 0 TMA producer (Vp slices by TMA, r2
 // coordinates and column scales by 1-D bulk copies; no multicast), warp 1 MMA issuer and TMEM
-// allocator, warps 2-3 idle, warps 4-11 compute (TMEM lane quarter w % 4, r2 / column half (w-4)/4).
+// allocator, warps 2-3 idle, warps 4-19 compute (TMEM lane quarter w % 4, r2 / column part (w-4)/4).
 // Every mbarrier wait is bounded; on expiry the kernel records a status code, drains its own copies
 // and MMAs with bounded waits, frees TMEM and returns.
 #include <cuda.h>
@@ -43,6 +43,13 @@ namespace tc {
 namespace {
 
 constexpr int kPairStages = 3;
+// 16 compute warps: four column / r2 parts per TMEM lane quarter.  With 8 (two parts, 64 T columns a thread) the per-pair
+// chains left the schedulers two warps each (48.1 -> 36.2 ms per launch at 65,536 x 65,536 points x 300 columns,
+// results unchanged to the bit); a thread's 32 double-float columns leave
+// room for 112 registers.  Register split: 640 threads x 96 at launch = 61440 = 128 x 32 + 512 x 112
+constexpr int kPairParts = 4, kPairWarps = 4 * kPairParts, kPairThreads = 128 + 32 * kPairWarps;
+constexpr int kPairRegsProducer = 32, kPairRegsCompute = 112;
+static_assert(128 * kPairRegsProducer + 32 * kPairWarps * kPairRegsCompute <= kPairThreads * 96, "register split exceeds the launch allocation");
 // X tile buffers: two where shared memory allows (GEMM of block g - 1 overlaps the writing of block g)
 __host__ __device__ constexpr int pairXBuffers(int NB) { return NB == 128 ? 1 : 2; }
 constexpr int kPairXSlices = 4;   // h, m, l/256, m/256
@@ -72,8 +79,8 @@ struct __align__(1024) PairSmem {
   uint8_t x[XBUF][kPairXSlices][BM * BK * 2];      // X tile slices: SW128 K-major [128 rows][64]
   float4 coords[NSTAGE][BK];                       // r2 block as 32 pairs
   float cinv[NSTAGE][NB];                          // inverse column scales of the block's chunk columns
-  float cinvT[NCW][2][NB / 2];                     // each compute warp's columns' scales, by block parity
-  float rowmax[2][2][BM];                          // [block parity][r2 half][row]
+  float cinvT[kPairWarps][2][NB / kPairParts];     // each compute warp's columns' scales, by block parity
+  float rowmax[2][kPairParts][BM];                 // [block parity][r2 part][row]
   uint64_t full[NSTAGE], empty[NSTAGE];
   uint64_t xfull[XBUF], xfree[XBUF];
   uint64_t tfull[2], tfree[2];                     // T accumulator buffers
@@ -168,11 +175,11 @@ __device__ __forceinline__ void decodePairItem(PairParams const & P, int item, i
   split = r % P.nSplit;
 }
 
-// Adds T buffer tb of block f (this thread's row and NB/2 columns) with the block's scales into the
+// Adds T buffer tb of block f (this thread's row and NB / kPairParts columns) with the block's scales into the
 // double-float accumulators by Fast2Sum and hands the buffer back to the MMA issuer.
 template <int NB, class SmemT>
-__device__ __forceinline__ bool flushPairBlock(SmemT & S, uint32_t taddr, uint32_t f, int cw, float fac, uint64_t (&hi)[NB / 4],
-                                               uint64_t (&lo)[NB / 4], int lane, volatile int * abortFlag, int * status)
+__device__ __forceinline__ bool flushPairBlock(SmemT & S, uint32_t taddr, uint32_t f, int cw, float fac, uint64_t (&hi)[NB / (2 * kPairParts)],
+                                               uint64_t (&lo)[NB / (2 * kPairParts)], int lane, volatile int * abortFlag, int * status)
 {
   int const tb = f & 1;
   if (!waitBar(&S.tfull[tb], (f >> 1) & 1, abortFlag, status, 131)) return false;
@@ -181,7 +188,7 @@ __device__ __forceinline__ bool flushPairBlock(SmemT & S, uint32_t taddr, uint32
   uint64_t const k256 = f2pack(256.0f, 256.0f);
   uint64_t const ff = f2pack(fac, fac);
   uint32_t const base = taddr + uint32_t(tb * 2 * NB);
-  constexpr int NQ = NB / 16;
+  constexpr int NQ = NB / (8 * kPairParts);
   float hh[2][8], mm[2][8];
   tmemLoad8(base, hh[0]);
   tmemLoad8(base + NB, mm[0]);
@@ -212,7 +219,7 @@ __device__ __forceinline__ bool flushPairBlock(SmemT & S, uint32_t taddr, uint32
 }
 
 template <int NB, int KIND>
-__global__ void __launch_bounds__(NTHREADS, 1)
+__global__ void __launch_bounds__(kPairThreads, 1)
     kPairTc(const __grid_constant__ PairParams P, const __grid_constant__ CUtensorMap mapH, const __grid_constant__ CUtensorMap mapM,
             const __grid_constant__ CUtensorMap mapL)
 {
@@ -228,11 +235,11 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   int const nItems = P.nTiles * P.nChunks * P.nSplit;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < NSTAGE; ++s) { mbarInit(&S.full[s], 1); mbarInit(&S.empty[s], 1 + NCW); }
-    for (int b = 0; b < XBUF; ++b) { mbarInit(&S.xfull[b], NCW); mbarInit(&S.xfree[b], 1); }
+    for (int s = 0; s < NSTAGE; ++s) { mbarInit(&S.full[s], 1); mbarInit(&S.empty[s], 1 + kPairWarps); }
+    for (int b = 0; b < XBUF; ++b) { mbarInit(&S.xfull[b], kPairWarps); mbarInit(&S.xfree[b], 1); }
     for (int b = 0; b < 2; ++b) {
-      mbarInit(&S.tfull[b], 1); mbarInit(&S.tfree[b], NCW);
-      for (int q = 0; q < 4; ++q) mbarInit(&S.rmax[b][q], 2);
+      mbarInit(&S.tfull[b], 1); mbarInit(&S.tfree[b], kPairWarps);
+      for (int q = 0; q < 4; ++q) mbarInit(&S.rmax[b][q], kPairParts);
     }
     mbarInit(&S.done, 1);
     S.abort = 0;
@@ -248,7 +255,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   uint32_t const tmem = S.tmemBase;
 
   if (warp < 4) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsProducer));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPairRegsProducer));
     if (warp == 0) {
       // ---------------------------------------------------------------- TMA producer
       if (lane == 0) {
@@ -330,17 +337,17 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
     }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsCompute));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kPairRegsCompute));
     // ---------------------------------------------------------------- compute warps
     int const cw = warp - 4;
     int const quarter = warp & 3;
-    int const half = cw >> 2;
+    int const part = cw >> 2;
     int const row = quarter * 32 + lane;
     uint32_t const laneBase = uint32_t(quarter * 32) << 16;
-    uint32_t const tAddr = tmem + laneBase + uint32_t(half * (NB / 2));
+    uint32_t const tAddr = tmem + laneBase + uint32_t(part * (NB / kPairParts));
     uint32_t g = 0;
     bool ok = true;
-    uint64_t ahi[NB / 4], alo[NB / 4];
+    uint64_t ahi[NB / (2 * kPairParts)], alo[NB / (2 * kPairParts)];
     uint64_t const kInv256 = f2pack(1.0f / 256.0f, 1.0f / 256.0f), kM256 = f2pack(-256.0f, -256.0f);
     uint64_t const kMagic = f2pack(12582912.0f, 12582912.0f);   // 1.5 * 2^23: adding it rounds |x| < 2^22 to an integer
     uint64_t const kInv65536 = f2pack(1.0f / 65536.0f, 1.0f / 65536.0f), kM65536 = f2pack(-65536.0f, -65536.0f);
@@ -353,7 +360,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       int const r1 = tile * BM + row;
       float4 const p1 = P.r1xyz[r1];
 #pragma unroll
-      for (int c = 0; c < NB / 4; ++c) { ahi[c] = 0; alo[c] = 0; }
+      for (int c = 0; c < NB / (2 * kPairParts); ++c) { ahi[c] = 0; alo[c] = 0; }
       float pendingFac = 0.0f;
       bool pending = false;
       uint64_t const p1x = f2pack(p1.x, p1.x), p1y = f2pack(p1.y, p1.y), p1z = f2pack(p1.z, p1.z);
@@ -361,11 +368,12 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         int const s = g % NSTAGE, b = g & 1, xb = g % XBUF;
         if (!(ok = waitBar(&S.full[s], (g / NSTAGE) & 1, abortFlag, P.status, 132))) break;
         // this warp's column scales, kept for the flush of block g after the stage is released
-        for (int c = lane; c < NB / 2; c += 32) S.cinvT[cw][b][c] = S.cinv[s][half * (NB / 2) + c];
-        float4 const * cc = S.coords[s] + half * 32;
-        uint64_t xv[16];
+        for (int c = lane; c < NB / kPairParts; c += 32) S.cinvT[cw][b][c] = S.cinv[s][part * (NB / kPairParts) + c];
+        constexpr int PAIRS = BK / (2 * kPairParts);   // r2 pairs per thread
+        float4 const * cc = S.coords[s] + part * 2 * PAIRS;
+        uint64_t xv[PAIRS];
 #pragma unroll
-        for (int pr = 0; pr < 16; ++pr) {
+        for (int pr = 0; pr < PAIRS; ++pr) {
           float4 const qa = cc[2 * pr], qb = cc[2 * pr + 1];
           uint64_t const dx = f2sub(p1x, f2pack(qa.x, qa.y));
           uint64_t const dy = f2sub(p1y, f2pack(qa.z, qa.w));
@@ -373,19 +381,20 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           uint64_t const r2 = f2fma(dx, dx, f2fma(dy, dy, f2mul(dz, dz)));
           xv[pr] = pairKernel<KIND>(P, dx, dy, dz, r2, p1.w);
         }
-        // row maximum of |X| over the block's 64 r2 points: this warp's 32 and the other half's
+        // row maximum of |X| over the block's 64 r2 points: this warp's share and the other parts'
         float mx = 0.0f;
 #pragma unroll
-        for (int pr = 0; pr < 16; ++pr) {
+        for (int pr = 0; pr < PAIRS; ++pr) {
           float xa, xb2;
           f2unpack(xv[pr], xa, xb2);
           mx = fmaxf(mx, fmaxf(fabsf(xa), fabsf(xb2)));
         }
-        S.rowmax[b][half][row] = mx;
+        S.rowmax[b][part][row] = mx;
         __syncwarp();
         if (lane == 0) mbarArrive(&S.rmax[b][quarter]);
         if (!(ok = waitBar(&S.rmax[b][quarter], (g >> 1) & 1, abortFlag, P.status, 135))) break;
-        mx = fmaxf(mx, S.rowmax[b][half ^ 1][row]);
+#pragma unroll
+        for (int q = 0; q < kPairParts; ++q) mx = fmaxf(mx, S.rowmax[b][q][row]);
         // scale bs = 2^(23 - E), E = floor(log2 mx) (clamped below): |X bs| < 2^24
         int const E = max(int((__float_as_uint(mx) >> 23) & 0xFF) - 127, kMinExp);
         float const bs = __uint_as_float(uint32_t(127 + 23 - E) << 23);
@@ -394,8 +403,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         if (g >= uint32_t(XBUF) && !(ok = waitBar(&S.xfree[xb], ((g / XBUF) - 1) & 1, abortFlag, P.status, 134))) break;
         uint64_t const bb = f2pack(bs, bs);
 #pragma unroll
-        for (int ch = 0; ch < 4; ++ch) {
-          uint32_t const off = sw128(row, half * 4 + ch);
+        for (int ch = 0; ch < PAIRS / 4; ++ch) {
+          uint32_t const off = sw128(row, part * (PAIRS / 4) + ch);
           // t = X bs = 65536 h + 256 m + l: h = rint(t / 65536), m = rint(r / 256), l = r - 256 m with
           // r = t - 65536 h; slices h, m, l/256 (rounded to nearest BF16: it feeds only the cross
           // accumulator), m/256
@@ -428,8 +437,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       if (r1 < P.n1) {
         double * T = P.T + int64_t(split) * P.tStride + int64_t(r1) * P.ldt;
 #pragma unroll
-        for (int c = 0; c < NB / 2; ++c) {
-          int const col = chunk * NB + half * (NB / 2) + c;
+        for (int c = 0; c < NB / kPairParts; ++c) {
+          int const col = chunk * NB + part * (NB / kPairParts) + c;
           float h0, h1, l0, l1;
           f2unpack(ahi[c / 2], h0, h1);
           f2unpack(alo[c / 2], l0, l1);
@@ -448,7 +457,7 @@ int launchPairs(tcscf_ctx * ctx, PairParams const & P, CUtensorMap const (&maps)
   size_t const smem = sizeof(PairSmem<NB>) + 1024;
   static_assert(sizeof(PairSmem<NB>) + 1024 <= 232448, "shared memory per CTA");
   TCSCF_CUDA(ctx, cudaFuncSetAttribute(kPairTc<NB, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-  kPairTc<NB, KIND><<<grid, NTHREADS, smem, ctx->stream>>>(P, maps[0], maps[1], maps[2]);
+  kPairTc<NB, KIND><<<grid, kPairThreads, smem, ctx->stream>>>(P, maps[0], maps[1], maps[2]);
   TCSCF_LAUNCH(ctx);
   return TCSCF_OK;
 }
