@@ -35,6 +35,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "tc_device.cuh"
 
@@ -104,8 +105,9 @@ __device__ __forceinline__ uint64_t f2rcp(uint64_t s)
 }
 
 // Kernel values of two pairs (packed): d = r1 - r2 components, r2sq = |d|^2.
-template <int KIND>
-__device__ __forceinline__ uint64_t pairKernel(PairParams const & P, uint64_t dx, uint64_t dy, uint64_t dz, uint64_t r2sq, float thr)
+// DROP: those below thr give 0; otherwise the smallest |d|^2 seen goes to mn
+template <int KIND, bool DROP>
+__device__ __forceinline__ uint64_t pairKernel(PairParams const & P, uint64_t dx, uint64_t dy, uint64_t dz, uint64_t r2sq, float thr, float & mn)
 {
   float r2a, r2b;
   f2unpack(r2sq, r2a, r2b);
@@ -130,6 +132,10 @@ __device__ __forceinline__ uint64_t pairKernel(PairParams const & P, uint64_t dx
       g = f2mul(f2mul(up, y), d);
     }
   }
+  if constexpr (!DROP) {
+    mn = min3(mn, r2a, r2b);
+    return g;
+  }
   float ga, gb;
   f2unpack(g, ga, gb);
   ga = r2a >= thr ? ga : 0.0f;
@@ -137,33 +143,9 @@ __device__ __forceinline__ uint64_t pairKernel(PairParams const & P, uint64_t dx
   return f2pack(ga, gb);
 }
 
-__device__ __forceinline__ uint32_t bf16PairRnP(uint64_t ab)
-{
-  float a, b;
-  f2unpack(ab, a, b);
-  __nv_bfloat162 const h = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<uint32_t const *>(&h);
-}
-__device__ __forceinline__ uint32_t bf16PairExactP(uint64_t ab)
-{
-  float a, b;
-  f2unpack(ab, a, b);
-  return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
-}
-
 __host__ __device__ constexpr uint32_t idescBf16(int M, int N)
 {
   return (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(N >> 3) << 17) | (uint32_t(M >> 4) << 24);
-}
-
-__device__ __forceinline__ void mmaBf16P(uint32_t tmemD, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate)
-{
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmemD),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
-      : "memory");
 }
 
 __device__ __forceinline__ void decodePairItem(PairParams const & P, int item, int & tile, int & chunk, int & split)
@@ -289,6 +271,8 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       if (lane == 0) {
         constexpr uint32_t idesc = idescBf16(BM, NB);
         constexpr uint32_t idescX2 = idescBf16(BM, 2 * NB);   // h x [h'; m']: adjacent slices, adjacent accumulators
+        constexpr uint32_t kXStep = BM * BK * 2 / 16, kVStep = NB * BK * 2 / 16;
+        uint32_t const xLo = descLo(smemAddr(S.x[0][0])), vLo = descLo(smemAddr(S.v[0][0])), hi = descHi(1024, 2);
         uint32_t g = 0;
         bool ok = true;
         for (int item = blockIdx.x; item < nItems && ok; item += gridDim.x) {
@@ -303,20 +287,17 @@ __global__ void __launch_bounds__(kPairThreads, 1)
             if (!(ok = waitBar(&S.xfull[xb], (g / XBUF) & 1, abortFlag, P.status, 123))) break;
             fenceAfterSync();
             uint32_t const dA = tmem + uint32_t(tb * 2 * NB), dB = dA + NB;
-            uint32_t aX[kPairXSlices];
-#pragma unroll
-            for (int k = 0; k < kPairXSlices; ++k) aX[k] = smemAddr(S.x[xb][k]);
-            uint32_t const bV[3] = {smemAddr(S.v[s][0]), smemAddr(S.v[s][1]), smemAddr(S.v[s][2])};
-            auto dxa = [&](int sl, int k) { return smemDesc(aX[sl] + 32 * k, 1024, 2); };
-            auto dvb = [&](int sl, int k) { return smemDesc(bV[sl] + 32 * k, 1024, 2); };
+            uint32_t const aLo = xLo + uint32_t(xb) * kPairXSlices * kXStep, bLo = vLo + uint32_t(s) * 3 * kVStep;
+            auto dxa = [&](int sl, int k) { return aLo + sl * kXStep + 2 * k; };
+            auto dvb = [&](int sl, int k) { return bLo + sl * kVStep + 2 * k; };
 #pragma unroll
             for (int k = 0; k < BK / 16; ++k) {
-              uint32_t const acc = k > 0 ? 1u : 0u;
-              mmaBf16P(dA, dxa(0, k), dvb(0, k), idescX2, acc);   // A += hX hV, B += hX mV
-              mmaBf16P(dB, dxa(1, k), dvb(0, k), idesc, 1);       // B += mX hV
-              mmaBf16P(dB, dxa(0, k), dvb(2, k), idesc, 1);       // B += hX lV/256
-              mmaBf16P(dB, dxa(3, k), dvb(1, k), idesc, 1);       // B += m/256 X mV
-              mmaBf16P(dB, dxa(2, k), dvb(0, k), idesc, 1);       // B += l/256 X hV
+              if (k == 0) mmaF16<0>(dA, dxa(0, k), dvb(0, k), hi, idescX2);   // A += hX hV, B += hX mV
+              else mmaF16<1>(dA, dxa(0, k), dvb(0, k), hi, idescX2);
+              mmaF16<1>(dB, dxa(1, k), dvb(0, k), hi, idesc);                  // B += mX hV
+              mmaF16<1>(dB, dxa(0, k), dvb(2, k), hi, idesc);                  // B += hX lV/256
+              mmaF16<1>(dB, dxa(3, k), dvb(1, k), hi, idesc);                  // B += m/256 X mV
+              mmaF16<1>(dB, dxa(2, k), dvb(0, k), hi, idesc);                  // B += l/256 X hV
             }
             mmaCommit(&S.xfree[xb]);
             mmaCommit(&S.empty[s]);
@@ -348,9 +329,6 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     uint32_t g = 0;
     bool ok = true;
     uint64_t ahi[NB / (2 * kPairParts)], alo[NB / (2 * kPairParts)];
-    uint64_t const kInv256 = f2pack(1.0f / 256.0f, 1.0f / 256.0f), kM256 = f2pack(-256.0f, -256.0f);
-    uint64_t const kMagic = f2pack(12582912.0f, 12582912.0f);   // 1.5 * 2^23: adding it rounds |x| < 2^22 to an integer
-    uint64_t const kInv65536 = f2pack(1.0f / 65536.0f, 1.0f / 65536.0f), kM65536 = f2pack(-65536.0f, -65536.0f);
     for (int item = blockIdx.x; item < nItems && ok; item += gridDim.x) {
       int tile, chunk, split;
       decodePairItem(P, item, tile, chunk, split);
@@ -372,14 +350,26 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         constexpr int PAIRS = BK / (2 * kPairParts);   // r2 pairs per thread
         float4 const * cc = S.coords[s] + part * 2 * PAIRS;
         uint64_t xv[PAIRS];
+        // pairs below the FP32 resolution of r1 are dropped in a second pass over the few blocks that hold one (in kFlashTc, with
+        // half the warps and twice the registers a thread, the second body cost more than the test it saves)
+        auto generate = [&](auto dropTest, uint64_t x, uint64_t y1, uint64_t z) {
+          float mn = 3.0e38f;
 #pragma unroll
-        for (int pr = 0; pr < PAIRS; ++pr) {
-          float4 const qa = cc[2 * pr], qb = cc[2 * pr + 1];
-          uint64_t const dx = f2sub(p1x, f2pack(qa.x, qa.y));
-          uint64_t const dy = f2sub(p1y, f2pack(qa.z, qa.w));
-          uint64_t const dz = f2sub(p1z, f2pack(qb.x, qb.y));
-          uint64_t const r2 = f2fma(dx, dx, f2fma(dy, dy, f2mul(dz, dz)));
-          xv[pr] = pairKernel<KIND>(P, dx, dy, dz, r2, p1.w);
+          for (int pr = 0; pr < PAIRS; ++pr) {
+            float4 const qa = cc[2 * pr], qb = cc[2 * pr + 1];
+            uint64_t const dx = f2sub(x, f2pack(qa.x, qa.y));
+            uint64_t const dy = f2sub(y1, f2pack(qa.z, qa.w));
+            uint64_t const dz = f2sub(z, f2pack(qb.x, qb.y));
+            uint64_t const r2 = f2fma(dx, dx, f2fma(dy, dy, f2mul(dz, dz)));
+            xv[pr] = pairKernel<KIND, decltype(dropTest)::value>(P, dx, dy, dz, r2, p1.w, mn);
+          }
+          return mn;
+        };
+        if (__any_sync(0xffffffffu, !(generate(std::false_type{}, p1x, p1y, p1z) >= p1.w))) {
+          // r1 through opaque registers: the second pass shares no values with the first, whose registers stay free
+          uint64_t x = p1x, y1 = p1y, z = p1z;
+          asm volatile("" : "+l"(x), "+l"(y1), "+l"(z));
+          generate(std::true_type{}, x, y1, z);
         }
         // row maximum of |X| over the block's 64 r2 points: this warp's share and the other parts'
         float mx = 0.0f;
@@ -387,7 +377,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         for (int pr = 0; pr < PAIRS; ++pr) {
           float xa, xb2;
           f2unpack(xv[pr], xa, xb2);
-          mx = fmaxf(mx, fmaxf(fabsf(xa), fabsf(xb2)));
+          mx = absMax3(mx, xa, xb2);
         }
         S.rowmax[b][part][row] = mx;
         __syncwarp();
@@ -397,7 +387,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         for (int q = 0; q < kPairParts; ++q) mx = fmaxf(mx, S.rowmax[b][q][row]);
         // scale bs = 2^(23 - E), E = floor(log2 mx) (clamped below): |X bs| < 2^24
         int const E = max(int((__float_as_uint(mx) >> 23) & 0xFF) - 127, kMinExp);
-        float const bs = __uint_as_float(uint32_t(127 + 23 - E) << 23);
+        float const bs = __uint_as_float(uint32_t(127 + 7 - E) << 23);   // 2^(23 - E) / 65536: the slices' h in integers
         // a block's sum_r2 X Vp = 2^24 (256 A + B) / (bs cs) = 2^(E+1) cinv (256 A + B)
         float const fac = __uint_as_float(uint32_t(127 + E + 1) << 23);
         if (g >= uint32_t(XBUF) && !(ok = waitBar(&S.xfree[xb], ((g / XBUF) - 1) & 1, abortFlag, P.status, 134))) break;
@@ -405,21 +395,9 @@ __global__ void __launch_bounds__(kPairThreads, 1)
 #pragma unroll
         for (int ch = 0; ch < PAIRS / 4; ++ch) {
           uint32_t const off = sw128(row, part * (PAIRS / 4) + ch);
-          // t = X bs = 65536 h + 256 m + l: h = rint(t / 65536), m = rint(r / 256), l = r - 256 m with
-          // r = t - 65536 h; slices h, m, l/256 (rounded to nearest BF16: it feeds only the cross
-          // accumulator), m/256
           uint32_t sh[4], sm[4], sl[4], sms[4];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            uint64_t const t = f2mul(xv[ch * 4 + e], bb);
-            uint64_t const h = f2sub(f2fma(t, kInv65536, kMagic), kMagic);
-            uint64_t const r = f2fma(h, kM65536, t);
-            uint64_t const m = f2sub(f2fma(r, kInv256, kMagic), kMagic);
-            sh[e] = bf16PairExactP(h);
-            sm[e] = bf16PairExactP(m);
-            sl[e] = bf16PairRnP(f2mul(f2fma(m, kM256, r), kInv256));
-            sms[e] = bf16PairExactP(f2mul(m, kInv256));
-          }
+          for (int e = 0; e < 4; ++e) sliceX24(xv[ch * 4 + e], bb, sh[e], sm[e], sl[e], sms[e]);
           *reinterpret_cast<uint4 *>(S.x[xb][0] + off) = make_uint4(sh[0], sh[1], sh[2], sh[3]);
           *reinterpret_cast<uint4 *>(S.x[xb][1] + off) = make_uint4(sm[0], sm[1], sm[2], sm[3]);
           *reinterpret_cast<uint4 *>(S.x[xb][2] + off) = make_uint4(sl[0], sl[1], sl[2], sl[3]);

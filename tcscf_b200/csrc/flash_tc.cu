@@ -61,6 +61,10 @@ constexpr int kMinExp = -100;
 // TMEM columns: rho buffers b = 0, 1 at 128 b (hi*hi) and 128 b + 64 (cross); T at TCOL0 (hi*hi) and
 // TCOL0 + NB (cross)
 constexpr uint32_t TCOL0 = 256;
+// T accumulator buffers: two where TMEM holds them, so that GEMM2 of block g does not wait for the flush of block g - 1
+// (4190 -> 4122 us at 59,000 points x 40 columns).  At NB = 128 one fills its half of TMEM; splitting it into two areas of 64
+// columns, flushed in turn, took 252 against 224 ms at 406,000 points x 120 columns: twice the MMAs of half the width
+__host__ __device__ constexpr int tBuffersFor(int NB) { return NB == 64 ? 2 : 1; }
 
 // RP: padded rank of rho (GEMM1 K): 32 (64-byte rows, 64B swizzle) or 64 (128-byte rows, 128B swizzle)
 template <int NB, int RP, int XS, int NS>
@@ -79,7 +83,7 @@ struct __align__(1024) Smem {
   uint64_t full[NSTAGE], empty[NSTAGE];
   uint64_t sfull[2], sfree[2], xfull[2], xfree[2];   // xfull / xfree: per X buffer
   uint64_t rmax[2][4];                     // [block parity][lane quarter]: both r2 halves posted their maxima
-  uint64_t tfull, tfree;
+  uint64_t tfull[2], tfree[2];             // per T buffer
   uint64_t p1full, p1free, done;
   uint32_t tmemBase;
   int abort;
@@ -89,16 +93,6 @@ struct __align__(1024) Smem {
 __host__ __device__ constexpr uint32_t instrDescBf16(int M, int N)
 {
   return (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(N >> 3) << 17) | (uint32_t(M >> 4) << 24);
-}
-
-__device__ __forceinline__ void mmaBf16(uint32_t tmemD, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate)
-{
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmemD),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
-      : "memory");
 }
 
 // the BF16 pair {a, b} rounded to nearest
@@ -125,7 +119,10 @@ template <int NB, class SmemT>
 __device__ __forceinline__ bool flushBlock(SmemT & S, uint32_t taddr, uint32_t f, int cw, float fac, uint64_t (&hi)[NB / 4],
                                            uint64_t (&lo)[NB / 4], int lane, volatile int * abortFlag, int * status)
 {
-  if (!waitBar(&S.tfull, f & 1, abortFlag, status, 31)) return false;
+  constexpr uint32_t TBUF = tBuffersFor(NB);
+  uint32_t const tb = f % TBUF;
+  if (!waitBar(&S.tfull[tb], (f / TBUF) & 1, abortFlag, status, 31)) return false;
+  taddr += tb * 2 * NB;
   fenceAfterSync();
   float const * cs = S.cinvT[cw][f & 1];
   uint64_t const k256 = f2pack(256.0f, 256.0f);
@@ -161,7 +158,7 @@ __device__ __forceinline__ bool flushBlock(SmemT & S, uint32_t taddr, uint32_t f
   }
   fenceBeforeSync();
   __syncwarp();
-  if (lane == 0) mbarArrive(&S.tfree);
+  if (lane == 0) mbarArrive(&S.tfree[tb]);
   return true;
 }
 
@@ -179,7 +176,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   int const warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   volatile int * abortFlag = &S.abort;
 
-  static_assert(TCOL0 + 2 * NB <= 512, "TMEM columns");
+  static_assert(TCOL0 + tBuffersFor(NB) * 2 * NB <= 512, "TMEM columns");
   constexpr uint32_t kStageBytes = 3 * NB * BK * 2 + 3 * BK * RP * 2 + BK * sizeof(float4) + BK * sizeof(float) + NB * sizeof(float);
   constexpr uint32_t kPsi1Bytes = 4 * BM * RP * 2;
 
@@ -190,7 +187,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       mbarInit(&S.xfull[b], NCW); mbarInit(&S.xfree[b], 1);
       for (int q = 0; q < 4; ++q) mbarInit(&S.rmax[b][q], 2);
     }
-    mbarInit(&S.tfull, 1); mbarInit(&S.tfree, NCW);
+    for (int b = 0; b < 2; ++b) { mbarInit(&S.tfull[b], 1); mbarInit(&S.tfree[b], NCW); }
     mbarInit(&S.p1full, 1); mbarInit(&S.p1free, 1); mbarInit(&S.done, 1);
     S.abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -258,7 +255,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       // the B rows continue), and the two accumulators are adjacent in TMEM (A then B)
       constexpr uint32_t idesc1x2 = instrDescBf16(BM, 2 * BK);
       constexpr uint32_t idesc2x2 = instrDescBf16(BM, 2 * NB);
-      uint32_t const aPsi1[4] = {smemAddr(S.psi1[0]), smemAddr(S.psi1[1]), smemAddr(S.psi1[2]), smemAddr(S.psi1[3])};
+      constexpr uint32_t kPsi1Step = BM * RP * 2 / 16, kPsi2Step = BK * RP * 2 / 16, kXStep = BM * BK * 2 / 16, kVStep = NB * BK * 2 / 16;
+      uint32_t const psi1Lo = descLo(smemAddr(S.psi1[0])), psi2Lo = descLo(smemAddr(S.psi2[0][0])), xLo = descLo(smemAddr(S.x[0][0])),
+                     vLo = descLo(smemAddr(S.v[0][0]));
+      uint32_t const hi1 = descHi(RP == 64 ? 1024 : 512, RP == 64 ? 2 : 4), hi2 = descHi(1024, 2);
       uint32_t blockCount = 0;   // global block counter: selects stage, rho / X buffers, T phase
       uint32_t p1Use = 0;
       bool ok = true;
@@ -281,19 +281,18 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           if (g >= 2 && !waitBar(&S.sfree[b], ((g >> 1) - 1) & 1, abortFlag, P.status, 23)) return false;
           fenceAfterSync();
           uint32_t const dHH = tmem + b * 2 * BK, dX = dHH + BK;
-          uint32_t const bPsi2[3] = {smemAddr(S.psi2[s][0]), smemAddr(S.psi2[s][1]), smemAddr(S.psi2[s][2])};
-          constexpr uint32_t sbo = RP == 64 ? 1024 : 512, swz = RP == 64 ? 2 : 4;
-          auto da = [&](int sl, int k) { return smemDesc(aPsi1[sl] + 32 * k, sbo, swz); };
-          auto db = [&](int sl, int k) { return smemDesc(bPsi2[sl] + 32 * k, sbo, swz); };
+          uint32_t const bLo = psi2Lo + uint32_t(s) * 3 * kPsi2Step;
+          auto da = [&](int sl, int k) { return psi1Lo + sl * kPsi1Step + 2 * k; };
+          auto db = [&](int sl, int k) { return bLo + sl * kPsi2Step + 2 * k; };
 #pragma unroll
           for (int k = 0; k < RP / 16; ++k) {
-            uint32_t const acc = k > 0 ? 1u : 0u;
             // B: h m' + m h' + h l'/256 + l/256 h' + m/256 m'; A: h h'
-            mmaBf16(dHH, da(0, k), db(0, k), idesc1x2, acc);   // A += h h', B += h m'
-            mmaBf16(dX, da(1, k), db(0, k), idesc1, 1);
-            mmaBf16(dX, da(0, k), db(2, k), idesc1, 1);
-            mmaBf16(dX, da(2, k), db(0, k), idesc1, 1);
-            mmaBf16(dX, da(3, k), db(1, k), idesc1, 1);
+            if (k == 0) mmaF16<0>(dHH, da(0, k), db(0, k), hi1, idesc1x2);   // A += h h', B += h m'
+            else mmaF16<1>(dHH, da(0, k), db(0, k), hi1, idesc1x2);
+            mmaF16<1>(dX, da(1, k), db(0, k), hi1, idesc1);
+            mmaF16<1>(dX, da(0, k), db(2, k), hi1, idesc1);
+            mmaF16<1>(dX, da(2, k), db(0, k), hi1, idesc1);
+            mmaF16<1>(dX, da(3, k), db(1, k), hi1, idesc1);
           }
           mmaCommit(&S.sfull[b]);
           return true;
@@ -303,37 +302,36 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           if (jj + 1 < nblk && !(ok = gemm1(jj + 1))) break;
           uint32_t const g = base + jj;
           int const s = g % NSTAGE;
-          // the T accumulators are free once the compute warps flushed block g - 1
-          if (g >= 1 && !(ok = waitBar(&S.tfree, (g - 1) & 1, abortFlag, P.status, 24))) break;
+          // T buffer tb is free once the compute warps flushed block g - TBUF
+          constexpr uint32_t TBUF = tBuffersFor(NB);
+          uint32_t const tb = g % TBUF;
+          if (g >= TBUF && !(ok = waitBar(&S.tfree[tb], ((g / TBUF) - 1) & 1, abortFlag, P.status, 24))) break;
           int const xb = g % XBUF;
           if (!(ok = waitBar(&S.xfull[xb], (g / XBUF) & 1, abortFlag, P.status, 25))) break;
           fenceAfterSync();
-          uint32_t const dHH = tmem + TCOL0, dX = dHH + NB;
-          uint32_t aX[XSL];
-#pragma unroll
-          for (int k = 0; k < XSL; ++k) aX[k] = smemAddr(S.x[xb][k]);
-          uint32_t const bV[3] = {smemAddr(S.v[s][0]), smemAddr(S.v[s][1]), smemAddr(S.v[s][2])};
-          auto dxa = [&](int sl, int k) { return smemDesc(aX[sl] + 32 * k, 1024, 2); };
-          auto dvb = [&](int sl, int k) { return smemDesc(bV[sl] + 32 * k, 1024, 2); };
+          uint32_t const dHH = tmem + TCOL0 + tb * 2 * NB, dX = dHH + NB;
+          uint32_t const aLo = xLo + uint32_t(xb) * XSL * kXStep, bLo = vLo + uint32_t(s) * 3 * kVStep;
+          auto dxa = [&](int sl, int k) { return aLo + sl * kXStep + 2 * k; };
+          auto dvb = [&](int sl, int k) { return bLo + sl * kVStep + 2 * k; };
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k) {
-            uint32_t const acc = k > 0 ? 1u : 0u;
-            mmaBf16(dHH, dxa(0, k), dvb(0, k), idesc2x2, acc);   // A += hX hV, B += hX mV
+            if (k == 0) mmaF16<0>(dHH, dxa(0, k), dvb(0, k), hi2, idesc2x2);   // A += hX hV, B += hX mV
+            else mmaF16<1>(dHH, dxa(0, k), dvb(0, k), hi2, idesc2x2);
             if constexpr (XS == 3) {
               // B += mX hV + hX lV/256 + m/256 mV + l/256 hV
-              mmaBf16(dX, dxa(1, k), dvb(0, k), idesc2, 1);
-              mmaBf16(dX, dxa(0, k), dvb(2, k), idesc2, 1);
-              mmaBf16(dX, dxa(3, k), dvb(1, k), idesc2, 1);
-              mmaBf16(dX, dxa(2, k), dvb(0, k), idesc2, 1);
+              mmaF16<1>(dX, dxa(1, k), dvb(0, k), hi2, idesc2);
+              mmaF16<1>(dX, dxa(0, k), dvb(2, k), hi2, idesc2);
+              mmaF16<1>(dX, dxa(3, k), dvb(1, k), hi2, idesc2);
+              mmaF16<1>(dX, dxa(2, k), dvb(0, k), hi2, idesc2);
             } else {
               // B += lX hV + hX lV/256
-              mmaBf16(dX, dxa(1, k), dvb(0, k), idesc2, 1);
-              mmaBf16(dX, dxa(0, k), dvb(2, k), idesc2, 1);
+              mmaF16<1>(dX, dxa(1, k), dvb(0, k), hi2, idesc2);
+              mmaF16<1>(dX, dxa(0, k), dvb(2, k), hi2, idesc2);
             }
           }
           mmaCommit(&S.xfree[xb]);
           mmaCommit(&S.empty[s]);
-          mmaCommit(&S.tfull);
+          mmaCommit(&S.tfull[tb]);
           if (jj == nblk - 1) mmaCommit(&S.p1free);
         }
         blockCount += nblk;
@@ -365,7 +363,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     uint64_t ahi[NB / 4], alo[NB / 4];   // T of this thread's row and columns as FP32 hi + lo, column pairs
     uint64_t const k256 = f2pack(256.0f, 256.0f), kInv256 = f2pack(1.0f / 256.0f, 1.0f / 256.0f), kM256 = f2pack(-256.0f, -256.0f);
     uint64_t const kMagic = f2pack(12582912.0f, 12582912.0f);   // 1.5 * 2^23: adding it rounds |x| < 2^22 to an integer
-    uint64_t const kInv65536 = f2pack(1.0f / 65536.0f, 1.0f / 65536.0f), kM65536 = f2pack(-65536.0f, -65536.0f);
     uint64_t const mOne = f2pack(-1.0f, -1.0f), mHalf = f2pack(-0.5f, -0.5f);
     for (int item = blockIdx.x; item < nItems && ok; item += gridDim.x) {
       int ii, tile, split;
@@ -453,7 +450,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         for (int pr = 0; pr < 16; ++pr) {
           float xa, xb;
           f2unpack(xv[pr], xa, xb);
-          mx = fmaxf(mx, fmaxf(fabsf(xa), fabsf(xb)));
+          mx = absMax3(mx, xa, xb);
         }
         S.rowmax[b][half][row] = mx;
         __syncwarp();
@@ -469,27 +466,15 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         // X buffer xb is free once GEMM2 of block g - XBUF completed
         int const xb = g % XBUF;
         if (g >= uint32_t(XBUF) && !(ok = waitBar(&S.xfree[xb], ((g / XBUF) - 1) & 1, abortFlag, P.status, 34))) break;
-        uint64_t const bb = f2pack(bs, bs);
+        // XS = 3: X' bs / 65536, the slices' h in integers
+        uint64_t const bb = XS == 3 ? f2pack(bs * (1.0f / 65536.0f), bs * (1.0f / 65536.0f)) : f2pack(bs, bs);
 #pragma unroll
         for (int ch = 0; ch < 4; ++ch) {
           uint32_t const off = sw128(row, half * 4 + ch);
           if constexpr (XS == 3) {
-            // t = X' bs = 65536 h + 256 m + l: h = rint(t / 65536), m = rint(r / 256), l = r - 256 m,
-            // r = t - 65536 h; slices h, m, l/256, m/256
             uint32_t sh[4], sm[4], sl[4], sms[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              uint64_t const t = f2mul(xv[ch * 4 + e], bb);
-              uint64_t const h = f2sub(f2fma(t, kInv65536, kMagic), kMagic);
-              uint64_t const r = f2fma(h, kM65536, t);
-              uint64_t const m = f2sub(f2fma(r, kInv256, kMagic), kMagic);
-              // the lowest slice only feeds the cross accumulator, which rounds 2^-8 below the result:
-              // it is stored rounded to nearest BF16 (8 significant bits), not rounded to an integer
-              sh[e] = bf16PairExact(h);
-              sm[e] = bf16PairExact(m);
-              sl[e] = bf16PairRn(f2mul(f2fma(m, kM256, r), kInv256));
-              sms[e] = bf16PairExact(f2mul(m, kInv256));
-            }
+            for (int e = 0; e < 4; ++e) sliceX24(xv[ch * 4 + e], bb, sh[e], sm[e], sl[e], sms[e]);
             *reinterpret_cast<uint4 *>(S.x[xb][0] + off) = make_uint4(sh[0], sh[1], sh[2], sh[3]);
             *reinterpret_cast<uint4 *>(S.x[xb][1] + off) = make_uint4(sm[0], sm[1], sm[2], sm[3]);
             *reinterpret_cast<uint4 *>(S.x[xb][2] + off) = make_uint4(sl[0], sl[1], sl[2], sl[3]);

@@ -160,6 +160,25 @@ __device__ __forceinline__ void mmaCommit(uint64_t * bar)
 
 __device__ __forceinline__ void fenceBeforeSync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fenceAfterSync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+
+// The MMA issuer is one thread on the critical path of every block, so its operands cost one 32-bit add each: the low
+// word of a descriptor (address / 16 in 14 bits, which no tile here overflows) moves by 2 per 16 columns of K
+// and by bytes / 16 per buffer, the high word is a constant of the layout (against 64-bit descriptors built per MMA: kFlashTc
+// 4237 -> 4190 us at 59,000 points x 40 columns, kPairTc 36.2 -> 35.3 ms at 65,536 x 65,536 points x 300).
+__device__ __forceinline__ uint32_t descLo(uint32_t smemAddrBytes) { return uint32_t(smemDesc(smemAddrBytes, 1024, 2)); }
+__device__ __forceinline__ uint32_t descHi(uint32_t sbo, uint32_t swz) { return uint32_t(smemDesc(0, sbo, swz) >> 32); }
+template <uint32_t ACC>
+__device__ __forceinline__ void mmaF16(uint32_t tmemD, uint32_t aLo, uint32_t bLo, uint32_t hi, uint32_t idesc)
+{
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+      "mov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p;\n\t}" ::"r"(tmemD),
+      "r"(aLo), "r"(bLo), "r"(hi), "r"(idesc), "n"(ACC)
+      : "memory");
+}
+
 __device__ __forceinline__ void fenceProxyAsync() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 __device__ __forceinline__ void tmemLoad16(uint32_t taddr, float * v)
@@ -238,6 +257,49 @@ __device__ __forceinline__ float rsqrtApprox(float x)
 __device__ __forceinline__ uint32_t sw128(int row, int chunk)
 {
   return uint32_t((row >> 3) * 1024 + (row & 7) * 128 + ((chunk ^ (row & 7)) << 4));
+}
+
+// max(m, |a|, |b|) and min(m, a, b) (NaN if any is) in one instruction each
+__device__ __forceinline__ float absMax3(float m, float a, float b)
+{
+  float r;
+  asm("{\n\t.reg .f32 x, y;\n\tabs.f32 x, %2;\n\tabs.f32 y, %3;\n\tmax.f32 %0, %1, x, y;\n\t}" : "=f"(r) : "f"(m), "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float min3(float m, float a, float b)
+{
+  float r;
+  asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(m), "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ uint32_t bf16x2Mul256(uint32_t v)   // exact: a power of two
+{
+  uint32_t r;
+  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(0x43804380u));
+  return r;
+}
+// The 24-bit slices of two X values x with u = x scale = h + m/256 + l/65536 (scale a power of two, |u| < 256): h and m integers by
+// rounding to nearest, l the rest; stored as h, m, l/256 (rounded to nearest BF16: it feeds only the cross
+// accumulator) and m/256.  Working in units of h, m/256 falls out of the rounding itself and the two
+// scalings are one BF16-pair multiply each (with absMax3: kFlashTc 4122 -> 3820 us at 59,000 points x 40 columns, kPairTc
+// 35.3 -> 34.9 ms; the slices are the same bits).
+__device__ __forceinline__ void sliceX24(uint64_t x, uint64_t scale, uint32_t & sh, uint32_t & sm, uint32_t & sl, uint32_t & sms)
+{
+  uint64_t const kMagic = f2pack(12582912.0f, 12582912.0f);   // 1.5 * 2^23: adding it rounds |u| < 2^22 to an integer
+  uint64_t const kMagic8 = f2pack(49152.0f, 49152.0f);        // 1.5 * 2^15: to a multiple of 1/256
+  uint64_t const u = f2mul(x, scale);
+  uint64_t const h = f2sub(f2add(u, kMagic), kMagic);
+  uint64_t const r = f2sub(u, h);
+  uint64_t const m = f2sub(f2add(r, kMagic8), kMagic8);
+  float a, b;
+  f2unpack(h, a, b);
+  sh = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+  f2unpack(m, a, b);
+  sms = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+  sm = bf16x2Mul256(sms);
+  f2unpack(f2sub(r, m), a, b);
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(sl) : "f"(b), "f"(a));
+  sl = bf16x2Mul256(sl);
 }
 
 }  // namespace tc
