@@ -652,73 +652,102 @@ __global__ void kPackCoordPairs(int64_t n, int64_t npad, const double * pts, con
 // r1 tile's diagonal, which the tensor kernel skips, added to the potential:
 //   VH[r] += sum_{j < BM tile(r)} g(r, j) c(j)
 // with the tensor kernel's FP32 arithmetic on the same packed points (its drop rule and its
-// Newton-refined rsqrt), FP32 sums per 64-point block added in FP64.  One block of 64 threads per
-// (r1 tile, chunk of its lower r2 blocks), the tiles with the most pairs first; each thread takes two
-// rows of the tile (r and r + 64), so that every r2 point it loads serves both.  Each chunk's row sums
+// Newton-refined rsqrt), FP32 sums per 64-point block added in FP64.  One block of kLowerThreads threads per
+// (r1 tile, chunk of its lower r2 blocks), the tiles with the most pairs first; each thread takes kLowerRows
+// rows of the tile, so that every r2 point it loads serves them all.  Each chunk's row sums
 // go to an FP64 partial, and the partials of a row are added in chunk order (deterministic).
-__device__ __forceinline__ uint64_t coulombPair(uint64_t px, uint64_t py, uint64_t pz, float thr, float4 qa, float4 qb)
+// FMA pipe bound (11 packed operations per two pairs).  Two rows a thread, a test of every pair and 8 chunks a tile took 815 us at
+// 59,000 points, 33.5 ms at 406,000; four rows (half the shared-memory reads), the test out of the loop and 16 chunks: 703 us and
+// 32.0 ms, 79 % of that pipe.  With 8 chunks the 3,688 one-warp blocks of the smaller grid are little more than fit at once (822 us)
+constexpr int kLowerRows = 4, kLowerThreads = BM / kLowerRows;
+
+// v[u] = this thread's sums over one 64-point block.  DROP: pairs below a row's resolution (its w) count 0; otherwise they are
+// left in, and false is returned if there is one
+template <bool DROP>
+__device__ __forceinline__ bool coulombBlock(float4 const * sq, float4 const (&p)[kLowerRows], uint64_t (&v)[kLowerRows])
 {
   uint64_t const mOne = f2pack(-1.0f, -1.0f), mHalf = f2pack(-0.5f, -0.5f);
-  uint64_t const dx = f2sub(px, f2pack(qa.x, qa.y));
-  uint64_t const dy = f2sub(py, f2pack(qa.z, qa.w));
-  uint64_t const dz = f2sub(pz, f2pack(qb.x, qb.y));
-  uint64_t const r2 = f2fma(dx, dx, f2fma(dy, dy, f2mul(dz, dz)));
-  float r2a, r2b;
-  f2unpack(r2, r2a, r2b);
-  uint64_t y = f2pack(rsqrtApprox(r2a), rsqrtApprox(r2b));
-  uint64_t const em = f2fma(f2mul(r2, y), y, mOne);
-  y = f2fma(f2mul(y, mHalf), em, y);
-  float ya, yb;
-  f2unpack(y, ya, yb);
-  ya = r2a >= thr ? ya : 0.0f;
-  yb = r2b >= thr ? yb : 0.0f;
-  return f2pack(ya, yb);
+  float mn[kLowerRows];
+#pragma unroll
+  for (int u = 0; u < kLowerRows; ++u) { v[u] = 0; mn[u] = 3.0e38f; }
+#pragma unroll(DROP ? 1 : 4)
+  for (int e = 0; e < BK / 2; ++e) {
+    float4 const qa = sq[2 * e], qb = sq[2 * e + 1];
+#pragma unroll
+    for (int u = 0; u < kLowerRows; ++u) {
+      uint64_t const dx = f2sub(f2pack(p[u].x, p[u].x), f2pack(qa.x, qa.y));
+      uint64_t const dy = f2sub(f2pack(p[u].y, p[u].y), f2pack(qa.z, qa.w));
+      uint64_t const dz = f2sub(f2pack(p[u].z, p[u].z), f2pack(qb.x, qb.y));
+      uint64_t const r2 = f2fma(dx, dx, f2fma(dy, dy, f2mul(dz, dz)));
+      float r2a, r2b;
+      f2unpack(r2, r2a, r2b);
+      uint64_t y = f2pack(rsqrtApprox(r2a), rsqrtApprox(r2b));
+      uint64_t const em = f2fma(f2mul(r2, y), y, mOne);
+      y = f2fma(f2mul(y, mHalf), em, y);
+      if constexpr (DROP) {
+        float ya, yb;
+        f2unpack(y, ya, yb);
+        y = f2pack(r2a >= p[u].w ? ya : 0.0f, r2b >= p[u].w ? yb : 0.0f);
+      } else {
+        mn[u] = min3(mn[u], r2a, r2b);
+      }
+      v[u] = f2fma(y, f2pack(qb.z, qb.w), v[u]);
+    }
+  }
+  bool far = true;
+#pragma unroll
+  for (int u = 0; u < kLowerRows; ++u) far = far && mn[u] >= p[u].w;
+  return far;
 }
 
 // The lower rows of one r1 tile of one contraction over the r2 blocks [jb, je) (a chunk of the blocks
-// before the tile): out[t] and out[t + 64] receive the two rows' sums (rows r = BM tile + t, r + 64)
+// before the tile): out[row] receives the sum of each of the tile's rows (those of thread t: t + kLowerThreads u)
 __device__ __forceinline__ void coulombLowerChunk(int tile, int jb, int je, const float4 * __restrict__ r1xyz, const float4 * __restrict__ r2pairs,
                                                   double * out)
 {
-  // the r2 points pass through shared memory in 64-point blocks (64 float4 in pair layout, one per
-  // thread), the next block's load in flight while the current one is summed
+  // the r2 points pass through shared memory in 64-point blocks (64 float4 in pair layout),
+  // the next block's load in flight while the current one is summed
   __shared__ float4 sq[2][BK];
+  constexpr int LOADS = BK / kLowerThreads;
   int const t = threadIdx.x;
-  int64_t const r0 = int64_t(tile) * BM + t, r1 = r0 + BM / 2;
-  float4 const pa = r1xyz[r0], pb = r1xyz[r1];
-  uint64_t const ax = f2pack(pa.x, pa.x), ay = f2pack(pa.y, pa.y), az = f2pack(pa.z, pa.z);
-  uint64_t const bx = f2pack(pb.x, pb.x), by = f2pack(pb.y, pb.y), bz = f2pack(pb.z, pb.z);
-  double vha = 0.0, vhb = 0.0;
-  if (je > jb) sq[0][t] = r2pairs[int64_t(jb) * BK + t];
+  float4 p[kLowerRows], nxt[LOADS];
+  double vh[kLowerRows];
+#pragma unroll
+  for (int u = 0; u < kLowerRows; ++u) {
+    p[u] = r1xyz[int64_t(tile) * BM + t + kLowerThreads * u];
+    vh[u] = 0.0;
+  }
+  if (je > jb)
+#pragma unroll
+    for (int i = 0; i < LOADS; ++i) sq[0][t + i * kLowerThreads] = r2pairs[int64_t(jb) * BK + t + i * kLowerThreads];
   __syncthreads();
   for (int j = jb; j < je; ++j) {
     int const buf = (j - jb) & 1;
     bool const more = j + 1 < je;
-    float4 const nxt = more ? r2pairs[int64_t(j + 1) * BK + t] : make_float4(0, 0, 0, 0);
-    uint64_t va = 0, vb = 0;
-#pragma unroll 4
-    for (int e = 0; e < BK / 2; ++e) {
-      float4 const qa = sq[buf][2 * e], qb = sq[buf][2 * e + 1];
-      uint64_t const c = f2pack(qb.z, qb.w);
-      va = f2fma(coulombPair(ax, ay, az, pa.w, qa, qb), c, va);
-      vb = f2fma(coulombPair(bx, by, bz, pb.w, qa, qb), c, vb);
+#pragma unroll
+    for (int i = 0; i < LOADS; ++i) nxt[i] = more ? r2pairs[int64_t(j + 1) * BK + t + i * kLowerThreads] : make_float4(0, 0, 0, 0);
+    uint64_t v[kLowerRows];
+    // few blocks hold a pair to drop: those are summed again with the test of each pair
+    if (!coulombBlock<false>(sq[buf], p, v)) coulombBlock<true>(sq[buf], p, v);
+#pragma unroll
+    for (int u = 0; u < kLowerRows; ++u) {
+      float u0, u1;
+      f2unpack(v[u], u0, u1);
+      vh[u] += double(u0 + u1);
     }
-    float u0, u1;
-    f2unpack(va, u0, u1);
-    vha += double(u0 + u1);
-    f2unpack(vb, u0, u1);
-    vhb += double(u0 + u1);
-    if (more) sq[buf ^ 1][t] = nxt;   // block j - 1's buffer: every thread finished it before the last barrier
+    if (more)   // block j - 1's buffer: every thread finished it before the last barrier
+#pragma unroll
+      for (int i = 0; i < LOADS; ++i) sq[buf ^ 1][t + i * kLowerThreads] = nxt[i];
     __syncthreads();
   }
-  out[t] = vha;
-  out[t + BM / 2] = vhb;
+#pragma unroll
+  for (int u = 0; u < kLowerRows; ++u) out[t + kLowerThreads * u] = vh[u];
 }
 
 // The lower blocks of tile p (its 2 p r2 blocks before the diagonal) in kLowerChunks chunks, chunk c the
 // blocks [c 2p / S, (c + 1) 2p / S): heavy tiles in short pieces, so that no single block's work sets
 // the kernel's tail
-constexpr int kLowerChunks = 8;
+constexpr int kLowerChunks = 16;
 __device__ __forceinline__ void lowerChunkRange(int tile, int c, int & jb, int & je)
 {
   int const n = tile * (BM / BK);
@@ -728,7 +757,7 @@ __device__ __forceinline__ void lowerChunkRange(int tile, int c, int & jb, int &
 
 // one block per (tile >= 1, chunk), the tiles with the most pairs first: the chunk's row sums into
 // part[((tile - 1) kLowerChunks + chunk) BM + row]
-__global__ void __launch_bounds__(BM / 2) kCoulombLower(int nTiles, const float4 * __restrict__ r1xyz, const float4 * __restrict__ r2pairs,
+__global__ void __launch_bounds__(kLowerThreads) kCoulombLower(int nTiles, const float4 * __restrict__ r1xyz, const float4 * __restrict__ r2pairs,
                                                        double * part)
 {
   int const tile = nTiles - 1 - int(blockIdx.x) / kLowerChunks, c = int(blockIdx.x) % kLowerChunks;
@@ -759,7 +788,7 @@ struct CoulombLowerJob {
   int64_t n1;
 };
 // one block per (listed (job, tile), chunk): the chunk's row sums into part[(entry kLowerChunks + chunk) BM + row]
-__global__ void __launch_bounds__(BM / 2) kCoulombLowerBatch(const CoulombLowerJob * __restrict__ jobs, const int2 * __restrict__ tiles,
+__global__ void __launch_bounds__(kLowerThreads) kCoulombLowerBatch(const CoulombLowerJob * __restrict__ jobs, const int2 * __restrict__ tiles,
                                                             double * part)
 {
   int const entry = int(blockIdx.x) / kLowerChunks, c = int(blockIdx.x) % kLowerChunks;
@@ -1115,7 +1144,7 @@ size_t lowerPartBytes(int64_t nTiles) { return size_t(std::max<int64_t>(nTiles, 
 int coulombLower(tcscf_ctx * ctx, tc::Instance const & I, Contraction const & c, double * part)
 {
   if (!hasLowerRows(I, c)) return TCSCF_OK;
-  tc::kCoulombLower<<<unsigned((I.nTiles - 1) * tc::kLowerChunks), tc::BM / 2, 0, ctx->stream>>>(I.nTiles, I.r1xyz, I.r2pairs, part);
+  tc::kCoulombLower<<<unsigned((I.nTiles - 1) * tc::kLowerChunks), tc::kLowerThreads, 0, ctx->stream>>>(I.nTiles, I.r1xyz, I.r2pairs, part);
   TCSCF_LAUNCH(ctx);
   tc::kCoulombLowerSum<<<gridBlocks(c.n1, 256), 256, 0, ctx->stream>>>(c.n1, part, c.VH);
   TCSCF_LAUNCH(ctx);
@@ -1296,7 +1325,7 @@ int tensorRun(tcscf_ctx * ctx, TensorPrep * const * preps, int count, bool recor
     auto * dPart = reinterpret_cast<double *>(static_cast<char *>(q) + jobBytes + tileBytes);
     TCSCF_CUDA(ctx, cudaMemcpyAsync(dJobs, jobs.data(), sizeof(tc::CoulombLowerJob) * jobs.size(), cudaMemcpyHostToDevice, ctx->stream));
     TCSCF_CUDA(ctx, cudaMemcpyAsync(dTiles, lowerTiles.data(), sizeof(int2) * lowerTiles.size(), cudaMemcpyHostToDevice, ctx->stream));
-    tc::kCoulombLowerBatch<<<unsigned(lowerTiles.size() * tc::kLowerChunks), tc::BM / 2, 0, ctx->stream>>>(dJobs, dTiles, dPart);
+    tc::kCoulombLowerBatch<<<unsigned(lowerTiles.size() * tc::kLowerChunks), tc::kLowerThreads, 0, ctx->stream>>>(dJobs, dTiles, dPart);
     TCSCF_LAUNCH(ctx);
     tc::kCoulombLowerBatchSum<<<unsigned(lowerTiles.size()), tc::BM, 0, ctx->stream>>>(dJobs, dTiles, dPart);
     TCSCF_LAUNCH(ctx);
