@@ -1,4 +1,4 @@
-// FP64 CUDA-core r12 contractions and Fock-matrix reductions.
+// FP64 r12 contractions and Fock-matrix reductions, on the FP64 tensor cores.
 //
 // The r12 contraction is written flash-style: for a tile of r1 points the kernel streams r2 in
 // blocks, generates g(r1,r2) from the point coordinates (never stored), forms the density-matrix
