@@ -51,17 +51,29 @@ __device__ __forceinline__ double z3norm(Z3 const & a)
   return a.x.x * a.x.x + a.x.y * a.x.y + a.y.x * a.y.x + a.y.y * a.y.y + a.z.x * a.z.x + a.z.y * a.z.y;
 }
 
-// Device view of one TC build: inputs and the per-point intermediates ([2] = spin).
+struct R3 {
+  double x, y, z;
+};
+__device__ __forceinline__ double2 zrfma(double a, double2 b, double2 c) { return make_double2(fma(a, b.x, c.x), fma(a, b.y, c.y)); }
+__device__ __forceinline__ void z3axpy(Z3 & a, double2 s, R3 const & b)
+{
+  a.x = zrfma(b.x, s, a.x);
+  a.y = zrfma(b.y, s, a.y);
+  a.z = zrfma(b.z, s, a.z);
+}
+__device__ __forceinline__ double2 z3dot(R3 const & a, Z3 const & b) { return zrfma(a.x, b.x, zrfma(a.y, b.y, zscale(a.z, b.z))); }
+
+// Device view of one TC build in the real-harmonic basis: inputs (the kept tensors' planes as they are) and the
+// per-point intermediates ([2] = spin).
 struct TcView {
   int64_t n1;
-  int nb, nelMax;
+  int nb, nelMax, ld, ps;                // ld, ps: tensorStride(nb), tensorPlane(nb)
   int nel[2];
-  int fcx;                               // Fji complex (3-D r2 grid) or real
-  const double * Fs;                     // [n1][nb][nb]
+  const double * Fs;                     // [n1][ps]
   const double * Fo;
-  const double2 * Vs;                    // [n1][nb][nb][3]
-  const double2 * Vo;
-  const double2 * vals;                  // [n1][nb]
+  const double * Vs;                     // [n1][3][ps]
+  const double * Vo;
+  const double * vals;                   // [n1][nb]
   const double2 * grads;                 // [n1][nb][3]
   const double * w;                      // [n1]
   const double2 * D;                     // [2][nb][nb], D_s(i,j) at [s][i][j]
@@ -83,14 +95,11 @@ struct TcView {
   double2 * SCV;                         // [2][n1][3]   sum_b conj(V-tilde_b) occ_b
 };
 
-__device__ __forceinline__ double2 fget(TcView const & t, const double * F, int64_t r, int j, int i)
+__device__ __forceinline__ double fget(TcView const & t, const double * F, int64_t r, int j, int i) { return F[r * t.ps + j * t.ld + i]; }
+__device__ __forceinline__ R3 vget(TcView const & t, const double * V, int64_t r, int j, int i)
 {
-  int64_t const o = (r * t.nb + j) * t.nb + i;
-  return t.fcx ? reinterpret_cast<const double2 *>(F)[o] : make_double2(F[o], 0.0);
-}
-__device__ __forceinline__ Z3 vget(TcView const & t, const double2 * V, int64_t r, int j, int i)
-{
-  return z3load(V + ((r * t.nb + j) * t.nb + i) * 3);
+  const double * p = V + 3 * r * t.ps + j * t.ld + i;
+  return {p[0], p[t.ps], p[2 * t.ps]};
 }
 __device__ __forceinline__ double2 dget(TcView const & t, int s, int i, int j) { return t.D[(int64_t(s) * t.nb + i) * t.nb + j]; }
 __device__ __forceinline__ double2 cget(TcView const & t, int s, int i, int b) { return (s == 0 ? t.C0 : t.C1)[int64_t(b) * t.nb + i]; }
@@ -110,18 +119,18 @@ __global__ void kTcPoint(TcView t)
     double2 faa = make_double2(0, 0), occ = make_double2(0, 0);
     Z3 vt = z3zero(), sg = z3zero();
     for (int j = 0; j < nb; ++j) {
-      double2 const cvj = zconj(t.vals[r * nb + j]);
+      double const vj = t.vals[r * nb + j];
       for (int i = 0; i < nb; ++i) {
         double2 const ds = dget(t, s, i, j), dop = dget(t, so, i, j);
-        faa = zadd(faa, zadd(zmul(fget(t, t.Fs, r, j, i), ds), zmul(fget(t, t.Fo, r, j, i), dop)));
+        faa = zrfma(fget(t, t.Fs, r, j, i), ds, zrfma(fget(t, t.Fo, r, j, i), dop, faa));
         z3axpy(vt, ds, vget(t, t.Vs, r, j, i));
         z3axpy(vt, dop, vget(t, t.Vo, r, j, i));
-        z3axpy(sg, zmul(ds, cvj), gget(t, r, i));
+        z3axpy(sg, zscale(vj, ds), gget(t, r, i));
       }
     }
     for (int k = 0; k < nb; ++k) {
-      double2 const cvk = zconj(t.vals[r * nb + k]);
-      for (int l = 0; l < nb; ++l) occ = zadd(occ, zmul(zmul(dget(t, s, l, k), cvk), t.vals[r * nb + l]));
+      double const vk = t.vals[r * nb + k];
+      for (int l = 0; l < nb; ++l) occ = zrfma(vk * t.vals[r * nb + l], dget(t, s, l, k), occ);
     }
     t.Faa[idx] = faa;
     z3store(t.VT + idx * 3, vt);
@@ -147,15 +156,15 @@ __global__ void kTcPointI(TcView t)
       double2 kv = make_double2(0, 0), kc = make_double2(0, 0);
       Z3 kg = z3zero();
       for (int k = 0; k < nb; ++k) {
-        kv = zadd(kv, zmul(dget(t, s, k, j), t.vals[r * nb + k]));
+        kv = zrfma(t.vals[r * nb + k], dget(t, s, k, j), kv);
         z3axpy(kg, dget(t, s, k, j), gget(t, r, k));
-        kc = zadd(kc, zmul(dget(t, s, j, k), zconj(t.vals[r * nb + k])));
+        kc = zrfma(t.vals[r * nb + k], dget(t, s, j, k), kc);
       }
-      Z3 const vji = vget(t, t.Vs, r, j, i);
-      fai = zadd(fai, zmul(kv, fget(t, t.Fs, r, j, i)));
+      R3 const vji = vget(t, t.Vs, r, j, i);
+      fai = zrfma(fget(t, t.Fs, r, j, i), kv, fai);
       vai = zadd(vai, z3dot(vji, kg));
       z3axpy(vts, kv, vji);                              // sum_k (sum_l D(l,k) v_l) V(k,i), k := j
-      z3axpy(vja, kc, vget(t, t.Vs, r, i, j));           // row i of Vja: sum_j (sum_k D(j,k) v_k^*) V(i,j)
+      z3axpy(vja, kc, vji);                              // row i of Vja: sum_j (sum_k D(j,k) v_k) V(i,j), V symmetric
     }
     t.Fai[idx] = fai;
     t.Vai[idx] = vai;
@@ -217,7 +226,7 @@ __global__ void kTcVab(TcView t)
     Z3 cs = z3zero();
     for (int k = 0; k < nb; ++k) {
       Z3 const vk = z3conj(z3load(t.VTs + (idx * nb + k) * 3));
-      for (int l = 0; l < nb; ++l) z3axpy(cs, zmul(dget(t, s, l, k), t.vals[r * nb + l]), vk);
+      for (int l = 0; l < nb; ++l) z3axpy(cs, zscale(t.vals[r * nb + l], dget(t, s, l, k)), vk);
     }
     z3store(t.SCV + idx * 3, cs);
   }
@@ -254,23 +263,23 @@ __global__ void kTcReduce(TcView t, double2 * out)
   for (int64_t r = threadIdx.x; r < t.n1; r += blockDim.x) {
     int64_t const ps = int64_t(s) * t.n1 + r, po = int64_t(so) * t.n1 + r;
     double const w = t.w[r];
-    double2 const vi = t.vals[r * nb + i], cvj = zconj(t.vals[r * nb + j]);
+    double const vi = t.vals[r * nb + i], vj = t.vals[r * nb + j];
     Z3 const gi = gget(t, r, i);
-    Z3 const vsji = vget(t, t.Vs, r, j, i), voji = vget(t, t.Vo, r, j, i);
+    R3 const vsji = vget(t, t.Vs, r, j, i), voji = vget(t, t.Vo, r, j, i);
     // two-body scalar
-    sc = zadd(sc, zscale(w, zmul(cvj, zsub(zmul(t.Faa[ps], vi), t.Fai[ps * nb + i]))));
+    sc = zadd(sc, zscale(w * vj, zsub(zscale(vi, t.Faa[ps]), t.Fai[ps * nb + i])));
     // two-body vector
     Z3 const vt = z3load(t.VT + ps * 3), vto = z3load(t.VT + po * 3);
-    double2 va = zmul(cvj, zsub(z3dot(vt, gi), t.Vai[ps * nb + i]));
+    double2 va = zscale(vj, zsub(z3dot(vt, gi), t.Vai[ps * nb + i]));
     va = zadd(va, z3dot(vsji, z3load(t.SG + ps * 3)));
     va = zadd(va, z3dot(voji, z3load(t.SG + po * 3)));
     va = zsub(va, z3dot(z3load(t.Vja + (ps * nb + j) * 3), gi));
     ve = zadd(ve, zscale(w, va));
     // three-body
     Z3 const vti = z3load(t.VTs + (ps * nb + i) * 3), vtj = z3load(t.VTs + (ps * nb + j) * 3);
-    double2 x = zmul(zscale(z3norm(vt) - t.sumNs[ps] - t.sumNo[po], cvj), vi);
-    x = zadd(x, zscale(2.0, zmul(cvj, zsub(t.SVD[ps * nb + i], z3dot(vt, vti)))));
-    x = zadd(x, zscale(2.0, zmul(zsub(zconj(t.SVD[ps * nb + j]), z3dot(z3conj(vtj), vt)), vi)));
+    double2 x = make_double2((z3norm(vt) - t.sumNs[ps] - t.sumNo[po]) * vj * vi, 0.0);
+    x = zadd(x, zscale(2.0 * vj, zsub(t.SVD[ps * nb + i], z3dot(vt, vti))));
+    x = zadd(x, zscale(2.0 * vi, zsub(zconj(t.SVD[ps * nb + j]), z3dot(z3conj(vtj), vt))));
     double2 sbS = make_double2(0, 0), sbO = make_double2(0, 0);
     for (int b = 0; b < ne; ++b) {
       int64_t const oj = ((ps * nb + j) * nm + b) * 3, oi = ((ps * nb + i) * nm + b) * 3;
@@ -330,11 +339,11 @@ __global__ void kRealToZ(int n, const double * in, double2 * out)
 }
 
 // ---- fused per-point build (nb <= kFusedMaxNb) -------------------------------------------------------
-// The kernels above keep every per-point intermediate in HBM and read the tensors several times over.  kTcFused
-// reads them once, in the form they are kept in: real symmetric [nb][nb] planes in the real-harmonic
+// Both forms of the build work on the tensors as they are kept: real symmetric [nb][nb] planes in the real-harmonic
 // basis, where the basis values are real too and only densities, orbitals and gradients are complex
 // (every term pairs one conjugated and one plain index, so the sums transform back as one matrix each,
-// kSumsToReference).  A block walks the points p = block, block + grid, ...; one point's planes (Vs, Vo
+// kSumsToReference).  The kernels above keep every per-point intermediate in HBM and read the tensors several times
+// over; kTcFused reads them once.  A block walks the points p = block, block + grid, ...; one point's planes (Vs, Vo
 // components, Fs, Fo) arrive in shared memory by bulk copies while the block before them is still at its
 // outer products.  Everything that is a contraction runs on the FP64 tensor cores:
 //   (1) V(j,i) x_i for all vectors x at once (columns: sum_k D(k,i) v_k, sum_k D(i,k) v_k, sum_k D(k,i) g_k and the
@@ -370,7 +379,6 @@ __device__ __forceinline__ double2 zcfma(double2 a, double2 b, double2 c)  // co
 {
   return make_double2(fma(a.x, b.x, fma(a.y, b.y, c.x)), fma(a.x, b.y, fma(-a.y, b.x, c.y)));
 }
-__device__ __forceinline__ double2 zrfma(double a, double2 b, double2 c) { return make_double2(fma(a, b.x, c.x), fma(a, b.y, c.y)); }
 
 // Shared-memory layout of kTcFused in doubles.  NB: the basis size rounded up to 4, the planes' row stride; every vector is
 // padded to it with zeros, so that the loops and offsets are constants.  What depends on the electron counts comes last
@@ -793,6 +801,30 @@ __global__ void __launch_bounds__(256) kTcPartials(int nparts, int n, const doub
   out[e] = a;
 }
 
+// C_R(k, b) = sum_i conj(U[k][i]) C(i, b) of the occupied orbitals, stored (i, b) at [b nb + i]: n0 of them at C0, the rest at C1
+__global__ void kOrbitalsToReal(int n0, int n, int nb, const DevSto * sto, const double2 * C0, const double2 * C1, double2 * CR)
+{
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n * nb; e += gridDim.x * blockDim.x) {
+    int const b = e / nb, k = e % nb, q = sto[k].partner;
+    const double2 * C = b < n0 ? C0 + b * nb : C1 + (b - n0) * nb;
+    double2 c = zmul(zconj(uRow(sto, k, k)), C[k]);
+    if (q >= 0) c = zadd(c, zmul(zconj(uRow(sto, k, q)), C[q]));
+    CR[e] = c;
+  }
+}
+
+// g_R(r, k) = sum_i U[k][i] g(r, i) of the basis gradients [rows][nb][3]
+__global__ void kGradsToReal(int64_t rows, int nb, const DevSto * sto, const double2 * g, double2 * gR)
+{
+  TC_GRID_LOOP(rows * nb * 3)
+  {
+    int const k = int(idx / 3 % nb), q = sto[k].partner;
+    double2 a = zmul(uRow(sto, k, k), g[idx]);
+    if (q >= 0) a = zadd(a, zmul(uRow(sto, k, q), g[idx + 3 * (q - k)]));
+    gR[idx] = a;
+  }
+}
+
 // X(j,i) = sum_{k,l} U[k][j] XR(k,l) conj(U[l][i]) of `count` complex matrices
 __global__ void kSumsToReference(int count, int nb, const DevSto * s, const double2 * XR, double2 * X)
 {
@@ -921,46 +953,58 @@ int tcFockBuildDevice(tcscf_ctx * ctx, TcInputs const & in, int nup, int ndown, 
     TCSCF_CUDA(ctx, cudaMemcpyAsync(hostStatus, dStatus, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     return TCSCF_OK;
   }
-  // larger bases: the tensors in the reference's layout, a chunk of points (at most 1 GiB of them) at a time
-  size_t const nn = size_t(nb) * nb, fElem = in.F[0]->isComplex ? 2 : 1;
-  size_t const perRow = sizeof(double) * nn * (2 * fElem + 12);
-  int64_t const chunk = std::max<int64_t>(1, std::min<int64_t>(n1, int64_t((size_t(1) << 30) / perRow)));
-  int const chunks = int((n1 + chunk - 1) / chunk);
+  // larger bases (or electron counts): the per-intermediate kernels on the same planes, over all points at once so that
+  // the one-thread-per-point kernels fill the machine; in chunks only where the intermediates do not fit
+  // the device beside the tensors.  Planes read in place, against expanding them to the complex layout in chunks of 1 GiB: 65,536 points,
+  // 2 + 2 electrons: 138 -> 101 ms at 40 functions, 561 -> 328 ms at 64 (16,384 points 36.9 -> 22.8 and 140 -> 73 ms)
+  size_t const nn = size_t(nb) * nb;
   size_t const perPoint = 1 + nb + 3 + 3 + nb + 3 * nb + 3 * nb + 2 * 3 * size_t(nb) * nm + nb + 3;   // double2 units
-  size_t const bytes = sizeof(double2) * (2 * size_t(chunk) * perPoint + 6 * nn * (size_t(chunks) + 1)) + sizeof(double) * 2 * 3 * size_t(chunk) +
-                       perRow * chunk + 1024;
+  int64_t chunk = n1;
   void * p = nullptr;
-  TCSCF_TRY(scratch(ctx, "tc_terms", bytes, &p));
+  size_t bytes = 0;
+  for (int st = TCSCF_ERR_CUDA; st != TCSCF_OK;) {
+    size_t const chunks = size_t((n1 + chunk - 1) / chunk);
+    bytes = sizeof(double2) * (2 * size_t(chunk) * perPoint + size_t(chunk) * nb * 3 + 6 * nn * (chunks + 2) + 2 * nn + size_t(nup + ndown) * nb) +
+            sizeof(double) * 2 * 3 * size_t(chunk) + 1024;
+    st = scratch(ctx, "tc_terms", bytes, &p);
+    if (st == TCSCF_OK) break;
+    cudaGetLastError();   // the failed allocation is not the next launch's error
+    if (chunk <= 1024) return st;
+    chunk = (chunk + 1) / 2;
+  }
+  int const chunks = int((n1 + chunk - 1) / chunk);
   double2 * z = static_cast<double2 *>(p);
   auto take = [&](size_t n) { double2 * r = z; z += n; return r; };
   size_t const n2 = 2 * size_t(chunk);
   TcView t{};
   t.nb = nb; t.nelMax = nm; t.nel[0] = nup; t.nel[1] = ndown;
-  t.fcx = in.F[0]->isComplex;
-  t.D = dD; t.C0 = dC0; t.C1 = dC1;
-  double2 * V[2] = {take(size_t(chunk) * nn * 3), take(size_t(chunk) * nn * 3)};
-  t.Vs = V[0]; t.Vo = V[1];
+  t.ld = tensorStride(nb); t.ps = tensorPlane(nb);
+  double2 * DR = take(2 * nn);
+  double2 * C0 = take(size_t(nup) * nb);
+  double2 * C1 = take(size_t(ndown) * nb);
+  double2 * grads = take(size_t(chunk) * nb * 3);
+  t.D = DR; t.C0 = C0; t.C1 = C1; t.grads = grads;
   t.Faa = take(n2); t.Fai = take(n2 * nb); t.VT = take(n2 * 3); t.SG = take(n2 * 3);
   t.Vai = take(n2 * nb); t.Vja = take(n2 * nb * 3); t.VTs = take(n2 * nb * 3);
   t.Vjbs = take(n2 * nb * nm * 3); t.Vjbo = take(n2 * nb * nm * 3); t.SVD = take(n2 * nb); t.SCV = take(n2 * 3);
-  double2 * part = take(6 * nn * chunks);
   double2 * sums = take(6 * nn);
+  double2 * sumsR = take(6 * nn);
+  double2 * part = take(6 * nn * chunks);
   double * dr = reinterpret_cast<double *>(z);
   t.occD = dr; t.sumNs = dr + n2; t.sumNo = dr + 2 * n2;
-  double * F[2] = {dr + 3 * n2, dr + 3 * n2 + size_t(chunk) * nn * fElem};
-  t.Fs = F[0]; t.Fo = F[1];
-  TCSCF_CHECK(ctx, reinterpret_cast<char *>(F[1] + size_t(chunk) * nn * fElem) <= static_cast<char *>(p) + bytes, TCSCF_ERR_INVALID_ARGUMENT,
-              "internal: tc scratch");
+  TCSCF_CHECK(ctx, reinterpret_cast<char *>(dr + 3 * n2) <= static_cast<char *>(p) + bytes, TCSCF_ERR_INVALID_ARGUMENT, "internal: tc scratch");
+  for (int s = 0; s < 2; ++s) TCSCF_TRY(densityToRealLaunch(ctx, nb, g.dsto, dD + s * nn, DR + s * nn));
+  kOrbitalsToReal<<<gridBlocks(int64_t(nup + ndown) * nb, 256), 256, 0, ctx->stream>>>(nup, nup + ndown, nb, g.dsto, dC0, dC1, C0);
+  TCSCF_LAUNCH(ctx);
   for (int c = 0; c < chunks; ++c) {
     int64_t const r0 = c * chunk, rows = std::min(chunk, n1 - r0);
-    for (int k = 0; k < 2; ++k) {
-      TCSCF_TRY(tensorToReference(ctx, *in.F[k], g.dsto, r0, rows, F[k]));
-      TCSCF_TRY(tensorToReference(ctx, *in.V[k], g.dsto, r0, rows, reinterpret_cast<double *>(V[k])));
-    }
     t.n1 = rows;
-    t.vals = reinterpret_cast<const double2 *>(g.vals) + r0 * nb;
-    t.grads = reinterpret_cast<const double2 *>(g.grads) + r0 * nb * 3;
+    t.Fs = in.F[0]->d + r0 * t.ps; t.Fo = in.F[1]->d + r0 * t.ps;
+    t.Vs = in.V[0]->d + 3 * r0 * t.ps; t.Vo = in.V[1]->d + 3 * r0 * t.ps;
+    t.vals = g.phiR + r0 * nb;
     t.w = g.w + r0;
+    kGradsToReal<<<gridBlocks(rows * nb * 3, 256), 256, 0, ctx->stream>>>(rows, nb, g.dsto, reinterpret_cast<const double2 *>(g.grads) + r0 * nb * 3, grads);
+    TCSCF_LAUNCH(ctx);
     kTcPoint<<<gridBlocks(2 * rows, 128), 128, 0, ctx->stream>>>(t);
     TCSCF_LAUNCH(ctx);
     kTcPointI<<<gridBlocks(2 * rows * nb, 128), 128, 0, ctx->stream>>>(t);
@@ -971,10 +1015,14 @@ int tcFockBuildDevice(tcscf_ctx * ctx, TcInputs const & in, int nup, int ndown, 
     TCSCF_LAUNCH(ctx);
     kTcSvd<<<gridBlocks(2 * rows * nb, 128), 128, 0, ctx->stream>>>(t);
     TCSCF_LAUNCH(ctx);
-    kTcReduce<<<unsigned(2 * nb * nb), 256, 0, ctx->stream>>>(t, part + 6 * nn * c);
+    kTcReduce<<<unsigned(2 * nb * nb), 256, 0, ctx->stream>>>(t, chunks == 1 ? sumsR : part + 6 * nn * c);
     TCSCF_LAUNCH(ctx);
   }
-  kTcPartials<<<unsigned((6 * nn + 31) / 32), 256, 0, ctx->stream>>>(chunks, int(6 * nn), part, sums);
+  if (chunks > 1) {
+    kTcPartials<<<unsigned((6 * nn + 31) / 32), 256, 0, ctx->stream>>>(chunks, int(6 * nn), part, sumsR);
+    TCSCF_LAUNCH(ctx);
+  }
+  kSumsToReference<<<gridBlocks(int64_t(6 * nn), 256), 256, 0, ctx->stream>>>(6, nb, g.dsto, sumsR, sums);
   TCSCF_LAUNCH(ctx);
   kTcAssemble<<<gridBlocks(2 * nb * nb, 256), 256, 0, ctx->stream>>>(nb, sums, dH, respectSym, dG2, dG3);
   TCSCF_LAUNCH(ctx);
