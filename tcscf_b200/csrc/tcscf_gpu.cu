@@ -221,7 +221,7 @@ __device__ __forceinline__ void twoSum(double a, double b, double & s, double & 
 // (b.im, b.re), so fragments are plain 8-byte loads and the sign goes with the weight of A.  One block: a 32 x 32 tile (i tile <= j tile: S and H are Hermitian, the rest
 // is mirrored) over a chunk of points, 4 warps of 8 x 32; the points' values pass through shared memory 8 at
 // a time, the next ones loaded into registers meanwhile.  chunks == 1 writes S and H, else the partials
-// [chunk][S, H][nb][nb] for kQuadSum.  Bound by the FP64 MMAs.  One block per element, reading two columns with
+// [chunk][S, and H with gradients][nb][nb] for kQuadSum.  Bound by the FP64 MMAs.  One block per element, reading two columns with
 // a stride of nb: 59,000 points x 40 functions 2,995 -> 334 us.
 constexpr int kQuadPts = 8;
 struct QuadArgs {
@@ -363,14 +363,15 @@ int quadLaunch(tcscf_ctx * ctx, Grid const & g, int Z, bool withH, double2 * out
   int64_t const chunk = ((g.n + want - 1) / want + kQuadPts - 1) / kQuadPts * kQuadPts;
   int const chunks = int((g.n + chunk - 1) / chunk);
   double2 * part = chunks == 1 ? out : out + 2 * nn;
+  int const m = (withH ? 2 : 1) * nn;   // elements of a chunk's partials: without H only those of S exist
   QuadArgs a{g.n, chunk, nb, Z, g.pts, g.w, reinterpret_cast<const double2 *>(g.vals), withH ? reinterpret_cast<const double2 *>(g.grads) : nullptr,
-             part, part + nn, 2 * int64_t(nn)};
+             part, part + nn, m};
   dim3 const grid{unsigned(chunks), unsigned(t * (t + 1) / 2)};
   if (withH) kQuadOverlapCore<true><<<grid, 128, 0, ctx->stream>>>(a);
   else kQuadOverlapCore<false><<<grid, 128, 0, ctx->stream>>>(a);
   TCSCF_LAUNCH(ctx);
   if (chunks > 1) {
-    kQuadSum<<<unsigned((2 * nn + 31) / 32), 256, 0, ctx->stream>>>(2 * nn, chunks, part, out);
+    kQuadSum<<<unsigned((m + 31) / 32), 256, 0, ctx->stream>>>(m, chunks, part, out);
     TCSCF_LAUNCH(ctx);
   }
   return TCSCF_OK;
