@@ -325,6 +325,51 @@ __global__ void __launch_bounds__(128, 3) kQuadOverlapCore(QuadArgs a)
   }
 }
 
+// S_ij and (with gradients) H_ij for small sums: one block per (i, j), the threads over the points.  Latency bound; its reads of two
+// columns nb apart cost more than the tiles' MMAs only from some size on (quadPerElement)
+__global__ void __launch_bounds__(256) kQuadElements(int64_t n, int nb, int Z, const double * pts, const double * w, const double2 * vals,
+                                                     const double2 * grads, double2 * S, double2 * H)
+{
+  int const i = blockIdx.x / nb, j = blockIdx.x % nb;
+  double v[4] = {0, 0, 0, 0};   // S and H, re and im
+  for (int64_t p = threadIdx.x; p < n; p += blockDim.x) {
+    double2 const a = vals[p * nb + i], b = vals[p * nb + j];
+    double const ovRe = a.x * b.x + a.y * b.y, ovIm = a.x * b.y - a.y * b.x;   // conj(a) b
+    v[0] += w[p] * ovRe;
+    v[1] += w[p] * ovIm;
+    if (grads) {
+      double const r = norm3d(pts[p], pts[n + p], pts[2 * n + p]);
+      double kRe = 0, kIm = 0;
+      for (int d = 0; d < 3; ++d) {
+        double2 const ga = grads[(p * nb + i) * 3 + d], gb = grads[(p * nb + j) * 3 + d];
+        kRe += ga.x * gb.x + ga.y * gb.y;
+        kIm += ga.x * gb.y - ga.y * gb.x;
+      }
+      v[2] += w[p] * (0.5 * kRe - Z * ovRe / r);
+      v[3] += w[p] * (0.5 * kIm - Z * ovIm / r);
+    }
+  }
+  __shared__ double red[8][4];
+  for (int q = 0; q < 4; ++q) {
+    for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][q] = v[q];
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (int q = 0; q < 4; ++q)
+    for (int k = 1; k < 8; ++k) v[q] += red[k][q];
+  S[blockIdx.x] = make_double2(v[0], v[1]);
+  if (grads) H[blockIdx.x] = make_double2(v[2], v[3]);
+}
+// Where one block per element is the faster form.  Its time grows with n (latency of a thread's points) and n nb^2 (reads); the tiles'
+// starts higher (a second launch, 8-point groups of whole 32 x 32 tiles) and stays flat up to about 8,000 points.  Whole calls,
+// per element / tiled: with H 37 / 55 us at 50 points and 47 / 59 at 2,500 (1 function), 46 / 61 at 500 and 70 / 60 at
+// 2,500 (20), 74 / 65 at 500 (40); S alone 22 / 33 at 50 points, 43 / 46 at 32,768 (5), 33 / 35 at 2,500 (20), 60 / 37 (40)
+bool quadPerElement(int64_t n, int nb, bool withH)
+{
+  return nb <= 48 && (withH ? n * (nb * nb + 100) <= 610000 : n * (nb * nb + 20) <= 1800000);
+}
+
 // out[e] = sum over the chunks c of part[c n + e]: 32 elements per block, 8 warps taking every eighth chunk each, added in warp order
 __global__ void __launch_bounds__(256) kQuadSum(int n, int chunks, const double2 * part, double2 * out)
 {
@@ -359,6 +404,12 @@ int quadChunks(tcscf_ctx * ctx, Grid const & g)
 int quadLaunch(tcscf_ctx * ctx, Grid const & g, int Z, bool withH, double2 * out, int maxChunks)
 {
   int const nb = g.nb, nn = nb * nb, t = (nb + 31) / 32;
+  if (quadPerElement(g.n, nb, withH)) {
+    kQuadElements<<<unsigned(nn), 256, 0, ctx->stream>>>(g.n, nb, Z, g.pts, g.w, reinterpret_cast<const double2 *>(g.vals),
+                                                       withH ? reinterpret_cast<const double2 *>(g.grads) : nullptr, out, out + nn);
+    TCSCF_LAUNCH(ctx);
+    return TCSCF_OK;
+  }
   int const want = std::min(maxChunks, quadChunks(ctx, g));
   int64_t const chunk = ((g.n + want - 1) / want + kQuadPts - 1) / kQuadPts * kQuadPts;
   int const chunks = int((g.n + chunk - 1) / chunk);
