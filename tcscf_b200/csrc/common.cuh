@@ -82,7 +82,7 @@ struct tcscf_ctx {
   cusolverDnHandle_t solver = nullptr;
   cublasHandle_t blas = nullptr;   // created on first use (4- and 6-index tensors)
   // stream-ordered pool of the grid buffers (points, weights, basis values and gradients, the
-  // packed tensor-path operand): grids created and destroyed between SCF runs reuse its memory
+  // packed tensor-path operand) and kept tensors: grids and tensors created and destroyed between SCF runs reuse its memory
   // without driver allocations or the device-wide synchronisation of cudaFree
   cudaMemPool_t gridPool = nullptr;
   std::string err;

@@ -2270,8 +2270,9 @@ int tcscf_ctx_create(int device, tcscf_ctx ** out)
       delete ctx;
       return TCSCF_ERR_CUDA;
     }
-    // memory of destroyed grids stays in the pool up to this much (a few Kr-sized grids); the rest
-    // goes back to the device at the next synchronisation
+    // memory of destroyed grids and tensors stays in the pool up to this much (a few Kr-sized grids, the tensors of a Be-TC
+    // cycle); the rest goes back to the device at the next synchronisation, and what stays when a cudaMalloc in this
+    // process, by the context's scratch or by another user of the device, would fail without it
     uint64_t keep = uint64_t(4) << 30;
     cudaMemPoolSetAttribute(ctx->gridPool, cudaMemPoolAttrReleaseThreshold, &keep);
   }
@@ -2639,6 +2640,9 @@ int tcscf_tensor_destroy(tcscf_ctx * ctx, int handle)
   TCSCF_CHECK(ctx, it != ctx->tensors.end(), TCSCF_ERR_INVALID_ARGUMENT, "unknown tensor handle");
   tensorRelease(ctx, it->second);
   ctx->tensors.erase(it);
+  // the pool gives back what it holds beyond its threshold when the stream is synchronised, so the memory is the
+  // device's again when this returns
+  cudaStreamSynchronize(ctx->stream);
   return TCSCF_OK;
 }
 
