@@ -726,9 +726,11 @@ __global__ void kComplexFactors(int nb, int nkeep, const int * keep, const doubl
 // shared memory (rows 4 mod 16 doubles apart: conflict-free fragments), the products on the FP64 tensor
 // cores, four column tiles at a time.  Bound by HBM.  As three kernels, each reading its operands again (one
 // thread per (r, b), the phi row from global memory): Kr (406,000 points, 120 columns, rank 18) 984 -> 375 us.
+// The functions pass through shared memory `panel` (a multiple of 4) at a time: all of them where they fit, and bases of about a
+// thousand functions and more in panels that are read again for every 32 columns
 struct OrbitalArgs {
   int64_t n;
-  int nb, R, ldx, ld, rows;
+  int nb, R, ldx, ld, rows, panel;
   double scale;
   const double * phi;
   const double * w;
@@ -741,51 +743,60 @@ struct OrbitalArgs {
 __global__ void __launch_bounds__(256) kOrbitals(OrbitalArgs a)
 {
   extern __shared__ double sm[];
-  int const nb = a.nb, nb4 = (nb + 3) / 4 * 4, R8 = (a.R + 7) / 8 * 8, lp = fragStride(nb4), lx = fragStride(R8);
+  int const nb = a.nb, nb4 = (nb + 3) / 4 * 4, kp = a.panel, R8 = (a.R + 7) / 8 * 8, lp = fragStride(kp), lx = fragStride(R8);
   int const t = threadIdx.x, warp = t >> 5, lane = t & 31, fr = lane >> 2, fq = lane & 3;
-  double * sX = sm;                                // [nb4][lx], then the same of Xc
-  double * sXc = sX + nb4 * lx;
-  double * sPhi = sXc + (a.Xc ? nb4 * lx : 0);     // [rows][lp]
+  double * sX = sm;                                // [kp][lx], then the same of Xc
+  double * sXc = sX + kp * lx;
+  double * sPhi = sXc + (a.Xc ? kp * lx : 0);      // [rows][lp]
   int64_t const r0 = int64_t(blockIdx.x) * a.rows;
   int const nr = int(min(int64_t(a.rows), a.n - r0));
-  for (int k = warp; k < nb4; k += 8)
-    for (int b = lane; b < R8; b += 32) {
-      bool const in = k < nb && b < a.R;
-      sX[k * lx + b] = in ? a.X[int64_t(k) * a.ldx + b] : 0.0;
-      if (a.Xc) sXc[k * lx + b] = in ? a.Xc[int64_t(k) * a.ldx + b] : 0.0;
-    }
-  // the block's phi rows are one contiguous range: every load in flight at once
-  for (int r = warp; r < a.rows; r += 8)
+  auto load = [&](int k0, int kn) {
+    for (int k = warp; k < kn; k += 8)
+      for (int b = lane; b < R8; b += 32) {
+        bool const in = k0 + k < nb && b < a.R;
+        sX[k * lx + b] = in ? a.X[int64_t(k0 + k) * a.ldx + b] : 0.0;
+        if (a.Xc) sXc[k * lx + b] = in ? a.Xc[int64_t(k0 + k) * a.ldx + b] : 0.0;
+      }
+    // with all functions in one panel the block's phi rows are one contiguous range: every load in flight at once
+    for (int r = warp; r < a.rows; r += 8)
 #pragma unroll 4
-    for (int c = lane; c < nb4; c += 32) {
-      bool const in = r < nr && c < nb;
-      cpAsync<8>(&sPhi[r * lp + c], in ? a.phi + (r0 + r) * nb + c : a.phi, in ? 8 : 0);
-    }
-  cpAsyncCommit();
-  cpAsyncWait<0>();
-  __syncthreads();
-  if (a.V)
-    for (int r = warp; r < nr; r += 8) {
-      double const f = a.scale * a.w[r0 + r];
-#pragma unroll 4
-      for (int c = lane; c < nb; c += 32) a.V[(r0 + r) * nb + c] = f * sPhi[r * lp + c];
-    }
-  if (8 * warp >= a.rows) return;
+      for (int c = lane; c < kn; c += 32) {
+        bool const in = r < nr && k0 + c < nb;
+        cpAsync<8>(&sPhi[r * lp + c], in ? a.phi + (r0 + r) * nb + k0 + c : a.phi, in ? 8 : 0);
+      }
+    cpAsyncCommit();
+    cpAsyncWait<0>();
+    __syncthreads();
+  };
   int const row = 8 * warp + fr;
   double s = 0;
   for (int b0 = 0; b0 < R8; b0 += 32) {
     double q[4][2], qc[4][2];
 #pragma unroll
     for (int j = 0; j < 4; ++j) q[j][0] = q[j][1] = qc[j][0] = qc[j][1] = 0.0;
-    for (int k = fq; k < nb4; k += 4) {
-      double const p = sPhi[row * lp + k];
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (b0 + 8 * j < R8) dmma(q[j], p, sX[k * lx + b0 + 8 * j + fr]);
-      if (a.Xc) {
+    for (int k0 = 0; k0 < nb4; k0 += kp) {
+      int const kn = min(kp, nb4 - k0);
+      if (b0 == 0 || kp < nb4) {
+        if (b0 + k0 > 0) __syncthreads();   // every warp is done with the panel before
+        load(k0, kn);
+        if (a.V && b0 == 0)
+          for (int r = warp; r < nr; r += 8) {
+            double const f = a.scale * a.w[r0 + r];
+#pragma unroll 4
+            for (int c = lane; c < min(kn, nb - k0); c += 32) a.V[(r0 + r) * nb + k0 + c] = f * sPhi[r * lp + c];
+          }
+      }
+      if (8 * warp >= a.rows) continue;
+      for (int k = fq; k < kn; k += 4) {
+        double const p = sPhi[row * lp + k];
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          if (b0 + 8 * j < R8) dmma(qc[j], p, sXc[k * lx + b0 + 8 * j + fr]);
+          if (b0 + 8 * j < R8) dmma(q[j], p, sX[k * lx + b0 + 8 * j + fr]);
+        if (a.Xc) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (b0 + 8 * j < R8) dmma(qc[j], p, sXc[k * lx + b0 + 8 * j + fr]);
+        }
       }
     }
 #pragma unroll
@@ -805,12 +816,15 @@ __global__ void __launch_bounds__(256) kOrbitals(OrbitalArgs a)
 
 int orbitals(tcscf_ctx * ctx, OrbitalArgs a)
 {
+  // the limit of the entry points, and its status, as they have always been
   TCSCF_CHECK(ctx, size_t(a.nb) * a.R * sizeof(double) <= 48 * 1024, TCSCF_ERR_CUDA, "orbital factor (basis size x density rank) above 6144 elements");
-  int const nb4 = (a.nb + 3) / 4 * 4, R8 = (a.R + 7) / 8 * 8;
-  auto bytes = [&](int rows) { return sizeof(double) * (size_t(nb4) * fragStride(R8) * (a.Xc ? 2 : 1) + size_t(rows) * fragStride(nb4)); };
+  int const R8 = (a.R + 7) / 8 * 8;
+  auto bytes = [&](int rows) { return sizeof(double) * (size_t(a.panel) * fragStride(R8) * (a.Xc ? 2 : 1) + size_t(rows) * fragStride(a.panel)); };
+  a.panel = (a.nb + 3) / 4 * 4;
   a.rows = 64;
   while (a.rows > 8 && bytes(a.rows) > 200 * 1024) a.rows /= 2;
-  TCSCF_CHECK(ctx, bytes(a.rows) <= 227 * 1024, TCSCF_ERR_UNSUPPORTED, "basis too large for the orbital kernel");
+  if (bytes(a.rows) > 227 * 1024) { a.panel = 256; a.rows = 64; }   // more than 908 functions, so at most 6 columns: 182 KB
+  TCSCF_CHECK(ctx, bytes(a.rows) <= 227 * 1024, TCSCF_ERR_UNSUPPORTED, "internal: orbital panel beyond the shared memory");
   TCSCF_CUDA(ctx, cudaFuncSetAttribute(kOrbitals, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes(a.rows))));
   kOrbitals<<<unsigned((a.n + a.rows - 1) / a.rows), 256, bytes(a.rows), ctx->stream>>>(a);
   TCSCF_LAUNCH(ctx);
@@ -1472,7 +1486,7 @@ int fockBuildDevice(tcscf_ctx * ctx, Grid & g1, Grid & g2, int nspin, const doub
     if (f.complex) complexSpin |= 1 << s;
     for (int part = 0; part < (f.complex ? 2 : 1); ++part) {
       double const * X1 = part == 0 ? f.X1 : f.X1im;
-      OrbitalArgs o1{n1, nb, R, f.ldx, ldpsi, 0, scale, g1.phiR, g1.w, X1, nullptr, psi1, nullptr, nullptr};
+      OrbitalArgs o1{n1, nb, R, f.ldx, ldpsi, 0, 0, scale, g1.phiR, g1.w, X1, nullptr, psi1, nullptr, nullptr};
       // the r2 side (the r1 side where the two are one): psi2, the Coulomb source with the r1-side factor on
       // the r2 points (rho(r2, r2)), and V for the first spin
       OrbitalArgs o2 = o1;
@@ -1639,7 +1653,7 @@ int fockBuildBatch(tcscf_ctx * ctx, int count, Grid * const * g1s, Grid * const 
       eligible = nl->count == 0;
     }
     if (!eligible) continue;
-    OrbitalArgs o1{n1, nb, f.R, f.ldx, nb, 0, scale, g1.phiR, g1.w, f.X1, nullptr, psi1, nullptr, nullptr};
+    OrbitalArgs o1{n1, nb, f.R, f.ldx, nb, 0, 0, scale, g1.phiR, g1.w, f.X1, nullptr, psi1, nullptr, nullptr};
     OrbitalArgs o2 = o1;
     o2.n = n2; o2.phi = g2.phiR; o2.w = g2.w; o2.coul = coul; o2.V = V;
     if (!sym) {
@@ -2116,7 +2130,7 @@ int scfGraph(tcscf_ctx * ctx, Grid & g1, Grid & g2, int nocc, const double * S, 
       TCSCF_CUDA(ctx, cudaMemsetAsync(Tb, 0, sizeof(double) * size_t(n1) * nb, ctx->stream));
       TCSCF_CUDA(ctx, cudaMemsetAsync(VH, 0, sizeof(double) * size_t(n1), ctx->stream));
     } else {
-    OrbitalArgs o{n2, nb, nocc, nocc, ldpsi, 0, scale, g2.phiR, g2.w, C, nullptr, sym ? psi1 : psi2, coul, nullptr};
+    OrbitalArgs o{n2, nb, nocc, nocc, ldpsi, 0, 0, scale, g2.phiR, g2.w, C, nullptr, sym ? psi1 : psi2, coul, nullptr};
     TCSCF_TRY(orbitals(ctx, o));
     if (!sym) {
       o.n = n1; o.phi = g1.phiR; o.w = g1.w; o.psi = psi1; o.coul = nullptr;
