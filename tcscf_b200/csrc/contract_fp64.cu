@@ -156,7 +156,10 @@ __global__ void __launch_bounds__(32 * contractWarps(RT), contractBlocks(NTL, RT
   // one pointer step from row to row, so a lane's pointers and byte counts are formed once.
   constexpr int W = 8 * NTL;
   int const cols = ncol - col0;
-  int const psiLanes = R4 <= 4 ? 4 : (R4 <= 8 ? 8 : (R4 <= 16 ? 16 : 32)), psiRows = 32 / psiLanes;
+  // lanes of a psi2 row: at least so many that the block's rows of one step are no more than a stage's
+  constexpr int kMinPsiLanes = kWarps * 32 / BK;
+  static_assert(kMinPsiLanes >= 4 && kWarps * (32 / kMinPsiLanes) <= BK, "psi2 rows of a copy step within the stage");
+  int const psiLanes = max(kMinPsiLanes, R4 <= 4 ? 4 : (R4 <= 8 ? 8 : (R4 <= 16 ? 16 : 32))), psiRows = 32 / psiLanes;
   int const pk = warp * psiRows + lane / psiLanes, pb = lane % psiLanes;
   int const vb0 = min(16, max(0, 8 * (cols - 2 * lane))), vb1 = min(16, max(0, 8 * (cols - 64 - 2 * lane)));
   const double * const vsrc = a.V + int64_t(warp) * a.ldv + col0 + (vb0 ? 2 * lane : 0);
