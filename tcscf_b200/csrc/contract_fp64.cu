@@ -541,7 +541,9 @@ int launchOne(tcscf_ctx * ctx, KArgs const & a, dim3 grid, size_t smem)
 }
 
 // the rank in steps of 4 as a template parameter where small (its loops and strides are then constants): 0 (the
-// precompute form), 1, 2, 3, 5, or -1 for any other; contractSteps rounds 4 up to 5
+// precompute form), 1, 2, 3, 5, or -1 for any other; contractSteps rounds 4 up to 5.  Against -1 for all, 16,384 x 16,000 points x
+// 40 columns: rank 1 1.53 -> 1.10 ms, rank 9 1.23, rank 18 1.40; a 4 of its own would take ranks 13 to 16 from 1.39 to 1.31
+// (each value is 12 more kernels to compile, so the set stops where it does)
 constexpr int kAnySteps = -1;
 int contractSteps(int rt, int R)
 {
@@ -568,7 +570,6 @@ int launchKind(tcscf_ctx * ctx, int nt, int rt, int kr, KArgs const & a, dim3 gr
 {
   if constexpr (KIND == 0) {
     if (rt == 1) {
-      if (nt == 4) return launchOne<0, 4, 1, kAnySteps>(ctx, a, grid, smem);
       if (nt == 8) return launchOne<0, 8, 1, kAnySteps>(ctx, a, grid, smem);
       return launchOne<0, 16, 1, kAnySteps>(ctx, a, grid, smem);
     }
@@ -597,10 +598,15 @@ int launchKind(tcscf_ctx * ctx, int nt, int rt, int kr, KArgs const & a, dim3 gr
   }
 }
 
-// the smallest instantiated tile count that holds nt tiles
+// The smallest instantiated tile count that holds nt tiles.  Direct builds pay for padded tiles with MMAs: every count up to 6, then
+// sets with at most one padded tile (16,384 x 16,000 points, rank 5, with / without a kernel of its own: 7 tiles 1.49 / 1.63 ms, 9 1.75 /
+// 1.87, 11 2.05 / 2.13, 14 2.38 / 2.60; counts of 4, 8 and 16 alone 0.95 for 1 tile's 0.55, 2.57 for 9).  The transcorrelated kernels'
+// time is g first: four counts, 13 being the three groups of the 300 pair products of 24 functions (8,192 x 8,000 points: 3.10 ms, with 16 tiles 3.36);
+// the padding of 9 tiles to 13 costs them 13 to 17 %, of 6 to 8 2 to 30 %.  More of either is compile time: all 16 counts double it.
+// Eight warps of one row tile: factors too wide for the shared memory of two, which only bases above 32 columns (8 or 16 tiles) have
 int contractTiles(int kind, int rt, int nt)
 {
-  static int const direct[] = {1, 2, 3, 4, 5, 6, 8, 10, 12, 13, 15, 16}, wideRank[] = {4, 8, 16}, tc[] = {4, 8, 13, 16};
+  static int const direct[] = {1, 2, 3, 4, 5, 6, 8, 10, 12, 13, 15, 16}, wideRank[] = {8, 16}, tc[] = {4, 8, 13, 16};
   auto pick = [&](auto const & v) { for (int t : v) if (t >= nt) return t; return 16; };
   return kind != 0 ? pick(tc) : (rt == 1 ? pick(wideRank) : pick(direct));
 }
