@@ -212,17 +212,17 @@ struct OchiDev {
   double c[8][2];
 };
 
-// 1/r12 from r12^2 >= 0, 0 for an exactly coincident pair.  The hardware estimate y (rsqrt.approx.ftz.f64 works
-// on the high word: no conversions, about 20 bits) is refined by the binomial series of (1 - e)^(-1/2) to
-// second order, y + y e (1/2 + 3/8 e) with e = 1 - x y^2 (Householder's third-order step): the next
-// term, (5/16) e^3, is below 2^-58, so one step of five FP64 operations does what two quadratic Newton
-// steps (seven) do.  The estimate of a zero is cleared on the ALU (the high word of a non-negative double is
-// 0 only for 0 and for values below 2^-1042), which leaves the FP64 pipe alone.
+// 1/r12 from a finite r12^2 >= 0, 0 for an exactly coincident pair.  The hardware estimate y (rsqrt.approx.ftz.f64 works
+// on the high word: no conversions) is refined by the binomial series of (1 - e)^(-1/2) to
+// second order, y + y e (1/2 + 3/8 e) with e = 1 - x y^2 (Householder's third-order step), so one step of five FP64 operations
+// does what two quadratic Newton steps (seven) do: within 1.24 x 2^-53 over all exponents (tests/test_gpu_inv_r12.py), the
+// rounding of the step itself (1.5 at most), so the series' next term is below the last place.  The estimate of zero, and of the subnormal
+// numbers the instruction takes for zero (points closer than 2^-511), is cleared on the ALU by the high word, which leaves the FP64 pipe alone.
 __device__ __forceinline__ double invR12(double r2)
 {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2));
-  y = __hiloint2double(__double2hiint(r2) == 0 ? 0 : __double2hiint(y), 0);
+  y = __hiloint2double(__double2hiint(r2) < 0x00100000 ? 0 : __double2hiint(y), 0);
   double const e = fma(-r2 * y, y, 1.0);
   return fma(y * e, fma(0.375, e, 0.5), y);
 }
