@@ -48,8 +48,8 @@ struct Grid {
 
 // A kept Fji / Vji tensor.  The r12 kernels are real and each element integrates a product of two basis functions, so in the
 // real-harmonic basis the tensor is real and symmetric: it is kept as planes [n1][1 or 3][plane] of nb rows
-// (tensorStride(nb) doubles apart, zeros behind and below), half the complex [nb][nb](3) layout of the reference basis, which
-// tensorToReference forms where a routine or the host wants it
+// tensorStride(nb) doubles apart, half the complex [nb][nb](3) layout of the reference basis (a 2-D r2 grid's real Fji: the
+// same), which tensorToReference forms where a routine or the host wants it
 struct Tensor {
   double * d = nullptr;
   int64_t n1 = 0;
@@ -57,10 +57,12 @@ struct Tensor {
   int isComplex = 1;   // of the reference layout (0: a 2-D r2 grid's real Fji)
   int vec = 0;         // 3 components (Vji)
 };
-// row stride of a plane, and doubles per plane: 4 (mod 8), which puts the fragments of 8 planes on different shared-memory
-// banks and every plane on a 16-byte boundary
-__host__ __device__ constexpr int tensorStride(int nb) { return (nb + 3) / 4 * 4; }
-__host__ __device__ constexpr int tensorPlane(int nb) { return tensorStride(nb) * tensorStride(nb) + 4; }
+// Row stride of a plane, and doubles per plane.  Up to kTensorPadNb functions, where the fused transcorrelated build copies planes
+// as they are, rows are padded to a multiple of 4 and planes to 4 (mod 8), zeros behind and below: the fragments of 8 planes
+// then lie on different shared-memory banks and every plane on a 16-byte boundary (24 functions 580 doubles for 576, 7 functions 68 for 49)
+constexpr int kTensorPadNb = 32;
+__host__ __device__ constexpr int tensorStride(int nb) { return nb > kTensorPadNb ? nb : (nb + 3) / 4 * 4; }
+__host__ __device__ constexpr int tensorPlane(int nb) { return tensorStride(nb) * tensorStride(nb) + (nb > kTensorPadNb ? 0 : 4); }
 
 struct Scratch {
   void * p = nullptr;

@@ -365,7 +365,7 @@ __global__ void kRealToZ(int n, const double * in, double2 * out)
 // barriers between the phases (two blocks per SM fill each other's): 65,536 points x 24 functions, 2 + 2
 // electrons, 8.0 -> 2.6 ms against FP64 FMAs from shared memory on the complex layout (4.8 GB); the sums with run-time
 // sizes took 3.4 ms (address arithmetic).
-constexpr int kFusedMaxNb = 32;
+constexpr int kFusedMaxNb = kTensorPadNb;
 constexpr int kFusedWaitCode = 60;
 __host__ __device__ constexpr int fusedWarps(int ntb) { return ntb == 4 ? 16 : 8; }
 // column tiles (5) or row tiles (4) a warp accumulates

@@ -58,3 +58,19 @@ def test_scratch_takes_the_memory_the_pool_keeps(fresh):
         del held
         torch.cuda.empty_cache()
     assert F.shape == (16, 64, 64)
+
+
+@pytest.mark.parametrize("dim2", [2, 3])
+def test_kept_tensor_above_32_functions_has_no_padding(fresh, dim2):
+    # 33 functions: 1,089 doubles a point for either kind of r2 grid
+    n1, basis = 400000, BASIS[:16] + BASIS[16:28] + BASIS[34:39]
+    assert len(basis) == 33
+    G1, G2 = api.QMCGrid(fresh, grids.qmc_grid(3, n1, 1)), api.QMCGrid(fresh, grids.qmc_grid(dim2, 16, 2))
+    for G in (G1, G2):
+        G.setBasisFunctions(basis)
+    t = [api.computeF(G1, G2, keep=True, copy=False)[1]]   # the call's scratch is there from here on
+    before = _free()
+    t += [api.computeF(G1, G2, keep=True, copy=False)[1] for _ in range(2)]
+    assert before - _free() <= 2 * n1 * 33 * 33 * 8 + 128 * MIB
+    for x in t:
+        x.close()
