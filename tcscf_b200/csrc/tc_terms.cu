@@ -189,8 +189,8 @@ __global__ void kTcVjb(TcView t)
     if (b < t.nel[s]) {
       for (int i = 0; i < nb; ++i) {
         double2 const c = cget(t, s, i, b);
-        z3axpy(rs, c, vget(t, t.Vs, r, j, i));
-        z3axpy(ro, c, vget(t, t.Vo, r, j, i));
+        z3axpy(rs, c, vget(t, t.Vs, r, i, j));   // V(j,i), read so that the lanes' j are adjacent
+        z3axpy(ro, c, vget(t, t.Vo, r, i, j));
       }
     }
     z3store(t.Vjbs + idx * 3, rs);
@@ -956,7 +956,7 @@ int tcFockBuildDevice(tcscf_ctx * ctx, TcInputs const & in, int nup, int ndown, 
   // larger bases (or electron counts): the per-intermediate kernels on the same planes, over all points at once so that
   // the one-thread-per-point kernels fill the machine; in chunks only where the intermediates do not fit
   // the device beside the tensors.  Planes read in place, against expanding them to the complex layout in chunks of 1 GiB: 65,536 points,
-  // 2 + 2 electrons: 138 -> 101 ms at 40 functions, 561 -> 328 ms at 64 (16,384 points 36.9 -> 22.8 and 140 -> 73 ms)
+  // 2 + 2 electrons: 138 -> 101 ms at 40 functions, 561 -> 321 ms at 64 (16,384 points 36.9 -> 23.2 and 140 -> 72 ms)
   size_t const nn = size_t(nb) * nb;
   size_t const perPoint = 1 + nb + 3 + 3 + nb + 3 * nb + 3 * nb + 2 * 3 * size_t(nb) * nm + nb + 3;   // double2 units
   int64_t chunk = n1;
