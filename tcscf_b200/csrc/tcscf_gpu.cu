@@ -2144,10 +2144,10 @@ int scfGraph(tcscf_ctx * ctx, Grid & g1, Grid & g2, int nocc, const double * S, 
       TCSCF_TRY(contractFp64(ctx, c));
     }
     }
-    // the exchange of T' and of the skipped pairs in sums of their own, not M + M^T as the single builds: that G is
-    // symmetric to the last bit, so the Jacobi solver never turns a degenerate shell, and split-BF16 loops (whose
-    // energies carry a few 1e-8 Eh of rounding per build) can sit in a cycle (Ne, 40 x 110 points: no two
-    // energies within 1e-9 in 60 iterations, against 13 to 16)
+    // The exchange of T' and of the skipped pairs in sums of their own.  A split-BF16 build's energies carry a few 1e-8 Eh of
+    // rounding, so at which iteration such a loop passes a stop test of that size is chance: any order of these sums moves it, none is
+    // better.  Stop test 1e-8 Eh, at most 60 iterations: over 60 Ne grids 12.0 on average in this order, 12.5 as M + M^T (the
+    // single builds' form); over 40 Kr grids 43.9 (16 did not pass) and 47.1 (18)
     double const cJ[2] = {2.0, 0.0}, none[2] = {0.0, 0.0};
     TCSCF_TRY(reduceFockReal(ctx, n1, nb, 1, g1.phiR, g1.w, VH, cJ, Tb, 0, nb, FR));
     if (sym) TCSCF_TRY(reduceFockReal(ctx, n1, nb, 1, g1.phiR, g1.w, nullptr, none, Tb, 0, nb, FRhalf));
