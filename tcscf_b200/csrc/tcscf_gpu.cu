@@ -1013,18 +1013,19 @@ int fockFinish(tcscf_ctx * ctx, int nspin, int nb, RealSums const & gr, const do
 // planes, for complex D = DR [nspin][nb][nb]; re and im parts apart.  One block of 8 warps per point at a time: warp w
 // takes plane rows k = w, w + 8, ... with the lanes over the columns; from the row of D^T it forms q_k = sum_m
 // D(m,k) phi_m (lanes, then shuffles), the row's share of Faa, and adds q_k F(k, .) to the lanes' columns of Fai; the warps'
-// sums meet in shared memory.  Every plane is read once for both spins.  Bound by HBM and the shuffles; the
+// sums meet in shared memory.  Every plane is read once for both spins.  The row stride and plane come as arguments (ld, ps): formed
+// from nb in the kernel they cost 293 us a build where this takes 272.  Bound by HBM and the shuffles; the
 // complex layout, read once per spin and sum: 16,384 points x 40 functions 337 -> 136 us, and the complex
 // reduction after it (16 blocks of 1,024 rows) 1,188 -> 22 us as two real ones.
 constexpr int kFaiMaxNb = 64;
 template <int NSPIN>
-__global__ void __launch_bounds__(256) kFaaFai(int64_t n1, int nb, const double * __restrict__ F, const double * __restrict__ phi, const double2 * DR,
+__global__ void __launch_bounds__(256) kFaaFai(int64_t n1, int nb, int ld, int ps, const double * __restrict__ F, const double * __restrict__ phi, const double2 * DR,
                                               double * FaaRe, double * FaaIm, double * FaiRe, double * FaiIm)
 {
   extern __shared__ double2 sDT[];   // [NSPIN][nb][nb]: D_s(m, k) at [s][k][m]
   __shared__ double2 sFai[8][NSPIN][kFaiMaxNb];
   __shared__ double2 sFaa[8];
-  int const nn = nb * nb, ps = tensorPlane(nb), ld = tensorStride(nb), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  int const nn = nb * nb, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   for (int e = tid; e < NSPIN * nn; e += 256) {
     int const s = e / nn, k = e % nn / nb, m = e % nb;
     sDT[e] = DR[s * nn + m * nb + k];
@@ -2784,7 +2785,7 @@ int tcscf_fock_build_precomputed(tcscf_ctx * ctx, int r1, int fji, int nspin, co
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm));
     int per = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, 256, sm);
-    kernel<<<unsigned(std::min<int64_t>(n1, int64_t(sms) * std::max(per, 1))), 256, sm, ctx->stream>>>(n1, nb, t.d, g1->phiR, DR, FaaRe, FaaIm, FaiRe, FaiIm);
+    kernel<<<unsigned(std::min<int64_t>(n1, int64_t(sms) * std::max(per, 1))), 256, sm, ctx->stream>>>(n1, nb, tensorStride(nb), tensorPlane(nb), t.d, g1->phiR, DR, FaaRe, FaaIm, FaiRe, FaiIm);
   };
   if (nspin == 1) launch(kFaaFai<1>);
   else launch(kFaaFai<2>);
