@@ -84,7 +84,7 @@ typedef enum tcscf_kernel {
 } tcscf_kernel;
 
 /* Precision of the r12 contraction (the direct Fock build; computeF / computeV take FP64 and BF16X3).
- * FP64: CUDA-core FP64 throughout.  BF16X3: tcgen05 tensor cores on fixed-point BF16
+ * FP64: FP64 throughout (CUDA cores and FP64 tensor cores).  BF16X3: tcgen05 tensor cores on fixed-point BF16
  * slices of every operand (24 bits for the orbital factors and the weighted basis, 16 or 24 bits for
  * g * rho; power-of-two scales per row / column / r2 block of 64), so the tensor-core sum of the
  * leading slices is exact; each block is added into double-float (FP32 hi + lo) accumulators.

@@ -120,10 +120,11 @@ __host__ __device__ constexpr int contractBlocks(int nt, int rt, int kind)
 // shared memory and no barrier separates the generation of g from the GEMM: the warps of an SM
 // drift apart.  Columns are interleaved in pairs (n and n + 1 of two tiles), so one 16-byte load serves two
 // MMAs.  Blocks are 4 warps (8 where RT = 1), r2 in stages of BK points through a two-stage cp.async
-// pipeline.  Bound by the FP64 pipe and the instruction issue together: an m8n8k4 MMA takes 16 issue cycles of its
-// scheduler and nothing overlaps it, so the time is 16 x MMAs plus the other instructions; they are kept
+// pipeline.  With RT = 2 rho takes m16n8k4 MMAs and T m16n8k8 ones, with RT = 1 both take m8n8k4.  Bound by the FP64 pipe and the
+// instruction issue together: an MMA takes 16 issue cycles of its scheduler per 8 x 8 x 4 product whatever its shape (32 for m16n8k4, 64 for
+// m16n8k8) and nothing overlaps it, so the time is 16 x products plus the other instructions; they are kept
 // few (copies without index arithmetic, the rank a template parameter, no masks in full stages, the
-// half weight applied once).  Forming the next group's X beside the GEMM, MMAs of m8n8k4 or m16n8k8 and
+// half weight applied once).  Forming the next group's X beside the GEMM, MMAs of m8n8k4 and
 // volatile ordering all measured the same.  Against a kernel that passed X through shared memory between
 // two barriers: 59,000 points x 40 columns (rank 5, symmetric) 21.1 -> 7.2 ms; 81,200 points x 120
 // columns (rank 18, symmetric) 58.6 -> 32.1 ms, 0.81 of the FP64 matmul rate counting the padded MMAs.

@@ -259,7 +259,7 @@ __device__ __forceinline__ uint32_t sw128(int row, int chunk)
   return uint32_t((row >> 3) * 1024 + (row & 7) * 128 + ((chunk ^ (row & 7)) << 4));
 }
 
-// max(m, |a|, |b|) and min(m, a, b) (NaN if any is) in one instruction each
+// max(m, |a|, |b|), which passes over NaN, and min(m, a, b), NaN if any is, in one instruction each
 __device__ __forceinline__ float absMax3(float m, float a, float b)
 {
   float r;
