@@ -658,7 +658,7 @@ __global__ void kPackCoordPairs(int64_t n, int64_t npad, const double * pts, con
 // go to an FP64 partial, and the partials of a row are added in chunk order (deterministic).
 // FMA pipe bound (11 packed operations per two pairs).  Two rows a thread, a test of every pair and 8 chunks a tile took 815 us at
 // 59,000 points, 33.5 ms at 406,000; four rows (half the shared-memory reads), the test out of the loop and 16 chunks: 703 us and
-// 32.0 ms, 79 % of that pipe.  With 8 chunks the 3,688 one-warp blocks of the smaller grid are little more than fit at once (822 us)
+// 32.0 ms, 76 % of that pipe (121,800 points).  With 8 chunks the 3,688 one-warp blocks of the smaller grid are little more than fit at once (822 us)
 constexpr int kLowerRows = 4, kLowerThreads = BM / kLowerRows;
 
 // v[u] = this thread's sums over one 64-point block.  DROP: pairs below a row's resolution (its w) count 0; otherwise they are
