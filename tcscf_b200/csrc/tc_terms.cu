@@ -107,35 +107,53 @@ __device__ __forceinline__ Z3 gget(TcView const & t, int64_t r, int k) { return 
 
 #define TC_GRID_LOOP(total) for (int64_t idx = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; idx < (total); idx += int64_t(gridDim.x) * blockDim.x)
 
-// per (spin, r1): Faa (calculateIaa on both Fji, :1119-1124), V-tilde (calculateIaa on Vji :1125-1126
-// and calculateVTilde :397-434 are the same sum), scaled gradients (:102-140), occupied density (:530-567)
-__global__ void kTcPoint(TcView t)
+// per r1, both spins: Faa (calculateIaa on both Fji, :1119-1124), V-tilde (calculateIaa on Vji :1125-1126
+// and calculateVTilde :397-434 are the same sum), scaled gradients (:102-140), occupied density (:530-567).  A warp per
+// point, the lanes over the elements (i, j) of its planes: F(j,i) D(i,j) = F(i,j) D(i,j) element by element, the planes being
+// symmetric.  A thread per (spin, point), each walking the eight planes of its own: 65,536 points 13.6 -> 1.1 ms (33 functions), 59 -> 3.8 (64)
+__global__ void __launch_bounds__(128) kTcPoint(TcView t)
 {
-  int const nb = t.nb;
-  TC_GRID_LOOP(2 * t.n1)
-  {
-    int const s = int(idx / t.n1), so = 1 - s;
-    int64_t const r = idx % t.n1;
-    double2 faa = make_double2(0, 0), occ = make_double2(0, 0);
-    Z3 vt = z3zero(), sg = z3zero();
-    for (int j = 0; j < nb; ++j) {
-      double const vj = t.vals[r * nb + j];
-      for (int i = 0; i < nb; ++i) {
-        double2 const ds = dget(t, s, i, j), dop = dget(t, so, i, j);
-        faa = zrfma(fget(t, t.Fs, r, j, i), ds, zrfma(fget(t, t.Fo, r, j, i), dop, faa));
-        z3axpy(vt, ds, vget(t, t.Vs, r, j, i));
-        z3axpy(vt, dop, vget(t, t.Vo, r, j, i));
-        z3axpy(sg, zscale(vj, ds), gget(t, r, i));
+  int const nb = t.nb, lane = threadIdx.x & 31;
+  for (int64_t r = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; r < t.n1; r += int64_t(gridDim.x) * blockDim.x >> 5) {
+    double2 faa[2], occ[2];
+    Z3 vt[2], sg[2];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      faa[s] = occ[s] = make_double2(0, 0);
+      vt[s] = sg[s] = z3zero();
+    }
+    for (int e = lane; e < nb * t.ld; e += 32) {
+      int const i = e / t.ld, j = e - i * t.ld;
+      if (j >= nb) continue;
+      double2 const d[2] = {dget(t, 0, i, j), dget(t, 1, i, j)};
+      double const fs = fget(t, t.Fs, r, i, j), fo = fget(t, t.Fo, r, i, j), vj = t.vals[r * nb + j], vi = t.vals[r * nb + i];
+      R3 const vs = vget(t, t.Vs, r, i, j), vo = vget(t, t.Vo, r, i, j);
+      Z3 const g = gget(t, r, i);
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        faa[s] = zrfma(fs, d[s], zrfma(fo, d[1 - s], faa[s]));
+        z3axpy(vt[s], d[s], vs);
+        z3axpy(vt[s], d[1 - s], vo);
+        z3axpy(sg[s], zscale(vj, d[s]), g);
+        occ[s] = zrfma(vj * vi, d[s], occ[s]);
       }
     }
-    for (int k = 0; k < nb; ++k) {
-      double const vk = t.vals[r * nb + k];
-      for (int l = 0; l < nb; ++l) occ = zrfma(vk * t.vals[r * nb + l], dget(t, s, l, k), occ);
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      double * const v[15] = {&faa[s].x, &faa[s].y, &vt[s].x.x, &vt[s].x.y, &vt[s].y.x, &vt[s].y.y, &vt[s].z.x, &vt[s].z.y,
+                              &sg[s].x.x, &sg[s].x.y, &sg[s].y.x, &sg[s].y.y, &sg[s].z.x, &sg[s].z.y, &occ[s].x};
+#pragma unroll
+      for (int q = 0; q < 15; ++q)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) *v[q] += __shfl_xor_sync(0xffffffffu, *v[q], o);
+      if (lane == 0) {
+        int64_t const idx = s * t.n1 + r;
+        t.Faa[idx] = faa[s];
+        z3store(t.VT + idx * 3, vt[s]);
+        z3store(t.SG + idx * 3, sg[s]);
+        t.occD[idx] = occ[s].x;
+      }
     }
-    t.Faa[idx] = faa;
-    z3store(t.VT + idx * 3, vt);
-    z3store(t.SG + idx * 3, sg);
-    t.occD[idx] = occ.x;
   }
 }
 
@@ -954,9 +972,9 @@ int tcFockBuildDevice(tcscf_ctx * ctx, TcInputs const & in, int nup, int ndown, 
     return TCSCF_OK;
   }
   // larger bases (or electron counts): the per-intermediate kernels on the same planes, over all points at once so that
-  // the one-thread-per-point kernels fill the machine; in chunks only where the intermediates do not fit
+  // kernels with a thread or warp per point fill the machine; in chunks only where the intermediates do not fit
   // the device beside the tensors.  Planes read in place, against expanding them to the complex layout in chunks of 1 GiB: 65,536 points,
-  // 2 + 2 electrons: 138 -> 101 ms at 40 functions, 561 -> 321 ms at 64 (16,384 points 36.9 -> 23.2 and 140 -> 72 ms)
+  // 2 + 2 electrons: 138 -> 84 ms at 40 functions, 562 -> 274 ms at 64 (16,384 points 36.9 -> 21.0 and 140 -> 66 ms)
   size_t const nn = size_t(nb) * nb;
   size_t const perPoint = 1 + nb + 3 + 3 + nb + 3 * nb + 3 * nb + 2 * 3 * size_t(nb) * nm + nb + 3;   // double2 units
   int64_t chunk = n1;
@@ -1005,7 +1023,7 @@ int tcFockBuildDevice(tcscf_ctx * ctx, TcInputs const & in, int nup, int ndown, 
     t.w = g.w + r0;
     kGradsToReal<<<gridBlocks(rows * nb * 3, 256), 256, 0, ctx->stream>>>(rows, nb, g.dsto, reinterpret_cast<const double2 *>(g.grads) + r0 * nb * 3, grads);
     TCSCF_LAUNCH(ctx);
-    kTcPoint<<<gridBlocks(2 * rows, 128), 128, 0, ctx->stream>>>(t);
+    kTcPoint<<<gridBlocks(32 * rows, 128), 128, 0, ctx->stream>>>(t);
     TCSCF_LAUNCH(ctx);
     kTcPointI<<<gridBlocks(2 * rows * nb, 128), 128, 0, ctx->stream>>>(t);
     TCSCF_LAUNCH(ctx);
