@@ -40,6 +40,21 @@ class _Build:
             x.close()
 
 
+def _oracle(b):
+    uo, nb, g = oracle.ochi(U["a"], U["a12"], U["terms"]), len(BASIS), [b.g1, b.g2, b.g3]
+    vals = [oracle.basis_values(x.points, BASIS) for x in g[1:]]
+    o = [oracle.compute_F(g[0].points, g[1].points, g[1].weights, vals[0], nb, k, uo) for k in KS[:2]]
+    o += [oracle.compute_V(g[0].points, g[2].points, g[2].weights, vals[1], nb, k, uo) for k in KS[2:]]
+    v1, d1 = oracle.basis_values(g[0].points, BASIS, gradients=True)
+    return oracle.tc_fock_build(*o, v1, d1, g[0].weights, b.D, *b.nel, *b.occ, b.h)
+
+
+def _check(got, ref):
+    for a, r in zip(got[:3], ref[:3]):
+        assert np.abs(a - r).max() <= 1e-10 * max(1.0, np.abs(r).max())
+    assert abs(got[3] - ref[3]) <= 1e-10 * max(1.0, abs(ref[3]))
+
+
 def _kernels(f):
     with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
         f()
@@ -77,17 +92,15 @@ def test_chunks_under_memory_pressure(ctx, dim2):
         finally:
             del held
             torch.cuda.empty_cache()
-        g1, g2, g3 = b.g1, b.g2, b.g3
         b.close()
     for a, w in zip(parts[:3], whole[:3]):
         assert np.abs(a - w).max() <= 1e-12 * max(1.0, np.abs(w).max())
-    uo = oracle.ochi(U["a"], U["a12"], U["terms"])
-    vals = [oracle.basis_values(g.points, BASIS) for g in (g2, g3)]
-    nb = len(BASIS)
-    o = [oracle.compute_F(g1.points, g2.points, g2.weights, vals[0], nb, k, uo) for k in KS[:2]]
-    o += [oracle.compute_V(g1.points, g3.points, g3.weights, vals[1], nb, k, uo) for k in KS[2:]]
-    v1, d1 = oracle.basis_values(g1.points, BASIS, gradients=True)
-    ref = oracle.tc_fock_build(*o, v1, d1, g1.weights, b.D, *nel, *b.occ, b.h)
-    for a, r in zip(parts[:3], ref[:3]):
-        assert np.abs(a - r).max() <= 1e-10 * max(1.0, np.abs(r).max())
-    assert abs(parts[3] - ref[3]) <= 1e-10 * max(1.0, abs(ref[3]))
+    _check(parts, _oracle(b))
+
+
+@pytest.mark.parametrize("nel", [(0, 2), (1, 0)])
+def test_one_spin_empty(ctx, nel):
+    b = _Build(ctx, 37, nel)
+    got = b.run()
+    b.close()
+    _check(got, _oracle(b))
