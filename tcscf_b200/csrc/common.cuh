@@ -64,6 +64,9 @@ constexpr int kTensorPadNb = 32;
 __host__ __device__ constexpr int tensorStride(int nb) { return nb > kTensorPadNb ? nb : (nb + 3) / 4 * 4; }
 __host__ __device__ constexpr int tensorPlane(int nb) { return tensorStride(nb) * tensorStride(nb) + (nb > kTensorPadNb ? 0 : 4); }
 
+// what the context's pool keeps of released memory
+constexpr uint64_t kPoolKeepBytes = uint64_t(4) << 30;
+
 struct Scratch {
   void * p = nullptr;
   size_t bytes = 0;

@@ -2288,7 +2288,7 @@ int tcscf_ctx_create(int device, tcscf_ctx ** out)
     // memory of destroyed grids and tensors stays in the pool up to this much (a few Kr-sized grids, the tensors of a Be-TC
     // cycle); the rest goes back to the device at the next synchronisation, and what stays when a cudaMalloc in this
     // process, by the context's scratch or by another user of the device, would fail without it
-    uint64_t keep = uint64_t(4) << 30;
+    uint64_t keep = kPoolKeepBytes;
     cudaMemPoolSetAttribute(ctx->gridPool, cudaMemPoolAttrReleaseThreshold, &keep);
   }
   for (auto & e : ctx->ev) cudaEventCreate(&e);
@@ -2661,8 +2661,10 @@ int tcscf_tensor_destroy(tcscf_ctx * ctx, int handle)
   tensorRelease(ctx, it->second);
   ctx->tensors.erase(it);
   // the pool gives back what it holds beyond its threshold when the stream is synchronised, so the memory is the
-  // device's again when this returns
-  cudaStreamSynchronize(ctx->stream);
+  // device's again when this returns; below the threshold there is nothing to wait for (4 us of a 47 us computeF and destroy)
+  uint64_t held = 0;
+  if (cudaMemPoolGetAttribute(ctx->gridPool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess || held > kPoolKeepBytes)
+    cudaStreamSynchronize(ctx->stream);
   return TCSCF_OK;
 }
 
