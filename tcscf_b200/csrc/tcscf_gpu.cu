@@ -2660,11 +2660,13 @@ int tcscf_tensor_destroy(tcscf_ctx * ctx, int handle)
   TCSCF_CHECK(ctx, it != ctx->tensors.end(), TCSCF_ERR_INVALID_ARGUMENT, "unknown tensor handle");
   tensorRelease(ctx, it->second);
   ctx->tensors.erase(it);
-  // the pool gives back what it holds beyond its threshold when the stream is synchronised, so the memory is the
-  // device's again when this returns; below the threshold there is nothing to wait for (4 us of a 47 us computeF and destroy)
-  uint64_t held = 0;
-  if (cudaMemPoolGetAttribute(ctx->gridPool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess || held > kPoolKeepBytes)
-    cudaStreamSynchronize(ctx->stream);
+  // the pool gives memory back when the stream is synchronised: here where it holds more unused memory than it is to keep, so that
+  // the rest is the device's again when this returns (always: 4 us of a 47 us computeF and destroy, and memory that the next tensors
+  // would take again goes to the device and back)
+  uint64_t held = 0, used = 0;
+  cudaMemPoolGetAttribute(ctx->gridPool, cudaMemPoolAttrReservedMemCurrent, &held);
+  cudaMemPoolGetAttribute(ctx->gridPool, cudaMemPoolAttrUsedMemCurrent, &used);
+  if (held - used > kPoolKeepBytes) cudaStreamSynchronize(ctx->stream);
   return TCSCF_OK;
 }
 
